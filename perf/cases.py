@@ -8,6 +8,7 @@ operators, `work` counts what the call cannot do without, and `tolerance` says h
 import math
 
 import torch
+import torch.nn.functional as F
 
 from mimir_b200 import tensor as T
 
@@ -71,6 +72,11 @@ def _run_product(c, s):
     return T.product_2d(s["a"], s["b"], post=c["post"], bias=s["bias"])
 
 
+def _exact_product(c, s):
+    y = s["a"].double() @ s["b"].double()
+    return y if c["post"] == "id" else (y + s["bias"].double()).clamp_(min=0)
+
+
 def _work_product(c):
     m, n, k = c["m"], c["n"], c["k"]
     return c["batch"] * _size(c) * (m * k + k * n + m * n) + (4 * n if c["post"] != "id" else 0), 2 * c["batch"] * m * n * k
@@ -96,6 +102,17 @@ def _run_attention(c, s):
     return T.attention(s["q"], s["k"], s["v"], scale=1.0 / math.sqrt(c["d"]), causal=c["causal"])
 
 
+def _exact_attention(c, s):
+    out = torch.empty(s["q"].shape, dtype=torch.float64, device=s["q"].device)
+    hidden = torch.ones((c["sq"], c["sk"]), dtype=torch.bool, device=out.device).triu_(c["sk"] - c["sq"] + 1) if c["causal"] else None
+    for i in range(c["bh"]):
+        scores = (s["q"][i].double() @ s["k"][i].double().t()).mul_(1.0 / math.sqrt(c["d"]))
+        if hidden is not None:
+            scores.masked_fill_(hidden, -math.inf)
+        out[i] = torch.softmax(scores, -1) @ s["v"][i].double()
+    return out
+
+
 def _work_attention(c):
     bh, sq, sk, d = c["bh"], c["sq"], c["sk"], c["d"]
     scores = sq * sk - (sq * (sq - 1) // 2 if c["causal"] else 0)
@@ -117,6 +134,11 @@ def _prepare_rows(c, g):
 
 def _run_rows(c, s):
     return T.softmax(1, s["x"], out_dtype=BF16), T.rmsnorm(s["x"], s["gamma"], 1e-6, out_dtype=BF16)
+
+
+def _exact_rows(c, s):
+    x = s["x"].double()
+    return torch.softmax(x, 1), x * torch.rsqrt(x.square().mean(1, keepdim=True) + 1e-6) * s["gamma"].double()
 
 
 def _work_rows(c):
@@ -143,6 +165,11 @@ def _run_stats(c, s):
     return T.reduce("sum", 1, x), T.reduce_fused("sum", 1, x, "square"), T.binary_ax("mul", 1, x, s["scale"], then="relu")
 
 
+def _exact_stats(c, s):
+    x = s["x"].double()
+    return x.sum(1), x.square().sum(1), (x * s["scale"].double().unsqueeze(1)).clamp_(min=0)
+
+
 def _work_stats(c):
     cells = c["outer"] * c["length"] * c["inner"]
     return _size(c) * (2 * cells + 3 * c["outer"] * c["inner"]), 5 * cells
@@ -162,6 +189,11 @@ def _prepare_mlp(c, g):
 
 def _run_mlp(c, s):
     return T.mlp_gated(s["x"], s["w1"], s["w3"], s["w2"])
+
+
+def _exact_mlp(c, s):
+    x = s["x"].double()
+    return (F.silu(x @ s["w1"].double()) * (x @ s["w3"].double())) @ s["w2"].double()
 
 
 def _work_mlp(c):
@@ -201,6 +233,17 @@ def _run_train(c, s):
             "w1": T.product_2d(T.transpose(x, (1, 0)), d1), "b1": T.reduce("sum", 0, d1)}
 
 
+def _exact_train(c, s):
+    x, y, w1, w2, w3, b1, b2, b3 = (s[k].double() for k in ("x", "y", "w1", "w2", "w3", "b1", "b2", "b3"))
+    h1 = torch.tanh(x @ w1 + b1)
+    h2 = torch.tanh(h1 @ w2 + b2)
+    logits = h2 @ w3 + b3
+    d3 = torch.softmax(logits, 1) - y
+    d2 = d3 @ w3.t() * (1 - h2 * h2)
+    d1 = d2 @ w2.t() * (1 - h1 * h1)
+    return {"logits": logits, "w3": h2.t() @ d3, "b3": d3.sum(0), "w2": h1.t() @ d2, "b2": d2.sum(0), "w1": x.t() @ d1, "b1": d1.sum(0)}
+
+
 def _work_train(c):
     b, i, h, o = c["batch"], c["inputs"], c["hidden"], c["classes"]
     weights = i * h + h * h + h * o
@@ -226,6 +269,15 @@ def _run_conv(c, s):
     return T.pool("max", T.unary("relu", y), (2, 2))
 
 
+def _exact_conv(c, s):
+    w = s["w"].double().flatten(1)
+    y = []
+    for x in s["x"].double().split(1):
+        oh, ow = (c["h"] - 1) // c["stride"] + 1, (c["w"] - 1) // c["stride"] + 1
+        y.append((w @ F.unfold(x, c["k"], padding=c["k"] // 2, stride=c["stride"])).view(1, c["cout"], oh, ow))
+    return F.max_pool2d(torch.cat(y).clamp_(min=0), 2)
+
+
 def _work_conv(c):
     oh, ow = (c["h"] - 1) // c["stride"] + 1, (c["w"] - 1) // c["stride"] + 1
     taps = c["cin"] * c["k"] ** 2
@@ -235,13 +287,13 @@ def _work_conv(c):
 
 # ------------------------------------------------------------------------------------------------------------------- common
 KINDS = {
-    "product": (_draw_product, _prepare_product, _run_product, _work_product),
-    "attention": (_draw_attention, _prepare_attention, _run_attention, _work_attention),
-    "rows": (_draw_rows, _prepare_rows, _run_rows, _work_rows),
-    "stats": (_draw_stats, _prepare_stats, _run_stats, _work_stats),
-    "mlp": (_draw_mlp, _prepare_mlp, _run_mlp, _work_mlp),
-    "train": (_draw_train, _prepare_train, _run_train, _work_train),
-    "conv": (_draw_conv, _prepare_conv, _run_conv, _work_conv),
+    "product": (_draw_product, _prepare_product, _run_product, _work_product, _exact_product),
+    "attention": (_draw_attention, _prepare_attention, _run_attention, _work_attention, _exact_attention),
+    "rows": (_draw_rows, _prepare_rows, _run_rows, _work_rows, _exact_rows),
+    "stats": (_draw_stats, _prepare_stats, _run_stats, _work_stats, _exact_stats),
+    "mlp": (_draw_mlp, _prepare_mlp, _run_mlp, _work_mlp, _exact_mlp),
+    "train": (_draw_train, _prepare_train, _run_train, _work_train, _exact_train),
+    "conv": (_draw_conv, _prepare_conv, _run_conv, _work_conv, _exact_conv),
 }
 # how often each kind is drawn: contractions and attention are most of what programs do
 WEIGHTS = {"product": 4, "attention": 4, "rows": 2, "stats": 1, "mlp": 2, "train": 1, "conv": 2}
@@ -298,6 +350,11 @@ def run(state):
 def work(case):
     nbytes, flops = KINDS[case["kind"]][3](case)
     return {"bytes": nbytes, "flops": flops}
+
+
+def exact(case, seed):
+    """What `run` returns for these inputs, as plain torch gives it in 64 bits."""
+    return KINDS[case["kind"]][4](case, prepare(case, seed))
 
 
 def tolerance(case):
