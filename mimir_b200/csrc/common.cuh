@@ -151,6 +151,28 @@ __device__ __forceinline__ float apply_op(int op, float a, float b) {
     if (op & MIMK_OP_COMPOSED_BASE) return apply_op_plain((op >> 8) & 0xff, apply_op_plain(op & 0xff, a, b), 0.f);
     return apply_op_plain(op, a, b);
 }
+// The same on N elements with one dispatch: a[i] = op(a[i], b[i]).
+template <int N>
+__device__ __forceinline__ void apply_op_plain_n(int op, float (&a)[N], const float (&b)[N]) {
+#define MIMK_CASE(OP)                                                              \
+    case OP:                                                                       \
+        _Pragma("unroll") for (int i = 0; i < N; ++i) a[i] = apply_op_plain(OP, a[i], b[i]); \
+        break;
+    switch (op) {
+        MIMK_CASE(MIMK_OP_ADD) MIMK_CASE(MIMK_OP_SUB) MIMK_CASE(MIMK_OP_MUL) MIMK_CASE(MIMK_OP_DIV) MIMK_CASE(MIMK_OP_MAX)
+        MIMK_CASE(MIMK_OP_MIN) MIMK_CASE(MIMK_OP_SUBEXP) MIMK_CASE(MIMK_OP_RELU) MIMK_CASE(MIMK_OP_TANH) MIMK_CASE(MIMK_OP_EXP)
+        MIMK_CASE(MIMK_OP_SILU) MIMK_CASE(MIMK_OP_NEG) MIMK_CASE(MIMK_OP_SQUARE) MIMK_CASE(MIMK_OP_ABS) MIMK_CASE(MIMK_OP_SQRT)
+        MIMK_CASE(MIMK_OP_RSQRT) MIMK_CASE(MIMK_OP_LOG) MIMK_CASE(MIMK_OP_EXP2) MIMK_CASE(MIMK_OP_LOG2) MIMK_CASE(MIMK_OP_SIGMOID)
+        default: break;
+    }
+#undef MIMK_CASE
+}
+template <int N>
+__device__ __forceinline__ void apply_op_n(int op, float (&a)[N], const float (&b)[N]) {
+    const bool composed = op & MIMK_OP_COMPOSED_BASE;
+    apply_op_plain_n(composed ? op & 0xff : op, a, b);
+    if (composed) apply_op_plain_n((op >> 8) & 0xff, a, b);
+}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
