@@ -270,6 +270,12 @@ extern "C" int mimk_attn_fwd(const mimk_attn_desc* d, void* stream) {
     if (paired && attn_tc_pair_supported(*d)) return attn_tc_pair(*d, s);
     if (attn_tc_persistent_supported(*d)) return attn_tc_persistent(*d, s);
     static int composed = -1;  // MIMK_ATTN_COMPOSED=0 keeps every such problem on the one-launch CUDA-core kernel
+    static int f32_tc = -1;
+    if (f32_tc < 0) {
+        const char* e = getenv("MIMK_F32_TC");
+        f32_tc        = (e && e[0] == '0') ? 0 : 1;
+    }
+    if (f32_tc && attn_f32_tc_supported(*d)) return attn_f32_tc(*d, s);
     if (composed < 0) {
         const char* e = getenv("MIMK_ATTN_COMPOSED");
         composed      = (e && e[0] == '0') ? 0 : 1;

@@ -108,6 +108,9 @@ MrpPlan mrp_plan(const mimk_mrp_desc& d);
 int permute_copy(const void* in, void* out, int esize, int rank, const int64_t* out_shape, const int* perm, cudaStream_t s);
 int attn_simt(const mimk_attn_desc& d, cudaStream_t s);
 // f32, and bf16 with other head dims, at scale: the composition S = Q K^T, softmax, O = P V on the contraction and row
+// f32, head_dim up to 128: fused, on the tensor cores, three bf16 pieces per value (attn_f32_tc.cu)
+int attn_f32_tc_supported(const mimk_attn_desc& d);
+int attn_f32_tc(const mimk_attn_desc& d, cudaStream_t s);
 // kernels (attn_composed.cu)
 int attn_composed_supported(const mimk_attn_desc& d);
 int attn_composed(const mimk_attn_desc& d, cudaStream_t s);

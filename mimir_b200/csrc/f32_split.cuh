@@ -1,0 +1,103 @@
+// f32 operands for the bf16 tensor cores: every value as the exact sum of three bf16 pieces, and the shared-memory tiles that
+// hold the pieces.
+//
+// An f32 significand has 24 bits and a bf16 one 8, so cutting x after its first 8 bits, and what is left after its next 8,
+// gives x = h + m + l exactly (below the bf16 range of small numbers the last bits are lost, as in any product that
+// underflows). Of the nine products of two such sums the six with at least 2^-16 of the value are taken,
+//     h h,  h m + m h,  h l + m m + l h,
+// the three left out are below 2^-22 of it. An infinite or NaN operand leaves NaN in a piece, so every cell it reaches
+// comes out non-finite and is computed again by the scalar fold.
+//
+// Tiles: [rows x 32] bf16, K contiguous, 64-byte rows, 64-byte swizzle (16-byte unit u of row r lies at u ^ ((r >> 1) & 3)).
+#pragma once
+
+#include "common.cuh"
+#include "sm100.cuh"
+
+namespace mimk {
+namespace f32split {
+
+constexpr int BK = 32;  // k per tile row
+
+__device__ __forceinline__ uint32_t upper_halves(float a, float b) {
+    return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+}
+__device__ __forceinline__ float lower_part(float x) { return x - __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
+
+__device__ __forceinline__ void st_shared16(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+
+// Eight consecutive k of one row, cut into pieces and stored at `addr` of the three piece tiles (`piece_bytes` apart). Values
+// that are bf16 already are their own first piece (PIECES = 1).
+template <int PIECES = 3>
+__device__ __forceinline__ void split_store8(uint32_t addr, uint32_t piece_bytes, const float (&x)[8]) {
+    st_shared16(addr, upper_halves(x[0], x[1]), upper_halves(x[2], x[3]), upper_halves(x[4], x[5]), upper_halves(x[6], x[7]));
+    if constexpr (PIECES == 3) {
+        float r[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) r[i] = lower_part(x[i]);
+        st_shared16(addr + piece_bytes, upper_halves(r[0], r[1]), upper_halves(r[2], r[3]), upper_halves(r[4], r[5]),
+                    upper_halves(r[6], r[7]));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) r[i] = lower_part(r[i]);
+        st_shared16(addr + 2 * piece_bytes, upper_halves(r[0], r[1]), upper_halves(r[2], r[3]), upper_halves(r[4], r[5]),
+                    upper_halves(r[6], r[7]));
+    }
+}
+__device__ __forceinline__ uint32_t unit_offset(int row, int unit) { return uint32_t(row * 64 + ((unit ^ ((row >> 1) & 3)) << 4)); }
+
+// Shared-memory matrix descriptor of such a tile: K-major, 64-byte swizzle (layout 4), 512 bytes between groups of eight rows.
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t saddr) {
+    uint64_t d = 0;
+    d |= uint64_t((saddr & 0x3FFFFu) >> 4);
+    d |= uint64_t(1) << 16;
+    d |= uint64_t(512 >> 4) << 32;
+    d |= uint64_t(1) << 46;
+    d |= uint64_t(4) << 61;
+    return d;
+}
+
+// D (+)= A B^T over one 32-wide k-block, the six products, smallest first (the tensor core cuts off what its accumulator
+// update cannot hold, which costs least while the accumulator is small). `a` / `b`: the h piece; m and l follow. PIECES = 1: the
+// product of the h pieces alone.
+template <int PIECES = 3>
+__device__ __forceinline__ void mma_six(uint32_t d, uint32_t a, uint32_t a_piece, uint32_t b, uint32_t b_piece, uint32_t idesc) {
+    constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0}, FIRST = PIECES == 1 ? 5 : 0;
+#pragma unroll
+    for (int t = FIRST; t < 6; ++t)
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            sm100::mma_f16_ss(d, smem_desc_sw64(a + PA[t] * a_piece + k * 32), smem_desc_sw64(b + PB[t] * b_piece + k * 32), idesc,
+                              (t > FIRST || k > 0) ? 1u : 0u);
+}
+
+__device__ __forceinline__ float load1(const float* p) { return __ldg(p); }
+__device__ __forceinline__ float load1(const __nv_bfloat16* p) {
+    return __uint_as_float(uint32_t(__ldg(reinterpret_cast<const unsigned short*>(p))) << 16);
+}
+// Eight consecutive elements from `at`, as f32: `left` of them exist (zeros for the rest), none where the row is not there. vec:
+// `at` is 16-byte aligned.
+__device__ __forceinline__ void load8(float (&x)[8], const __nv_bfloat16* at, bool there, int left, bool vec) {
+    if (there && vec && left >= 8) {
+        const uint4 v       = __ldg(reinterpret_cast<const uint4*>(at));
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[2 * i] = __uint_as_float(w[i] << 16), x[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = there && i < left ? load1(at + i) : 0.f;
+    }
+}
+__device__ __forceinline__ void load8(float (&x)[8], const float* at, bool there, int left, bool vec) {
+    if (there && vec && left >= 8) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(at)), b = __ldg(reinterpret_cast<const float4*>(at + 4));
+        x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w, x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = there && i < left ? load1(at + i) : 0.f;
+    }
+}
+
+}  // namespace f32split
+}  // namespace mimk

@@ -54,3 +54,40 @@ def test_folds_and_maps_along_a_middle_axis(T, outer, length, inner, dtype):
     assert torch.equal(d64(T.reduce("max", 1, x)), xd.amax(1)) and torch.equal(d64(T.reduce("min", 1, x)), xd.amin(1))
     want = (xd * yd[:, None]).clamp(min=0)
     close_cells(T.binary_ax("mul", 1, x, y, then="relu"), want, want.abs() + 1e-30, tol)
+
+
+def attention_reference(q, k, v, scale, causal):
+    s = d64(q) @ d64(k).transpose(1, 2) * scale
+    if causal:
+        hidden = torch.ones(s.shape[1:], dtype=torch.bool).triu_(s.shape[2] - s.shape[1] + 1)
+        s = s.masked_fill(hidden, -math.inf)
+        p = torch.softmax(s, -1).masked_fill(hidden, 0.0)
+        p = p.masked_fill(hidden.all(1)[None, :, None], 0.0)
+    else:
+        p = torch.softmax(s, -1)
+    return p @ d64(v), torch.logsumexp(s, -1)
+
+
+@pytest.mark.parametrize("bh,sq,sk,d,causal", [
+    (2, 128, 64, 64, False), (3, 129, 65, 32, False), (2, 300, 191, 33, False), (2, 257, 257, 96, True), (1, 130, 200, 97, True),
+    (2, 200, 100, 128, True), (1, 1, 1000, 80, False), (2, 127, 63, 1, True), (40, 150, 150, 64, False)])
+def test_f32_attention_of_any_length(T, bh, sq, sk, d, causal):
+    q, k, v = rnd((bh, sq, d), 1), rnd((bh, sk, d), 2), rnd((bh, sk, d), 3)
+    got, lse = T.attention(q, k, v, scale=d ** -0.5, causal=causal, return_lse=True)
+    T.device_status()
+    want, want_lse = attention_reference(q, k, v, d ** -0.5, causal)
+    # scores off by F32_CELL of their terms, which the exponential turns into a relative error of the weights
+    assert ((d64(got) - want).abs() <= 64 * F32_CELL).all()
+    seen = want_lse.isfinite()
+    assert torch.equal(d64(lse).isfinite(), seen) and ((d64(lse) - want_lse).abs()[seen] <= 64 * F32_CELL).all()
+    assert torch.equal(got, T.attention(q, k, v, scale=d ** -0.5, causal=causal))
+
+
+def test_f32_attention_with_infinities_takes_the_general_path(T):
+    q, k, v = rnd((2, 300, 64), 1), rnd((2, 200, 64), 2), rnd((2, 200, 64), 3)
+    q[0, 5, 3], k[1, 7, 2], v[0, 9, 1], v[1, 8, 1] = math.inf, -math.inf, math.nan, math.inf
+    got = T.attention(q, k, v, scale=0.125)
+    want, _ = attention_reference(q, k, v, 0.125, False)
+    g = d64(got)
+    assert torch.equal(g.isnan(), want.isnan()) and torch.equal(g.isinf(), want.isinf())
+    assert ((g - want).abs()[want.isfinite()] <= 64 * F32_CELL).all()
