@@ -276,6 +276,7 @@ extern "C" int mimk_attn_fwd(const mimk_attn_desc* d, void* stream) {
         f32_tc        = (e && e[0] == '0') ? 0 : 1;
     }
     if (f32_tc && attn_f32_tc_supported(*d)) return attn_f32_tc(*d, s);
+    if (attn_few_supported(*d)) return attn_few(*d, s);
     if (composed < 0) {
         const char* e = getenv("MIMK_ATTN_COMPOSED");
         composed      = (e && e[0] == '0') ? 0 : 1;

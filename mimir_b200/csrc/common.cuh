@@ -124,6 +124,9 @@ int attn_tc_pair(const mimk_attn_desc& d, cudaStream_t s);
 // ---- device side ----------------------------------------------------------------------------------
 #ifdef __CUDACC__
 // the scalar meaning of MIMK_OP_* (unary ones ignore b)
+// bf16, head_dim 64 or 128, up to 16 query rows: streams K and V once (attn_few.cu)
+int attn_few_supported(const mimk_attn_desc& d);
+int attn_few(const mimk_attn_desc& d, cudaStream_t s);
 __device__ __forceinline__ float apply_op_plain(int op, float a, float b) {
     switch (op) {
         case MIMK_OP_ADD: return a + b;

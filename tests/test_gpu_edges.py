@@ -91,3 +91,28 @@ def test_f32_attention_with_infinities_takes_the_general_path(T):
     g = d64(got)
     assert torch.equal(g.isnan(), want.isnan()) and torch.equal(g.isinf(), want.isinf())
     assert ((g - want).abs()[want.isfinite()] <= 64 * F32_CELL).all()
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("bh,sq,sk,causal", [
+    (3, 1, 1, False), (2, 1, 15, False), (5, 16, 17, True), (2, 16, 9, True), (1, 9, 4097, True), (160, 2, 300, False), (300, 1, 70, True),
+    (1, 1, 5000, False), (7, 5, 1024, False)])
+def test_attention_of_a_few_queries(T, bh, sq, sk, d, causal):
+    q, k, v = rnd((bh, sq, d), 1, BF16), rnd((bh, sk, d), 2, BF16), rnd((bh, sk, d), 3, BF16)
+    got, lse = T.attention(q, k, v, scale=d ** -0.5, causal=causal, return_lse=True)
+    T.device_status()
+    want, want_lse = attention_reference(q, k, v, d ** -0.5, causal)
+    # weights and result are rounded to bf16: 2^-9 of every term
+    weights = attention_reference(q, k, v.abs(), d ** -0.5, causal)[0]
+    assert ((d64(got) - want).abs() <= BF16_ROUND * (want.abs() + weights) + 1e-6).all()
+    seen = want_lse.isfinite()
+    assert torch.equal(d64(lse).isfinite(), seen) and ((d64(lse) - want_lse).abs()[seen] <= 1e-4).all()
+
+
+def test_attention_of_a_few_queries_does_not_read_hidden_keys(T):
+    q, k, v = rnd((2, 4, 64), 1, BF16), rnd((2, 40, 64), 2, BF16), rnd((2, 40, 64), 3, BF16)
+    v[0, 39, 5], v[1, 38, 7] = math.inf, math.nan   # seen by the last query, and by the last two
+    got = d64(T.attention(q, k, v, scale=0.125, causal=True))
+    assert got[0, :3].isfinite().all() and got[0, 3, 5].isinf() and got[1, :2].isfinite().all() and got[1, 2:, 7].isnan().all()
+    want, _ = attention_reference(q, k, v.nan_to_num(0, 0, 0), 0.125, True)
+    assert ((got - want).abs()[0, :3] <= 0.03).all() and ((got - want).abs()[1, :2] <= 0.03).all()
