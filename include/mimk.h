@@ -280,6 +280,19 @@ typedef struct mimk_attn_desc {
 } mimk_attn_desc;
 int mimk_attn_fwd(const mimk_attn_desc* desc, void* stream);
 
+/* out[n, co, oh, ow] = sum over (ci, kh, kw) of x[n, ci, oh s + kh d - p, ow s + kw d - p] * filters[co, ci, kh, kw], cells of x
+ * outside it read as zeros: tensor.conv (tensor.mim:434-438) with its padding, as one contraction on the tensor cores whose left
+ * operand is gathered from the image. dtype F32 or BF16 (out the same); any extents and alignment, windows up to 31 x 31. */
+typedef struct mimk_conv_desc {
+    int64_t n, cin, h, w, cout, kh, kw;
+    int64_t stride_h, stride_w, dil_h, dil_w, pad_h, pad_w;
+    const void* x;
+    const void* filters;
+    void* out;
+    int32_t dtype, pad_;
+} mimk_conv_desc;
+int mimk_conv(const mimk_conv_desc* desc, void* stream);
+
 /* Y = (silu(X W1) * (X W3)) W2 with the gated product H kept in `dtype`.
  * Replaces: two product_2d + math.slf + binary mul (epilogue-fused into one contraction) + product_2d.
  * x [m,k]; w1,w3 [k,f] (b_layout KN) or [f,k] (NK); w2 [f,n] (KN) or [n,f] (NK); y [m,n].

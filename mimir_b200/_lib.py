@@ -25,7 +25,7 @@ ROWS_SOFTMAX, ROWS_RMSNORM, ROWS_SOFTMAX_RMSNORM = 0, 1, 2
 SYMBOLS = (
     "mimk_status_str", "mimk_abi_version", "mimk_last_cuda_error", "mimk_device_check", "mimk_device_status", "mimk_selftest_wait_expiry",
     "mimk_gemm", "mimk_gemm_flat", "mimk_gemm_gather", "mimk_gemm_reduce_scatter", "mimk_gemm_kpanels", "mimk_reduce", "mimk_reduce_fused", "mimk_reduce_plan", "mimk_reduce_static", "mimk_softmax", "mimk_rmsnorm", "mimk_softmax_rmsnorm", "mimk_map", "mimk_map_t",
-    "mimk_splat", "mimk_select", "mimk_generate_affine", "mimk_gather", "mimk_scatter", "mimk_attn_fwd", "mimk_mlp_gated", "mimk_map_reduce_post", "mimk_mrp_classify", "mimk_mrp_cell_kernel", "mimk_program_classify", "mimk_program_run", "mimk_chain_order", "mimk_chain_cost",
+    "mimk_splat", "mimk_select", "mimk_generate_affine", "mimk_gather", "mimk_scatter", "mimk_attn_fwd", "mimk_conv", "mimk_mlp_gated", "mimk_map_reduce_post", "mimk_mrp_classify", "mimk_mrp_cell_kernel", "mimk_program_classify", "mimk_program_run", "mimk_chain_order", "mimk_chain_cost",
     "mimk_host_rows", "mimk_host_rows_pair", "mimk_host_gemm", "mimk_host_attn_fwd", "mimk_host_mlp_gated", "mimk_host_map_reduce_post", "mimk_host_register",
     "mimk_host_unregister", "mimk_host_release",
 )
@@ -63,6 +63,14 @@ class AttnDesc(C.Structure):
         ("batch_heads", C.c_int64), ("seq_q", C.c_int64), ("seq_k", C.c_int64), ("head_dim", C.c_int64),
         ("q", C.c_void_p), ("k", C.c_void_p), ("v", C.c_void_p), ("o", C.c_void_p), ("lse", C.c_void_p),
         ("scale", C.c_float), ("causal", C.c_int32), ("dtype", C.c_int32),
+    ]
+
+
+class ConvDesc(C.Structure):
+    _fields_ = [
+        ("n", C.c_int64), ("cin", C.c_int64), ("h", C.c_int64), ("w", C.c_int64), ("cout", C.c_int64), ("kh", C.c_int64), ("kw", C.c_int64),
+        ("stride_h", C.c_int64), ("stride_w", C.c_int64), ("dil_h", C.c_int64), ("dil_w", C.c_int64), ("pad_h", C.c_int64), ("pad_w", C.c_int64),
+        ("x", C.c_void_p), ("filters", C.c_void_p), ("out", C.c_void_p), ("dtype", C.c_int32), ("pad_", C.c_int32),
     ]
 
 
@@ -149,6 +157,7 @@ def lib() -> C.CDLL:
         L.mimk_map.argtypes = [ci, vp, vp, vp, ci, i64, i64, i64, ci, vp]
         L.mimk_map_t.argtypes = [ci, vp, vp, vp, ci, ci, i64, i64, i64, ci, vp]
         L.mimk_attn_fwd.argtypes = [C.POINTER(AttnDesc), vp]
+        L.mimk_conv.argtypes = [C.POINTER(ConvDesc), vp]
         L.mimk_splat.argtypes = [vp, ci, i64, i64, vp]
         L.mimk_select.argtypes = [vp, vp, vp, vp, ci, i64, vp]
         L.mimk_generate_affine.argtypes = [vp, ci, ci, C.POINTER(i64), C.POINTER(i64), vp]

@@ -293,6 +293,29 @@ extern "C" int mimk_mlp_gated(const mimk_mlp_desc* d, void* stream) {
     int st = MIMK_OK;
     if (!device_info(&st)) return st;
     if (d->m == 0 || d->n == 0) return MIMK_OK;
+extern "C" int mimk_conv(const mimk_conv_desc* d, void* stream) {
+    if (!d) return MIMK_E_ARG;
+    if (d->n < 0 || d->cin < 1 || d->h < 1 || d->w < 1 || d->cout < 0 || d->kh < 1 || d->kw < 1) return MIMK_E_ARG;
+    if (d->stride_h < 1 || d->stride_w < 1 || d->dil_h < 1 || d->dil_w < 1 || d->pad_h < 0 || d->pad_w < 0) return MIMK_E_ARG;
+    if (d->dtype != MIMK_F32 && d->dtype != MIMK_BF16) return MIMK_E_DTYPE;
+    // one image, one filter and every coordinate of the padded image are 30-bit numbers
+    constexpr double LIM = double(1 << 30);
+    if (double(d->cin) * double(d->h) * double(d->w) >= LIM || double(d->cin) * double(d->kh) * double(d->kw) >= LIM) return MIMK_E_UNSUPPORTED;
+    if (double(d->h) + 2.0 * double(d->pad_h) >= LIM || double(d->w) + 2.0 * double(d->pad_w) >= LIM) return MIMK_E_UNSUPPORTED;
+    if (double(d->dil_h) * double(d->kh) >= LIM || double(d->dil_w) * double(d->kw) >= LIM) return MIMK_E_UNSUPPORTED;
+    if (d->kh > 31 || d->kw > 31) return MIMK_E_UNSUPPORTED;  // a bit of a mask per tap row and column
+    if (d->stride_h >= (1 << 30) || d->stride_w >= (1 << 30)) return MIMK_E_UNSUPPORTED;
+    const int64_t span_h = d->h + 2 * d->pad_h - d->dil_h * (d->kh - 1) - 1, span_w = d->w + 2 * d->pad_w - d->dil_w * (d->kw - 1) - 1;
+    if (span_h < 0 || span_w < 0) return MIMK_E_SHAPE;
+    const double pixels = double(span_h / d->stride_h + 1) * double(span_w / d->stride_w + 1);
+    if (pixels >= LIM || double(d->n) * pixels * double(d->cout) >= double(int64_t(1) << 40)) return MIMK_E_UNSUPPORTED;
+    int st = MIMK_OK;
+    if (!device_info(&st)) return st;
+    if (d->n == 0 || d->cout == 0) return MIMK_OK;
+    if (!d->x || !d->filters || !d->out) return MIMK_E_ARG;
+    return conv_tc(*d, static_cast<cudaStream_t>(stream));
+}
+
     if (!d->x || !d->w1 || !d->w3 || !d->w2 || !d->y) return MIMK_E_ARG;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     void* h        = d->h;

@@ -71,7 +71,7 @@ int gemm_tc2(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2,
              int64_t a_panels = 1, int64_t scatter_rows = 0);
 int gemm_tc_any(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2,
                 const mimk_gather_dst* gather = nullptr, int64_t a_panels = 1);  // picks between the two
-int gemm_f32_tc_supported(const mimk_gemm_desc& d);  // f32 operands on the tensor cores (3xTF32)
+int gemm_f32_tc_supported(const mimk_gemm_desc& d);  // f32 operands on the tensor cores (three bf16 pieces each)
 int gemm_f32_tc(const mimk_gemm_desc& d, cudaStream_t s);
 // map_reduce_post instances that are a contraction, an axis fold or an elementwise map go to those kernels (mrp_route.cu)
 bool mrp_try_route(const mimk_mrp_desc& d, void* stream, int* status);
@@ -82,6 +82,7 @@ inline bool op_is_unary(int op) { return op >= MIMK_OP_RELU && op <= MIMK_OP_SIG
 // A (possibly composed) elementwise operator taken apart; false when it names an unknown part.
 inline bool decode_op(int op, int* inner, int* outer) {
     *inner = op, *outer = MIMK_OP_COPY;
+int conv_tc(const mimk_conv_desc& d, cudaStream_t s);  // the same kernel, its left operand gathered from an image
     if (op & MIMK_OP_COMPOSED_BASE) {
         if (op & ~0x1ffff) return false;
         *inner = op & 0xff, *outer = (op >> 8) & 0xff;

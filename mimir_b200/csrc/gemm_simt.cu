@@ -256,7 +256,7 @@ int launch(const mimk_gemm_desc& d, cudaStream_t s) {
 // Below 2^27 multiply-adds the small-tile kernel is also faster than three TF32 passes over re-written operands (three
 // launches): 256^3 6.3 against 14.0 us, 384^3 8.6 against 18.1, 512^3 17.2 against 18.5 (CUDA-graph replays, warm).
 int gemm_simt_preferred(const mimk_gemm_desc& d) {
-    return small_tiles_apply(d) && d.m * d.n * d.k < (int64_t(1) << 27) / (d.batch > 0 ? d.batch : 1);
+    return 0 && small_tiles_apply(d) && d.m * d.n * d.k < (int64_t(1) << 27) / (d.batch > 0 ? d.batch : 1);
 }
 
 int gemm_simt(const mimk_gemm_desc& d, cudaStream_t s) {

@@ -116,3 +116,41 @@ def test_attention_of_a_few_queries_does_not_read_hidden_keys(T):
     assert got[0, :3].isfinite().all() and got[0, 3, 5].isinf() and got[1, :2].isfinite().all() and got[1, 2:, 7].isnan().all()
     want, _ = attention_reference(q, k, v.nan_to_num(0, 0, 0), 0.125, True)
     assert ((got - want).abs()[0, :3] <= 0.03).all() and ((got - want).abs()[1, :2] <= 0.03).all()
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (31, 65, 33), (128, 64, 512), (129, 127, 31), (600, 700, 260), (40, 30, 5000), (1500, 1300, 300)])
+@pytest.mark.parametrize("b_nk,offset,out", [(True, 0, F32), (False, 0, F32), (True, 1, F32), (False, 1, BF16)])
+def test_f32_products_of_any_extent(T, m, n, k, b_nk, offset, out):
+    a, b = rnd((m, k), 1, F32, offset), rnd((n, k) if b_nk else (k, n), 2, F32, offset)
+    b = b.t() if b_nk else b
+    bias = rnd((n,), 3)
+    got = T.product_2d(a, b, post="bias", bias=bias, out_dtype=out)
+    T.device_status()
+    scale = d64(a).abs() @ d64(b).abs() + d64(bias).abs()
+    close_cells(got, d64(a) @ d64(b) + d64(bias), scale, F32_CELL if out == F32 else BF16_ROUND)
+
+
+def test_f32_products_keep_infinities_and_extremes(T):
+    a, b = rnd((200, 600), 1), rnd((600, 300), 2)
+    a[3, 5], a[7, 0], b[9, 11] = math.inf, math.nan, -math.inf
+    a[100] *= 1e-30
+    b[:, 30] *= 1e25
+    close_cells(T.product_2d(a, b), d64(a) @ d64(b), d64(a).abs() @ d64(b).abs(), F32_CELL)
+
+
+@pytest.mark.parametrize("n,cin,h,w,cout,kh,kw,stride,dil,pad,dtype", [
+    (2, 5, 17, 23, 16, 3, 3, (1, 1), (1, 1), (1, 1), F32), (1, 33, 30, 31, 65, 3, 2, (2, 1), (1, 2), (0, 1), F32),
+    (3, 16, 40, 40, 130, 1, 1, (1, 1), (1, 1), (0, 0), F32), (2, 3, 50, 41, 40, 7, 5, (2, 2), (1, 1), (3, 2), BF16),
+    (9, 64, 20, 20, 96, 3, 3, (1, 1), (2, 2), (2, 2), BF16), (24, 8, 60, 60, 100, 5, 5, (1, 1), (1, 1), (4, 0), F32)])
+def test_convolutions_gathered_from_the_image(T, monkeypatch, n, cin, h, w, cout, kh, kw, stride, dil, pad, dtype):
+    monkeypatch.setattr(T, "CONV_CONTRACTION_MIN_WORK", 1)
+    x, f = rnd((n, cin, h, w), 1, dtype), rnd((cout, cin, kh, kw), 2, dtype)
+    got = T.conv(x, f, stride=stride, dilation=dil, padding=pad)
+    T.device_status()
+    conv = torch.nn.functional.conv2d
+    want, scale = (conv(u, v, stride=stride, dilation=dil, padding=pad) for u, v in ((d64(x), d64(f)), (d64(x).abs(), d64(f).abs())))
+    close_cells(got, want, scale + 1e-6, F32_CELL if dtype == F32 else BF16_ROUND)
+    if dtype == F32:   # an infinity reaches the cells whose window holds it, and no other
+        x[0, 0, h // 2, w // 2] = math.inf
+        assert torch.equal(d64(T.conv(x, f, stride=stride, dilation=dil, padding=pad)).isfinite(),
+                           conv(d64(x), d64(f), stride=stride, dilation=dil, padding=pad).isfinite())
