@@ -112,6 +112,10 @@ int gemm_tc_any(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* 
         const char* e = getenv("MIMK_GEMM_2CTA");
         allow_pair    = (e && e[0] == '0') ? 0 : ((e && e[0] == '2') ? 2 : 1);
     }
+    int st                = MIMK_OK;
+    const DeviceInfo* dev = device_info(&st);
+    if (!dev) return st;
+    if (allow_pair != 2 && !gather && a_panels == 1 && gemm_tc_split_preferred(d, gated, dev->sm_count)) return gemm_tc_split(d, s, gated, b2);
     // the paired kernel takes one launch per batch entry; long batches go to the one-CTA kernel, which walks
     // (batch, tile) pairs in a single launch
     if (allow_pair == 2 && d.batch <= 64 && gemm_tc_supported(d)) return gemm_tc2(d, s, gated, b2, gather, a_panels);
@@ -179,6 +183,10 @@ extern "C" int mimk_gemm(const mimk_gemm_desc* d, void* stream) {
     if (!d->c || (d->k > 0 && (!d->a || !d->b))) return MIMK_E_ARG;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (gemm_tc_supported(*d)) return gemm_tc_any(*d, s, 0, nullptr);
+    if (d->in_dtype == MIMK_BF16) {
+        const int r = gemm_tc_ragged(*d, s);
+        if (r != MIMK_E_UNSUPPORTED) return r;
+    }
     static int f32_tc = -1;  // MIMK_F32_TC=0 keeps f32 contractions on the CUDA cores (for A/B measurements)
     if (f32_tc < 0) {
         const char* e = getenv("MIMK_F32_TC");
@@ -268,6 +276,7 @@ extern "C" int mimk_attn_fwd(const mimk_attn_desc* d, void* stream) {
         paired        = (e && e[0] == '1') ? 1 : 0;
     }
     if (paired && attn_tc_pair_supported(*d)) return attn_tc_pair(*d, s);
+    if (attn_few_supported(*d)) return attn_few(*d, s);
     if (attn_tc_persistent_supported(*d)) return attn_tc_persistent(*d, s);
     static int composed = -1;  // MIMK_ATTN_COMPOSED=0 keeps every such problem on the one-launch CUDA-core kernel
     static int f32_tc = -1;
@@ -276,7 +285,6 @@ extern "C" int mimk_attn_fwd(const mimk_attn_desc* d, void* stream) {
         f32_tc        = (e && e[0] == '0') ? 0 : 1;
     }
     if (f32_tc && attn_f32_tc_supported(*d)) return attn_f32_tc(*d, s);
-    if (attn_few_supported(*d)) return attn_few(*d, s);
     if (composed < 0) {
         const char* e = getenv("MIMK_ATTN_COMPOSED");
         composed      = (e && e[0] == '0') ? 0 : 1;
@@ -285,14 +293,6 @@ extern "C" int mimk_attn_fwd(const mimk_attn_desc* d, void* stream) {
     return attn_simt(*d, s);
 }
 
-extern "C" int mimk_mlp_gated(const mimk_mlp_desc* d, void* stream) {
-    if (!d) return MIMK_E_ARG;
-    if (d->m < 0 || d->k < 0 || d->f < 0 || d->n < 0) return MIMK_E_ARG;
-    if (d->dtype != MIMK_BF16) return MIMK_E_DTYPE;
-    if (d->b_layout != MIMK_B_KN && d->b_layout != MIMK_B_NK) return MIMK_E_ARG;
-    int st = MIMK_OK;
-    if (!device_info(&st)) return st;
-    if (d->m == 0 || d->n == 0) return MIMK_OK;
 extern "C" int mimk_conv(const mimk_conv_desc* d, void* stream) {
     if (!d) return MIMK_E_ARG;
     if (d->n < 0 || d->cin < 1 || d->h < 1 || d->w < 1 || d->cout < 0 || d->kh < 1 || d->kw < 1) return MIMK_E_ARG;
@@ -316,6 +316,14 @@ extern "C" int mimk_conv(const mimk_conv_desc* d, void* stream) {
     return conv_tc(*d, static_cast<cudaStream_t>(stream));
 }
 
+extern "C" int mimk_mlp_gated(const mimk_mlp_desc* d, void* stream) {
+    if (!d) return MIMK_E_ARG;
+    if (d->m < 0 || d->k < 0 || d->f < 0 || d->n < 0) return MIMK_E_ARG;
+    if (d->dtype != MIMK_BF16) return MIMK_E_DTYPE;
+    if (d->b_layout != MIMK_B_KN && d->b_layout != MIMK_B_NK) return MIMK_E_ARG;
+    int st = MIMK_OK;
+    if (!device_info(&st)) return st;
+    if (d->m == 0 || d->n == 0) return MIMK_OK;
     if (!d->x || !d->w1 || !d->w3 || !d->w2 || !d->y) return MIMK_E_ARG;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     void* h        = d->h;

@@ -63,16 +63,26 @@ int gemm_simt_preferred(const mimk_gemm_desc& d);  // small f32 product: the 32 
 int gemm_tc_supported(const mimk_gemm_desc& d);
 // a_panels > 1: A is given as that many row-major [m, k / a_panels] matrices one after another (the layout an all-gather
 // of column slabs delivers); k / a_panels must then be a multiple of 64
+// pitch: operands whose rows are that many elements apart, and a result of any pitch and alignment (plain stores)
+struct GemmPitch {
+    int64_t a, b;
+};
 int gemm_tc(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, const mimk_gather_dst* gather = nullptr,
-            int64_t a_panels = 1);
+            int64_t a_panels = 1, const GemmPitch* pitch = nullptr);
+int gemm_tc_ragged(const mimk_gemm_desc& d, cudaStream_t s);  // bf16 with extents or pointers TMA cannot take as they are
+// few tiles: narrower ones, their k-blocks dealt out to a cluster (gemm_tc_split.cu); takes what gemm_tc takes, one destination
+int gemm_tc_split_preferred(const mimk_gemm_desc& d, int gated, int sm_count);
+int gemm_tc_split(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, const GemmPitch* pitch = nullptr);
+int gemm_tc2_enough(int64_t m, int64_t n, int gated);        // the paired kernel has tiles for every pair of SMs
 int gemm_tc2_supported(const mimk_gemm_desc& d, int gated);  // the paired-SM (cta_group::2) form
 // scatter_rows > 0 (gemm_tc2 only): rows [t scatter_rows, (t + 1) scatter_rows) of the f32 result are added into gather->dst[t]
 int gemm_tc2(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, const mimk_gather_dst* gather = nullptr,
-             int64_t a_panels = 1, int64_t scatter_rows = 0);
+             int64_t a_panels = 1, int64_t scatter_rows = 0, const GemmPitch* pitch = nullptr);
 int gemm_tc_any(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2,
                 const mimk_gather_dst* gather = nullptr, int64_t a_panels = 1);  // picks between the two
 int gemm_f32_tc_supported(const mimk_gemm_desc& d);  // f32 operands on the tensor cores (three bf16 pieces each)
 int gemm_f32_tc(const mimk_gemm_desc& d, cudaStream_t s);
+int conv_tc(const mimk_conv_desc& d, cudaStream_t s);  // the same kernel, its left operand gathered from an image
 // map_reduce_post instances that are a contraction, an axis fold or an elementwise map go to those kernels (mrp_route.cu)
 bool mrp_try_route(const mimk_mrp_desc& d, void* stream, int* status);
 // What a descriptor's access maps spell, whatever its size (the router itself leaves small instances on the per-cell
@@ -82,7 +92,6 @@ inline bool op_is_unary(int op) { return op >= MIMK_OP_RELU && op <= MIMK_OP_SIG
 // A (possibly composed) elementwise operator taken apart; false when it names an unknown part.
 inline bool decode_op(int op, int* inner, int* outer) {
     *inner = op, *outer = MIMK_OP_COPY;
-int conv_tc(const mimk_conv_desc& d, cudaStream_t s);  // the same kernel, its left operand gathered from an image
     if (op & MIMK_OP_COMPOSED_BASE) {
         if (op & ~0x1ffff) return false;
         *inner = op & 0xff, *outer = (op >> 8) & 0xff;
@@ -115,6 +124,9 @@ int attn_f32_tc(const mimk_attn_desc& d, cudaStream_t s);
 // kernels (attn_composed.cu)
 int attn_composed_supported(const mimk_attn_desc& d);
 int attn_composed(const mimk_attn_desc& d, cudaStream_t s);
+// bf16, head_dim 64 or 128, up to 16 query rows: streams K and V once (attn_few.cu)
+int attn_few_supported(const mimk_attn_desc& d);
+int attn_few(const mimk_attn_desc& d, cudaStream_t s);
 // bf16, head_dim 64 or 128: one CTA per SM pulls (head, query-tile pair) items, hand-over between items pipelined
 int attn_tc_persistent_supported(const mimk_attn_desc& d);
 int attn_tc_persistent(const mimk_attn_desc& d, cudaStream_t s);
@@ -125,9 +137,6 @@ int attn_tc_pair(const mimk_attn_desc& d, cudaStream_t s);
 // ---- device side ----------------------------------------------------------------------------------
 #ifdef __CUDACC__
 // the scalar meaning of MIMK_OP_* (unary ones ignore b)
-// bf16, head_dim 64 or 128, up to 16 query rows: streams K and V once (attn_few.cu)
-int attn_few_supported(const mimk_attn_desc& d);
-int attn_few(const mimk_attn_desc& d, cudaStream_t s);
 __device__ __forceinline__ float apply_op_plain(int op, float a, float b) {
     switch (op) {
         case MIMK_OP_ADD: return a + b;

@@ -16,6 +16,7 @@
 // Two accumulator buffers in TMEM let the epilogue of tile i overlap the main loop of tile i+1.
 // Every mbarrier wait is bounded; on expiry the CTA records MIMK_E_DEVICE_WAIT and unwinds (frees TMEM, exits).
 #include "common.cuh"
+#include "gemm_epilogue.cuh"
 #include "sm100.cuh"
 
 namespace mimk {
@@ -78,7 +79,8 @@ __device__ __forceinline__ void tile_coords(int64_t tile, int64_t tiles_m, int64
 }
 
 // BN: output-tile width per B operand (256 plain, 128 gated). B_MN: B stored [K,N] (N contiguous).
-template <int BN, bool B_MN, bool GATED, class TOut>
+// DIRECT: the one destination is written by plain stores (store_piece).
+template <int BN, bool B_MN, bool GATED, class TOut, bool DIRECT>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ OutMaps om, const Params p) {
@@ -246,17 +248,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         tc_fence_before();
                         mbar_arrive(smem_u32(&bars->acc_empty[acc]));
                     }
-                    if (p.post != MIMK_POST_ID && row < p.M) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            const int64_t col = n0 + c + i;
-                            if (col < p.N) {
-                                const float rowv = p.post_row ? __ldg(p.post_row + col) : 0.f;
-                                const float full = post_full ? float(post_full[zoff + row * p.N + col]) : 0.f;
-                                v[i]             = apply_post(p.post, v[i], rowv, full);
-                            }
-                        }
-                    }
+                    if (p.post != MIMK_POST_ID && row < p.M)
+                        apply_post_32(p.post, v, p.post_row, post_full ? post_full + zoff + row * p.N : nullptr, n0 + c, p.N);
                     // this thread's row of the piece: 16-byte units at (unit ^ (row & 7)), the 128-byte swizzle
                     const uint32_t row_addr = buf + lane * 128;
                     if (sizeof(TOut) == 2) {
@@ -279,6 +272,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                          : "memory");
                         }
                     }
+                }
+                if (DIRECT) {
+                    __syncwarp();
+                    store_piece(smem_raw + (buf - raw_addr), static_cast<TOut*>(p.dst[0]) + zoff + row0 * p.ldc + n0 + c0, p.ldc, p.M - row0,
+                                p.N - n0 - c0, lane);
+                    continue;  // the next piece goes to the other buffer, and the one after waits for this warp above
                 }
                 fence_proxy_async_smem();  // the bulk store reads shared memory through the async proxy
                 __syncwarp();
@@ -324,10 +323,10 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-template <int BN, bool B_MN, bool GATED, class TOut>
+template <int BN, bool B_MN, bool GATED, class TOut, bool DIRECT = false>
 int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tB2, const OutMaps& om, const Params& p,
            int sm_count, cudaStream_t s) {
-    auto kern = gemm_tc_kernel<BN, B_MN, GATED, TOut>;
+    auto kern = gemm_tc_kernel<BN, B_MN, GATED, TOut, DIRECT>;
     static bool configured[64] = {};  // per template instance and device: the attribute is a per-device setting
     int dev = 0;
     MIMK_CUDA_TRY(cudaGetDevice(&dev));
@@ -339,6 +338,66 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tB2,
     const int grid      = int(tiles < sm_count ? tiles : sm_count);
     kern<<<grid, NUM_THREADS, SMEM_BYTES, s>>>(tA, tB, tB2, om, p);
     return launch_status();
+}
+
+// Rows of `cols` bf16, one after another, copied to rows of `pitch` (a multiple of 8) elements, 16 bytes per thread; up to two
+// such matrices in one launch. What lies between cols and pitch is never read (the tensor maps end at cols) and gets zeros.
+// Sources start at any element: words are read aligned and shifted together, single elements where a word would reach outside.
+struct PackJob {
+    const uint16_t* src;
+    uint16_t* dst;
+    int64_t rows, cols, pitch;
+};
+__device__ __forceinline__ void pack_unit(const PackJob& j, int64_t i) {
+    const int64_t units = j.pitch >> 3, r = i / units, c = (i - r * units) * 8;
+    const uint16_t* s = j.src + r * j.cols + c;
+    const int64_t here = r * j.cols + c, total = j.rows * j.cols;
+    uint32_t w[4];
+    if (c + 8 <= j.cols && here >= 1 && here + 9 <= total) {
+        const bool shifted  = (reinterpret_cast<uintptr_t>(s) >> 1) & 1;
+        const uint32_t* a   = reinterpret_cast<const uint32_t*>(s - (shifted ? 1 : 0));
+        const uint32_t q[5] = {__ldg(a), __ldg(a + 1), __ldg(a + 2), __ldg(a + 3), shifted ? __ldg(a + 4) : 0u};
+#pragma unroll
+        for (int t = 0; t < 4; ++t) w[t] = shifted ? __funnelshift_r(q[t], q[t + 1], 16) : q[t];
+    } else {
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const uint32_t lo = c + 2 * t < j.cols ? s[2 * t] : 0u, hi = c + 2 * t + 1 < j.cols ? s[2 * t + 1] : 0u;
+            w[t] = lo | (hi << 16);
+        }
+    }
+    *reinterpret_cast<uint4*>(j.dst + r * j.pitch + c) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+__global__ void __launch_bounds__(256) pack_rows_kernel(const PackJob a, const PackJob b) {
+    const int64_t na = a.rows * (a.pitch >> 3), nb = b.rows * (b.pitch >> 3);
+    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < na + nb; i += int64_t(gridDim.x) * blockDim.x) {
+        if (i < na) pack_unit(a, i);
+        else pack_unit(b, i - na);
+    }
+}
+
+// How the operands of a bf16 contraction have to be laid out for TMA (16-byte pitch, base and batch stride).
+struct RaggedPlan {
+    bool pack_a, pack_b;
+    int64_t rows_a, cols_a, pitch_a, rows_b, cols_b, pitch_b;
+    size_t bytes_a, bytes_b;
+};
+bool ragged_plan(const mimk_gemm_desc& d, RaggedPlan* r) {
+    if (d.in_dtype != MIMK_BF16 || d.k <= 0) return false;
+    constexpr int64_t LIM = int64_t(1) << 31;
+    if (d.m >= LIM || d.n >= LIM || d.k >= LIM || d.batch >= LIM) return false;
+    const bool b_mn = d.b_layout == MIMK_B_KN;
+    const int64_t row_b = b_mn ? d.n : d.k, out_b = b_mn ? d.k : d.n;
+    const bool a_b = d.batch > 1 && d.stride_a != 0, b_b = d.batch > 1 && d.stride_b != 0;
+    // batches: one after another, or shared by all entries; results that lie one after another
+    if ((a_b && d.stride_a != d.m * d.k) || (b_b && d.stride_b != d.n * d.k) || (d.batch > 1 && d.stride_c != d.m * d.n)) return false;
+    r->rows_a = (a_b ? d.batch : 1) * d.m, r->cols_a = d.k, r->pitch_a = (d.k + 7) & ~int64_t(7);
+    r->rows_b = (b_b ? d.batch : 1) * out_b, r->cols_b = row_b, r->pitch_b = (row_b + 7) & ~int64_t(7);
+    r->pack_a = d.k % 8 != 0 || !aligned16(d.a) || (a_b && d.stride_a % 8 != 0);
+    r->pack_b = row_b % 8 != 0 || !aligned16(d.b) || (b_b && d.stride_b % 8 != 0);
+    r->bytes_a = r->pack_a ? (size_t(r->rows_a) * r->pitch_a * 2 + 255) & ~size_t(255) : 0;
+    r->bytes_b = r->pack_b ? size_t(r->rows_b) * r->pitch_b * 2 : 0;
+    return double(r->rows_a) * double(r->pitch_a) < double(int64_t(1) << 38) && double(r->rows_b) * double(r->pitch_b) < double(int64_t(1) << 38);
 }
 
 }  // namespace
@@ -417,7 +476,7 @@ int gemm_tc_supported(const mimk_gemm_desc& d) {
 }
 
 int gemm_tc(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, const mimk_gather_dst* gather,
-            int64_t a_panels) {
+            int64_t a_panels, const GemmPitch* pitch) {
     int st          = MIMK_OK;
     DeviceInfo* dev = device_info(&st);
     if (!dev) return st;
@@ -427,21 +486,22 @@ int gemm_tc(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, 
     const bool a_b = d.batch > 1 && d.stride_a != 0, b_b = d.batch > 1 && d.stride_b != 0;
     const uint64_t na = a_b ? uint64_t(d.batch) : 1, nb = b_b ? uint64_t(d.batch) : 1;
     // (the outermost stride of a one-entry operand is never used; it only has to be a legal value)
-    const uint64_t row_b = (b_mn ? uint64_t(d.n) : uint64_t(d.k)) * 2;
-    const uint64_t whole_a = uint64_t(d.m) * uint64_t(d.k) * 2, whole_b = uint64_t(d.n) * uint64_t(d.k) * 2;
-    const uint64_t sa = a_b ? uint64_t(d.stride_a) * 2 : (whole_a < (uint64_t(1) << 40) ? whole_a : uint64_t(d.k) * 2);
+    const uint64_t lda = pitch ? uint64_t(pitch->a) : uint64_t(d.k), ldb = pitch ? uint64_t(pitch->b) : (b_mn ? uint64_t(d.n) : uint64_t(d.k));
+    const uint64_t row_b = ldb * 2;
+    const uint64_t whole_a = uint64_t(d.m) * lda * 2, whole_b = (b_mn ? uint64_t(d.k) : uint64_t(d.n)) * row_b;
+    const uint64_t sa = a_b ? uint64_t(d.stride_a) * 2 : (whole_a < (uint64_t(1) << 40) ? whole_a : lda * 2);
     const uint64_t sb = b_b ? uint64_t(d.stride_b) * 2 : (whole_b < (uint64_t(1) << 40) ? whole_b : row_b);
     const void* B2 = b2 ? b2 : d.b;
     CUtensorMap tA, tB, tB2;
     if (a_panels < 1 || (a_panels > 1 && (d.batch != 1 || d.k % a_panels != 0 || (d.k / a_panels) % BK != 0))) return MIMK_E_UNSUPPORTED;
     const uint64_t kp = uint64_t(d.k / a_panels);  // A as a [panels * m, k / panels] matrix: panel g starts at row g * m
-    MIMK_TRY(make_tmap_bf16_3d(&tA, d.a, kp, uint64_t(d.m) * uint64_t(a_panels), na, kp * 2, sa, BK, BM));
+    MIMK_TRY(make_tmap_bf16_3d(&tA, d.a, kp, uint64_t(d.m) * uint64_t(a_panels), na, pitch ? lda * 2 : kp * 2, sa, BK, BM));
     if (b_mn) {
-        MIMK_TRY(make_tmap_bf16_3d(&tB, d.b, uint64_t(d.n), uint64_t(d.k), nb, uint64_t(d.n) * 2, sb, 64, BK));
-        MIMK_TRY(make_tmap_bf16_3d(&tB2, B2, uint64_t(d.n), uint64_t(d.k), nb, uint64_t(d.n) * 2, sb, 64, BK));
+        MIMK_TRY(make_tmap_bf16_3d(&tB, d.b, uint64_t(d.n), uint64_t(d.k), nb, row_b, sb, 64, BK));
+        MIMK_TRY(make_tmap_bf16_3d(&tB2, B2, uint64_t(d.n), uint64_t(d.k), nb, row_b, sb, 64, BK));
     } else {
-        MIMK_TRY(make_tmap_bf16_3d(&tB, d.b, uint64_t(d.k), uint64_t(d.n), nb, uint64_t(d.k) * 2, sb, BK, uint32_t(bn)));
-        MIMK_TRY(make_tmap_bf16_3d(&tB2, B2, uint64_t(d.k), uint64_t(d.n), nb, uint64_t(d.k) * 2, sb, BK, uint32_t(bn)));
+        MIMK_TRY(make_tmap_bf16_3d(&tB, d.b, uint64_t(d.k), uint64_t(d.n), nb, row_b, sb, BK, uint32_t(bn)));
+        MIMK_TRY(make_tmap_bf16_3d(&tB2, B2, uint64_t(d.k), uint64_t(d.n), nb, row_b, sb, BK, uint32_t(bn)));
     }
     Params p;
     p.M = d.m, p.N = d.n, p.K = d.k;
@@ -464,13 +524,22 @@ int gemm_tc(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, 
     p.status    = dev->status_dev;
     // destination maps: [batch, M, N] windows (row pitch ldc) starting at column col_off, boxes of 32 rows x 128 bytes
     const uint64_t out_size = d.out_dtype == MIMK_BF16 ? 2 : 4;
-    const uint64_t pitch    = uint64_t(p.ldc) * out_size;
-    const uint64_t whole_c  = uint64_t(d.m) * pitch;
-    const uint64_t sc = d.batch > 1 ? uint64_t(d.stride_c) * out_size : (whole_c < (uint64_t(1) << 40) ? whole_c : pitch);
+    const uint64_t row_c    = uint64_t(p.ldc) * out_size;
+    const uint64_t whole_c  = uint64_t(d.m) * row_c;
+    const uint64_t sc = d.batch > 1 ? uint64_t(d.stride_c) * out_size : (whole_c < (uint64_t(1) << 40) ? whole_c : row_c);
     OutMaps om;
+    if (pitch) {  // any pitch and alignment of the result: plain stores, no maps
+        if (gated || gather) return MIMK_E_UNSUPPORTED;
+        om = OutMaps{};
+        if (d.out_dtype == MIMK_BF16)
+            return b_mn ? launch<256, true, false, __nv_bfloat16, true>(tA, tB, tB2, om, p, dev->sm_count, s)
+                        : launch<256, false, false, __nv_bfloat16, true>(tA, tB, tB2, om, p, dev->sm_count, s);
+        return b_mn ? launch<256, true, false, float, true>(tA, tB, tB2, om, p, dev->sm_count, s)
+                    : launch<256, false, false, float, true>(tA, tB, tB2, om, p, dev->sm_count, s);
+    }
     for (int t = 0; t < p.n_dst; ++t) {
         const uint8_t* base = static_cast<const uint8_t*>(p.dst[t]) + size_t(p.col_off) * out_size;
-        MIMK_TRY(make_tmap_3d(&om.m[t], d.out_dtype == MIMK_F32, base, uint64_t(d.n), uint64_t(d.m), uint64_t(d.batch), pitch, sc,
+        MIMK_TRY(make_tmap_3d(&om.m[t], d.out_dtype == MIMK_F32, base, uint64_t(d.n), uint64_t(d.m), uint64_t(d.batch), row_c, sc,
                               uint32_t(128 / out_size), 32));
     }
     for (int t = p.n_dst; t < MIMK_MAX_GATHER; ++t) om.m[t] = om.m[0];
@@ -484,6 +553,53 @@ int gemm_tc(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, 
                     : launch<256, false, false, __nv_bfloat16>(tA, tB, tB2, om, p, dev->sm_count, s);
     return b_mn ? launch<256, true, false, float>(tA, tB, tB2, om, p, dev->sm_count, s)
                 : launch<256, false, false, float>(tA, tB, tB2, om, p, dev->sm_count, s);
+}
+
+// bf16 contractions whose extents or alignment break TMA's 16-byte rules: operands that do are copied to rows of an aligned
+// pitch first, and the result is written by plain stores. Returns MIMK_E_UNSUPPORTED, with nothing launched, where the CUDA-core
+// kernel is the better or the only way.
+//
+// Floor of the rule: below 2^22 multiply-adds one launch of the CUDA-core kernel is as fast as the copies and the tensor-core
+// kernel's start. Copies are kept in the cached buffer, which a captured graph must not hold on to, and a buffer that cannot be
+// had is no reason to fail: both stay on the CUDA-core kernel.
+int gemm_tc_ragged(const mimk_gemm_desc& d, cudaStream_t s) {
+    RaggedPlan r;
+    if (!ragged_plan(d, &r)) return MIMK_E_UNSUPPORTED;
+    if (double(d.m) * double(d.n) * double(d.k) * double(d.batch) < double(1 << 22)) return MIMK_E_UNSUPPORTED;
+    mimk_gemm_desc t = d;
+    int st           = MIMK_OK;
+    DeviceInfo* dev  = device_info(&st);
+    if (!dev) return st;
+    if (r.pack_a || r.pack_b) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        MIMK_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
+        if (cap != cudaStreamCaptureStatusNone) return MIMK_E_UNSUPPORTED;
+        void* scratch = nullptr;
+        if (get_scratch(r.bytes_a + r.bytes_b, &scratch, s) != MIMK_OK) {
+            cudaGetLastError();
+            return MIMK_E_UNSUPPORTED;
+        }
+        PackJob a{}, b{};
+        if (r.pack_a) {
+            a   = PackJob{static_cast<const uint16_t*>(d.a), static_cast<uint16_t*>(scratch), r.rows_a, r.cols_a, r.pitch_a};
+            t.a = scratch;
+            if (d.batch > 1 && d.stride_a != 0) t.stride_a = d.m * r.pitch_a;
+        }
+        if (r.pack_b) {
+            uint8_t* at = static_cast<uint8_t*>(scratch) + r.bytes_a;
+            b   = PackJob{static_cast<const uint16_t*>(d.b), reinterpret_cast<uint16_t*>(at), r.rows_b, r.cols_b, r.pitch_b};
+            t.b = at;
+            if (d.batch > 1 && d.stride_b != 0) t.stride_b = (d.b_layout == MIMK_B_KN ? d.k : d.n) * r.pitch_b;
+        }
+        const int64_t units = a.rows * (a.pitch >> 3) + b.rows * (b.pitch >> 3), blocks = (units + 255) / 256;
+        const int64_t cap_blocks = int64_t(dev->sm_count) * 8;
+        pack_rows_kernel<<<unsigned(blocks < cap_blocks ? blocks : cap_blocks), 256, 0, s>>>(a, b);
+        MIMK_TRY(launch_status());
+    }
+    const GemmPitch pitch{r.pitch_a, r.pitch_b};
+    if (gemm_tc_split_preferred(t, 0, dev->sm_count)) return gemm_tc_split(t, s, 0, nullptr, &pitch);
+    if (t.batch <= 64 && gemm_tc2_enough(t.m, t.n, 0)) return gemm_tc2(t, s, 0, nullptr, nullptr, 1, 0, &pitch);
+    return gemm_tc(t, s, 0, nullptr, nullptr, 1, &pitch);
 }
 
 }  // namespace mimk

@@ -15,6 +15,7 @@
 // Every wait is bounded; a CTA that gives up records MIMK_E_DEVICE_WAIT, and both CTAs meet at a final cluster barrier
 // before either releases shared or tensor memory.
 #include "common.cuh"
+#include "gemm_epilogue.cuh"
 #include "sm100.cuh"
 
 namespace mimk {
@@ -136,7 +137,8 @@ __device__ __forceinline__ void tile_coords(int64_t tile, int64_t tiles_m, int64
 }
 
 // BN: output-tile width per B operand (256 plain, 128 gated); this CTA stages BN/2 rows of each B operand.
-template <int BN, bool B_MN, bool GATED, class TOut>
+// DIRECT: the one destination is written by plain stores (store_piece).
+template <int BN, bool B_MN, bool GATED, class TOut, bool DIRECT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NUM_THREADS, 1)
 gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                 const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ OutMaps om, const Params p) {
@@ -308,17 +310,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         tc_fence_before();
                         mbar_arrive_cluster(acc_empty_even);
                     }
-                    if (p.post != MIMK_POST_ID && row < p.M) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            const int64_t col = n0 + c + i;
-                            if (col < p.N) {
-                                const float rowv = p.post_row ? __ldg(p.post_row + col) : 0.f;
-                                const float full = post_full ? float(post_full[row * p.N + col]) : 0.f;
-                                v[i]             = apply_post(p.post, v[i], rowv, full);
-                            }
-                        }
-                    }
+                    if (p.post != MIMK_POST_ID && row < p.M)
+                        apply_post_32(p.post, v, p.post_row, post_full ? post_full + row * p.N : nullptr, n0 + c, p.N);
                     // this thread's row of the tile: 16-byte pieces at (piece ^ (row & 7)), the 128-byte swizzle
                     const uint32_t row_addr = buf + lane * 128;
                     if (sizeof(TOut) == 2) {
@@ -341,6 +334,12 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                                          : "memory");
                         }
                     }
+                }
+                if (DIRECT) {
+                    __syncwarp();
+                    store_piece(smem_raw + (buf - raw_addr), static_cast<TOut*>(p.dst[0]) + row0 * p.ldc + n0 + c0, p.ldc, p.M - row0,
+                                p.N - n0 - c0, lane);
+                    continue;  // the next piece goes to the other buffer, and the one after waits for this warp above
                 }
                 fence_proxy_async_smem();  // the bulk store reads shared memory through the async proxy
                 __syncwarp();
@@ -377,10 +376,10 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     if (threadIdx.x == 0 && *abort_flag) *p.status = MIMK_E_DEVICE_WAIT;
 }
 
-template <int BN, bool B_MN, bool GATED, class TOut>
+template <int BN, bool B_MN, bool GATED, class TOut, bool DIRECT = false>
 int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tB2, const OutMaps& om, const Params& p,
            int sm_count, cudaStream_t s) {
-    auto kern = gemm_tc2_kernel<BN, B_MN, GATED, TOut>;
+    auto kern = gemm_tc2_kernel<BN, B_MN, GATED, TOut, DIRECT>;
     static bool configured[64] = {};  // per template instance and device: the attribute is a per-device setting
     int dev = 0;
     MIMK_CUDA_TRY(cudaGetDevice(&dev));
@@ -398,21 +397,22 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tB2,
 }  // namespace
 
 // Worth it only when there are enough 256-row tiles to go round; smaller problems stay on the one-CTA kernel.
-int gemm_tc2_supported(const mimk_gemm_desc& d, int gated) {
-    if (!gemm_tc_supported(d)) return 0;
+int gemm_tc2_enough(int64_t m, int64_t n, int gated) {
     const int bn = gated ? 128 : 256;
-    const int64_t tiles = ((d.m + 255) / 256) * ((d.n + bn - 1) / bn);
-    return d.m >= 512 && tiles >= 74;
+    const int64_t tiles = ((m + 255) / 256) * ((n + bn - 1) / bn);
+    return m >= 512 && tiles >= 74;
 }
+int gemm_tc2_supported(const mimk_gemm_desc& d, int gated) { return gemm_tc_supported(d) && gemm_tc2_enough(d.m, d.n, gated); }
 
 int gemm_tc2(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, const mimk_gather_dst* gather,
-             int64_t a_panels, int64_t scatter_rows) {
+             int64_t a_panels, int64_t scatter_rows, const GemmPitch* pitch) {
     int st          = MIMK_OK;
     DeviceInfo* dev = device_info(&st);
     if (!dev) return st;
     const bool b_mn = d.b_layout == MIMK_B_KN;
     const int bh    = gated ? 64 : 128;  // B rows (or columns, MN-major) staged per CTA and operand
     const size_t out_size = d.out_dtype == MIMK_BF16 ? 2 : 4;
+    const uint64_t row_b  = (pitch ? uint64_t(pitch->b) : uint64_t(b_mn ? d.n : d.k)) * 2;
     for (int64_t b = 0; b < d.batch; ++b) {
         const uint8_t* A  = static_cast<const uint8_t*>(d.a) + size_t(b * d.stride_a) * 2;
         const uint8_t* B  = static_cast<const uint8_t*>(d.b) + size_t(b * d.stride_b) * 2;
@@ -420,13 +420,13 @@ int gemm_tc2(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2,
         CUtensorMap tA, tB, tB2;
         if (a_panels < 1 || (a_panels > 1 && (d.batch != 1 || d.k % a_panels != 0 || (d.k / a_panels) % BK != 0))) return MIMK_E_UNSUPPORTED;
         const uint64_t kp = uint64_t(d.k / a_panels);  // A as a [panels * m, k / panels] matrix: panel g starts at row g * m
-        MIMK_TRY(make_tmap_bf16_2d(&tA, A, kp, uint64_t(d.m) * uint64_t(a_panels), kp * 2, BK, BM));
+        MIMK_TRY(make_tmap_bf16_2d(&tA, A, kp, uint64_t(d.m) * uint64_t(a_panels), pitch ? uint64_t(pitch->a) * 2 : kp * 2, BK, BM));
         if (b_mn) {
-            MIMK_TRY(make_tmap_bf16_2d(&tB, B, uint64_t(d.n), uint64_t(d.k), uint64_t(d.n) * 2, 64, BK));
-            MIMK_TRY(make_tmap_bf16_2d(&tB2, B2, uint64_t(d.n), uint64_t(d.k), uint64_t(d.n) * 2, 64, BK));
+            MIMK_TRY(make_tmap_bf16_2d(&tB, B, uint64_t(d.n), uint64_t(d.k), row_b, 64, BK));
+            MIMK_TRY(make_tmap_bf16_2d(&tB2, B2, uint64_t(d.n), uint64_t(d.k), row_b, 64, BK));
         } else {
-            MIMK_TRY(make_tmap_bf16_2d(&tB, B, uint64_t(d.k), uint64_t(d.n), uint64_t(d.k) * 2, BK, uint32_t(bh)));
-            MIMK_TRY(make_tmap_bf16_2d(&tB2, B2, uint64_t(d.k), uint64_t(d.n), uint64_t(d.k) * 2, BK, uint32_t(bh)));
+            MIMK_TRY(make_tmap_bf16_2d(&tB, B, uint64_t(d.k), uint64_t(d.n), row_b, BK, uint32_t(bh)));
+            MIMK_TRY(make_tmap_bf16_2d(&tB2, B2, uint64_t(d.k), uint64_t(d.n), row_b, BK, uint32_t(bh)));
         }
         Params p;
         p.M = d.m, p.N = d.n, p.K = d.k;
@@ -458,6 +458,17 @@ int gemm_tc2(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2,
         // destination maps: [M, N] windows (row pitch ldc) starting at column col_off, boxes of 32 rows x 128 bytes;
         // [scatter_rows, N] windows when the row blocks are scattered
         OutMaps om;
+        if (pitch) {  // any pitch and alignment of the result: plain stores, no maps
+            if (gated || gather) return MIMK_E_UNSUPPORTED;
+            om = OutMaps{};
+            if (d.out_dtype == MIMK_BF16)
+                MIMK_TRY((b_mn ? launch<256, true, false, __nv_bfloat16, true>(tA, tB, tB2, om, p, dev->sm_count, s)
+                               : launch<256, false, false, __nv_bfloat16, true>(tA, tB, tB2, om, p, dev->sm_count, s)));
+            else
+                MIMK_TRY((b_mn ? launch<256, true, false, float, true>(tA, tB, tB2, om, p, dev->sm_count, s)
+                               : launch<256, false, false, float, true>(tA, tB, tB2, om, p, dev->sm_count, s)));
+            continue;
+        }
         for (int t = 0; t < p.n_dst; ++t) {
             const uint8_t* base = static_cast<const uint8_t*>(p.dst[t]) + size_t(p.col_off) * out_size;
             MIMK_TRY(make_tmap_2d(&om.m[t], d.out_dtype == MIMK_F32, base, uint64_t(d.n),

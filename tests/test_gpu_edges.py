@@ -154,3 +154,51 @@ def test_convolutions_gathered_from_the_image(T, monkeypatch, n, cin, h, w, cout
         x[0, 0, h // 2, w // 2] = math.inf
         assert torch.equal(d64(T.conv(x, f, stride=stride, dilation=dil, padding=pad)).isfinite(),
                            conv(d64(x), d64(f), stride=stride, dilation=dil, padding=pad).isfinite())
+
+
+@pytest.mark.parametrize("m,n,k,b_nk,post,out,offset", [
+    (2000, 1003, 520, True, "bias_relu", BF16, 0), (300, 257, 1031, True, None, BF16, 0), (129, 255, 1033, False, "bias", F32, 0),
+    (640, 5003, 264, False, None, BF16, 0), (640, 5001, 257, True, "bias_tanh", F32, 1), (65, 2056, 512, True, None, BF16, 1),
+    (3, 9001, 513, False, None, BF16, 3), (1, 8193, 1024, True, "relu", BF16, 0),
+    (16, 4096, 4096, True, None, BF16, 0), (1, 520, 4104, False, None, F32, 0), (17, 130, 4096, True, "bias", BF16, 0),
+    (129, 72, 4160, False, "add", BF16, 0), (128, 64, 64, True, None, F32, 0), (700, 1000, 72, True, "bias_relu", BF16, 0)])
+def test_bf16_products_of_any_extent(T, m, n, k, b_nk, post, out, offset):
+    a = rnd((m, k), 1, BF16, offset)
+    b = rnd((n, k) if b_nk else (k, n), 2, BF16, offset)
+    b = b.t() if b_nk else b
+    bias = rnd((n,), 3) if post and post.startswith("bias") else None
+    full = rnd((m, n), 4, out) if post == "add" else None
+    got = T.product_2d(a, b, post=post, bias=bias, full=full, out_dtype=out)
+    T.device_status()
+    want = d64(a) @ d64(b)
+    scale = d64(a).abs() @ d64(b).abs() * 2.0 ** -14   # the f32 sums, next to the rounding of the result
+    want = want + (d64(bias) if bias is not None else 0) + (d64(full) if full is not None else 0)
+    rounding = want.abs() * (BF16_ROUND if out == BF16 else 2.0 ** -20)
+    if post and post.endswith("relu"):
+        want = want.clamp(min=0)
+    if post and post.endswith("tanh"):
+        want = want.tanh()
+    assert got.dtype == out and ((d64(got) - want).abs() <= rounding + scale + 1e-6).all()
+
+
+@pytest.mark.parametrize("B,m,n,k,b_nk", [(3, 129, 255, 67, True), (5, 40, 200, 286, False), (2, 130, 64, 1000, True), (70, 16, 24, 72, False)])
+def test_bf16_batches_of_any_extent(T, B, m, n, k, b_nk):
+    a, b = rnd((B, m, k), 1, BF16), rnd((B, n, k) if b_nk else (B, k, n), 2, BF16)
+    b = b.transpose(1, 2) if b_nk else b
+    got = T.bmm(a, b)
+    T.device_status()
+    want = d64(a) @ d64(b)
+    assert ((d64(got) - want).abs() <= want.abs() * BF16_ROUND + d64(a).abs() @ d64(b).abs() * 2.0 ** -14 + 1e-6).all()
+
+
+@pytest.mark.parametrize("m,k,f,n,b_nk", [(1, 512, 1024, 512, True), (17, 520, 1032, 264, False), (128, 1024, 2048, 512, False), (200, 512, 640, 520, True)])
+def test_gated_mlp_of_few_rows(T, m, k, f, n, b_nk):
+    x = rnd((m, k), 1, BF16)
+    w = [(rnd((o, i) if b_nk else (i, o), s, BF16) * 0.05) for s, (i, o) in enumerate([(k, f), (k, f), (f, n)], 2)]
+    w = [t.t() if b_nk else t for t in w]
+    got = T.mlp_gated(x, *w)
+    T.device_status()
+    h = torch.nn.functional.silu(d64(x) @ d64(w[0])) * (d64(x) @ d64(w[1]))
+    want, terms = h @ d64(w[2]), h.abs() @ d64(w[2]).abs()
+    # the hidden layer is rounded to bf16: 2^-9 of every term, like the result itself
+    assert ((d64(got) - want).abs() <= BF16_ROUND * (want.abs() + terms) + 1e-6).all()
