@@ -42,21 +42,29 @@ __device__ __forceinline__ void apply_post_32(int post, float (&v)[32], const fl
 // neighbouring elements, two bf16 per lane where the pair is aligned.
 __device__ __forceinline__ void store_piece(const uint8_t* buf, float* c, int64_t ldc, int64_t rows, int64_t cols, int lane) {
     const int n = int(rows < 32 ? rows : 32);
-#pragma unroll 4
+#pragma unroll 8
     for (int r = 0; r < n; ++r)
         if (lane < cols) c[r * ldc + lane] = *reinterpret_cast<const float*>(buf + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
 }
 __device__ __forceinline__ void store_piece(const uint8_t* buf, __nv_bfloat16* c, int64_t ldc, int64_t rows, int64_t cols, int lane) {
     const int n = int(rows < 32 ? rows : 32), m = int(cols < 64 ? cols : 64);
-#pragma unroll 4
-    for (int r = 0; r < n; ++r) {
-        uint16_t* dst = reinterpret_cast<uint16_t*>(c + r * ldc);
-        const int odd = int(reinterpret_cast<uintptr_t>(dst) >> 1) & 1;  // pairs start at element 0 or 1
-        auto at = [&](int e) { return *reinterpret_cast<const uint16_t*>(buf + r * 128 + (((e >> 3) ^ (r & 7)) << 4) + (e & 7) * 2); };
-        const int e = 2 * lane + odd;
-        if (e + 1 < m) *reinterpret_cast<uint32_t*>(dst + e) = uint32_t(at(e)) | (uint32_t(at(e + 1)) << 16);
-        else if (e < m) dst[e] = at(e);
-        if (odd && lane == 0 && m > 0) dst[0] = at(0);
+    uint16_t* dst = reinterpret_cast<uint16_t*>(c);
+    const int odd0 = int(reinterpret_cast<uintptr_t>(dst) >> 1) & 1, step = int(ldc) & 1;
+#pragma unroll 8
+    for (int r = 0; r < 32; ++r) {
+        if (r >= n) break;
+        // this lane's pair of the row, elements 2 lane and 2 lane + 1, and (shifted by one) the pair that straddles two words
+        const uint32_t w    = *reinterpret_cast<const uint32_t*>(buf + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
+        const uint32_t next = __shfl_down_sync(0xffffffffu, w, 1);
+        if (!((odd0 + r * step) & 1)) {  // the row starts on a word
+            if (2 * lane + 1 < m) reinterpret_cast<uint32_t*>(dst)[lane] = w;
+            else if (2 * lane < m) dst[2 * lane] = uint16_t(w);
+        } else {
+            if (2 * lane + 2 < m) *reinterpret_cast<uint32_t*>(dst + 2 * lane + 1) = __funnelshift_r(w, next, 16);
+            else if (2 * lane + 1 < m) dst[2 * lane + 1] = uint16_t(w >> 16);
+            if (lane == 0 && m > 0) dst[0] = uint16_t(w);
+        }
+        dst += ldc;
     }
 }
 

@@ -5,17 +5,17 @@
 // programs take. Each operand value is cut into three bf16 pieces that sum to it exactly, and the six products that matter
 // are accumulated by tcgen05.mma (f32_split.cuh).
 //
-//   loaders      8 or 16 warps: read the operands (next k-block into registers while the present one is cut and stored), write
-//                the pieces into shared-memory tiles, and add each finished k-block's accumulator to sums in registers
-//   last warp    one thread issues the MMAs: 128 x BN x 32 per k-block, every k-block into a fresh one of four accumulators
-// The tensor core does not round its accumulator updates to nearest; with one k-block (2 x 6 updates, the small terms first)
-// per accumulator and ordinary f32 adds between k-blocks, the error stays that of an f32 fold for any K (2-norm 1.1e-7 to
-// 1.3e-7 for K from 64 to 4096; the scalar fold has 1.5e-7 to 1.2e-6).
+//   warps 0..15   read the operands and write their pieces into shared-memory tiles (each eight-k unit of the next k-block is
+//                 requested as soon as the present one's has left its registers), add finished accumulators to sums in registers
+//   warp 16       one thread issues the MMAs, 128 x BN x 32 per k-block; every four k-blocks go into a fresh accumulator
+// The tensor core does not round its accumulator updates to nearest; with 8 updates by full-size terms per accumulator (the small
+// terms of each k-block first) and ordinary f32 adds between accumulators, the error stays below that of an f32 fold for any K.
+// The accumulators are added in order whatever the grid (up to K = 2048: beyond that a CTA of a cluster may first add its own).
 //
 // The operands are read as the caller has them: any extents, strides and alignment, no copies, no scratch. What bounds it:
-// the loaders' instructions and shared-memory bandwidth (a k-block of 128 x 128 moves 96 KB into the MMA and 48 KB from the
-// loaders, 1150 clocks, against 770 of arithmetic). Too few tiles for the chip: the k-blocks of one tile are dealt out to a
-// cluster of up to eight CTAs, which add their partial tiles through distributed shared memory in a fixed order.
+// shared-memory bandwidth (a k-block of 128 x 128 moves 96 KB into the MMA and 48 KB from the loaders; measured 100 clocks per
+// instruction of 64 clocks' arithmetic) next to the loaders' instructions. Too few tiles for the chip: the accumulators of one
+// tile are dealt out to a cluster of two, four or eight CTAs, which exchange them through distributed shared memory.
 #include <cstdlib>
 
 #include "common.cuh"
@@ -30,23 +30,25 @@ using namespace f32split;
 namespace {
 
 constexpr int BM = 128;
-constexpr int NBUF = 4;         // accumulators in tensor memory
-constexpr int LAG = 2;          // k-blocks between storing one and adding its accumulator
-constexpr int GROUP_M = 16;
+constexpr int CHUNK = 4;        // k-blocks per accumulator
+constexpr int LOADERS = 512, NUM_THREADS = LOADERS + 32, MMA_WARP = LOADERS / 32;
+constexpr int STAGES = 4, GROUP_M = 16;
 constexpr int A_PIECE = BM * BK * 2;
 
 template <int BN, class TIn> struct Cfg {
     static constexpr int PIECES  = sizeof(TIn) == 4 ? 3 : 1;
-    static constexpr int STAGES  = BN == 128 || PIECES == 1 ? 4 : 3;  // BN 64: two CTAs can share an SM
     static constexpr int B_PIECE = BN * BK * 2;
     static constexpr int STAGE_BYTES = PIECES * (A_PIECE + B_PIECE);
-    static constexpr int PITCH = BN + 4;  // floats per row of the partial tile, which lies over the stages
-    static constexpr int TILE_BYTES = STAGES * STAGE_BYTES > BM * PITCH * 4 ? STAGES * STAGE_BYTES : BM * PITCH * 4;
+    static constexpr int PITCH = BN + 4, PART_BYTES = BM * PITCH * 4;  // a partial tile; they lie over the stages
+    static constexpr int NACC  = 512 / BN;                             // accumulators in tensor memory
+    static constexpr int SLOTS = BN == 128 ? 2 : 4;                    // of them, what a CTA of a cluster may hold to the end
+    static constexpr int TILE_BYTES = STAGES * STAGE_BYTES > SLOTS * PART_BYTES ? STAGES * STAGE_BYTES : SLOTS * PART_BYTES;
     static constexpr int SMEM_BYTES = TILE_BYTES + 1024 + 256;
+    static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
 };
 
 struct Bars {
-    uint64_t full[4], empty[4], acc_full[NBUF];
+    uint64_t full[STAGES], empty[STAGES], acc_full[8];
     uint32_t tmem_base;
     int abort_flag;
 };
@@ -80,13 +82,6 @@ __device__ __forceinline__ float4 ld_cluster4(uint32_t saddr, uint32_t rank) {
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
     return v;
 }
-__device__ __forceinline__ float ld_cluster1(uint32_t saddr, uint32_t rank) {
-    uint32_t a;
-    float v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-    return v;
-}
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld_32x32(taddr, r); }
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld_32x16(taddr, r); }
 
@@ -105,11 +100,73 @@ __device__ __forceinline__ void tile_coords(int64_t tile, int64_t tiles_m, int64
     tn                      = in_group / gsize;
 }
 
-// LOADERS: 512 threads, and the SM for one CTA alone; or 256, and two CTAs (BN 64) that hide each other's waits.
-template <int BN, int LOADERS, class TIn, class TOut, bool CONV>
-__global__ void __launch_bounds__(LOADERS + 32, LOADERS == 512 ? 1 : 2) gemm_f32_tc_kernel(const Params p) {
+__device__ __forceinline__ int cv_pixels(const Params& p) { return p.conv.oh * p.conv.ow; }
+
+// four neighbouring results of one row; vec: they are one aligned store, and n is a multiple of 4
+template <class TOut>
+__device__ __forceinline__ void store4(TOut* row, int64_t col, int64_t n, float4 q, bool vec) {
+    if (col >= n) return;
+    if (vec) {
+        if (sizeof(TOut) == 4) *reinterpret_cast<float4*>(row + col) = q;
+        else *reinterpret_cast<uint2*>(row + col) = make_uint2(pack_bf16x2(q.x, q.y), pack_bf16x2(q.z, q.w));
+    } else {
+        row[col] = TOut(q.x);
+        if (col + 1 < n) row[col + 1] = TOut(q.y);
+        if (col + 2 < n) row[col + 2] = TOut(q.z);
+        if (col + 3 < n) row[col + 3] = TOut(q.w);
+    }
+}
+
+// The scalar fold of one cell -- ascending k, one fma per step, what the CUDA-core kernel computes -- for cells the pieces make
+// non-finite: an operand of the fold was inf / NaN, or the sum overflowed.
+template <class TIn, bool CONV>
+__device__ __noinline__ float scalar_fold(const Params& p, int64_t bz, int64_t row, int64_t col) {
+    const TIn* A = static_cast<const TIn*>(p.A) + bz * p.sa;
+    const TIn* B = static_cast<const TIn*>(p.B) + bz * p.sb;
+    float v = 0.f;
+    if (CONV) {  // padding read as zeros
+        const ConvShape& cv = p.conv;
+        const int pixels  = cv.oh * cv.ow;
+        const int64_t img = row / pixels;
+        const int y = int(row - img * pixels) / cv.ow, x = int(row - img * pixels) - y * cv.ow;
+        const TIn* im = A + img * (int64_t(cv.cin) * cv.h * cv.w);
+        const TIn* wt = B + col * p.K;
+        for (int ci = 0; ci < cv.cin; ++ci)
+            for (int kr = 0; kr < cv.kh; ++kr)
+                for (int kq = 0; kq < cv.kw; ++kq, ++wt) {
+                    const int iy = y * cv.stride_h - cv.pad_h + kr * cv.dil_h, ix = x * cv.stride_w - cv.pad_w + kq * cv.dil_w;
+                    const bool in = unsigned(iy) < unsigned(cv.h) && unsigned(ix) < unsigned(cv.w);
+                    v = fmaf(in ? load1(im + (int64_t(ci) * cv.h + iy) * cv.w + ix) : 0.f, load1(wt), v);
+                }
+    } else {
+        const TIn* ar = A + row * p.K;
+        const TIn* br = p.b_nk ? B + col * p.K : B + col;
+        const int64_t step = p.b_nk ? 1 : p.N;
+        for (int64_t k = 0; k < p.K; ++k) v = fmaf(load1(ar + k), load1(br + k * step), v);
+    }
+    return v;
+}
+
+// Four neighbouring sums of one row: non-finite ones folded again, `post`, stored.
+template <class TIn, class TOut>
+__device__ __forceinline__ void finish4(const Params& p, TOut* out, const TOut* post_full, int64_t bz, int64_t row, int64_t col, float4 q) {
+    if (row >= p.M || col >= p.N) return;
+    float v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        if (col + e >= p.N) break;
+        if (!isfinite(v[e])) v[e] = scalar_fold<TIn, false>(p, bz, row, col + e);
+        const float rowv = p.post_row ? __ldg(p.post_row + col + e) : 0.f;
+        const float full = post_full ? float(post_full[row * p.N + col + e]) : 0.f;
+        v[e]             = apply_post(p.post, v[e], rowv, full);
+    }
+    store4(out + row * p.N, col, p.N, make_float4(v[0], v[1], v[2], v[3]), p.vec_c);
+}
+
+template <int BN, class TIn, class TOut, bool CONV>
+__global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __grid_constant__ Params p) {
     using C = Cfg<BN, TIn>;
-    constexpr int PIECES = C::PIECES, MMA_WARP = LOADERS / 32;
+    constexpr int PIECES = C::PIECES;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
     const uint32_t base     = (raw_addr + 1023u) & ~1023u;
@@ -125,44 +182,39 @@ __global__ void __launch_bounds__(LOADERS + 32, LOADERS == 512 ? 1 : 2) gemm_f32
     const int64_t m0 = tm * BM, n0 = tn * BN;
     const TIn* A = static_cast<const TIn*>(p.A) + bz * p.sa;
     const TIn* B = static_cast<const TIn*>(p.B) + bz * p.sb;
-    const int64_t all_kb = (p.K + BK - 1) / BK, per = (all_kb + p.split - 1) / p.split;
-    const int64_t kb0    = rank * per < all_kb ? rank * per : all_kb;
-    const int num_kb     = int(kb0 + per < all_kb ? per : all_kb - kb0);
+    const int all_kb = int((p.K + BK - 1) / BK), chunks = (all_kb + CHUNK - 1) / CHUNK, per = (chunks + p.split - 1) / p.split;
+    const int ch0 = rank * per < chunks ? rank * per : chunks, ch1 = ch0 + per < chunks ? ch0 + per : chunks;
+    const int kb0 = ch0 * CHUNK, kb1 = ch1 * CHUNK < all_kb ? ch1 * CHUNK : all_kb;
+    // this CTA's accumulators stay in tensor memory to the end and leave one by one, or are added up as they are finished
+    const bool hold = p.split > 1 && per <= C::SLOTS;
 
-    // What a loader thread holds of one k-block: one or two eight-k units of A and at most one of B. Where memory runs along k a
-    // unit's row is u / 4; where it runs along the rows (B stored [K, N], the pixels of an image) a warp takes one unit of 32
-    // neighbouring rows. The first loads are on their way while the barriers and the tensor memory are set up.
-    constexpr int UA = BM * 4 / LOADERS;
-    static_assert(BN * 4 <= LOADERS, "one unit of B per thread");
-    const int across = (warp >> 2) * 32 + lane, unit = warp & 3;
-    const bool has_b = BN * 4 == LOADERS || tid < BN * 4;
-    const int b_row = p.b_nk ? tid >> 2 : across, b_unit = p.b_nk ? tid & 3 : unit;
-    float fa[UA][8], fb[8];
-    const TIn* a_at[UA];           // CONV: the first tap of the pixel's window; else the thread's row of A, at its unit
-    int rows_in[UA], cols_in[UA];  // CONV: bit i: tap row / column i of this pixel lies inside the image
-    const ConvShape& cv = p.conv;
-#pragma unroll
-    for (int i = 0; i < UA; ++i) {
-        rows_in[i] = cols_in[i] = 0;
-        if (CONV) {
-            const int64_t row = m0 + across + i * (LOADERS / 4);
-            const int pixels  = cv.oh * cv.ow;
-            const int64_t img = row / pixels;
-            const int pix = int(row - img * pixels), y = pix / cv.ow;
-            const int ih0 = y * cv.stride_h - cv.pad_h, iw0 = (pix - y * cv.ow) * cv.stride_w - cv.pad_w;
-            a_at[i] = A + img * (int64_t(cv.cin) * cv.h * cv.w) + (int64_t(ih0) * cv.w + iw0);  // only taps inside are read
-            if (row < p.M) {
-                for (int r = 0; r < cv.kh; ++r) rows_in[i] |= int(unsigned(ih0 + r * cv.dil_h) < unsigned(cv.h)) << r;
-                for (int q = 0; q < cv.kw; ++q) cols_in[i] |= int(unsigned(iw0 + q * cv.dil_w) < unsigned(cv.w)) << q;
-            }
-        } else {
-            const int u = tid + i * LOADERS;
-            a_at[i] = A + (m0 + (u >> 2)) * p.K + (u & 3) * 8;
-        }
-    }
+    // A thread's part of a k-block: an eight-k unit of A and at most one of B. Where memory runs along k a unit's row is tid / 4;
+    // where it runs along the rows (B stored [K, N], the pixels of an image) a warp takes one unit of 32 neighbouring rows.
+    const int across = (warp >> 2) * 32 + lane, along = tid >> 2, unit = warp & 3;
+    const int a_row = CONV ? across : along, a_unit = CONV ? unit : tid & 3;
+    const int b_row = p.b_nk ? along : across, b_unit = p.b_nk ? tid & 3 : unit;
+    const bool has_b = BN == 128 || tid < BN * 4, a_there = m0 + a_row < p.M, b_there = n0 + b_row < p.N;
+    float fa[8], fb[8];
+    const TIn* a_at;                // CONV: the first tap of the pixel's window; else the thread's row of A, at its unit
     const TIn* b_at = p.b_nk ? B + (n0 + b_row) * p.K + b_unit * 8 : B + int64_t(b_unit * 8) * p.N + n0 + b_row;
-    auto fetch = [&](int kb) {
-        const int64_t k0 = (kb0 + kb) * BK;
+    int rows_in = 0, cols_in = 0;   // CONV: bit i: tap row / column i of this pixel lies inside the image
+    const ConvShape& cv = p.conv;
+    if (CONV) {
+        const int64_t row = m0 + a_row;
+        const int pixels  = cv.oh * cv.ow;
+        const int64_t img = row / pixels;
+        const int pix = int(row - img * pixels), y = pix / cv.ow;
+        const int ih0 = y * cv.stride_h - cv.pad_h, iw0 = (pix - y * cv.ow) * cv.stride_w - cv.pad_w;
+        a_at = A + img * (int64_t(cv.cin) * cv.h * cv.w) + (int64_t(ih0) * cv.w + iw0);  // only taps inside are read
+        if (a_there) {
+            for (int r = 0; r < cv.kh; ++r) rows_in |= int(unsigned(ih0 + r * cv.dil_h) < unsigned(cv.h)) << r;
+            for (int q = 0; q < cv.kw; ++q) cols_in |= int(unsigned(iw0 + q * cv.dil_w) < unsigned(cv.w)) << q;
+        }
+    } else {
+        a_at = A + (m0 + a_row) * p.K + a_unit * 8;
+    }
+    auto fetch_a = [&](int kb) {
+        const int64_t k0 = int64_t(kb) * BK;
         if (CONV) {
             const int k = int(k0) + unit * 8, taps = cv.kh * cv.kw;
             const int ci = k / taps;
@@ -171,11 +223,8 @@ __global__ void __launch_bounds__(LOADERS + 32, LOADERS == 512 ? 1 : 2) gemm_f32
             const int next_row = cv.dil_h * cv.w - cv.kw * cv.dil_w, next_plane = cv.h * cv.w - cv.kh * cv.dil_h * cv.w;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-#pragma unroll
-                for (int i = 0; i < UA; ++i) {
-                    const bool in = (rows_in[i] >> r) & (cols_in[i] >> q) & int(k + j < int(p.K));
-                    fa[i][j]      = in ? load1(a_at[i] + off) : 0.f;
-                }
+                const bool in = (rows_in >> r) & (cols_in >> q) & int(k + j < int(p.K));
+                fa[j]         = in ? load1(a_at + off) : 0.f;
                 off += cv.dil_w;
                 if (++q == cv.kw) {
                     q = 0, off += next_row;
@@ -183,45 +232,37 @@ __global__ void __launch_bounds__(LOADERS + 32, LOADERS == 512 ? 1 : 2) gemm_f32
                 }
             }
         } else {
-#pragma unroll
-            for (int i = 0; i < UA; ++i) {
-                const int u = tid + i * LOADERS;
-                load8(fa[i], a_at[i] + k0, m0 + (u >> 2) < p.M, int(p.K - k0) - (u & 3) * 8, p.vec_a);
-            }
-        }
-        if (has_b) {
-            const bool there = n0 + b_row < p.N;
-            const int left   = int(p.K - k0) - b_unit * 8;
-            if (p.b_nk) {
-                load8(fb, b_at + k0, there, left, p.vec_b);
-            } else {
-                const TIn* at = b_at + k0 * p.N;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) fb[j] = there && j < left ? load1(at + j * p.N) : 0.f;
-            }
+            load8(fa, a_at + k0, a_there, int(p.K - k0) - a_unit * 8, p.vec_a);
         }
     };
-    auto store = [&](uint32_t s0) {
+    auto fetch_b = [&](int kb) {
+        if (!has_b) return;
+        const int64_t k0 = int64_t(kb) * BK;
+        const int left   = int(p.K - k0) - b_unit * 8;
+        if (p.b_nk) {
+            load8(fb, b_at + k0, b_there, left, p.vec_b);
+        } else {
+            const TIn* at = b_at + k0 * p.N;
 #pragma unroll
-        for (int i = 0; i < UA; ++i) {
-            const int u = tid + i * LOADERS;
-            split_store8<PIECES>(s0 + (CONV ? unit_offset(across + i * (LOADERS / 4), unit) : unit_offset(u >> 2, u & 3)), A_PIECE, fa[i]);
+            for (int j = 0; j < 8; ++j) fb[j] = b_there && j < left ? load1(at + j * p.N) : 0.f;
         }
-        if (has_b) split_store8<PIECES>(s0 + PIECES * A_PIECE + unit_offset(b_row, b_unit), C::B_PIECE, fb);
     };
-    if (warp < MMA_WARP && num_kb > 0) fetch(0);
+    if (warp < MMA_WARP && kb0 < kb1) {  // on their way while the barriers and the tensor memory are set up
+        fetch_a(kb0);
+        fetch_b(kb0);
+    }
 
     if (tid == 0) {
-        for (int s = 0; s < C::STAGES; ++s) {
+        for (int s = 0; s < STAGES; ++s) {
             mbar_init(smem_u32(&bars->full[s]), LOADERS / 32);
             mbar_init(smem_u32(&bars->empty[s]), 1);
         }
-        for (int b = 0; b < NBUF; ++b) mbar_init(smem_u32(&bars->acc_full[b]), 1);
+        for (int b = 0; b < C::NACC; ++b) mbar_init(smem_u32(&bars->acc_full[b]), 1);
         bars->abort_flag = 0;
         fence_barrier_init();
     }
     if (warp == MMA_WARP) {
-        tmem_alloc(smem_u32(&bars->tmem_base), NBUF * BN);
+        tmem_alloc(smem_u32(&bars->tmem_base), 512);
         tmem_relinquish();
     }
     tc_fence_before();
@@ -233,150 +274,127 @@ __global__ void __launch_bounds__(LOADERS + 32, LOADERS == 512 ? 1 : 2) gemm_f32
         if (lane == 0) {
             const uint32_t idesc = idesc_bf16_f32(BM, BN, 0, 0);
             uint32_t stage = 0, phase = 0;
-            for (int kb = 0; kb < num_kb; ++kb) {
-                // A full stage also says that every loader warp has read the accumulator of k-block kb - 1 - LAG, so the buffer
-                // of kb - NBUF is free.
+            for (int kb = kb0; kb < kb1; ++kb) {
+                // A full stage also says that every warp has added up the chunk that ended four or more k-blocks before it, so an
+                // accumulator is free when its turn comes again (they are three or more in number).
                 if (!mbar_wait(smem_u32(&bars->full[stage]), phase, abort_flag)) break;
                 tc_fence_after();
-                const uint32_t s0 = base + stage * C::STAGE_BYTES;
-                mma_six<PIECES>(tmem_base + (kb & (NBUF - 1)) * BN, s0, A_PIECE, s0 + PIECES * A_PIECE, C::B_PIECE, idesc);
+                const uint32_t s0 = base + stage * C::STAGE_BYTES, acc = uint32_t((kb - kb0) / CHUNK) % C::NACC;
+                mma_six<PIECES>(tmem_base + acc * BN, s0, A_PIECE, s0 + PIECES * A_PIECE, C::B_PIECE, idesc, (kb - kb0) % CHUNK ? 1u : 0u);
                 mma_commit(smem_u32(&bars->empty[stage]));
-                mma_commit(smem_u32(&bars->acc_full[kb & (NBUF - 1)]));
-                if (++stage == C::STAGES) stage = 0, phase ^= 1u;
+                if ((kb - kb0) % CHUNK == CHUNK - 1 || kb + 1 == kb1) mma_commit(smem_u32(&bars->acc_full[acc]));
+                if (++stage == STAGES) stage = 0, phase ^= 1u;
             }
         }
         __syncwarp();
     } else {
-        static_assert(NBUF > LAG + 1, "an accumulator is read before its buffer comes round again");
-        constexpr int COLS = BN / (LOADERS / 128);  // accumulator columns per warp
+        static_assert(C::NACC >= 3, "an accumulator is added up before its turn comes again");
+        constexpr int COLS = BN / 4;  // accumulator columns per warp
+        const uint32_t quarter = uint32_t(warp & 3), col0 = uint32_t(warp >> 2) * COLS, lanes = (quarter * 32u) << 16;
         float sum[COLS];
 #pragma unroll
         for (int i = 0; i < COLS; ++i) sum[i] = 0.f;
-        const uint32_t quarter = uint32_t(warp & 3), col0 = uint32_t(warp >> 2) * COLS;
-        auto drain = [&](int kb) {
-            const int b = kb & (NBUF - 1);
-            if (!warp_wait(smem_u32(&bars->acc_full[b]), uint32_t(kb / NBUF) & 1u, abort_flag)) return false;
+        auto take = [&](int c, uint32_t (&r)[COLS]) {  // this CTA's chunk c
+            const uint32_t acc = uint32_t(c) % C::NACC;
+            if (!warp_wait(smem_u32(&bars->acc_full[acc]), uint32_t(c / C::NACC) & 1u, abort_flag)) return false;
             tc_fence_after();
-            uint32_t r[COLS];
-            tmem_ld_cols(tmem_base + b * BN + col0 + ((quarter * 32u) << 16), r);
+            tmem_ld_cols(tmem_base + acc * BN + col0 + lanes, r);
             tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < COLS; ++i) sum[i] += __uint_as_float(r[i]);
             tc_fence_before();
             return true;
         };
+        auto add = [&](int c) {
+            uint32_t r[COLS];
+            if (!take(c, r)) return false;
+#pragma unroll
+            for (int i = 0; i < COLS; ++i) sum[i] += __uint_as_float(r[i]);
+            return true;
+        };
         uint32_t stage = 0, phase = 0;
-        bool ok = true;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        bool ok   = true;
+        int added = 0;
+        for (int kb = kb0; kb < kb1; ++kb) {
             if (!(ok = warp_wait(smem_u32(&bars->empty[stage]), phase ^ 1u, abort_flag))) break;
-            store(base + stage * C::STAGE_BYTES);
+            const uint32_t s0 = base + stage * C::STAGE_BYTES;
+            split_store8<PIECES>(s0 + unit_offset(a_row, a_unit), A_PIECE, fa);
+            if (kb + 1 < kb1) fetch_a(kb + 1);
+            if (has_b) split_store8<PIECES>(s0 + PIECES * A_PIECE + unit_offset(b_row, b_unit), C::B_PIECE, fb);
+            if (kb + 1 < kb1) fetch_b(kb + 1);
             fence_proxy_async_smem();  // the MMA reads shared memory through the async proxy
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bars->full[stage]));
-            if (++stage == C::STAGES) stage = 0, phase ^= 1u;
-            if (kb + 1 < num_kb) fetch(kb + 1);
-            if (kb >= LAG && !(ok = drain(kb - LAG))) break;
+            if (++stage == STAGES) stage = 0, phase ^= 1u;
+            // the chunk before this one: with four stages its MMAs are complete by now
+            if (!hold && (kb - kb0) % CHUNK == CHUNK - 1 && kb - kb0 >= 2 * CHUNK - 1)
+                if (!(ok = add(added++))) break;
         }
-        for (int kb = num_kb > LAG ? num_kb - LAG : 0; kb < num_kb && ok; ++kb) ok = drain(kb);
-        // every MMA of this CTA is complete: the stages become the partial tile
+        auto part = [&](int slot, const float (&x)[COLS]) {
+            const uint32_t a = base + slot * C::PART_BYTES + (uint32_t(quarter * 32 + lane) * C::PITCH + col0) * 4;
 #pragma unroll
-        for (int i = 0; i < COLS; i += 4) {
-            const uint32_t a = base + (uint32_t(quarter * 32 + lane) * C::PITCH + col0 + i) * 4;
-            st_shared16(a, __float_as_uint(sum[i]), __float_as_uint(sum[i + 1]), __float_as_uint(sum[i + 2]), __float_as_uint(sum[i + 3]));
+            for (int i = 0; i < COLS; i += 4)
+                st_shared16(a + i * 4, __float_as_uint(x[i]), __float_as_uint(x[i + 1]), __float_as_uint(x[i + 2]), __float_as_uint(x[i + 3]));
+        };
+        // Once the last chunk is finished every MMA of this CTA is complete, and the stages become its partial tiles.
+        if (hold) {
+            uint32_t r[COLS];
+            if (ok && ch1 > ch0) ok = take(ch1 - ch0 - 1, r);
+            for (int c = 0; c < ch1 - ch0 && ok; ++c) {
+                if (!(ok = take(c, r))) break;
+#pragma unroll
+                for (int i = 0; i < COLS; ++i) sum[i] = __uint_as_float(r[i]);
+                part(c, sum);
+            }
+        } else {
+            for (; added < ch1 - ch0 && ok; ++added) ok = add(added);
+            part(0, sum);
         }
     }
     __syncthreads();
     // (an abandoned wait leaves MMAs that read the stages; their results are marked invalid by the status word)
     if (p.split > 1) cluster_sync();
-
-    if (CONV && warp < MMA_WARP) {
-        // the filters' planes: neighbouring lanes take neighbouring pixels (a thread keeps one pixel: the rows divide the threads)
-        const int rows = BM / p.split, r = rank * rows + tid % rows, pixels = cv.oh * cv.ow;
-        const int64_t row = m0 + r;
-        if (row < p.M) {
-            const int64_t img = row / pixels;
-            TOut* out         = static_cast<TOut*>(p.C) + img * p.N * pixels + (row - img * pixels);
-            for (int col = tid / rows; col < BN && n0 + col < p.N; col += LOADERS / rows) {
-                const uint32_t a = base + uint32_t(r * C::PITCH + col) * 4;
-                float v          = 0.f;
-                for (int s = 0; s < p.split; ++s)
-                    v += p.split > 1 ? ld_cluster1(a, uint32_t(s)) : *reinterpret_cast<const float*>(smem_raw + (a - raw_addr));
-                if (!isfinite(v)) {  // the scalar fold, ascending k, padding read as zeros
-                    const int y = int(row - img * pixels) / cv.ow, x = int(row - img * pixels) - y * cv.ow;
-                    const TIn* im = A + img * (int64_t(cv.cin) * cv.h * cv.w);
-                    const TIn* wt = B + (n0 + col) * p.K;
-                    v = 0.f;
-                    for (int ci = 0; ci < cv.cin; ++ci)
-                        for (int kr = 0; kr < cv.kh; ++kr)
-                            for (int kq = 0; kq < cv.kw; ++kq, ++wt) {
-                                const int iy = y * cv.stride_h - cv.pad_h + kr * cv.dil_h, ix = x * cv.stride_w - cv.pad_w + kq * cv.dil_w;
-                                const bool in = unsigned(iy) < unsigned(cv.h) && unsigned(ix) < unsigned(cv.w);
-                                v = fmaf(in ? load1(im + (int64_t(ci) * cv.h + iy) * cv.w + ix) : 0.f, load1(wt), v);
-                            }
-                }
-                out[(n0 + col) * pixels] = TOut(v);
-            }
-        }
-    } else if (warp < MMA_WARP) {
-        constexpr int LPR = BN / 4, RPW = 32 / LPR;  // lanes per row, rows per warp and step
-        const int rows = BM / p.split, col = (lane % LPR) * 4;
-        const int64_t gcol = n0 + col;
+    {
+        // the accumulators in order, each CTA a share of the rows
+        const int rows = BM / p.split, held = hold ? per : 1, used = hold ? chunks : (chunks + per - 1) / per;
         TOut* out             = static_cast<TOut*>(p.C) + bz * p.sc;
         const TOut* post_full = p.post_full ? static_cast<const TOut*>(p.post_full) + bz * p.sc : nullptr;
-        for (int r = rank * rows + warp * RPW + lane / LPR; r < (rank + 1) * rows; r += MMA_WARP * RPW) {
-            const int64_t row = m0 + r;
+        for (int i = tid; i < rows * (BN / 4); i += NUM_THREADS) {
+            // CONV: neighbouring threads take neighbouring pixels, else neighbouring columns
+            const int r = rank * rows + (CONV ? i % rows : i / (BN / 4)), col = (CONV ? i / rows : i % (BN / 4)) * 4;
+            const int64_t row = m0 + r, gcol = n0 + col;
             if (row >= p.M || gcol >= p.N) continue;
             const uint32_t a = base + uint32_t(r * C::PITCH + col) * 4;
-            float v[4]       = {0.f, 0.f, 0.f, 0.f};
-            for (int s = 0; s < p.split; ++s) {
-                const float4 q = p.split > 1 ? ld_cluster4(a, uint32_t(s)) : *reinterpret_cast<const float4*>(smem_raw + (a - raw_addr));
-                v[0] += q.x, v[1] += q.y, v[2] += q.z, v[3] += q.w;
+            float4 q         = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int t = 0; t < used; ++t) {
+                const float4 w = ld_cluster4(a + (t % held) * C::PART_BYTES, uint32_t(t / held));
+                q.x += w.x, q.y += w.y, q.z += w.z, q.w += w.w;
             }
+            if (CONV) {
+                const int pixels  = cv_pixels(p);
+                const int64_t img = row / pixels;
+                TOut* plane       = out + (img * p.N + gcol) * pixels + (row - img * pixels);
+                const float v[4]  = {q.x, q.y, q.z, q.w};
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int64_t n = gcol + i;
-                if (n >= p.N) break;
-                // A non-finite cell: an operand of its fold was inf / NaN, or the sum overflowed. Such cells take the scalar
-                // fold of the CUDA-core kernel -- ascending k, one fma per step -- from the caller's operands.
-                if (!isfinite(v[i])) {
-                    const TIn* ar = A + row * p.K;
-                    const TIn* br = p.b_nk ? B + n * p.K : B + n;
-                    const int64_t step = p.b_nk ? 1 : p.N;
-                    float acc = 0.f;
-                    for (int64_t k = 0; k < p.K; ++k) acc = fmaf(load1(ar + k), load1(br + k * step), acc);
-                    v[i] = acc;
-                }
-                const float rowv = p.post_row ? __ldg(p.post_row + n) : 0.f;
-                const float full = post_full ? float(post_full[row * p.N + n]) : 0.f;
-                v[i]             = apply_post(p.post, v[i], rowv, full);
-            }
-            TOut* dst = out + row * p.N + gcol;
-            if (p.vec_c) {  // four results are one aligned store, and N is a multiple of 4
-                if (sizeof(TOut) == 4)
-                    *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
-                else
-                    *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+                for (int e = 0; e < 4; ++e)
+                    if (gcol + e < p.N) plane[int64_t(e) * pixels] = TOut(isfinite(v[e]) ? v[e] : scalar_fold<TIn, CONV>(p, bz, row, gcol + e));
             } else {
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (gcol + i < p.N) dst[i] = TOut(v[i]);
+                finish4<TIn, TOut>(p, out, post_full, bz, row, gcol, q);
             }
         }
     }
-    if (p.split > 1) cluster_sync();  // no CTA of the cluster exits while another may read its partial tile
+    if (p.split > 1) cluster_sync();  // no CTA of the cluster exits while another may read its partial tiles
 
     tc_fence_before();
     __syncthreads();
     if (warp == MMA_WARP) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, NBUF * BN);
+        tmem_dealloc(tmem_base, 512);
     }
     if (tid == 0 && *abort_flag) *p.status = MIMK_E_DEVICE_WAIT;
 }
 
-template <int BN, int LOADERS, class TIn, class TOut, bool CONV>
+template <int BN, class TIn, class TOut, bool CONV>
 int launch(const Params& p, int64_t ctas, cudaStream_t s) {
-    auto kern = gemm_f32_tc_kernel<BN, LOADERS, TIn, TOut, CONV>;
+    auto kern = gemm_f32_tc_kernel<BN, TIn, TOut, CONV>;
     constexpr int SMEM = Cfg<BN, TIn>::SMEM_BYTES;
     static bool configured[64] = {};  // per template instance and device: the attribute is a per-device setting
     int dev = 0;
@@ -386,7 +404,7 @@ int launch(const Params& p, int64_t ctas, cudaStream_t s) {
         configured[dev & 63] = true;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned(ctas)), cfg.blockDim = dim3(LOADERS + 32), cfg.dynamicSmemBytes = SMEM, cfg.stream = s;
+    cfg.gridDim = dim3(unsigned(ctas)), cfg.blockDim = dim3(NUM_THREADS), cfg.dynamicSmemBytes = SMEM, cfg.stream = s;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = unsigned(p.split), attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
@@ -394,23 +412,29 @@ int launch(const Params& p, int64_t ctas, cudaStream_t s) {
     return note_cuda_error(cudaLaunchKernelEx(&cfg, kern, p));
 }
 
-// Tile width and split. Tiles of 128 x 128 read a third less shared memory per flop; 128 x 64 puts two CTAs on an SM, which
-// hides the start and end of a tile, and leaves a smaller last wave.
+// Tile width and split: the pair with the least estimated time, rounds * (fixed + k-blocks per CTA * per k-block), a round being
+// the tiles that are on the chip at once (one CTA per SM; clusters of eight and four leave SMs of a partly filled GPC idle).
 template <class TIn, class TOut, bool CONV>
 int plan_and_launch(Params& p, int64_t batch, int sm_count, cudaStream_t s) {
     p.tiles_m = (p.M + BM - 1) / BM;
-    const int64_t kb = (p.K + BK - 1) / BK, wide = p.tiles_m * ((p.N + 127) / 128) * batch;
-    int bn = p.N > 64 && wide >= sm_count && kb >= 8 ? 128 : 64;
-    if (getenv("SW_BN")) bn = atoi(getenv("SW_BN"));
+    const int kb = int((p.K + BK - 1) / BK), chunks = (kb + CHUNK - 1) / CHUNK;
+    int bn = 64;
+    double best = 1e300;
+    p.split     = 1;
+    for (int wide = 0; wide < 2; ++wide)
+        for (int split = 1; split <= 8 && split <= chunks; split *= 2) {
+            if (getenv("SW_BN") && atoi(getenv("SW_BN")) != (wide ? 128 : 64)) continue;
+            if (getenv("SW_SPLIT") && atoi(getenv("SW_SPLIT")) != split) continue;
+            const int64_t items = p.tiles_m * ((p.N + (wide ? 127 : 63)) / (wide ? 128 : 64)) * batch;
+            const int64_t room  = split == 1 ? sm_count : split == 2 ? sm_count / 2 - 4 : split == 4 ? sm_count / 4 - 5 : sm_count / 8 - 4;
+            const double rounds = double((items + room - 1) / room);
+            const int per       = (chunks + split - 1) / split * CHUNK;
+            const double time   = rounds * ((split > 1 ? 6.0 : 4.0) + (per < kb ? per : kb) * (wide ? 0.7 : 0.5));
+            if (time < best) best = time, bn = wide ? 128 : 64, p.split = split;
+        }
     p.tiles_n = (p.N + bn - 1) / bn;
-    const int64_t items = p.tiles_m * p.tiles_n * batch;
-    p.split = 1;
-    while (p.split < 8 && items * p.split * 2 <= sm_count && kb >= p.split * 2) p.split *= 2;
-    if (getenv("SW_SPLIT")) p.split = atoi(getenv("SW_SPLIT"));
-    const int64_t ctas = items * p.split;
-    if (bn == 128) return launch<128, 512, TIn, TOut, CONV>(p, ctas, s);
-    if (getenv("SW_LD") ? atoi(getenv("SW_LD")) == 512 : ctas <= sm_count) return launch<64, 512, TIn, TOut, CONV>(p, ctas, s);
-    return launch<64, 256, TIn, TOut, CONV>(p, ctas, s);
+    const int64_t ctas = p.tiles_m * p.tiles_n * batch * p.split;
+    return bn == 128 ? launch<128, TIn, TOut, CONV>(p, ctas, s) : launch<64, TIn, TOut, CONV>(p, ctas, s);
 }
 
 }  // namespace

@@ -12,8 +12,6 @@
 //   warps 2..5  accumulator -> f32 partial tile in shared memory, over the stages
 //   all         after a cluster barrier: the partial tiles are added in rank order through distributed shared memory, each CTA
 //               a share of the cells, `post`, and stored with neighbouring lanes on neighbouring columns (any pitch and alignment)
-#include <cstdlib>
-
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -252,11 +250,14 @@ int pick(int bn, bool gated, const CUtensorMap& tA, const CUtensorMap& tB, const
 
 }  // namespace
 
-int gemm_tc_split_preferred(const mimk_gemm_desc& d, int gated, int sm_count) {
-    const char* e = getenv("SW_TCS");
-    if (e) return e[0] != '0';
-    const int64_t tiles = ((d.m + BM - 1) / BM) * ((d.n + 255) / 256) * d.batch;
-    return tiles * (gated ? 2 : 1) < sm_count;
+// Few tiles of the one-CTA kernel's 128 x 256 (gated 128 x 128), and K long enough to deal out. The one-CTA kernel takes about
+// 0.3 us per k-block of its single round; this one starts and merges 4 us slower and works on several k-blocks of a tile at once:
+// 16 x 14336 x 4096 (56 tiles): 32.9 -> 24.3 us; 256 x 4096 x 4096 (32): 23.6 -> 17.7; 5000 x 64 x 8192 (40): 40.6 -> 17.7;
+// 300 x 200 x 16000 (3): 74.6 -> 16.7. Beyond the rule: 128 x 8192 x 1024: 10.0 against 12.1; 700 x 3008 x 8192 (72): 43.5 / 42.4;
+// 2048 x 1024 x 4096 (64): 24.1 / 27.1; 256^3: 6.3 / 7.0. With few rows the bytes of B decide, and more SMs fetch them faster.
+int gemm_tc_split_preferred(const mimk_gemm_desc& d, int gated) {
+    const int64_t width = gated ? 128 : 256, tiles = ((d.m + BM - 1) / BM) * ((d.n + width - 1) / width) * d.batch;
+    return d.k >= 24 * BK && tiles <= (d.m <= BM ? 74 : 40);
 }
 
 int gemm_tc_split(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, const GemmPitch* pitch) {
@@ -270,8 +271,8 @@ int gemm_tc_split(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void
     // (the outermost stride of a one-entry operand is never used; it only has to be a legal value)
     const uint64_t sa = a_b ? uint64_t(d.stride_a) * 2 : lda * 2, sb = b_b ? uint64_t(d.stride_b) * 2 : ldb * 2;
     const int64_t tiles_m = (d.m + BM - 1) / BM, kb = (d.k + BK - 1) / BK;
-    int bn = gated ? 128 : (tiles_m * ((d.n + 127) / 128) * d.batch * 2 >= dev->sm_count ? 128 : 64);
-    if (getenv("SW_BN") && !gated) bn = atoi(getenv("SW_BN"));
+    // 128 columns, or 64 where the result is narrow or eight CTAs for each tile would not fill the chip
+    const int bn  = gated || (d.n > 64 && tiles_m * ((d.n + 127) / 128) * d.batch * 8 >= dev->sm_count) ? 128 : 64;
     const int bno = gated ? 64 : bn;
     Params p{};
     p.M = d.m, p.N = d.n, p.K = d.k, p.stride_c = d.batch > 1 ? d.stride_c : 0;
@@ -284,7 +285,6 @@ int gemm_tc_split(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void
     const int64_t items = p.tiles_m * p.tiles_n * d.batch;
     p.split = 1;
     while (p.split < 8 && items * p.split * 2 <= 2 * dev->sm_count && kb >= p.split * 8) p.split *= 2;
-    if (getenv("SW_SPLIT")) p.split = atoi(getenv("SW_SPLIT"));
     p.C = d.c, p.post_row = static_cast<const float*>(d.post_row), p.post_full = d.post_full, p.post = d.post;
     p.vec_c  = d.n % 4 == 0 && aligned16(d.c) && p.stride_c % 4 == 0;
     p.status = dev->status_dev;

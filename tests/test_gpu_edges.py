@@ -191,7 +191,7 @@ def test_bf16_batches_of_any_extent(T, B, m, n, k, b_nk):
     assert ((d64(got) - want).abs() <= want.abs() * BF16_ROUND + d64(a).abs() @ d64(b).abs() * 2.0 ** -14 + 1e-6).all()
 
 
-@pytest.mark.parametrize("m,k,f,n,b_nk", [(1, 512, 1024, 512, True), (17, 520, 1032, 264, False), (128, 1024, 2048, 512, False), (200, 512, 640, 520, True)])
+@pytest.mark.parametrize("m,k,f,n,b_nk", [(1, 2048, 1024, 512, True), (17, 1544, 2056, 264, False), (128, 1536, 2048, 512, False), (200, 1600, 640, 520, True)])
 def test_gated_mlp_of_few_rows(T, m, k, f, n, b_nk):
     x = rnd((m, k), 1, BF16)
     w = [(rnd((o, i) if b_nk else (i, o), s, BF16) * 0.05) for s, (i, o) in enumerate([(k, f), (k, f), (f, n)], 2)]
