@@ -4,24 +4,20 @@
 // What bounds it is reading K and V once: with r query rows a loaded byte carries 2 r flops, far below the chip's ridge. The
 // tcgen05 kernel has 128-row tiles, so it would do 8 to 128 times the exponentials and could give each head to one SM only.
 // Here the keys of a head are dealt out to a cluster of up to eight CTAs of four warps, and every warp streams its own run of
-// keys, 16 at a time, into mma.sync fragments (16 rows are exactly its M). Each lane requests one row of the step's K or V by a bulk
-// copy (one instruction for 128 or 256 bytes) into the warp's own ring; no barrier is shared by warps in the loop. Both products
-// may take their contracted index in any order as long as both operands use the same one, so
+// keys, 16 at a time, into mma.sync fragments (16 rows are exactly its M). The copies are asynchronous, each lane reads from
+// shared memory only what it fetched itself, and so there is no barrier in the loop. Both products may take their contracted
+// index in any order as long as both operands use the same one, so
 //   K   a lane takes 16 consecutive bytes of a key (head_dim 8c .. 8c+7 of each 32), which are the fragments of two k-steps
 //   V   a lane takes 16 consecutive bytes of four keys; pairs of keys are interleaved by byte permutes, and the eight elements
 //       belong to eight different column tiles of the result
+// Measured: 128 heads x 1 x 4096 x 128, 61 us (4.4 TB/s, as the 128-row kernel); 8 x 1 x 8192 x 128, 22 us; causal 32 x 11 x 5000
+// x 128, 26 us. One bulk copy per key instead of 16 lanes' copies was slower (69, 32 and 29 us), registers instead of the ring too.
 // Each warp keeps its own running maximum, sum and output; they are merged through (distributed) shared memory in a fixed order.
 #include <math_constants.h>
 
-#include <cstdlib>
-
 #include "common.cuh"
-#include "sm100.cuh"
 
 namespace mimk {
-
-using namespace sm100;
-
 namespace {
 
 constexpr int ROWS = 16, WARPS = 4, THREADS = WARPS * 32, STEP = 16;
@@ -29,8 +25,8 @@ constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
 
 template <int D> struct Ring {
     static constexpr int STAGES = D == 128 ? 3 : 4;
-    static constexpr int PITCH  = D * 2 + 16;  // bytes between rows: the lanes of a 16-byte read phase spread over the banks
-    static constexpr int STAGE_BYTES = 2 * STEP * PITCH, WARP_BYTES = STAGES * STAGE_BYTES;
+    static constexpr int CHUNKS = D / 8;  // 16-byte pieces per lane and step: half K, half V
+    static constexpr int WARP_BYTES = STAGES * CHUNKS * 32 * 16;
     static_assert(WARP_BYTES >= ROWS * D * 4, "a warp's part of the output lies over its ring");
 };
 
@@ -41,16 +37,14 @@ struct Params {
     int64_t sq, sk;
     float scale;
     int causal, split;
-    int* status;
 };
 
 __device__ __forceinline__ uint4 ld_row(const __nv_bfloat16* p, bool there) {
     return there ? __ldg(reinterpret_cast<const uint4*>(p)) : make_uint4(0, 0, 0, 0);
 }
-__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
+// 16 bytes to shared memory, or zeros
+__device__ __forceinline__ void copy16(uint32_t dst, const __nv_bfloat16* src, bool there) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");
 }
 __device__ __forceinline__ uint4 ld_shared16(uint32_t a) {
     uint4 v;
@@ -95,8 +89,6 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
     auto part_o = [&](int w) { return reinterpret_cast<float*>(ring + w * R::WARP_BYTES); };  // [ROWS][D], once the loop is over
     __shared__ float part_m[WARPS][ROWS], part_l[WARPS][ROWS];
     __shared__ float cta_m[ROWS], cta_l[ROWS];
-    __shared__ uint64_t full[WARPS][R::STAGES];
-    __shared__ volatile int abort_flag;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c = lane & 3;
     const int rank  = int(blockIdx.x % unsigned(p.split));  // a cluster is `split` consecutive CTAs
     const int64_t h = blockIdx.x / unsigned(p.split);
@@ -107,22 +99,26 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
     const int64_t s0 = (rank * WARPS + warp) * per, s1 = s0 + per < steps ? s0 + per : steps;
     const float scale2 = p.scale * LOG2E;
 
-    const uint32_t mine = smem_u32(ring) + warp * R::WARP_BYTES, bars = smem_u32(full[warp]);
-    if (tid == 0) abort_flag = 0;
-    if (lane == 0)
-        for (int i = 0; i < R::STAGES; ++i) mbar_init(bars + i * 8, 1);
-    fence_barrier_init();
-    __syncthreads();
-    auto fetch = [&](int64_t step) {  // lanes 0..15 a row of the step's K, lanes 16..31 of its V; rows past the end stay as they are
-        __syncwarp();                 // every lane has read what lay there
-        if (step >= s1) return;
-        const unsigned stage = unsigned(step - s0) % R::STAGES;
-        const int64_t rows   = p.sk - step * STEP < STEP ? p.sk - step * STEP : STEP;
-        if (lane == 0) mbar_expect_tx(bars + stage * 8, uint32_t(rows) * 2 * D * 2);
-        __syncwarp();
-        const int r = lane & 15;
-        if (r < rows)
-            bulk_copy(mine + stage * R::STAGE_BYTES + lane * R::PITCH, (lane < 16 ? K : V) + (step * STEP + r) * D, D * 2, bars + stage * 8);
+    const uint32_t mine = uint32_t(__cvta_generic_to_shared(ring)) + warp * R::WARP_BYTES + lane * 16;
+    auto slot  = [&](int64_t step, int piece) { return mine + (unsigned(step - s0) % R::STAGES * R::CHUNKS + piece) * 512; };
+    auto fetch = [&](int64_t step) {  // this lane's pieces of the step's K and V; a step that is not there is an empty group
+        if (step < s1) {
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+#pragma unroll
+                for (int i = 0; i < G; ++i) {
+                    const int64_t key = step * STEP + t * 8 + g;
+                    copy16(slot(step, t * G + i), key < p.sk ? K + key * D + i * 32 + c * 8 : K, key < p.sk);
+                }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int ch = 0; ch < CH; ++ch) {
+                    const int64_t key = step * STEP + (j >> 1) * 8 + 2 * c + (j & 1);
+                    copy16(slot(step, 2 * G + j * CH + ch), key < p.sk ? V + key * D + ch * 64 + g * 8 : V, key < p.sk);
+                }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
 #pragma unroll
     for (int i = 0; i < R::STAGES - 1; ++i) fetch(s0 + i);
@@ -149,20 +145,18 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
     const int64_t seen_by_all = p.causal && p.sk - p.sq + 1 < p.sk ? p.sk - p.sq + 1 : p.sk;
 
     for (int64_t step = s0; step < s1; ++step) {
-        fetch(step + R::STAGES - 1);  // over the step before this one
-        const unsigned at = unsigned(step - s0), stage = at % R::STAGES;
-        if (!__all_sync(0xffffffffu, mbar_wait(bars + stage * 8, (at / R::STAGES) & 1u, &abort_flag))) break;
-        const uint32_t k_at = mine + stage * R::STAGE_BYTES + g * R::PITCH + c * 16, v_at = mine + stage * R::STAGE_BYTES + (STEP + 2 * c) * R::PITCH + g * 16;
+        fetch(step + R::STAGES - 1);  // over the step before this one, whose pieces are in registers or used up
+        asm volatile("cp.async.wait_group %0;" ::"n"(R::STAGES - 1) : "memory");
         // all of the step's fragments first: the copies into registers overlap one another and the first product
         uint4 kr[2][G], vr[4][CH];
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
-            for (int i = 0; i < G; ++i) kr[t][i] = ld_shared16(k_at + t * 8 * R::PITCH + i * 64);
+            for (int i = 0; i < G; ++i) kr[t][i] = ld_shared16(slot(step, t * G + i));
 #pragma unroll
         for (int j = 0; j < 4; ++j)
 #pragma unroll
-            for (int ch = 0; ch < CH; ++ch) vr[j][ch] = ld_shared16(v_at + ((j >> 1) * 8 + (j & 1)) * R::PITCH + ch * 128);
+            for (int ch = 0; ch < CH; ++ch) vr[j][ch] = ld_shared16(slot(step, 2 * G + j * CH + ch));
         float s[2][4] = {}, s2[2][4] = {};  // two chains of dependent products for each eight keys
 #pragma unroll
         for (int i = 0; i < G; ++i)
@@ -210,8 +204,8 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
 #pragma unroll
                     for (int e = 0; e < 4; ++e) o[ch][t][e] *= alpha[e >> 1];
         }
-        // A key that a row does not see (or that does not exist, whose row holds anything) must not reach it even as 0 times an
-        // infinity: such a block, where it holds one, is added cell by cell over the keys each row sees.
+        // A key that a row does not see must not reach it even as 0 times an infinity: such a block, where it holds one, is
+        // added cell by cell over the keys each row sees.
         bool odd_block = false;
         if (!whole) {
             bool bad = false;
@@ -255,6 +249,7 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
             }
         }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncwarp();  // every lane is done with the warp's ring
 
     // the warps' parts -> this CTA's part (in the first warp's place) -> the rows of the head, each CTA of the cluster some
@@ -308,7 +303,6 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
         if (p.lse && col == 0) p.lse[h * p.sq + row] = den > 0.f ? M * LN2 + logf(den) : -CUDART_INF_F;
     }
     if (p.split > 1) cluster_sync();  // no CTA of the cluster exits while another may read its part
-    if (tid == 0 && abort_flag) *p.status = MIMK_E_DEVICE_WAIT;
 }
 
 template <int D>
@@ -347,13 +341,12 @@ int attn_few(const mimk_attn_desc& d, cudaStream_t s) {
     Params p;
     p.q = static_cast<const __nv_bfloat16*>(d.q), p.k = static_cast<const __nv_bfloat16*>(d.k), p.v = static_cast<const __nv_bfloat16*>(d.v);
     p.o = static_cast<__nv_bfloat16*>(d.o), p.lse = d.lse;
-    p.sq = d.seq_q, p.sk = d.seq_k, p.scale = d.scale, p.causal = d.causal, p.status = dev->status_dev;
+    p.sq = d.seq_q, p.sk = d.seq_k, p.scale = d.scale, p.causal = d.causal;
     // As many CTAs per head as the SMs hold at once (two each): a second round of CTAs would pay the start of its stream and the
-    // merge, together several steps, again. Every warp has at least 64 keys.
-    const int64_t room = 2 * int64_t(dev->sm_count) / d.batch_heads, runs = d.seq_k / (WARPS * 64);
+    // merge, together several steps, again (128 heads x 4096 keys: split 1 / 2 / 4 / 8: 64 / 61 / 65 / 74 us; 8 x 8192: 118 / 64 /
+    // 36 / 22). Every warp has at least three steps.
     p.split = 1;
-    while (p.split < 8 && p.split < room && p.split < runs) ++p.split;
-    if (getenv("SW_FEW")) p.split = atoi(getenv("SW_FEW"));
+    while (p.split < 8 && d.batch_heads * p.split * 2 <= 2 * int64_t(dev->sm_count) && d.seq_k >= int64_t(p.split) * 2 * WARPS * 3 * STEP) p.split *= 2;
     return d.head_dim == 128 ? launch<128>(p, d.batch_heads * p.split, s) : launch<64>(p, d.batch_heads * p.split, s);
 }
 

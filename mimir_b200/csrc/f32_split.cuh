@@ -58,19 +58,23 @@ __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t saddr) {
     return d;
 }
 
-// D (+)= A B^T over one 32-wide k-block, the six products, smallest first (the tensor core cuts off what its accumulator
-// update cannot hold, which costs least while the accumulator is small). `a` / `b`: the h piece; m and l follow. PIECES = 1: the
-// product of the h pieces alone.
-template <int PIECES = 3>
-__device__ __forceinline__ void mma_six(uint32_t d, uint32_t a, uint32_t a_piece, uint32_t b, uint32_t b_piece, uint32_t idesc,
-                                        uint32_t accumulate) {
+// D = A B^T over `blocks` 32-wide k-blocks, the products smallest first over all of them: the tensor core cuts off what its
+// accumulator update cannot hold, which costs least while the accumulator is small (and so only 2 x blocks updates by full-size
+// terms count). stage[b]: block b's A tiles, its B tiles `b_off` behind; the h piece first. PIECES = 1: the product of the h pieces
+// alone.
+template <int PIECES>
+__device__ __forceinline__ void mma_six(uint32_t d, const uint32_t (&stage)[2], int blocks, uint32_t a_piece, uint32_t b_off,
+                                        uint32_t b_piece, uint32_t idesc) {
     constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0}, FIRST = PIECES == 1 ? 5 : 0;
 #pragma unroll
     for (int t = FIRST; t < 6; ++t)
 #pragma unroll
-        for (int k = 0; k < 2; ++k)
-            sm100::mma_f16_ss(d, smem_desc_sw64(a + PA[t] * a_piece + k * 32), smem_desc_sw64(b + PB[t] * b_piece + k * 32), idesc,
-                              (t > FIRST || k > 0) ? 1u : accumulate);
+        for (int b = 0; b < 2; ++b)
+            if (b < blocks)
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                    sm100::mma_f16_ss(d, smem_desc_sw64(stage[b] + PA[t] * a_piece + k * 32),
+                                      smem_desc_sw64(stage[b] + b_off + PB[t] * b_piece + k * 32), idesc, (t > FIRST || b > 0 || k > 0) ? 1u : 0u);
 }
 
 __device__ __forceinline__ float load1(const float* p) { return __ldg(p); }

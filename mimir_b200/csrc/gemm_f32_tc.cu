@@ -7,10 +7,10 @@
 //
 //   warps 0..15   read the operands and write their pieces into shared-memory tiles (each eight-k unit of the next k-block is
 //                 requested as soon as the present one's has left its registers), add finished accumulators to sums in registers
-//   warp 16       one thread issues the MMAs, 128 x BN x 32 per k-block; every four k-blocks go into a fresh accumulator
-// The tensor core does not round its accumulator updates to nearest; with 8 updates by full-size terms per accumulator (the small
-// terms of each k-block first) and ordinary f32 adds between accumulators, the error stays below that of an f32 fold for any K.
-// The accumulators are added in order whatever the grid (up to K = 2048: beyond that a CTA of a cluster may first add its own).
+//   warp 16       one thread issues the MMAs, 128 x BN x 32 per k-block; every two k-blocks go into a fresh accumulator
+// The tensor core does not round its accumulator updates to nearest; with four updates by full-size terms per accumulator (all
+// small terms first) and ordinary f32 adds between accumulators, the error stays below that of an f32 fold for any K.
+// The accumulators are added in order whatever the grid (up to K = 1536: beyond that a CTA of a cluster may first add its own).
 //
 // The operands are read as the caller has them: any extents, strides and alignment, no copies, no scratch. What bounds it:
 // shared-memory bandwidth (a k-block of 128 x 128 moves 96 KB into the MMA and 48 KB from the loaders; measured 100 clocks per
@@ -30,7 +30,7 @@ using namespace f32split;
 namespace {
 
 constexpr int BM = 128;
-constexpr int CHUNK = 4;        // k-blocks per accumulator
+constexpr int CHUNK = 2;        // k-blocks per accumulator
 constexpr int LOADERS = 512, NUM_THREADS = LOADERS + 32, MMA_WARP = LOADERS / 32;
 constexpr int STAGES = 4, GROUP_M = 16;
 constexpr int A_PIECE = BM * BK * 2;
@@ -41,7 +41,7 @@ template <int BN, class TIn> struct Cfg {
     static constexpr int STAGE_BYTES = PIECES * (A_PIECE + B_PIECE);
     static constexpr int PITCH = BN + 4, PART_BYTES = BM * PITCH * 4;  // a partial tile; they lie over the stages
     static constexpr int NACC  = 512 / BN;                             // accumulators in tensor memory
-    static constexpr int SLOTS = BN == 128 ? 2 : 4;                    // of them, what a CTA of a cluster may hold to the end
+    static constexpr int SLOTS = BN == 128 ? 3 : 4;                    // of them, what a CTA of a cluster may hold to the end
     static constexpr int TILE_BYTES = STAGES * STAGE_BYTES > SLOTS * PART_BYTES ? STAGES * STAGE_BYTES : SLOTS * PART_BYTES;
     static constexpr int SMEM_BYTES = TILE_BYTES + 1024 + 256;
     static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
@@ -55,8 +55,11 @@ struct Bars {
 
 // A convolution as a contraction: row = output pixel (image, oh, ow), k = (input channel, kh, kw), column = filter. Rows of the
 // patch matrix are gathered from the image as the loaders read them.
+// tap_major (channels a multiple of 8): k = (kh, kw, input channel) instead, so that the eight k of a unit share one tap: one test
+// whether it lies inside, and addresses a plane apart. With k in the order of the filters, every element has its own tap and
+// test: 16 x 128 x 56 x 56, 128 filters of 3 x 3: 207 us.
 struct ConvShape {
-    int cin, h, w, kh, kw, oh, ow, stride_h, stride_w, dil_h, dil_w, pad_h, pad_w;
+    int cin, h, w, kh, kw, oh, ow, stride_h, stride_w, dil_h, dil_w, pad_h, pad_w, tap_major;
 };
 
 struct Params {
@@ -215,7 +218,16 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
     }
     auto fetch_a = [&](int kb) {
         const int64_t k0 = int64_t(kb) * BK;
-        if (CONV) {
+        if (CONV && cv.tap_major) {
+            const int k = int(k0) + unit * 8, tap = k / cv.cin, r = tap / cv.kw, q = tap - r * cv.kw, plane = cv.h * cv.w;
+            const bool in = k < int(p.K) && ((rows_in >> r) & (cols_in >> q) & 1);
+            const TIn* at = a_at + (k - tap * cv.cin) * int64_t(plane) + (r * cv.dil_h * cv.w + q * cv.dil_w);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                fa[j] = in ? load1(at) : 0.f;
+                at += plane;
+            }
+        } else if (CONV) {
             const int k = int(k0) + unit * 8, taps = cv.kh * cv.kw;
             const int ci = k / taps;
             int r = (k - ci * taps) / cv.kw, q = k - ci * taps - r * cv.kw;
@@ -239,7 +251,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
         if (!has_b) return;
         const int64_t k0 = int64_t(kb) * BK;
         const int left   = int(p.K - k0) - b_unit * 8;
-        if (p.b_nk) {
+        if (CONV && cv.tap_major) {  // the filters are stored (input channel, kh, kw)
+            const int k = int(k0) + b_unit * 8, tap = k / cv.cin, taps = cv.kh * cv.kw;
+            const TIn* at = B + (n0 + b_row) * p.K + int64_t(k - tap * cv.cin) * taps + tap;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) fb[j] = b_there && left > 0 ? load1(at + j * taps) : 0.f;
+        } else if (p.b_nk) {
             load8(fb, b_at + k0, b_there, left, p.vec_b);
         } else {
             const TIn* at = b_at + k0 * p.N;
@@ -274,21 +291,31 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
         if (lane == 0) {
             const uint32_t idesc = idesc_bf16_f32(BM, BN, 0, 0);
             uint32_t stage = 0, phase = 0;
-            for (int kb = kb0; kb < kb1; ++kb) {
-                // A full stage also says that every warp has added up the chunk that ended four or more k-blocks before it, so an
-                // accumulator is free when its turn comes again (they are three or more in number).
-                if (!mbar_wait(smem_u32(&bars->full[stage]), phase, abort_flag)) break;
+            for (int kb = kb0, c = 0; kb < kb1; kb += CHUNK, ++c) {
+                // A full stage also says that every warp has added up the chunk three before this one, so an accumulator is free
+                // when its turn comes again.
+                uint32_t at[CHUNK], empty[CHUNK];
+                const int n = kb1 - kb < CHUNK ? kb1 - kb : CHUNK;
+                bool ok = true;
+#pragma unroll
+                for (int b = 0; b < CHUNK; ++b) {
+                    if (b < n && ok) ok = mbar_wait(smem_u32(&bars->full[stage]), phase, abort_flag);
+                    at[b] = base + stage * C::STAGE_BYTES, empty[b] = smem_u32(&bars->empty[stage]);
+                    if (b < n && ++stage == STAGES) stage = 0, phase ^= 1u;
+                }
+                if (!ok) break;
                 tc_fence_after();
-                const uint32_t s0 = base + stage * C::STAGE_BYTES, acc = uint32_t((kb - kb0) / CHUNK) % C::NACC;
-                mma_six<PIECES>(tmem_base + acc * BN, s0, A_PIECE, s0 + PIECES * A_PIECE, C::B_PIECE, idesc, (kb - kb0) % CHUNK ? 1u : 0u);
-                mma_commit(smem_u32(&bars->empty[stage]));
-                if ((kb - kb0) % CHUNK == CHUNK - 1 || kb + 1 == kb1) mma_commit(smem_u32(&bars->acc_full[acc]));
-                if (++stage == STAGES) stage = 0, phase ^= 1u;
+                const uint32_t acc = uint32_t(c) % C::NACC;
+                mma_six<PIECES>(tmem_base + acc * BN, at, n, A_PIECE, PIECES * A_PIECE, C::B_PIECE, idesc);
+#pragma unroll
+                for (int b = 0; b < CHUNK; ++b)
+                    if (b < n) mma_commit(empty[b]);
+                mma_commit(smem_u32(&bars->acc_full[acc]));
             }
         }
         __syncwarp();
     } else {
-        static_assert(C::NACC >= 3, "an accumulator is added up before its turn comes again");
+        static_assert(CHUNK == 2 && STAGES == 2 * CHUNK && C::NACC >= 3, "see the waits of the MMA warp");
         constexpr int COLS = BN / 4;  // accumulator columns per warp
         const uint32_t quarter = uint32_t(warp & 3), col0 = uint32_t(warp >> 2) * COLS, lanes = (quarter * 32u) << 16;
         float sum[COLS];
@@ -324,8 +351,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bars->full[stage]));
             if (++stage == STAGES) stage = 0, phase ^= 1u;
-            // the chunk before this one: with four stages its MMAs are complete by now
-            if (!hold && (kb - kb0) % CHUNK == CHUNK - 1 && kb - kb0 >= 2 * CHUNK - 1)
+            // two chunks before this one: with four stages its MMAs are complete by now
+            if (!hold && (kb - kb0) % CHUNK == CHUNK - 1 && kb - kb0 >= 3 * CHUNK - 1)
                 if (!(ok = add(added++))) break;
         }
         auto part = [&](int slot, const float (&x)[COLS]) {
@@ -364,9 +391,13 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
             if (row >= p.M || gcol >= p.N) continue;
             const uint32_t a = base + uint32_t(r * C::PITCH + col) * 4;
             float4 q         = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int t = 0; t < used; ++t) {
-                const float4 w = ld_cluster4(a + (t % held) * C::PART_BYTES, uint32_t(t / held));
-                q.x += w.x, q.y += w.y, q.z += w.z, q.w += w.w;
+            for (int t0 = 0; t0 < used; t0 += 4) {  // four on their way at a time, added in order
+                float4 w[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t)
+                    w[t] = t0 + t < used ? ld_cluster4(a + ((t0 + t) % held) * C::PART_BYTES, uint32_t((t0 + t) / held)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int t = 0; t < 4; ++t) q.x += w[t].x, q.y += w[t].y, q.z += w[t].z, q.w += w[t].w;
             }
             if (CONV) {
                 const int pixels  = cv_pixels(p);
@@ -473,7 +504,7 @@ int conv_tc(const mimk_conv_desc& d, cudaStream_t s) {
     p.A = d.x, p.B = d.filters, p.C = d.out;
     p.M = d.n * oh * ow, p.N = d.cout, p.K = d.cin * d.kh * d.kw;
     p.conv = ConvShape{int(d.cin), int(d.h), int(d.w), int(d.kh), int(d.kw), int(oh), int(ow), int(d.stride_h), int(d.stride_w),
-                       int(d.dil_h), int(d.dil_w), int(d.pad_h), int(d.pad_w)};
+                       int(d.dil_h), int(d.dil_w), int(d.pad_h), int(d.pad_w), d.cin % 8 == 0 && d.kh * d.kw > 1};
     p.b_nk   = 1;
     p.vec_b  = p.K % (d.dtype == MIMK_F32 ? 4 : 8) == 0 && aligned16(d.filters);
     p.status = dev->status_dev;

@@ -10,6 +10,7 @@ as ValueError before anything is launched; kernel-side failures raise MimkError.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
 
 import torch
@@ -29,7 +30,8 @@ _UNOP = {"relu": L.OP_RELU, "tanh": L.OP_TANH, "exp": L.OP_EXP, "silu": L.OP_SIL
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device, as torch.cuda.current_stream().cuda_stream without the Stream object."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _dt(t: torch.Tensor) -> int:
@@ -377,20 +379,25 @@ def compose_reshape(consumer_map, n_loops: int, s_view, s_in) -> AccessMap:
     return AccessMap([lin for _ in s_in], div=[math.prod(s_in[j + 1:]) for j in range(len(s_in))], mod=s_in)
 
 
-def _fill_map(dst, m, n_loops):
-    rows = len(m)
-    if rows > L.MRP_MAX_RANK:
+@functools.lru_cache(maxsize=256)
+def _affine(rows, div, mod, n_loops) -> L.AffineMap:
+    """An access map's C form (copied into every descriptor that names it)."""
+    if len(rows) > L.MRP_MAX_RANK:
         raise ValueError("access map has too many results")
-    dst.rows = rows
-    for j, row in enumerate(m):
-        row = [int(v) for v in row]
+    dst = L.AffineMap()
+    dst.rows = len(rows)
+    for j, row in enumerate(rows):
         if len(row) != n_loops + 1:
             raise ValueError("access map row must have n_loops + 1 coefficients (the last one is the constant)")
-        for l in range(n_loops):
-            dst.coef[j][l] = row[l]
-        dst.coef[j][n_loops] = row[n_loops]
-        dst.div[j] = getattr(m, "div", None)[j] if getattr(m, "div", None) else 0
-        dst.mod[j] = getattr(m, "mod", None)[j] if getattr(m, "mod", None) else 0
+        dst.coef[j][:n_loops + 1] = [int(v) for v in row]
+        dst.div[j] = int(div[j]) if div else 0
+        dst.mod[j] = int(mod[j]) if mod else 0
+    return dst
+
+
+def _map(m, n_loops) -> L.AffineMap:
+    div, mod = getattr(m, "div", None), getattr(m, "mod", None)
+    return _affine(tuple(map(tuple, m)), tuple(div) if div else None, tuple(mod) if mod else None, n_loops)
 
 
 def _mrp_desc(So, Sr, f, init, post, map_out, maps, in_meta, post_maps, post_meta, acc_dtype, out_dtype, out_ptr):
@@ -400,20 +407,16 @@ def _mrp_desc(So, Sr, f, init, post, map_out, maps, in_meta, post_maps, post_met
         raise ValueError("map_reduce_post: too many loops, axes or inputs for the generic kernel")
     d = L.MrpDesc()
     d.ro, d.rn, d.nis, d.nps = ro, rn, len(in_meta), len(post_meta)
-    for i, v in enumerate(Sr):
-        d.sr[i] = v
-    for i, v in enumerate(So):
-        d.so[i] = v
+    d.sr[:rn], d.so[:ro] = Sr, So
     for i, ((ptr, dt, shape), m) in enumerate(zip(in_meta, maps)):
         if len(shape) > L.MRP_MAX_RANK:
             raise ValueError("input rank too large for the generic kernel")
         d.in_[i] = ptr
         d.in_dtype[i] = _DT[dt]
-        for j, v in enumerate(shape):
-            d.in_shape[i][j] = v
+        d.in_shape[i][:len(shape)] = shape
         if len(m) != len(shape):
             raise ValueError("access map must have one result per input axis")
-        _fill_map(d.in_map[i], m, rn)
+        d.in_map[i] = _map(m, rn)
     for i, ((ptr, dt, shape), m) in enumerate(zip(post_meta, post_maps)):
         d.post_in[i] = ptr
         d.post_dtype[i] = _DT[dt]
@@ -421,10 +424,10 @@ def _mrp_desc(So, Sr, f, init, post, map_out, maps, in_meta, post_maps, post_met
             d.post_shape[i][j] = v
         if len(m) != len(shape):
             raise ValueError("epilogue access map must have one result per epilogue-input axis")
-        _fill_map(d.post_map[i], m, ro)
+        d.post_map[i] = _map(m, ro)
     if len(map_out) != ro:
         raise ValueError("map_out must have one result per output axis")
-    _fill_map(d.map_out, map_out, rn)
+    d.map_out = _map(map_out, rn)
     d.comb, d.post = f, post
     d.acc_dtype, d.out_dtype = _DT[acc_dtype], _DT[out_dtype]
     if acc_dtype == torch.float32:
@@ -480,7 +483,7 @@ def map_reduce_post(So, Sr, f: int, init, post: int, map_out, maps, ins, post_ma
         out_dtype = acc_dtype
     dev = ins[0].device if ins else (post_ins[0].device if post_ins else torch.device("cuda"))
     # a write map that stores loop vector o at o covers the whole result; anything else may leave cells untouched
-    covers = So == Sr[:len(So)] and [list(r) for r in map_out] == [list(r) for r in proj_map(len(Sr), range(len(So)))]
+    covers = So == Sr[:len(So)] and all(list(r) == u for r, u in zip(map_out, proj_map(len(Sr), range(len(So))))) and len(map_out) == len(So)
     out = (torch.empty if covers else torch.zeros)(So, dtype=out_dtype, device=dev)
     d = _mrp_desc(So, Sr, f, init, post, map_out, maps, [(t.data_ptr(), t.dtype, tuple(t.shape)) for t in ins], post_maps,
                   [(t.data_ptr(), t.dtype, tuple(t.shape)) for t in post_ins], acc_dtype, out_dtype, out.data_ptr())
@@ -641,8 +644,8 @@ def _mrp_into(out, Sr, f, init, post, map_out, maps, ins):
         d.in_dtype[i] = _dt(t)
         for j, v in enumerate(t.shape):
             d.in_shape[i][j] = v
-        _fill_map(d.in_map[i], m, rn)
-    _fill_map(d.map_out, map_out, rn)
+        d.in_map[i] = _map(m, rn)
+    d.map_out = _map(map_out, rn)
     d.comb, d.post = f, post
     acc = _acc(out)
     d.acc_dtype, d.out_dtype = _DT[acc], _dt(out)
