@@ -282,14 +282,16 @@ int mimk_attn_fwd(const mimk_attn_desc* desc, void* stream);
 
 /* out[n, co, oh, ow] = sum over (ci, kh, kw) of x[n, ci, oh s + kh d - p, ow s + kw d - p] * filters[co, ci, kh, kw], cells of x
  * outside it read as zeros: tensor.conv (tensor.mim:434-438) with its padding, as one contraction on the tensor cores whose left
- * operand is gathered from the image. dtype F32 or BF16 (out the same); any extents and alignment, windows up to 31 x 31. */
+ * operand is gathered from the image. dtype F32 or BF16 (out the same); any extents and alignment, windows up to 31 x 31.
+ * by_tap: the filters are given as [co, kh, kw, ci], ci a multiple of 8; then each load's place in the window is tested once for
+ * eight channels. */
 typedef struct mimk_conv_desc {
     int64_t n, cin, h, w, cout, kh, kw;
     int64_t stride_h, stride_w, dil_h, dil_w, pad_h, pad_w;
     const void* x;
     const void* filters;
     void* out;
-    int32_t dtype, pad_;
+    int32_t dtype, by_tap;
 } mimk_conv_desc;
 int mimk_conv(const mimk_conv_desc* desc, void* stream);
 

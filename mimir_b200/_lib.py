@@ -70,7 +70,7 @@ class ConvDesc(C.Structure):
     _fields_ = [
         ("n", C.c_int64), ("cin", C.c_int64), ("h", C.c_int64), ("w", C.c_int64), ("cout", C.c_int64), ("kh", C.c_int64), ("kw", C.c_int64),
         ("stride_h", C.c_int64), ("stride_w", C.c_int64), ("dil_h", C.c_int64), ("dil_w", C.c_int64), ("pad_h", C.c_int64), ("pad_w", C.c_int64),
-        ("x", C.c_void_p), ("filters", C.c_void_p), ("out", C.c_void_p), ("dtype", C.c_int32), ("pad_", C.c_int32),
+        ("x", C.c_void_p), ("filters", C.c_void_p), ("out", C.c_void_p), ("dtype", C.c_int32), ("by_tap", C.c_int32),
     ]
 
 

@@ -295,6 +295,7 @@ extern "C" int mimk_conv(const mimk_conv_desc* d, void* stream) {
     if (d->n < 0 || d->cin < 1 || d->h < 1 || d->w < 1 || d->cout < 0 || d->kh < 1 || d->kw < 1) return MIMK_E_ARG;
     if (d->stride_h < 1 || d->stride_w < 1 || d->dil_h < 1 || d->dil_w < 1 || d->pad_h < 0 || d->pad_w < 0) return MIMK_E_ARG;
     if (d->dtype != MIMK_F32 && d->dtype != MIMK_BF16) return MIMK_E_DTYPE;
+    if (d->by_tap && d->cin % 8 != 0) return MIMK_E_SHAPE;
     // one image, one filter and every coordinate of the padded image are 30-bit numbers
     constexpr double LIM = double(1 << 30);
     if (double(d->cin) * double(d->h) * double(d->w) >= LIM || double(d->cin) * double(d->kh) * double(d->kw) >= LIM) return MIMK_E_UNSUPPORTED;

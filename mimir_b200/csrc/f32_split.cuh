@@ -45,6 +45,21 @@ __device__ __forceinline__ void split_store8(uint32_t addr, uint32_t piece_bytes
                     upper_halves(r[6], r[7]));
     }
 }
+// Four consecutive k of a row, half a 16-byte unit.
+template <int PIECES = 3>
+__device__ __forceinline__ void split_store4(uint32_t addr, uint32_t piece_bytes, const float* x) {
+    float r[4] = {x[0], x[1], x[2], x[3]};
+#pragma unroll
+    for (int t = 0; t < PIECES; ++t) {
+        asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr + t * piece_bytes), "r"(upper_halves(r[0], r[1])), "r"(upper_halves(r[2], r[3]))
+                     : "memory");
+#pragma unroll
+        for (int i = 0; i < 4; ++i) r[i] = lower_part(r[i]);
+    }
+}
+__device__ __forceinline__ uint32_t half_unit_offset(int row, int half) {
+    return uint32_t(row * 64 + (((half >> 1) ^ ((row >> 1) & 3)) << 4) + (half & 1) * 8);
+}
 __device__ __forceinline__ uint32_t unit_offset(int row, int unit) { return uint32_t(row * 64 + ((unit ^ ((row >> 1) & 3)) << 4)); }
 
 // Shared-memory matrix descriptor of such a tile: K-major, 64-byte swizzle (layout 4), 512 bytes between groups of eight rows.
@@ -80,6 +95,26 @@ __device__ __forceinline__ void mma_six(uint32_t d, const uint32_t (&stage)[2], 
 __device__ __forceinline__ float load1(const float* p) { return __ldg(p); }
 __device__ __forceinline__ float load1(const __nv_bfloat16* p) {
     return __uint_as_float(uint32_t(__ldg(reinterpret_cast<const unsigned short*>(p))) << 16);
+}
+// Four consecutive elements from `at`, as f32, under the rules of load8 (vec: one aligned load).
+__device__ __forceinline__ void load4(float* x, const float* at, bool there, int left, bool vec) {
+    if (there && vec && left >= 4) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(at));
+        x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = there && i < left ? load1(at + i) : 0.f;
+    }
+}
+__device__ __forceinline__ void load4(float* x, const __nv_bfloat16* at, bool there, int left, bool vec) {
+    if (there && vec && left >= 4) {
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(at));
+        x[0] = __uint_as_float(v.x << 16), x[1] = __uint_as_float(v.x & 0xffff0000u);
+        x[2] = __uint_as_float(v.y << 16), x[3] = __uint_as_float(v.y & 0xffff0000u);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = there && i < left ? load1(at + i) : 0.f;
+    }
 }
 // Eight consecutive elements from `at`, as f32: `left` of them exist (zeros for the rest), none where the row is not there. vec:
 // `at` is 16-byte aligned.

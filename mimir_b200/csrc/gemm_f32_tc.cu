@@ -55,7 +55,7 @@ struct Bars {
 
 // A convolution as a contraction: row = output pixel (image, oh, ow), k = (input channel, kh, kw), column = filter. Rows of the
 // patch matrix are gathered from the image as the loaders read them.
-// tap_major (channels a multiple of 8): k = (kh, kw, input channel) instead, so that the eight k of a unit share one tap: one test
+// tap_major (channels a multiple of 8): k = (kh, kw, input channel) instead, in the filters too, so that the eight k of a unit share one tap: one test
 // whether it lies inside, and addresses a plane apart. With k in the order of the filters, every element has its own tap and
 // test: 16 x 128 x 56 x 56, 128 filters of 3 x 3: 207 us.
 struct ConvShape {
@@ -133,12 +133,14 @@ __device__ __noinline__ float scalar_fold(const Params& p, int64_t bz, int64_t r
         const int64_t img = row / pixels;
         const int y = int(row - img * pixels) / cv.ow, x = int(row - img * pixels) - y * cv.ow;
         const TIn* im = A + img * (int64_t(cv.cin) * cv.h * cv.w);
-        const TIn* wt = B + col * p.K;
+        const int taps = cv.kh * cv.kw;
         for (int ci = 0; ci < cv.cin; ++ci)
             for (int kr = 0; kr < cv.kh; ++kr)
-                for (int kq = 0; kq < cv.kw; ++kq, ++wt) {
+                for (int kq = 0; kq < cv.kw; ++kq) {
                     const int iy = y * cv.stride_h - cv.pad_h + kr * cv.dil_h, ix = x * cv.stride_w - cv.pad_w + kq * cv.dil_w;
                     const bool in = unsigned(iy) < unsigned(cv.h) && unsigned(ix) < unsigned(cv.w);
+                    const int tap = kr * cv.kw + kq;
+                    const TIn* wt = B + col * p.K + (cv.tap_major ? tap * cv.cin + ci : ci * taps + tap);
                     v = fmaf(in ? load1(im + (int64_t(ci) * cv.h + iy) * cv.w + ix) : 0.f, load1(wt), v);
                 }
     } else {
@@ -191,30 +193,30 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
     // this CTA's accumulators stay in tensor memory to the end and leave one by one, or are added up as they are finished
     const bool hold = p.split > 1 && per <= C::SLOTS;
 
-    // A thread's part of a k-block: an eight-k unit of A and at most one of B. Where memory runs along k a unit's row is tid / 4;
-    // where it runs along the rows (B stored [K, N], the pixels of an image) a warp takes one unit of 32 neighbouring rows.
-    const int across = (warp >> 2) * 32 + lane, along = tid >> 2, unit = warp & 3;
-    const int a_row = CONV ? across : along, a_unit = CONV ? unit : tid & 3;
-    const int b_row = p.b_nk ? along : across, b_unit = p.b_nk ? tid & 3 : unit;
-    const bool has_b = BN == 128 || tid < BN * 4, a_there = m0 + a_row < p.M, b_there = n0 + b_row < p.N;
+    // A thread's part of a k-block. Where memory runs along k: four k of one or two rows 64 apart, eight lanes to a row's 128
+    // bytes. Where it runs along the rows (B stored [K, N], the pixels of an image): eight k of one row, a warp's lanes on
+    // neighbouring rows.
+    const int across = (warp >> 2) * 32 + lane, unit = warp & 3, along = tid >> 3, half = tid & 7;
+    constexpr int NB = BN / 64;
+    const bool has_b = BN == 128 || p.b_nk || tid < BN * 4;
     float fa[8], fb[8];
-    const TIn* a_at;                // CONV: the first tap of the pixel's window; else the thread's row of A, at its unit
-    const TIn* b_at = p.b_nk ? B + (n0 + b_row) * p.K + b_unit * 8 : B + int64_t(b_unit * 8) * p.N + n0 + b_row;
+    const TIn* a_at;                // CONV: the first tap of the pixel's window; else the thread's first row of A
+    const TIn* b_at = p.b_nk ? B + (n0 + along) * p.K + half * 4 : B + int64_t(unit * 8) * p.N + n0 + across;
     int rows_in = 0, cols_in = 0;   // CONV: bit i: tap row / column i of this pixel lies inside the image
     const ConvShape& cv = p.conv;
     if (CONV) {
-        const int64_t row = m0 + a_row;
+        const int64_t row = m0 + across;
         const int pixels  = cv.oh * cv.ow;
         const int64_t img = row / pixels;
         const int pix = int(row - img * pixels), y = pix / cv.ow;
         const int ih0 = y * cv.stride_h - cv.pad_h, iw0 = (pix - y * cv.ow) * cv.stride_w - cv.pad_w;
         a_at = A + img * (int64_t(cv.cin) * cv.h * cv.w) + (int64_t(ih0) * cv.w + iw0);  // only taps inside are read
-        if (a_there) {
+        if (row < p.M) {
             for (int r = 0; r < cv.kh; ++r) rows_in |= int(unsigned(ih0 + r * cv.dil_h) < unsigned(cv.h)) << r;
             for (int q = 0; q < cv.kw; ++q) cols_in |= int(unsigned(iw0 + q * cv.dil_w) < unsigned(cv.w)) << q;
         }
     } else {
-        a_at = A + (m0 + a_row) * p.K + a_unit * 8;
+        a_at = A + (m0 + along) * p.K + half * 4;
     }
     auto fetch_a = [&](int kb) {
         const int64_t k0 = int64_t(kb) * BK;
@@ -244,24 +246,40 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
                 }
             }
         } else {
-            load8(fa, a_at + k0, a_there, int(p.K - k0) - a_unit * 8, p.vec_a);
+            const int left = int(p.K - k0) - half * 4;
+            load4(fa, a_at + k0, m0 + along < p.M, left, p.vec_a);
+            load4(fa + 4, a_at + k0 + 64 * p.K, m0 + along + 64 < p.M, left, p.vec_a);
         }
     };
     auto fetch_b = [&](int kb) {
         if (!has_b) return;
         const int64_t k0 = int64_t(kb) * BK;
-        const int left   = int(p.K - k0) - b_unit * 8;
-        if (CONV && cv.tap_major) {  // the filters are stored (input channel, kh, kw)
-            const int k = int(k0) + b_unit * 8, tap = k / cv.cin, taps = cv.kh * cv.kw;
-            const TIn* at = B + (n0 + b_row) * p.K + int64_t(k - tap * cv.cin) * taps + tap;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) fb[j] = b_there && left > 0 ? load1(at + j * taps) : 0.f;
-        } else if (p.b_nk) {
-            load8(fb, b_at + k0, b_there, left, p.vec_b);
+        if (p.b_nk) {
+            const int left = int(p.K - k0) - half * 4;
+            load4(fb, b_at + k0, n0 + along < p.N, left, p.vec_b);
+            if (NB == 2) load4(fb + 4, b_at + k0 + 64 * p.K, n0 + along + 64 < p.N, left, p.vec_b);
         } else {
-            const TIn* at = b_at + k0 * p.N;
+            const TIn* at  = b_at + k0 * p.N;
+            const int left = int(p.K - k0) - unit * 8;
+            const bool in  = n0 + across < p.N;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) fb[j] = b_there && j < left ? load1(at + j * p.N) : 0.f;
+            for (int j = 0; j < 8; ++j) fb[j] = in && j < left ? load1(at + j * p.N) : 0.f;
+        }
+    };
+    auto store_a = [&](uint32_t at) {
+        if (CONV) {
+            split_store8<PIECES>(at + unit_offset(across, unit), A_PIECE, fa);
+        } else {
+            split_store4<PIECES>(at + half_unit_offset(along, half), A_PIECE, fa);
+            split_store4<PIECES>(at + half_unit_offset(along + 64, half), A_PIECE, fa + 4);
+        }
+    };
+    auto store_b = [&](uint32_t at) {
+        if (p.b_nk) {
+            split_store4<PIECES>(at + half_unit_offset(along, half), C::B_PIECE, fb);
+            if (NB == 2) split_store4<PIECES>(at + half_unit_offset(along + 64, half), C::B_PIECE, fb + 4);
+        } else if (has_b) {
+            split_store8<PIECES>(at + unit_offset(across, unit), C::B_PIECE, fb);
         }
     };
     if (warp < MMA_WARP && kb0 < kb1) {  // on their way while the barriers and the tensor memory are set up
@@ -343,9 +361,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
         for (int kb = kb0; kb < kb1; ++kb) {
             if (!(ok = warp_wait(smem_u32(&bars->empty[stage]), phase ^ 1u, abort_flag))) break;
             const uint32_t s0 = base + stage * C::STAGE_BYTES;
-            split_store8<PIECES>(s0 + unit_offset(a_row, a_unit), A_PIECE, fa);
+            store_a(s0);
             if (kb + 1 < kb1) fetch_a(kb + 1);
-            if (has_b) split_store8<PIECES>(s0 + PIECES * A_PIECE + unit_offset(b_row, b_unit), C::B_PIECE, fb);
+            store_b(s0 + PIECES * A_PIECE);
             if (kb + 1 < kb1) fetch_b(kb + 1);
             fence_proxy_async_smem();  // the MMA reads shared memory through the async proxy
             __syncwarp();
@@ -504,7 +522,7 @@ int conv_tc(const mimk_conv_desc& d, cudaStream_t s) {
     p.A = d.x, p.B = d.filters, p.C = d.out;
     p.M = d.n * oh * ow, p.N = d.cout, p.K = d.cin * d.kh * d.kw;
     p.conv = ConvShape{int(d.cin), int(d.h), int(d.w), int(d.kh), int(d.kw), int(oh), int(ow), int(d.stride_h), int(d.stride_w),
-                       int(d.dil_h), int(d.dil_w), int(d.pad_h), int(d.pad_w), d.cin % 8 == 0 && d.kh * d.kw > 1};
+                       int(d.dil_h), int(d.dil_w), int(d.pad_h), int(d.pad_w), d.by_tap};
     p.b_nk   = 1;
     p.vec_b  = p.K % (d.dtype == MIMK_F32 ? 4 : 8) == 0 && aligned16(d.filters);
     p.status = dev->status_dev;

@@ -698,6 +698,9 @@ def conv(x: torch.Tensor, w: torch.Tensor, stride=(1, 1), dilation=(1, 1), paddi
         x, w = x.contiguous(), w.contiguous()
         out = torch.empty((n, cout, oh, ow), dtype=x.dtype, device=x.device)
         d = L.ConvDesc()
+        d.by_tap = cin % 8 == 0 and kh * kw > 1
+        if d.by_tap:
+            w = transpose(w.view(cout, cin, kh * kw), (0, 2, 1))
         d.n, d.cin, d.h, d.w, d.cout, d.kh, d.kw = n, cin, h, wd, cout, kh, kw
         d.stride_h, d.stride_w, d.dil_h, d.dil_w, d.pad_h, d.pad_w = *stride, *dilation, *padding
         d.x, d.filters, d.out, d.dtype = x.data_ptr(), w.data_ptr(), out.data_ptr(), _dt(x)
