@@ -16,8 +16,6 @@
 // shared-memory bandwidth (a k-block of 128 x 128 moves 96 KB into the MMA and 48 KB from the loaders; measured 100 clocks per
 // instruction of 64 clocks' arithmetic) next to the loaders' instructions. Too few tiles for the chip: the accumulators of one
 // tile are dealt out to a cluster of two, four or eight CTAs, which exchange them through distributed shared memory.
-#include <cstdlib>
-
 #include "common.cuh"
 #include "f32_split.cuh"
 #include "sm100.cuh"
@@ -462,7 +460,9 @@ int launch(const Params& p, int64_t ctas, cudaStream_t s) {
 }
 
 // Tile width and split: the pair with the least estimated time, rounds * (fixed + k-blocks per CTA * per k-block), a round being
-// the tiles that are on the chip at once (one CTA per SM; clusters of eight and four leave SMs of a partly filled GPC idle).
+// the tiles that are on the chip at once: one CTA per SM; clusters leave SMs of a partly filled group idle (15 of eight were on
+// the chip at once, 16 took two rounds; of four 32). Measured per k-block: 1.15 us (128 wide), 0.95 (64); fixed 8 us, 9 with the
+// exchange. 1000^3: 128 wide split 2, 29 us (128 / 1: 48, 64 / 1: 40); 300 x 300 x 3000: 64 wide split 8, 20 (64 / 1: 99).
 template <class TIn, class TOut, bool CONV>
 int plan_and_launch(Params& p, int64_t batch, int sm_count, cudaStream_t s) {
     p.tiles_m = (p.M + BM - 1) / BM;
@@ -472,13 +472,11 @@ int plan_and_launch(Params& p, int64_t batch, int sm_count, cudaStream_t s) {
     p.split     = 1;
     for (int wide = 0; wide < 2; ++wide)
         for (int split = 1; split <= 8 && split <= chunks; split *= 2) {
-            if (getenv("SW_BN") && atoi(getenv("SW_BN")) != (wide ? 128 : 64)) continue;
-            if (getenv("SW_SPLIT") && atoi(getenv("SW_SPLIT")) != split) continue;
             const int64_t items = p.tiles_m * ((p.N + (wide ? 127 : 63)) / (wide ? 128 : 64)) * batch;
-            const int64_t room  = split == 1 ? sm_count : split == 2 ? sm_count / 2 - 4 : split == 4 ? sm_count / 4 - 5 : sm_count / 8 - 4;
+            const int64_t room  = split == 1 ? sm_count : split == 2 ? sm_count / 2 - 4 : split == 4 ? sm_count / 4 - 5 : sm_count / 8 - 3;
             const double rounds = double((items + room - 1) / room);
             const int per       = (chunks + split - 1) / split * CHUNK;
-            const double time   = rounds * ((split > 1 ? 6.0 : 4.0) + (per < kb ? per : kb) * (wide ? 0.7 : 0.5));
+            const double time   = rounds * ((split > 1 ? 9.0 : 8.0) + (per < kb ? per : kb) * (wide ? 1.15 : 0.95));
             if (time < best) best = time, bn = wide ? 128 : 64, p.split = split;
         }
     p.tiles_n = (p.N + bn - 1) / bn;
