@@ -334,6 +334,17 @@ int attn_few_supported(const mimk_attn_desc& d) {
     return aligned16(d.q) && aligned16(d.k) && aligned16(d.v);
 }
 
+// The 128-row kernel gives each SM a head and at head_dim 128 streams it as fast as eight warps here do, so where its rounds of
+// heads leave few SMs idle it is ahead: 128 heads x 4096: 55.5 / 60.8 us; 256 x 8192: 202 / 215. Not so 64 x 1000: 18.1 / 17.3, or
+// at head_dim 64 (256 x 8192: 175 / 109).
+int attn_heads_fill(const mimk_attn_desc& d) {
+    int st          = MIMK_OK;
+    DeviceInfo* dev = device_info(&st);
+    if (!dev || d.head_dim != 128) return 0;
+    const int64_t rounds = (d.batch_heads + dev->sm_count - 1) / dev->sm_count;
+    return d.batch_heads * 5 >= rounds * dev->sm_count * 4;
+}
+
 int attn_few(const mimk_attn_desc& d, cudaStream_t s) {
     int st          = MIMK_OK;
     DeviceInfo* dev = device_info(&st);

@@ -16,6 +16,8 @@
 // shared-memory bandwidth (a k-block of 128 x 128 moves 96 KB into the MMA and 48 KB from the loaders; measured 100 clocks per
 // instruction of 64 clocks' arithmetic) next to the loaders' instructions. Too few tiles for the chip: the accumulators of one
 // tile are dealt out to a cluster of two, four or eight CTAs, which exchange them through distributed shared memory.
+#include <type_traits>
+
 #include "common.cuh"
 #include "f32_split.cuh"
 #include "sm100.cuh"
@@ -308,7 +310,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
             const uint32_t idesc = idesc_bf16_f32(BM, BN, 0, 0);
             uint32_t stage = 0, phase = 0;
             for (int kb = kb0, c = 0; kb < kb1; kb += CHUNK, ++c) {
-                // A full stage also says that every warp has added up the chunk three before this one, so an accumulator is free
+                // A full stage also says that every warp has added up the chunk four before this one, so an accumulator is free
                 // when its turn comes again.
                 uint32_t at[CHUNK], empty[CHUNK];
                 const int n = kb1 - kb < CHUNK ? kb1 - kb : CHUNK;
@@ -331,33 +333,30 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
         }
         __syncwarp();
     } else {
-        static_assert(CHUNK == 2 && STAGES == 2 * CHUNK && C::NACC >= 3, "see the waits of the MMA warp");
+        static_assert(CHUNK == 2 && STAGES == 2 * CHUNK && C::NACC >= 4, "see the waits of the MMA warp");
         constexpr int COLS = BN / 4;  // accumulator columns per warp
         const uint32_t quarter = uint32_t(warp & 3), col0 = uint32_t(warp >> 2) * COLS, lanes = (quarter * 32u) << 16;
         float sum[COLS];
 #pragma unroll
         for (int i = 0; i < COLS; ++i) sum[i] = 0.f;
-        auto take = [&](int c, uint32_t (&r)[COLS]) {  // this CTA's chunk c
-            const uint32_t acc = uint32_t(c) % C::NACC;
-            if (!warp_wait(smem_u32(&bars->acc_full[acc]), uint32_t(c / C::NACC) & 1u, abort_flag)) return false;
+        // sixteen columns, from `h` on, of this CTA's chunk c; the registers are valid after tmem_ld_wait
+        auto ready   = [&](int c) {
+            const bool ok = warp_wait(smem_u32(&bars->acc_full[uint32_t(c) % C::NACC]), uint32_t(c / C::NACC) & 1u, abort_flag);
             tc_fence_after();
-            tmem_ld_cols(tmem_base + acc * BN + col0 + lanes, r);
+            return ok;
+        };
+        auto request = [&](int c, int h, uint32_t (&r)[16]) { tmem_ld_32x16(tmem_base + uint32_t(c) % C::NACC * BN + col0 + lanes + h, r); };
+        auto add     = [&](auto h, const uint32_t (&r)[16]) {
             tmem_ld_wait();
-            tc_fence_before();
-            return true;
-        };
-        auto add = [&](int c) {
-            uint32_t r[COLS];
-            if (!take(c, r)) return false;
 #pragma unroll
-            for (int i = 0; i < COLS; ++i) sum[i] += __uint_as_float(r[i]);
-            return true;
+            for (int i = 0; i < 16; ++i) sum[decltype(h)::value + i] += __uint_as_float(r[i]);
+            tc_fence_before();
         };
+        using First  = std::integral_constant<int, 0>;
+        using Second = std::integral_constant<int, COLS == 32 ? 16 : 0>;
         uint32_t stage = 0, phase = 0;
-        bool ok   = true;
-        int added = 0;
-        for (int kb = kb0; kb < kb1; ++kb) {
-            if (!(ok = warp_wait(smem_u32(&bars->empty[stage]), phase ^ 1u, abort_flag))) break;
+        auto load_block = [&](int kb) {
+            if (!warp_wait(smem_u32(&bars->empty[stage]), phase ^ 1u, abort_flag)) return false;
             const uint32_t s0 = base + stage * C::STAGE_BYTES;
             store_a(s0);
             if (kb + 1 < kb1) fetch_a(kb + 1);
@@ -367,9 +366,23 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bars->full[stage]));
             if (++stage == STAGES) stage = 0, phase ^= 1u;
-            // two chunks before this one: with four stages its MMAs are complete by now
-            if (!hold && (kb - kb0) % CHUNK == CHUNK - 1 && kb - kb0 >= 3 * CHUNK - 1)
-                if (!(ok = add(added++))) break;
+            return true;
+        };
+        bool ok   = true;
+        int added = 0;
+        for (int c = 0; c < ch1 - ch0; ++c) {
+            // A read of tensor memory waits behind the MMAs in the queue (about 1200 clocks), so it is requested before a block is
+            // loaded and added after it. The chunk three before this one is complete: of its blocks' stages this one's take over.
+            uint32_t r[16];
+            const bool due = !hold && c >= 3, second = kb0 + c * CHUNK + 1 < kb1;
+            if (!(ok = !due || ready(added))) break;
+            if (due) request(added, 0, r);
+            if (!(ok = load_block(kb0 + c * CHUNK))) break;
+            if (due) add(First{}, r);
+            if (COLS == 32 && due) request(added, 16, r);
+            if (second && !(ok = load_block(kb0 + c * CHUNK + 1))) break;
+            if (COLS == 32 && due) add(Second{}, r);
+            added += due;
         }
         auto part = [&](int slot, const float (&x)[COLS]) {
             const uint32_t a = base + slot * C::PART_BYTES + (uint32_t(quarter * 32 + lane) * C::PITCH + col0) * 4;
@@ -379,16 +392,27 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
         };
         // Once the last chunk is finished every MMA of this CTA is complete, and the stages become its partial tiles.
         if (hold) {
-            uint32_t r[COLS];
-            if (ok && ch1 > ch0) ok = take(ch1 - ch0 - 1, r);
+            if (ok && ch1 > ch0) ok = ready(ch1 - ch0 - 1);
             for (int c = 0; c < ch1 - ch0 && ok; ++c) {
-                if (!(ok = take(c, r))) break;
+                if (!(ok = ready(c))) break;
+                uint32_t r[COLS];
+                tmem_ld_cols(tmem_base + uint32_t(c) % C::NACC * BN + col0 + lanes, r);
+                tmem_ld_wait();
 #pragma unroll
                 for (int i = 0; i < COLS; ++i) sum[i] = __uint_as_float(r[i]);
                 part(c, sum);
             }
         } else {
-            for (; added < ch1 - ch0 && ok; ++added) ok = add(added);
+            for (; added < ch1 - ch0 && ok; ++added) {
+                if (!(ok = ready(added))) break;
+                uint32_t r[16];
+                request(added, 0, r);
+                add(First{}, r);
+                if (COLS == 32) {
+                    request(added, 16, r);
+                    add(Second{}, r);
+                }
+            }
             part(0, sum);
         }
     }
