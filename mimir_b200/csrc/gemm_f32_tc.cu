@@ -371,17 +371,33 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
         bool ok   = true;
         int added = 0;
         for (int c = 0; c < ch1 - ch0; ++c) {
-            // A read of tensor memory waits behind the MMAs in the queue (about 1200 clocks), so it is requested before a block is
-            // loaded and added after it. The chunk three before this one is complete: of its blocks' stages this one's take over.
-            uint32_t r[16];
-            const bool due = !hold && c >= 3, second = kb0 + c * CHUNK + 1 < kb1;
-            if (!(ok = !due || ready(added))) break;
-            if (due) request(added, 0, r);
-            if (!(ok = load_block(kb0 + c * CHUNK))) break;
-            if (due) add(First{}, r);
-            if (COLS == 32 && due) request(added, 16, r);
-            if (second && !(ok = load_block(kb0 + c * CHUNK + 1))) break;
-            if (COLS == 32 && due) add(Second{}, r);
+            // A read of tensor memory waits behind the MMAs in the queue (about 1200 clocks). Where the loaders wait for memory too
+            // (an image's patches), it is requested before a block is loaded and added after it (16 x 128 x 56 x 56, 128 filters of
+            // 3 x 3: 241 -> 201 us; bf16 248 -> 279, 2048^3 163 -> 170, so not there). The chunk read is complete: its stages are in use again.
+            constexpr bool EARLY = CONV && PIECES == 3;
+            const int kb = kb0 + c * CHUNK;
+            const bool due = !hold && c >= (EARLY ? 3 : 2), second = kb + 1 < kb1;
+            if constexpr (EARLY) {
+                uint32_t r[16];
+                if (!(ok = !due || ready(added))) break;
+                if (due) request(added, 0, r);
+                if (!(ok = load_block(kb))) break;
+                if (due) add(First{}, r);
+                if (COLS == 32 && due) request(added, 16, r);
+                if (second && !(ok = load_block(kb + 1))) break;
+                if (COLS == 32 && due) add(Second{}, r);
+            } else {
+                if (!(ok = load_block(kb) && (!second || load_block(kb + 1)))) break;
+                if (due) {
+                    uint32_t r[COLS];
+                    if (!(ok = ready(added))) break;
+                    tmem_ld_cols(tmem_base + uint32_t(added) % C::NACC * BN + col0 + lanes, r);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < COLS; ++i) sum[i] += __uint_as_float(r[i]);
+                    tc_fence_before();
+                }
+            }
             added += due;
         }
         auto part = [&](int slot, const float (&x)[COLS]) {
