@@ -663,6 +663,11 @@ def _mrp_into(out, Sr, f, init, post, map_out, maps, ins):
 # and for integers, as ONE map_reduce_post on the per-cell kernel, which keeps the reference's ascending fold per output cell
 # bit for bit.
 CONV_CONTRACTION_MIN_WORK = 1 << 27
+# A bf16 patch matrix is worth writing where the contraction is long enough for the full-rate kernels (they take extents that are
+# multiples of 8): 16 x 128 x 56 x 56, 128 filters of 3 x 3 (2^32.8), 193 us against 240 gathered; 32 x 32 x 112 x 112, 32 filters
+# (2^31.8), 427 against 339.
+CONV_PATCH_MIN_WORK = 1 << 32
+_CONV_PATCH_BYTES = 1 << 30   # patches of at most this many bytes at a time (whole images per piece)
 
 
 def _conv_on_tensor_cores(dtype, n, cin, cout, kh, kw, oh, ow) -> bool:
@@ -681,6 +686,33 @@ def _conv_indexable(x, w, oh, ow, stride, dilation, padding) -> bool:
                     *stride) < 1 << 30)
 
 
+def _conv_as_contraction(xp, w, n, cin, cout, kh, kw, oh, ow, stride, dilation) -> torch.Tensor:
+    """conv as patches x weights: P[(n, oh, ow), (ci, kh, kw)] = xp[n, ci, oh*s + kh*d, ow*s + kw*d] gathered by one copy
+    operation (the read map conv_impl builds, tensor.mim:1254-1282, with the reduction loops turned into axes), then
+    P . W^T on the contraction kernels with W read through transpose_2d, then the channel axis moved forward by the tiled
+    permutation copy."""
+    k = cin * kh * kw
+    esize = xp.element_size()
+    per_image = oh * ow * k * esize
+    step = max(1, min(n, _CONV_PATCH_BYTES // max(per_image, 1)))
+    w2 = w.contiguous().view(cout, k)
+    out = torch.empty((n, cout, oh, ow), dtype=xp.dtype, device=xp.device)
+    # loops: 0 n, 1 oh, 2 ow, 3 ci, 4 kh, 5 kw
+    mi = [[0] * 7 for _ in range(4)]
+    mi[0][0] = 1
+    mi[1][3] = 1
+    mi[2][1], mi[2][4] = stride[0], dilation[0]
+    mi[3][2], mi[3][5] = stride[1], dilation[1]
+    for n0 in range(0, n, step):
+        nb = min(step, n - n0)
+        shape = (nb, oh, ow, cin, kh, kw)
+        patches = map_reduce_post(shape, shape, L.F_FIRST, 0.0, L.P_ID, id_map(6), [mi], [xp[n0:n0 + nb].contiguous()],
+                                  acc_dtype=torch.float32, out_dtype=xp.dtype)
+        y = product_2d(patches.view(nb * oh * ow, k), transpose_2d(w2))          # [(n, oh, ow), cout]
+        out[n0:n0 + nb] = transpose(y.view(nb, oh, ow, cout), (0, 3, 1, 2))
+    return out
+
+
 def conv(x: torch.Tensor, w: torch.Tensor, stride=(1, 1), dilation=(1, 1), padding=(0, 0)) -> torch.Tensor:
     """`conv R (stride, dilation, padding) (input, weight)`: NCHW input, [Cout, Cin, KH, KW] weight (tensor.mim:434-438).
     Loop vector (n, co, oh, ow, ci, kh, kw); the input is read at (n, ci, oh*s + kh*d, ow*s + kw*d) of the padded tensor
@@ -695,6 +727,10 @@ def conv(x: torch.Tensor, w: torch.Tensor, stride=(1, 1), dilation=(1, 1), paddi
     if _conv_on_tensor_cores(x.dtype, n, cin, cout, kh, kw, oh, ow) and _conv_indexable(x, w, oh, ow, stride, dilation, padding):
         if x.dtype != w.dtype:
             raise TypeError("conv: both operands share the ring's element type")
+        k = cin * kh * kw
+        if x.dtype == torch.bfloat16 and k % 8 == 0 and cout % 8 == 0 and n * cout * oh * ow * k >= CONV_PATCH_MIN_WORK:
+            xp = pad(x, (0, 0, padding[0], padding[1]), (0, 0, padding[0], padding[1])) if any(padding) else x
+            return _conv_as_contraction(xp, w, n, cin, cout, kh, kw, oh, ow, stride, dilation)
         x, w = x.contiguous(), w.contiguous()
         out = torch.empty((n, cout, oh, ow), dtype=x.dtype, device=x.device)
         d = L.ConvDesc()
