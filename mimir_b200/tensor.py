@@ -671,8 +671,15 @@ _CONV_PATCH_BYTES = 1 << 30   # patches of at most this many bytes at a time (wh
 
 
 def _conv_on_tensor_cores(dtype, n, cin, cout, kh, kw, oh, ow) -> bool:
-    return (dtype in (torch.float32, torch.bfloat16) and cout >= 16 and n * oh * ow >= 128
-            and n * cout * oh * ow * cin * kh * kw >= CONV_CONTRACTION_MIN_WORK)
+    k = cin * kh * kw
+    if dtype not in (torch.float32, torch.bfloat16) or n * cout * oh * ow * k < CONV_CONTRACTION_MIN_WORK:
+        return False
+    return (cout >= 16 and n * oh * ow >= 128) or (dtype == torch.bfloat16 and _whole_tiles(k, cout))
+
+
+def _whole_tiles(k, cout) -> bool:
+    """Extents the full-rate bf16 contraction takes as they are."""
+    return k % 8 == 0 and cout % 8 == 0
 
 
 def _conv_indexable(x, w, oh, ow, stride, dilation, padding) -> bool:
@@ -724,11 +731,14 @@ def conv(x: torch.Tensor, w: torch.Tensor, stride=(1, 1), dilation=(1, 1), paddi
         raise ValueError("contracting dims don't match")
     oh = (h + 2 * padding[0] - dilation[0] * (kh - 1) - 1) // stride[0] + 1
     ow = (wd + 2 * padding[1] - dilation[1] * (kw - 1) - 1) // stride[1] + 1
-    if _conv_on_tensor_cores(x.dtype, n, cin, cout, kh, kw, oh, ow) and _conv_indexable(x, w, oh, ow, stride, dilation, padding):
-        if x.dtype != w.dtype:
+    k = cin * kh * kw
+    contraction = _conv_on_tensor_cores(x.dtype, n, cin, cout, kh, kw, oh, ow) and _conv_indexable(x, w, oh, ow, stride, dilation, padding)
+    if contraction and x.dtype != w.dtype:
+        if x.dtype == torch.float32 or _whole_tiles(k, cout):
             raise TypeError("conv: both operands share the ring's element type")
-        k = cin * kh * kw
-        if x.dtype == torch.bfloat16 and k % 8 == 0 and cout % 8 == 0 and n * cout * oh * ow * k >= CONV_PATCH_MIN_WORK:
+        contraction = False   # the per-cell kernel takes operands of two element types
+    if contraction:
+        if x.dtype == torch.bfloat16 and _whole_tiles(k, cout) and n * cout * oh * ow * k >= CONV_PATCH_MIN_WORK:
             xp = pad(x, (0, 0, padding[0], padding[1]), (0, 0, padding[0], padding[1])) if any(padding) else x
             return _conv_as_contraction(xp, w, n, cin, cout, kh, kw, oh, ow, stride, dilation)
         x, w = x.contiguous(), w.contiguous()
