@@ -1,7 +1,7 @@
-// Attention at sizes where one warp per query row is far too slow and the fused tensor-core kernels do not apply (f32;
-// bf16 with a head_dim other than 64 / 128): the reference's own composition `softmax (q * transpose_2d k) * v`
+// Attention at sizes where one warp per query row is far too slow and the fused tensor-core kernels do not apply (f32 beyond
+// head_dim 128; bf16 with a head_dim other than 64 / 128): the reference's own composition `softmax (q * transpose_2d k) * v`
 // (MimIR lit/tensor/attn_exec.mim:20-22), stage by stage, on this library's kernels.
-//   S = Q K^T      batched contraction on the tensor cores, f32 result (f32 operands: three TF32 products per term)
+//   S = Q K^T      batched contraction on the tensor cores, f32 result (f32 operands: gemm_f32_tc.cu, gemm_tf32.cu)
 //   S = mask(scale * S), in place
 //   P = softmax rows of S (f32 in place; bf16 operands: P stored as bf16 beside S), one pass over HBM
 //   O = P V        batched contraction
@@ -128,7 +128,7 @@ int attn_composed(const mimk_attn_desc& d, cudaStream_t s) {
     const int64_t es       = half ? 2 : 4;
     const int64_t per_head = d.seq_q * d.seq_k;
     int64_t group = MAX_SCORE_BYTES / (per_head * (half ? 6 : 4));
-    if (group > 16) group = 16;  // the f32 tensor-core contraction takes batches of up to 16
+    if (group > 16) group = 16;  // the TF32 contraction takes batches of up to 16
     if (group > d.batch_heads) group = d.batch_heads;
     void* scratch = nullptr;
     MIMK_TRY(get_aux_scratch(size_t(group * per_head) * (half ? 6 : 4), &scratch, s));

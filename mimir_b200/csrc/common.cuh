@@ -59,7 +59,7 @@ inline size_t dtype_size(int dt) { return dt == MIMK_BF16 ? 2 : (dt == MIMK_I64 
 
 // kernels implemented in the other translation units
 int gemm_simt(const mimk_gemm_desc& d, cudaStream_t s);
-int gemm_simt_preferred(const mimk_gemm_desc& d);  // small f32 product: the 32 x 32-tile CUDA-core kernel beats 3xTF32
+int gemm_simt_preferred(const mimk_gemm_desc& d);  // f32 products the CUDA cores are ahead on
 int gemm_tc_supported(const mimk_gemm_desc& d);
 // a_panels > 1: A is given as that many row-major [m, k / a_panels] matrices one after another (the layout an all-gather
 // of column slabs delivers); k / a_panels must then be a multiple of 64
@@ -82,6 +82,9 @@ int gemm_tc_any(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* 
                 const mimk_gather_dst* gather = nullptr, int64_t a_panels = 1);  // picks between the two
 int gemm_f32_tc_supported(const mimk_gemm_desc& d);  // f32 operands on the tensor cores (three bf16 pieces each)
 int gemm_f32_tc(const mimk_gemm_desc& d, cudaStream_t s);
+// results with many tiles: the operands cut beforehand, three TF32 products (gemm_tf32.cu)
+int gemm_tf32_preferred(const mimk_gemm_desc& d, int sm_count, double pieces_us);
+int gemm_tf32(const mimk_gemm_desc& d, cudaStream_t s);
 int conv_tc(const mimk_conv_desc& d, cudaStream_t s);  // the same kernel, its left operand gathered from an image
 // map_reduce_post instances that are a contraction, an axis fold or an elementwise map go to those kernels (mrp_route.cu)
 bool mrp_try_route(const mimk_mrp_desc& d, void* stream, int* status);
@@ -117,11 +120,10 @@ MrpPlan mrp_plan(const mimk_mrp_desc& d);
 // axis permutation as a tiled copy (permute.cu); perm[j] = the output loop that indexes input axis j
 int permute_copy(const void* in, void* out, int esize, int rank, const int64_t* out_shape, const int* perm, cudaStream_t s);
 int attn_simt(const mimk_attn_desc& d, cudaStream_t s);
-// f32, and bf16 with other head dims, at scale: the composition S = Q K^T, softmax, O = P V on the contraction and row
 // f32, head_dim up to 128: fused, on the tensor cores, three bf16 pieces per value (attn_f32_tc.cu)
 int attn_f32_tc_supported(const mimk_attn_desc& d);
 int attn_f32_tc(const mimk_attn_desc& d, cudaStream_t s);
-// kernels (attn_composed.cu)
+// other head dims at scale: the composition S = Q K^T, softmax, O = P V on the contraction and row kernels (attn_composed.cu)
 int attn_composed_supported(const mimk_attn_desc& d);
 int attn_composed(const mimk_attn_desc& d, cudaStream_t s);
 // bf16, head_dim 64 or 128, up to 16 query rows: streams K and V once (attn_few.cu)

@@ -503,25 +503,32 @@ int launch(const Params& p, int64_t ctas, cudaStream_t s) {
 // the tiles that are on the chip at once: one CTA per SM; clusters leave SMs of a partly filled group idle (15 of eight were on
 // the chip at once, 16 took two rounds; of four 32). Measured per k-block: 1.15 us (128 wide), 0.95 (64); fixed 8 us, 9 with the
 // exchange. 1000^3: 128 wide split 2, 29 us (128 / 1: 48, 64 / 1: 40); 300 x 300 x 3000: 64 wide split 8, 20 (64 / 1: 99).
-template <class TIn, class TOut, bool CONV>
-int plan_and_launch(Params& p, int64_t batch, int sm_count, cudaStream_t s) {
-    p.tiles_m = (p.M + BM - 1) / BM;
-    const int kb = int((p.K + BK - 1) / BK), chunks = (kb + CHUNK - 1) / CHUNK;
-    int bn = 64;
-    double best = 1e300;
-    p.split     = 1;
+struct Plan {
+    int bn, split;
+    double us;
+};
+Plan make_plan(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count) {
+    const int64_t tiles_m = (m + BM - 1) / BM;
+    const int kb = int((k + BK - 1) / BK), chunks = (kb + CHUNK - 1) / CHUNK;
+    Plan best{64, 1, 1e300};
     for (int wide = 0; wide < 2; ++wide)
         for (int split = 1; split <= 8 && split <= chunks; split *= 2) {
-            const int64_t items = p.tiles_m * ((p.N + (wide ? 127 : 63)) / (wide ? 128 : 64)) * batch;
+            const int64_t items = tiles_m * ((n + (wide ? 127 : 63)) / (wide ? 128 : 64)) * batch;
             const int64_t room  = split == 1 ? sm_count : split == 2 ? sm_count / 2 - 4 : split == 4 ? sm_count / 4 - 5 : sm_count / 8 - 3;
             const double rounds = double((items + room - 1) / room);
             const int per       = (chunks + split - 1) / split * CHUNK;
             const double time   = rounds * ((split > 1 ? 9.0 : 8.0) + (per < kb ? per : kb) * (wide ? 1.15 : 0.95));
-            if (time < best) best = time, bn = wide ? 128 : 64, p.split = split;
+            if (time < best.us) best = Plan{wide ? 128 : 64, split, time};
         }
-    p.tiles_n = (p.N + bn - 1) / bn;
+    return best;
+}
+
+template <class TIn, class TOut, bool CONV>
+int plan_and_launch(Params& p, int64_t batch, int sm_count, cudaStream_t s) {
+    const Plan plan = make_plan(p.M, p.N, p.K, batch, sm_count);
+    p.split = plan.split, p.tiles_m = (p.M + BM - 1) / BM, p.tiles_n = (p.N + plan.bn - 1) / plan.bn;
     const int64_t ctas = p.tiles_m * p.tiles_n * batch * p.split;
-    return bn == 128 ? launch<128, TIn, TOut, CONV>(p, ctas, s) : launch<64, TIn, TOut, CONV>(p, ctas, s);
+    return plan.bn == 128 ? launch<128, TIn, TOut, CONV>(p, ctas, s) : launch<64, TIn, TOut, CONV>(p, ctas, s);
 }
 
 }  // namespace
@@ -537,6 +544,10 @@ int gemm_f32_tc(const mimk_gemm_desc& d, cudaStream_t s) {
     int st          = MIMK_OK;
     DeviceInfo* dev = device_info(&st);
     if (!dev) return st;
+    if (gemm_tf32_preferred(d, dev->sm_count, make_plan(d.m, d.n, d.k, d.batch, dev->sm_count).us)) {
+        const int r = gemm_tf32(d, s);
+        if (r != MIMK_E_UNSUPPORTED) return r;
+    }
     Params p{};
     p.A = d.a, p.B = d.b, p.C = d.c;
     p.M = d.m, p.N = d.n, p.K = d.k;

@@ -13,6 +13,9 @@ BF16, F32 = torch.bfloat16, torch.float32
 BF16_ROUND = 2.0 ** -8
 # an f32 product cut into bf16 pieces leaves out less than 2^-22 of each |a b|, its sums and the accumulators' updates lose no more
 F32_CELL = 2.0 ** -20
+# three TF32 products leave out less than 2^-20 of each |a b|; a chunk of 256 k is 96 updates of an accumulator that cut off at
+# most 2^-22 of it each
+TF32_CELL = 2.0 ** -15
 
 
 @pytest.fixture(scope="module")
@@ -118,7 +121,7 @@ def test_attention_of_a_few_queries_does_not_read_hidden_keys(T):
     assert ((got - want).abs()[0, :3] <= 0.03).all() and ((got - want).abs()[1, :2] <= 0.03).all()
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (31, 65, 33), (128, 64, 512), (129, 127, 31), (600, 700, 260), (40, 30, 5000), (1500, 1300, 300)])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (31, 65, 33), (128, 64, 512), (129, 127, 31), (600, 700, 260), (40, 30, 5000), (1500, 1301, 300)])
 @pytest.mark.parametrize("b_nk,offset,out", [(True, 0, F32), (False, 0, F32), (True, 1, F32), (False, 1, BF16)])
 def test_f32_products_of_any_extent(T, m, n, k, b_nk, offset, out):
     a, b = rnd((m, k), 1, F32, offset), rnd((n, k) if b_nk else (k, n), 2, F32, offset)
@@ -128,6 +131,29 @@ def test_f32_products_of_any_extent(T, m, n, k, b_nk, offset, out):
     T.device_status()
     scale = d64(a).abs() @ d64(b).abs() + d64(bias).abs()
     close_cells(got, d64(a) @ d64(b) + d64(bias), scale, F32_CELL if out == F32 else BF16_ROUND)
+
+
+@pytest.mark.parametrize("batch,m,n,k,b_nk,offset,out", [
+    (1, 1500, 1300, 300, True, 0, F32), (1, 1500, 1300, 301, False, 1, F32), (1, 1281, 1544, 257, True, 1, BF16),
+    (1, 1281, 1544, 260, False, 0, BF16), (3, 1153, 1156, 515, True, 0, F32), (2, 4100, 4100, 33, False, 0, F32)])
+def test_f32_products_with_many_tiles(T, batch, m, n, k, b_nk, offset, out):
+    lead = (batch,) if batch > 1 else ()
+    a, b = rnd(lead + (m, k), 1, F32, offset), rnd(lead + ((n, k) if b_nk else (k, n)), 2, F32, offset)
+    b = b.transpose(-1, -2) if b_nk else b
+    a[..., 5, 3], b[..., 7, 9] = math.inf, math.nan
+    run = lambda: T.bmm(a, b) if batch > 1 else T.product_2d(a, b, out_dtype=out)
+    run()
+    got = run()
+    T.device_status()
+    want, scale = d64(a) @ d64(b), (d64(a).abs() @ d64(b).abs()).nan_to_num(0, 0, 0)
+    close_cells(got, want, scale, TF32_CELL if out == F32 else BF16_ROUND)
+    # a captured call holds no buffer of the library: it takes the kernel that needs none, whose error is smaller
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = run()
+    graph.replay()
+    T.device_status()
+    close_cells(got, want, scale, F32_CELL if out == F32 else BF16_ROUND)
 
 
 def test_f32_products_keep_infinities_and_extremes(T):
@@ -154,6 +180,18 @@ def test_convolutions_gathered_from_the_image(T, monkeypatch, n, cin, h, w, cout
         x[0, 0, h // 2, w // 2] = math.inf
         assert torch.equal(d64(T.conv(x, f, stride=stride, dilation=dil, padding=pad)).isfinite(),
                            conv(d64(x), d64(f), stride=stride, dilation=dil, padding=pad).isfinite())
+
+
+@pytest.mark.parametrize("n,cin,h,w,cout,kh,kw,stride", [(2, 8, 64, 64, 128, 3, 3, (1, 1)), (1, 16, 65, 31, 256, 1, 5, (2, 1))])
+def test_bf16_convolutions_with_and_without_a_patch_matrix(T, monkeypatch, n, cin, h, w, cout, kh, kw, stride):
+    monkeypatch.setattr(T, "CONV_CONTRACTION_MIN_WORK", 1)
+    x, f = rnd((n, cin, h, w), 1, BF16), rnd((cout, cin, kh, kw), 2, BF16)
+    want, scale = (torch.nn.functional.conv2d(u, v, stride=stride) for u, v in ((d64(x), d64(f)), (d64(x).abs(), d64(f).abs())))
+    for least in (1, 2 ** 62):
+        monkeypatch.setattr(T, "CONV_PATCH_MIN_WORK", least)
+        got = T.conv(x, f, stride=stride)
+        T.device_status()
+        close_cells(got, want, scale + 1e-6, BF16_ROUND)
 
 
 @pytest.mark.parametrize("m,n,k,b_nk,post,out,offset", [
