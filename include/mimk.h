@@ -93,8 +93,8 @@ enum {
  * (src/mim/plug/tensor/tensor.mim:404-407, 480-486, 510-513, 1367-1423) and the kernel that
  * gpu::phase::LowerMapReduce::build_kernel generates for them (src/mim/plug/gpu/phase/lower_map_reduce.cpp:148-265).
  * in_dtype F32: f32-grade results -- small or oddly shaped problems fold each cell in ascending k on the CUDA cores,
- * larger ones run on the tensor cores as three TF32 products per term (head/tail split, about 21 mantissa bits per
- * product, f32 accumulation). in_dtype BF16: f32 accumulation on the tensor cores.
+ * larger ones run on the tensor cores, every value as the exact sum of three bf16 pieces (six products per term) or, with
+ * many tiles, as three TF32 products per term (head/tail split, about 21 mantissa bits per product); f32 accumulation. in_dtype BF16: f32 accumulation on the tensor cores.
  * out_dtype F32 or BF16 (round to nearest even). batch strides are in elements; 0 re-uses the operand. */
 typedef struct mimk_gemm_desc {
     int64_t batch, m, n, k;
@@ -264,7 +264,7 @@ int mimk_scatter(const void* input, const void* index, const void* updates, void
  * Replaces: the composed program `softmax (q * transpose_2d k) * v` (lit/tensor/attn_exec.mim:20-22), seven
  * map_reduce_post ops with a materialised score matrix; scale, mask and batching are extensions.
  * q,o: [batch_heads, seq_q, head_dim]; k,v: [batch_heads, seq_k, head_dim]; dtype F32 or BF16 (o same dtype);
- * bf16 with head_dim 64 or 128 runs fused on the tensor cores; f32, and bf16 with other head dims, from 2^24
+ * bf16 with head_dim 64 or 128 and f32 with head_dim up to 128 run fused on the tensor cores; other head dims from 2^24
  * score-products on run as the composition S = Q K^T, softmax, O = P V on the contraction and row kernels (the score
  * matrix lives in a cached library buffer; not when lse is requested); everything else on a warp-per-query CUDA-core kernel;
  * lse (optional, f32 [batch_heads, seq_q]) receives log-sum-exp of the scaled scores. */

@@ -15,7 +15,9 @@
 // The operands are read as the caller has them: any extents, strides and alignment, no copies, no scratch. What bounds it:
 // shared-memory bandwidth (a k-block of 128 x 128 moves 96 KB into the MMA and 48 KB from the loaders; measured 100 clocks per
 // instruction of 64 clocks' arithmetic) next to the loaders' instructions. Too few tiles for the chip: the accumulators of one
-// tile are dealt out to a cluster of two, four or eight CTAs, which exchange them through distributed shared memory.
+// tile are dealt out to a cluster of two, four or eight CTAs, which exchange them through distributed shared memory. Many tiles: the operands
+// are cut beforehand instead (gemm_tf32.cu). Measured: 1000^3 28 us (34 as three TF32 products, 2e-6 off; here 1.3e-7), 4096 x 128 x
+// 4096 45 (121), 64 of 512^3 220 (830 on the CUDA cores), 24 of 503 x 2052 x 407 342 (1062).
 #include <type_traits>
 
 #include "common.cuh"
@@ -55,8 +57,8 @@ struct Bars {
 
 // A convolution as a contraction: row = output pixel (image, oh, ow), k = (input channel, kh, kw), column = filter. Rows of the
 // patch matrix are gathered from the image as the loaders read them.
-// tap_major (channels a multiple of 8): k = (kh, kw, input channel) instead, in the filters too, so that the eight k of a unit share one tap: one test
-// whether it lies inside, and addresses a plane apart. With k in the order of the filters, every element has its own tap and
+// tap_major (channels a multiple of 8): k = (kh, kw, input channel) instead, in the filters too, so that the eight k of a unit
+// share one tap: one test whether it lies inside, and addresses a plane apart. With k in the order of the filters, every element has its own tap and
 // test: 16 x 128 x 56 x 56, 128 filters of 3 x 3: 207 us.
 struct ConvShape {
     int cin, h, w, kh, kw, oh, ow, stride_h, stride_w, dil_h, dil_w, pad_h, pad_w, tap_major;
