@@ -663,10 +663,6 @@ def _mrp_into(out, Sr, f, init, post, map_out, maps, ins):
 # and for integers, as ONE map_reduce_post on the per-cell kernel, which keeps the reference's ascending fold per output cell
 # bit for bit.
 CONV_CONTRACTION_MIN_WORK = 1 << 27
-# A bf16 patch matrix is worth writing where the contraction is long enough for the full-rate kernels (they take extents that are
-# multiples of 8): 16 x 128 x 56 x 56, 128 filters of 3 x 3 (2^32.8), 193 us against 240 gathered; 32 x 32 x 112 x 112, 32 filters
-# (2^31.8), 427 against 339.
-CONV_PATCH_MIN_WORK = 1 << 32
 _CONV_PATCH_BYTES = 1 << 30   # patches of at most this many bytes at a time (whole images per piece)
 
 
@@ -680,6 +676,27 @@ def _conv_on_tensor_cores(dtype, n, cin, cout, kh, kw, oh, ow) -> bool:
 def _whole_tiles(k, cout) -> bool:
     """Extents the full-rate bf16 contraction takes as they are."""
     return k % 8 == 0 and cout % 8 == 0
+
+
+def _patches_pay(dtype, pixels, cout, k, window, padded) -> bool:
+    """Whether a patch matrix and the full-rate contraction beat gathering the patches inside the contraction.
+
+    bf16: both estimated, in us. Gathered: rounds of a tile per SM, 14 + 1.85 per k-block of 32 (7 + 1.25 for up to 64 filters).
+    Patches: three or four operators' host time, 85 or 112, or where it is more the matrix at 1.3 per MB, the result at 2 (written
+    twice, read once) and 3.3 per round of contraction tiles. Measured, gathered / patches: 16 x 64 x 56 x 56, 256 filters of 3 x 3,
+    273 / 131; 32 x 128 x 56 x 56, 256 of 1 x 1, 237 / 154; 32 x 32 x 112 x 112, 64 of 3 x 3, 395 / 448; 8 x 128 x 56 x 56, 128 of
+    1 x 1, 45 / 83.
+    f32: the contraction that takes the patches writes two copies of them; only where each pixel is gathered again for many filters
+    without a window to blow it up: 32 x 256 x 56 x 56, 512 of 1 x 1, 595 / 536; 256 of them, 307 / 371."""
+    if dtype == torch.float32:
+        return window == 1 and cout > 256 and cout % 4 == 0 and pixels * cout * k >= 1 << 33
+    if not _whole_tiles(k, cout):
+        return False
+    wide = cout > 64
+    rounds = -(-(-(-pixels // 128) * -(-cout // (128 if wide else 64))) // 148)
+    gathered = rounds * ((14 + 1.85 * -(-k // 32)) if wide else (7 + 1.25 * -(-k // 32)))
+    passes = (1.3 * k + 2.0 * cout) * pixels * 2e-6 + 3.3 * -(-(-(-pixels // 128) * -(-cout // 256)) // 148)
+    return max(112 if padded else 85, passes) < gathered
 
 
 def _conv_indexable(x, w, oh, ow, stride, dilation, padding) -> bool:
@@ -738,7 +755,7 @@ def conv(x: torch.Tensor, w: torch.Tensor, stride=(1, 1), dilation=(1, 1), paddi
             raise TypeError("conv: both operands share the ring's element type")
         contraction = False   # the per-cell kernel takes operands of two element types
     if contraction:
-        if x.dtype == torch.bfloat16 and _whole_tiles(k, cout) and n * cout * oh * ow * k >= CONV_PATCH_MIN_WORK:
+        if _patches_pay(x.dtype, n * oh * ow, cout, k, kh * kw, any(padding)):
             xp = pad(x, (0, 0, padding[0], padding[1]), (0, 0, padding[0], padding[1])) if any(padding) else x
             return _conv_as_contraction(xp, w, n, cin, cout, kh, kw, oh, ow, stride, dilation)
         x, w = x.contiguous(), w.contiguous()

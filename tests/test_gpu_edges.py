@@ -182,16 +182,17 @@ def test_convolutions_gathered_from_the_image(T, monkeypatch, n, cin, h, w, cout
                            conv(d64(x), d64(f), stride=stride, dilation=dil, padding=pad).isfinite())
 
 
-@pytest.mark.parametrize("n,cin,h,w,cout,kh,kw,stride", [(2, 8, 64, 64, 128, 3, 3, (1, 1)), (1, 16, 65, 31, 256, 1, 5, (2, 1))])
-def test_bf16_convolutions_with_and_without_a_patch_matrix(T, monkeypatch, n, cin, h, w, cout, kh, kw, stride):
+@pytest.mark.parametrize("n,cin,h,w,cout,kh,kw,stride", [(2, 8, 64, 64, 128, 3, 3, (1, 1)), (1, 16, 65, 31, 256, 1, 5, (2, 1)), (2, 8, 30, 30, 40, 1, 1, (1, 1))])
+@pytest.mark.parametrize("dtype", [BF16, F32])
+def test_convolutions_with_and_without_a_patch_matrix(T, monkeypatch, n, cin, h, w, cout, kh, kw, stride, dtype):
     monkeypatch.setattr(T, "CONV_CONTRACTION_MIN_WORK", 1)
-    x, f = rnd((n, cin, h, w), 1, BF16), rnd((cout, cin, kh, kw), 2, BF16)
+    x, f = rnd((n, cin, h, w), 1, dtype), rnd((cout, cin, kh, kw), 2, dtype)
     want, scale = (torch.nn.functional.conv2d(u, v, stride=stride) for u, v in ((d64(x), d64(f)), (d64(x).abs(), d64(f).abs())))
-    for least in (1, 2 ** 62):
-        monkeypatch.setattr(T, "CONV_PATCH_MIN_WORK", least)
+    for patches in (True, False):
+        monkeypatch.setattr(T, "_patches_pay", lambda *sizes: patches)
         got = T.conv(x, f, stride=stride)
         T.device_status()
-        close_cells(got, want, scale + 1e-6, BF16_ROUND)
+        close_cells(got, want, scale + 1e-6, BF16_ROUND if dtype == BF16 else TF32_CELL)
 
 
 @pytest.mark.parametrize("m,n,k,b_nk,post,out,offset", [
