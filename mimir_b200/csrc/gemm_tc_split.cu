@@ -255,9 +255,13 @@ int pick(int bn, bool gated, const CUtensorMap& tA, const CUtensorMap& tB, const
 // 16 x 14336 x 4096 (56 tiles): 32.9 -> 24.3 us; 256 x 4096 x 4096 (32): 23.6 -> 17.7; 5000 x 64 x 8192 (40): 40.6 -> 17.7;
 // 300 x 200 x 16000 (3): 74.6 -> 16.7. Beyond the rule: 128 x 8192 x 1024: 10.0 against 12.1; 700 x 3008 x 8192 (72): 43.5 / 42.4;
 // 2048 x 1024 x 4096 (64): 24.1 / 27.1; 256^3: 6.3 / 7.0. With few rows the bytes of B decide, and more SMs fetch them faster.
+// A shorter K pays for the exchange with fewer tiles only: 16 x 14336 x 1024 (56): 10.9 -> 9.3 us; 256 x 1024 x 1024 (8): 11.2 -> 8.3;
+// the gated block 2 x 1024 x 1280 x 960: 48 -> 21, 300 x 1024 x 1024 x 1024 (24, then 12): 48 -> 27; not 1000 x 1024 x 768 (32):
+// 9.8 / 14.5, nor the second stage of 700 x 1280 x 1280 (30).
 int gemm_tc_split_preferred(const mimk_gemm_desc& d, int gated) {
     const int64_t width = gated ? 128 : 256, tiles = ((d.m + BM - 1) / BM) * ((d.n + width - 1) / width) * d.batch;
-    return d.k >= 24 * BK && tiles <= (d.m <= BM ? 74 : 40);
+    if (d.k >= 24 * BK) return tiles <= (d.m <= BM ? 74 : 40);
+    return d.m <= 32 ? d.k >= 8 * BK && tiles <= 74 : d.k >= 16 * BK && tiles <= (gated ? 24 : 16);
 }
 
 int gemm_tc_split(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, const GemmPitch* pitch) {

@@ -200,7 +200,7 @@ def test_convolutions_with_and_without_a_patch_matrix(T, monkeypatch, n, cin, h,
     (640, 5003, 264, False, None, BF16, 0), (640, 5001, 257, True, "bias_tanh", F32, 1), (65, 2056, 512, True, None, BF16, 1),
     (3, 9001, 513, False, None, BF16, 3), (1, 8193, 1024, True, "relu", BF16, 0),
     (16, 4096, 4096, True, None, BF16, 0), (1, 520, 4104, False, None, F32, 0), (17, 130, 4096, True, "bias", BF16, 0),
-    (129, 72, 4160, False, "add", BF16, 0), (128, 64, 64, True, None, F32, 0), (700, 1000, 72, True, "bias_relu", BF16, 0)])
+    (129, 72, 4160, False, "add", BF16, 0), (31, 1000, 512, False, None, BF16, 0), (250, 1016, 1032, True, "bias", F32, 0), (128, 64, 64, True, None, F32, 0), (700, 1000, 72, True, "bias_relu", BF16, 0)])
 def test_bf16_products_of_any_extent(T, m, n, k, b_nk, post, out, offset):
     a = rnd((m, k), 1, BF16, offset)
     b = rnd((n, k) if b_nk else (k, n), 2, BF16, offset)
