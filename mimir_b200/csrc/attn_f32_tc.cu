@@ -225,11 +225,12 @@ __global__ void __launch_bounds__(NUM_THREADS, DP <= 64 ? 2 : 1) attn_f32_tc_ker
             mx = fmaxf(mx, pair_max[(half ^ 1) * 128 + r]);
             const float m_new = fmaxf(m, mx);
             const float alpha = m == -CUDART_INF_F ? 0.f : expf(m - m_new);
+            const float from  = m_new == -CUDART_INF_F ? 0.f : m_new;  // keys that score minus infinity so far weigh nothing
             m                 = m_new;
             float part = 0.f;
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
-                const float e = i < left ? expf(__uint_as_float(sr[i]) - m_new) : 0.f;
+                const float e = i < left ? expf(__uint_as_float(sr[i]) - from) : 0.f;
                 part += e;
                 sr[i] = __float_as_uint(e);
             }
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(NUM_THREADS, DP <= 64 ? 2 : 1) attn_f32_tc_ker
         l += pair_sum[(half ^ 1) * 128 + r];
         // a row both of whose threads saw only finite results is written here, any other one below
         const float inv = l > 0.f ? 1.f / l : 0.f;
-        bool finite     = isfinite(l);
+        bool finite     = isfinite(l) && (l > 0.f || limit <= 0);  // (keys seen and no weight: the general path knows the answer)
 #pragma unroll
         for (int i = 0; i < HALF; ++i) {
             o[i] *= inv;

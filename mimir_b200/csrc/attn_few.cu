@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
             const int64_t n = limit[r] - step * STEP;
             left[r]         = n < 0 ? 0 : n > STEP ? STEP : int(n);
         }
-        float mx[2] = {-CUDART_INF_F, -CUDART_INF_F}, alpha[2];
+        float mx[2] = {-CUDART_INF_F, -CUDART_INF_F}, alpha[2], from[2];
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
@@ -187,13 +187,14 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
             const float m_new = fmaxf(m[r], quad_max(mx[r]));
             alpha[r]          = part_weight(m[r], m_new);
             m[r]              = m_new;
+            from[r]           = m_new == -CUDART_INF_F ? 0.f : m_new;  // keys that score minus infinity so far weigh nothing
             l[r] *= alpha[r];
         }
 #pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                s[t][e] = whole || t * 8 + 2 * c + (e & 1) < left[e >> 1] ? exp2f(s[t][e] - m[e >> 1]) : 0.f;
+                s[t][e] = whole || t * 8 + 2 * c + (e & 1) < left[e >> 1] ? exp2f(s[t][e] - from[e >> 1]) : 0.f;
                 l[e >> 1] += s[t][e];
             }
         if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {  // a maximum has grown (rare after the first steps)
@@ -298,7 +299,9 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
         } else {
             M = cta_m[row], sum = part_o(0)[i], den = cta_l[row];
         }
-        const float inv = den > 0.f ? 1.f / den : 0.f;
+        // no weight at all: zeros for a row that sees no key, else every score is minus infinity and the softmax has no value
+        const bool none = den == 0.f && (!p.causal || row + 1 + p.sk - p.sq > 0);
+        const float inv = none ? CUDART_NAN_F : den > 0.f ? 1.f / den : 0.f;
         p.o[(h * p.sq + row) * D + col] = __float2bfloat16_rn(sum * inv);
         if (p.lse && col == 0) p.lse[h * p.sq + row] = den > 0.f ? M * LN2 + logf(den) : -CUDART_INF_F;
     }

@@ -43,7 +43,8 @@ __device__ __forceinline__ void row(float* qs, const T* __restrict__ Q, const T*
         }
         const float m_new = fmaxf(m, warp_max(s));
         const float alpha = (m == -CUDART_INF_F) ? 0.f : expf(m - m_new);
-        const float p     = (j < limit) ? expf(s - m_new) : 0.f;
+        // (keys that score minus infinity, and none better so far, weigh nothing)
+        const float p     = (j < limit) ? expf(s - (m_new == -CUDART_INF_F ? 0.f : m_new)) : 0.f;
         l                 = l * alpha + warp_sum(p);
 #pragma unroll
         for (int t = 0; t < MAX_D / 32; ++t) o_acc[t] *= alpha;
@@ -60,7 +61,8 @@ __device__ __forceinline__ void row(float* qs, const T* __restrict__ Q, const T*
         m = m_new;
     }
     T* o            = O + (h * Sq + i) * D;
-    const float inv = l > 0.f ? 1.f / l : 0.f;
+    // no weight at all: zeros for a row that sees no key, else every score is minus infinity and the softmax has no value
+    const float inv = l > 0.f ? 1.f / l : l == 0.f && limit > 0 ? CUDART_NAN_F : 0.f;
 #pragma unroll
     for (int t = 0; t < MAX_D / 32; ++t) {
         const int d = lane + 32 * t;

@@ -121,6 +121,26 @@ def test_attention_of_a_few_queries_does_not_read_hidden_keys(T):
     assert ((got - want).abs()[0, :3] <= 0.03).all() and ((got - want).abs()[1, :2] <= 0.03).all()
 
 
+@pytest.mark.parametrize("dtype,d", [(BF16, 64), (BF16, 128), (BF16, 80), (F32, 64), (F32, 130)])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("sq,sk,hidden", [
+    (1, 17, [16]), (1, 49, [48]), (2, 49, range(32)), (3, 4096, range(3896, 4094)), (4, 4096, range(0, 300)), (16, 200, range(16)),
+    (2, 700, range(64, 700, 2)), (3, 129, range(0, 128)), (2, 40, range(40))])
+def test_attention_with_scores_of_minus_infinity(T, dtype, d, causal, sq, sk, hidden):
+    # keys hidden by a coordinate of minus infinity against a query coordinate of one, as padding is, anywhere among the keys
+    q, k, v = rnd((3, sq, d), 1, dtype), rnd((3, sk, d), 2, dtype), rnd((3, sk, d), 3, dtype)
+    q[..., 0], k[..., 0] = 1.0, 0.0
+    k[:, list(hidden), 0] = -math.inf
+    got, lse = T.attention(q, k, v, scale=d ** -0.5, causal=causal, return_lse=True)
+    T.device_status()
+    want, want_lse = attention_reference(q, k, v, d ** -0.5, causal)
+    tol = 64 * F32_CELL if dtype == F32 else BF16_ROUND * (want.abs() + attention_reference(q, k, v.abs(), d ** -0.5, causal)[0]) + 1e-6
+    g = d64(got)
+    assert torch.equal(g.isnan(), want.isnan())   # no value where no key that a row sees has a finite score
+    assert (((g - want).abs() <= tol) | want.isnan()).all()
+    assert torch.equal(d64(lse).isfinite(), want_lse.isfinite()) and ((d64(lse) - want_lse).abs()[want_lse.isfinite()] <= 1e-4).all()
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 1, 1), (31, 65, 33), (128, 64, 512), (129, 127, 31), (600, 700, 260), (40, 30, 5000), (1500, 1301, 300)])
 @pytest.mark.parametrize("b_nk,offset,out", [(True, 0, F32), (False, 0, F32), (True, 1, F32), (False, 1, BF16)])
 def test_f32_products_of_any_extent(T, m, n, k, b_nk, offset, out):
