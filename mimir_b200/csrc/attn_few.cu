@@ -16,6 +16,7 @@
 #include <math_constants.h>
 
 #include "common.cuh"
+#include "f32_split.cuh"
 
 namespace mimk {
 namespace {
@@ -78,10 +79,13 @@ __device__ __forceinline__ bool has_nonfinite(uint4 v) {
     auto bad = [](uint32_t w) { return (w & 0x7f80u) == 0x7f80u || (w & 0x7f800000u) == 0x7f800000u; };
     return bad(v.x) || bad(v.y) || bad(v.z) || bad(v.w);
 }
-// weight of a part whose running maximum (in powers of two) is m, in a whole of maximum M; a part without keys has none
-__device__ __forceinline__ float part_weight(float m, float M) { return m == -CUDART_INF_F ? 0.f : exp2f(m - M); }
+// Scores are kept in powers of two, or in powers of e where the weights are kept in f32.
+template <bool F32W> __device__ __forceinline__ float power(float x) { return F32W ? expf(x) : exp2f(x); }
+// weight of a part whose running maximum is m, in a whole of maximum M; a part without keys has none
+template <bool F32W> __device__ __forceinline__ float part_weight(float m, float M) { return m == -CUDART_INF_F ? 0.f : power<F32W>(m - M); }
 
-template <int D>
+// F32W: the weights enter the second product as three bf16 pieces that sum to the f32 value, not rounded to bf16.
+template <int D, bool F32W>
 __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(const Params p) {
     constexpr int G = D / 32, CH = D / 64;
     using R = Ring<D>;
@@ -97,7 +101,7 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
     const __nv_bfloat16* V = p.v + h * p.sk * D;
     const int64_t steps = (p.sk + STEP - 1) / STEP, per = (steps + p.split * WARPS - 1) / (p.split * WARPS);
     const int64_t s0 = (rank * WARPS + warp) * per, s1 = s0 + per < steps ? s0 + per : steps;
-    const float scale2 = p.scale * LOG2E;
+    const float scale = F32W ? p.scale : p.scale * LOG2E;
 
     const uint32_t mine = uint32_t(__cvta_generic_to_shared(ring)) + warp * R::WARP_BYTES + lane * 16;
     auto slot  = [&](int64_t step, int piece) { return mine + (unsigned(step - s0) % R::STAGES * R::CHUNKS + piece) * 512; };
@@ -179,13 +183,13 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
         for (int t = 0; t < 2; ++t)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                s[t][e] = (s[t][e] + s2[t][e]) * scale2;
+                s[t][e] = (s[t][e] + s2[t][e]) * scale;
                 if (whole || t * 8 + 2 * c + (e & 1) < left[e >> 1]) mx[e >> 1] = fmaxf(mx[e >> 1], s[t][e]);
             }
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
             const float m_new = fmaxf(m[r], quad_max(mx[r]));
-            alpha[r]          = part_weight(m[r], m_new);
+            alpha[r]          = part_weight<F32W>(m[r], m_new);
             m[r]              = m_new;
             from[r]           = m_new == -CUDART_INF_F ? 0.f : m_new;  // keys that score minus infinity so far weigh nothing
             l[r] *= alpha[r];
@@ -194,7 +198,7 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
         for (int t = 0; t < 2; ++t)
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-                s[t][e] = whole || t * 8 + 2 * c + (e & 1) < left[e >> 1] ? exp2f(s[t][e] - from[e >> 1]) : 0.f;
+                s[t][e] = whole || t * 8 + 2 * c + (e & 1) < left[e >> 1] ? power<F32W>(s[t][e] - from[e >> 1]) : 0.f;
                 l[e >> 1] += s[t][e];
             }
         if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {  // a maximum has grown (rare after the first steps)
@@ -217,27 +221,36 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
             odd_block = __any_sync(0xffffffffu, bad);
         }
         if (!odd_block) {
-            const uint32_t a0 = pack_bf16x2(s[0][0], s[0][1]), a1 = pack_bf16x2(s[0][2], s[0][3]);
-            const uint32_t a2 = pack_bf16x2(s[1][0], s[1][1]), a3 = pack_bf16x2(s[1][2], s[1][3]);
 #pragma unroll
-            for (int ch = 0; ch < CH; ++ch) {
-                const uint32_t w0[4] = {vr[0][ch].x, vr[0][ch].y, vr[0][ch].z, vr[0][ch].w}, w1[4] = {vr[1][ch].x, vr[1][ch].y, vr[1][ch].z, vr[1][ch].w};
-                const uint32_t w2[4] = {vr[2][ch].x, vr[2][ch].y, vr[2][ch].z, vr[2][ch].w}, w3[4] = {vr[3][ch].x, vr[3][ch].y, vr[3][ch].z, vr[3][ch].w};
+            for (int piece = 0; piece < (F32W ? 3 : 1); ++piece) {
+                uint32_t a[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    mma16816(o[ch][2 * u], a0, a1, a2, a3, __byte_perm(w0[u], w1[u], 0x5410), __byte_perm(w2[u], w3[u], 0x5410));
-                    mma16816(o[ch][2 * u + 1], a0, a1, a2, a3, __byte_perm(w0[u], w1[u], 0x7632), __byte_perm(w2[u], w3[u], 0x7632));
+                for (int i = 0; i < 4; ++i) {
+                    float &lo = s[i >> 1][(i & 1) * 2], &hi = s[i >> 1][(i & 1) * 2 + 1];
+                    a[i] = F32W ? f32split::upper_halves(lo, hi) : pack_bf16x2(lo, hi);
+                    if (F32W) lo = f32split::lower_part(lo), hi = f32split::lower_part(hi);
+                }
+#pragma unroll
+                for (int ch = 0; ch < CH; ++ch) {
+                    const uint32_t w0[4] = {vr[0][ch].x, vr[0][ch].y, vr[0][ch].z, vr[0][ch].w}, w1[4] = {vr[1][ch].x, vr[1][ch].y, vr[1][ch].z, vr[1][ch].w};
+                    const uint32_t w2[4] = {vr[2][ch].x, vr[2][ch].y, vr[2][ch].z, vr[2][ch].w}, w3[4] = {vr[3][ch].x, vr[3][ch].y, vr[3][ch].z, vr[3][ch].w};
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        mma16816(o[ch][2 * u], a[0], a[1], a[2], a[3], __byte_perm(w0[u], w1[u], 0x5410), __byte_perm(w2[u], w3[u], 0x5410));
+                        mma16816(o[ch][2 * u + 1], a[0], a[1], a[2], a[3], __byte_perm(w0[u], w1[u], 0x7632), __byte_perm(w2[u], w3[u], 0x7632));
+                    }
                 }
             }
         } else {
             for (int kk = 0; kk < STEP; ++kk) {
-                const int from    = (lane & ~3) | ((kk & 7) >> 1);
+                const int at      = (lane & ~3) | ((kk & 7) >> 1);
                 const int64_t key = step * STEP + kk;
                 float pr[2];
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
                     const float lo = kk < 8 ? s[0][2 * r] : s[1][2 * r], hi = kk < 8 ? s[0][2 * r + 1] : s[1][2 * r + 1];
-                    pr[r] = __bfloat162float(__float2bfloat16_rn(__shfl_sync(0xffffffffu, (kk & 1) ? hi : lo, from)));
+                    pr[r] = __shfl_sync(0xffffffffu, (kk & 1) ? hi : lo, at);
+                    if (!F32W) pr[r] = __bfloat162float(__float2bfloat16_rn(pr[r]));
                 }
 #pragma unroll
                 for (int ch = 0; ch < CH; ++ch)
@@ -277,7 +290,7 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
         float sum = 0.f, den = 0.f;
 #pragma unroll
         for (int w = 0; w < WARPS; ++w) {
-            const float wt = part_weight(part_m[w][row], M);
+            const float wt = part_weight<F32W>(part_m[w][row], M);
             sum += wt * part_o(w)[i];
             den += wt * part_l[w][row];
         }
@@ -292,7 +305,7 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
         if (p.split > 1) {
             for (int r = 0; r < p.split; ++r) M = fmaxf(M, ld_cluster(&cta_m[row], r));
             for (int r = 0; r < p.split; ++r) {
-                const float wt = part_weight(ld_cluster(&cta_m[row], r), M);
+                const float wt = part_weight<F32W>(ld_cluster(&cta_m[row], r), M);
                 sum += wt * ld_cluster(part_o(0) + i, r);
                 den += wt * ld_cluster(&cta_l[row], r);
             }
@@ -303,14 +316,14 @@ __global__ void __launch_bounds__(THREADS, D == 128 ? 2 : 3) attn_few_kernel(con
         const bool none = den == 0.f && (!p.causal || row + 1 + p.sk - p.sq > 0);
         const float inv = none ? CUDART_NAN_F : den > 0.f ? 1.f / den : 0.f;
         p.o[(h * p.sq + row) * D + col] = __float2bfloat16_rn(sum * inv);
-        if (p.lse && col == 0) p.lse[h * p.sq + row] = den > 0.f ? M * LN2 + logf(den) : -CUDART_INF_F;
+        if (p.lse && col == 0) p.lse[h * p.sq + row] = den > 0.f ? (F32W ? M : M * LN2) + logf(den) : -CUDART_INF_F;
     }
     if (p.split > 1) cluster_sync();  // no CTA of the cluster exits while another may read its part
 }
 
-template <int D>
+template <int D, bool F32W>
 int launch(const Params& p, int64_t ctas, cudaStream_t s) {
-    auto kern = attn_few_kernel<D>;
+    auto kern = attn_few_kernel<D, F32W>;
     constexpr int SMEM = WARPS * Ring<D>::WARP_BYTES;
     static bool configured[64] = {};  // per template instance and device: the attribute is a per-device setting
     int dev = 0;
@@ -361,7 +374,11 @@ int attn_few(const mimk_attn_desc& d, cudaStream_t s) {
     // 36 / 22). Every warp has at least three steps.
     p.split = 1;
     while (p.split < 8 && d.batch_heads * p.split * 2 <= 2 * int64_t(dev->sm_count) && d.seq_k >= int64_t(p.split) * 2 * WARPS * 3 * STEP) p.split *= 2;
-    return d.head_dim == 128 ? launch<128>(p, d.batch_heads * p.split, s) : launch<64>(p, d.batch_heads * p.split, s);
+    // The calls that the 128-row kernel takes too (attn_tc_p.cu) have weights rounded to bf16, as there; the others, whose general
+    // path keeps them in f32 (attn_row.cuh), keep them here.
+    const int64_t ctas = d.batch_heads * p.split;
+    if (attn_tc_persistent_supported(d)) return d.head_dim == 128 ? launch<128, false>(p, ctas, s) : launch<64, false>(p, ctas, s);
+    return d.head_dim == 128 ? launch<128, true>(p, ctas, s) : launch<64, true>(p, ctas, s);
 }
 
 }  // namespace mimk

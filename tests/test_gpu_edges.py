@@ -112,6 +112,19 @@ def test_attention_of_a_few_queries(T, bh, sq, sk, d, causal):
     assert torch.equal(d64(lse).isfinite(), seen) and ((d64(lse) - want_lse).abs()[seen] <= 1e-4).all()
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("bh,sq,sk,causal,scale", [(3, 1, 40, True, 0.1), (2, 16, 1000, True, 0.1), (9, 2, 5000, True, 0.1), (200, 3, 300, True, 0.1), (4, 5, 700, False, -0.1)])
+def test_attention_of_a_few_queries_keeps_f32_weights(T, bh, sq, sk, d, causal, scale):
+    # fewer queries than keys under a mask, or a negative scale: f32 weights, so that only the result is rounded to bf16
+    q, k, v = rnd((bh, sq, d), 1, BF16), rnd((bh, sk, d), 2, BF16), rnd((bh, sk, d), 3, BF16)
+    got = T.attention(q, k, v, scale=scale, causal=causal)
+    T.device_status()
+    want, _ = attention_reference(q, k, v, scale, causal)
+    weights = attention_reference(q, k, v.abs(), scale, causal)[0]
+    # half a unit in the last of eight bits: 2^-8 of the result; scores off by F32_CELL of their terms
+    assert ((d64(got) - want).abs() <= BF16_ROUND * want.abs() + 64 * F32_CELL * weights).all()
+
+
 def test_attention_of_a_few_queries_does_not_read_hidden_keys(T):
     q, k, v = rnd((2, 4, 64), 1, BF16), rnd((2, 40, 64), 2, BF16), rnd((2, 40, 64), 3, BF16)
     v[0, 39, 5], v[1, 38, 7] = math.inf, math.nan   # seen by the last query, and by the last two
