@@ -40,12 +40,6 @@ __device__ __forceinline__ void apply_post_32(int post, float (&v)[32], const fl
 // One 32-row piece of a staged result (128-byte-swizzled rows at `buf`) to a matrix that bulk stores cannot write (a row pitch
 // that is no multiple of 16 bytes, or a base that is not aligned): the warp stores each row with neighbouring lanes on
 // neighbouring elements, two bf16 per lane where the pair is aligned.
-__device__ __forceinline__ void store_piece(const uint8_t* buf, float* c, int64_t ldc, int64_t rows, int64_t cols, int lane) {
-    const int n = int(rows < 32 ? rows : 32);
-#pragma unroll 8
-    for (int r = 0; r < n; ++r)
-        if (lane < cols) c[r * ldc + lane] = *reinterpret_cast<const float*>(buf + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
-}
 __device__ __forceinline__ void store_piece(const uint8_t* buf, __nv_bfloat16* c, int64_t ldc, int64_t rows, int64_t cols, int lane) {
     const int n = int(rows < 32 ? rows : 32), m = int(cols < 64 ? cols : 64);
     uint16_t* dst = reinterpret_cast<uint16_t*>(c);

@@ -535,11 +535,26 @@ int plan_and_launch(Params& p, int64_t batch, int sm_count, cudaStream_t s) {
 
 }  // namespace
 
-int gemm_f32_tc_supported(const mimk_gemm_desc& d) {
-    if (d.in_dtype != MIMK_F32 || d.k <= 0) return 0;
+static int extents_fit(const mimk_gemm_desc& d) {
+    if (d.k <= 0) return 0;
     if (d.m >= (int64_t(1) << 31) || d.n >= (int64_t(1) << 31) || d.k >= (int64_t(1) << 31)) return 0;
     const int64_t tiles = ((d.m + BM - 1) / BM) * ((d.n + 63) / 64);
     return tiles < (int64_t(1) << 28) && d.batch < (int64_t(1) << 28) && tiles * d.batch < (int64_t(1) << 28);  // one grid
+}
+int gemm_f32_tc_supported(const mimk_gemm_desc& d) { return d.in_dtype == MIMK_F32 && extents_fit(d); }
+
+static Params product_params(const mimk_gemm_desc& d, const DeviceInfo& dev) {
+    Params p{};
+    p.A = d.a, p.B = d.b, p.C = d.c;
+    p.M = d.m, p.N = d.n, p.K = d.k;
+    p.sa = d.batch > 1 ? d.stride_a : 0, p.sb = d.batch > 1 ? d.stride_b : 0, p.sc = d.batch > 1 ? d.stride_c : 0;
+    p.post_row = static_cast<const float*>(d.post_row), p.post_full = d.post_full, p.post = d.post;
+    p.b_nk  = d.b_layout == MIMK_B_NK;
+    p.vec_a = d.k % 4 == 0 && aligned16(d.a) && p.sa % 4 == 0;
+    p.vec_b = d.k % 4 == 0 && aligned16(d.b) && p.sb % 4 == 0;
+    p.vec_c = d.n % 4 == 0 && aligned16(d.c) && p.sc % 4 == 0;
+    p.status = dev.status_dev;
+    return p;
 }
 
 int gemm_f32_tc(const mimk_gemm_desc& d, cudaStream_t s) {
@@ -550,18 +565,21 @@ int gemm_f32_tc(const mimk_gemm_desc& d, cudaStream_t s) {
         const int r = gemm_tf32(d, s);
         if (r != MIMK_E_UNSUPPORTED) return r;
     }
-    Params p{};
-    p.A = d.a, p.B = d.b, p.C = d.c;
-    p.M = d.m, p.N = d.n, p.K = d.k;
-    p.sa = d.batch > 1 ? d.stride_a : 0, p.sb = d.batch > 1 ? d.stride_b : 0, p.sc = d.batch > 1 ? d.stride_c : 0;
-    p.post_row = static_cast<const float*>(d.post_row), p.post_full = d.post_full, p.post = d.post;
-    p.b_nk  = d.b_layout == MIMK_B_NK;
-    p.vec_a = d.k % 4 == 0 && aligned16(d.a) && p.sa % 4 == 0;
-    p.vec_b = d.k % 4 == 0 && aligned16(d.b) && p.sb % 4 == 0;
-    p.vec_c = d.n % 4 == 0 && aligned16(d.c) && p.sc % 4 == 0;
-    p.status = dev->status_dev;
+    Params p = product_params(d, *dev);
     return d.out_dtype == MIMK_BF16 ? plan_and_launch<float, __nv_bfloat16, false>(p, d.batch, dev->sm_count, s)
                                     : plan_and_launch<float, float, false>(p, d.batch, dev->sm_count, s);
+}
+
+// bf16 operands, an f32 result, extents or alignment that TMA cannot take. One piece per value, accumulators of 64 k and f32 adds
+// between them: an accumulator kept over all of K (gemm_tc.cu) loses up to 2e-6 of a result that the CUDA-core fold gives to 4e-7,
+// which a result in f32 shows (2000 x 5003 x 2048).
+int gemm_bf16_chunked(const mimk_gemm_desc& d, cudaStream_t s) {
+    if (d.in_dtype != MIMK_BF16 || d.out_dtype != MIMK_F32 || !extents_fit(d)) return MIMK_E_UNSUPPORTED;
+    int st          = MIMK_OK;
+    DeviceInfo* dev = device_info(&st);
+    if (!dev) return st;
+    Params p = product_params(d, *dev);
+    return plan_and_launch<__nv_bfloat16, float, false>(p, d.batch, dev->sm_count, s);
 }
 
 int conv_tc(const mimk_conv_desc& d, cudaStream_t s) {

@@ -273,7 +273,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         }
                     }
                 }
-                if (DIRECT) {
+                if constexpr (DIRECT) {
                     __syncwarp();
                     store_piece(smem_raw + (buf - raw_addr), static_cast<TOut*>(p.dst[0]) + zoff + row0 * p.ldc + n0 + c0, p.ldc, p.M - row0,
                                 p.N - n0 - c0, lane);
@@ -528,14 +528,11 @@ int gemm_tc(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, 
     const uint64_t whole_c  = uint64_t(d.m) * row_c;
     const uint64_t sc = d.batch > 1 ? uint64_t(d.stride_c) * out_size : (whole_c < (uint64_t(1) << 40) ? whole_c : row_c);
     OutMaps om;
-    if (pitch) {  // any pitch and alignment of the result: plain stores, no maps
-        if (gated || gather) return MIMK_E_UNSUPPORTED;
+    if (pitch) {  // any pitch and alignment of the result, which is bf16: plain stores, no maps
+        if (gated || gather || d.out_dtype != MIMK_BF16) return MIMK_E_UNSUPPORTED;
         om = OutMaps{};
-        if (d.out_dtype == MIMK_BF16)
-            return b_mn ? launch<256, true, false, __nv_bfloat16, true>(tA, tB, tB2, om, p, dev->sm_count, s)
-                        : launch<256, false, false, __nv_bfloat16, true>(tA, tB, tB2, om, p, dev->sm_count, s);
-        return b_mn ? launch<256, true, false, float, true>(tA, tB, tB2, om, p, dev->sm_count, s)
-                    : launch<256, false, false, float, true>(tA, tB, tB2, om, p, dev->sm_count, s);
+        return b_mn ? launch<256, true, false, __nv_bfloat16, true>(tA, tB, tB2, om, p, dev->sm_count, s)
+                    : launch<256, false, false, __nv_bfloat16, true>(tA, tB, tB2, om, p, dev->sm_count, s);
     }
     for (int t = 0; t < p.n_dst; ++t) {
         const uint8_t* base = static_cast<const uint8_t*>(p.dst[t]) + size_t(p.col_off) * out_size;
@@ -556,7 +553,7 @@ int gemm_tc(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, 
 }
 
 // bf16 contractions whose extents or alignment break TMA's 16-byte rules: operands that do are copied to rows of an aligned
-// pitch first, and the result is written by plain stores. Returns MIMK_E_UNSUPPORTED, with nothing launched, where the CUDA-core
+// pitch first, and the result is written by plain stores. (A result in f32: gemm_bf16_chunked.) Returns MIMK_E_UNSUPPORTED, with nothing launched, where the CUDA-core
 // kernel is the better or the only way.
 //
 // Measured: 2000 x 5003 x 2048, 57 us (2240 on the CUDA cores; 38 with a width of 5008); K = 2047 as well, 75; 3 x 9000 x 5001, 23 to
@@ -568,6 +565,7 @@ int gemm_tc_ragged(const mimk_gemm_desc& d, cudaStream_t s) {
     RaggedPlan r;
     if (!ragged_plan(d, &r)) return MIMK_E_UNSUPPORTED;
     if (double(d.m) * double(d.n) * double(d.k) * double(d.batch) < double(1 << 22)) return MIMK_E_UNSUPPORTED;
+    if (d.out_dtype == MIMK_F32) return gemm_bf16_chunked(d, s);  // a result that would show the accumulator's lost bits
     mimk_gemm_desc t = d;
     int st           = MIMK_OK;
     DeviceInfo* dev  = device_info(&st);

@@ -335,7 +335,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         }
                     }
                 }
-                if (DIRECT) {
+                if constexpr (DIRECT) {
                     __syncwarp();
                     store_piece(smem_raw + (buf - raw_addr), static_cast<TOut*>(p.dst[0]) + row0 * p.ldc + n0 + c0, p.ldc, p.M - row0,
                                 p.N - n0 - c0, lane);
@@ -458,15 +458,11 @@ int gemm_tc2(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2,
         // destination maps: [M, N] windows (row pitch ldc) starting at column col_off, boxes of 32 rows x 128 bytes;
         // [scatter_rows, N] windows when the row blocks are scattered
         OutMaps om;
-        if (pitch) {  // any pitch and alignment of the result: plain stores, no maps
-            if (gated || gather) return MIMK_E_UNSUPPORTED;
+        if (pitch) {  // any pitch and alignment of the result, which is bf16: plain stores, no maps
+            if (gated || gather || d.out_dtype != MIMK_BF16) return MIMK_E_UNSUPPORTED;
             om = OutMaps{};
-            if (d.out_dtype == MIMK_BF16)
-                MIMK_TRY((b_mn ? launch<256, true, false, __nv_bfloat16, true>(tA, tB, tB2, om, p, dev->sm_count, s)
-                               : launch<256, false, false, __nv_bfloat16, true>(tA, tB, tB2, om, p, dev->sm_count, s)));
-            else
-                MIMK_TRY((b_mn ? launch<256, true, false, float, true>(tA, tB, tB2, om, p, dev->sm_count, s)
-                               : launch<256, false, false, float, true>(tA, tB, tB2, om, p, dev->sm_count, s)));
+            MIMK_TRY((b_mn ? launch<256, true, false, __nv_bfloat16, true>(tA, tB, tB2, om, p, dev->sm_count, s)
+                           : launch<256, false, false, __nv_bfloat16, true>(tA, tB, tB2, om, p, dev->sm_count, s)));
             continue;
         }
         for (int t = 0; t < p.n_dst; ++t) {

@@ -253,6 +253,20 @@ def test_bf16_products_of_any_extent(T, m, n, k, b_nk, post, out, offset):
     assert got.dtype == out and ((d64(got) - want).abs() <= rounding + scale + 1e-6).all()
 
 
+@pytest.mark.parametrize("batch,m,n,k,b_nk,offset", [
+    (1, 2000, 1003, 2048, True, 0), (1, 129, 255, 4001, False, 0), (1, 640, 1001, 2056, False, 1), (1, 65, 2056, 4096, True, 1), (3, 130, 203, 1030, True, 0)])
+def test_f32_results_of_bf16_products_of_any_extent(T, batch, m, n, k, b_nk, offset):
+    # as an f32 fold gives them (2^-20 of the terms, like an f32 product), whichever kernel the extents lead to
+    lead = (batch,) if batch > 1 else ()
+    a, b = rnd(lead + (m, k), 1, BF16, offset), rnd(lead + ((n, k) if b_nk else (k, n)), 2, BF16, offset)
+    a.abs_(), b.abs_()   # one sign: what an accumulator cuts off adds up
+    b = b.transpose(-1, -2) if b_nk else b
+    got = T.bmm(a, b, out_dtype=F32) if batch > 1 else T.product_2d(a, b, out_dtype=F32)
+    T.device_status()
+    want = d64(a) @ d64(b)
+    close_cells(got, want, want, F32_CELL)
+
+
 @pytest.mark.parametrize("B,m,n,k,b_nk", [(3, 129, 255, 67, True), (5, 40, 200, 286, False), (2, 130, 64, 1000, True), (70, 16, 24, 72, False)])
 def test_bf16_batches_of_any_extent(T, B, m, n, k, b_nk):
     a, b = rnd((B, m, k), 1, BF16), rnd((B, n, k) if b_nk else (B, k, n), 2, BF16)
