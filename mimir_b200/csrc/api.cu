@@ -302,6 +302,10 @@ extern "C" int mimk_conv(const mimk_conv_desc* d, void* stream) {
     if (double(d->h) + 2.0 * double(d->pad_h) >= LIM || double(d->w) + 2.0 * double(d->pad_w) >= LIM) return MIMK_E_UNSUPPORTED;
     if (double(d->dil_h) * double(d->kh) >= LIM || double(d->dil_w) * double(d->kw) >= LIM) return MIMK_E_UNSUPPORTED;
     if (d->kh > 31 || d->kw > 31) return MIMK_E_UNSUPPORTED;  // a bit of a mask per tap row and column
+    // the distance from a window's first tap to its last one in the last channel is a 31-bit number
+    const double reach = double(d->cin - 1) * double(d->h) * double(d->w) + double(d->kh - 1) * double(d->dil_h) * double(d->w) +
+                         double(d->kw - 1) * double(d->dil_w);
+    if (reach >= 2.0 * LIM) return MIMK_E_UNSUPPORTED;
     if (d->stride_h >= (1 << 30) || d->stride_w >= (1 << 30)) return MIMK_E_UNSUPPORTED;
     const int64_t span_h = d->h + 2 * d->pad_h - d->dil_h * (d->kh - 1) - 1, span_w = d->w + 2 * d->pad_w - d->dil_w * (d->kw - 1) - 1;
     if (span_h < 0 || span_w < 0) return MIMK_E_SHAPE;

@@ -235,12 +235,14 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
             const int k = int(k0) + unit * 8, taps = cv.kh * cv.kw;
             const int ci = k / taps;
             int r = (k - ci * taps) / cv.kw, q = k - ci * taps - r * cv.kw;
-            int off = ci * (cv.h * cv.w) + r * cv.dil_h * cv.w + q * cv.dil_w;
-            const int next_row = cv.dil_h * cv.w - cv.kw * cv.dil_w, next_plane = cv.h * cv.w - cv.kh * cv.dil_h * cv.w;
+            // offsets of taps that are read fit 31 bits (mimk_conv sees to it); the others wrap
+            const unsigned w = cv.w, plane = cv.h * w, down = cv.dil_h * w;
+            unsigned off = ci * plane + r * down + q * cv.dil_w;
+            const unsigned next_row = down - cv.kw * cv.dil_w, next_plane = plane - cv.kh * down;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const bool in = (rows_in >> r) & (cols_in >> q) & int(k + j < int(p.K));
-                fa[j]         = in ? load1(a_at + off) : 0.f;
+                fa[j]         = in ? load1(a_at + int(off)) : 0.f;
                 off += cv.dil_w;
                 if (++q == cv.kw) {
                     q = 0, off += next_row;

@@ -700,12 +700,13 @@ def _patches_pay(dtype, pixels, cout, k, window, padded) -> bool:
 
 
 def _conv_indexable(x, w, oh, ow, stride, dilation, padding) -> bool:
-    """What mimk_conv takes (30-bit coordinates, windows of up to 31 x 31); anything larger (or cropped by a negative padding) stays
-    on the per-cell kernel."""
-    n, _, h, wd = x.shape
+    """What mimk_conv takes (30-bit coordinates, windows of up to 31 x 31 whose last tap is less than 2^31 elements from the first);
+    anything larger (or cropped by a negative padding) stays on the per-cell kernel."""
+    n, cin, h, wd = x.shape
     cout, _, kh, kw = w.shape
     return (max(kh, kw) <= 31 and min(oh, ow) >= 1 and min(*stride, *dilation) >= 1 and min(padding) >= 0
             and n * cout * oh * ow < 1 << 40
+            and (cin - 1) * h * wd + (kh - 1) * dilation[0] * wd + (kw - 1) * dilation[1] < 1 << 31
             and max(x[0].numel(), w[0].numel(), oh * ow, h + 2 * padding[0], wd + 2 * padding[1], dilation[0] * kh, dilation[1] * kw,
                     *stride) < 1 << 30)
 

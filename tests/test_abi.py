@@ -140,3 +140,24 @@ def test_reduce_plan_fits_the_static_array_on_148_sms(lib):
     assert L.mimk_reduce_plan(1, 10 ** 6, 100000, 264, C.byref(n)) == 0 and n.value > cap   # a larger machine can exceed
     assert L.mimk_reduce_plan(-1, 4, 4, 148, C.byref(n)) == 1
     assert L.mimk_reduce_plan(1, 4, 4, 148, None) == 1
+
+
+@pytest.mark.parametrize("cin,h,w,kh,kw,dil,pad,fits", [
+    (8, 64, 65536, 3, 3, (40000, 1), (40000, 1), False),      # 2 x 40000 rows of 65536
+    (8, 64, 65536, 2, 3, (32000, 1), (15970, 1), True), (8, 64, 65536, 2, 3, (32766, 1), (16360, 1), False),
+    (1, 64, 65536, 1, 3, (40000, 1), (0, 1), True),           # no second tap row
+    (1, 1, 1 << 24, 3, 1, (100, 1), (100, 0), False), (3, 224, 224, 7, 7, (1, 1), (3, 3), True)])
+def test_convolution_offsets_fit_their_32_bits(lib, cin, h, w, kh, kw, dil, pad, fits):
+    """An image that a dilated window spans too widely for 32-bit offsets is refused before anything is launched, by the C entry
+    point and by the operator's choice of a kernel alike."""
+    import torch
+    from mimir_b200 import tensor as T
+    d = lib.ConvDesc()
+    d.n, d.cin, d.h, d.w, d.cout, d.kh, d.kw = 1, cin, h, w, 16, kh, kw
+    d.stride_h, d.stride_w, d.dil_h, d.dil_w, d.pad_h, d.pad_w = 1, 1, *dil, *pad
+    d.dtype, d.by_tap = lib.F32, 0
+    oh, ow = h + 2 * pad[0] - dil[0] * (kh - 1), w + 2 * pad[1] - dil[1] * (kw - 1)
+    x, f = torch.empty((1, cin, h, w), device="meta"), torch.empty((16, cin, kh, kw), device="meta")
+    assert T._conv_indexable(x, f, oh, ow, (1, 1), dil, pad) == fits
+    # (no operands: a shape that is taken fails at the next check, for want of a device or of a pointer)
+    assert (lib.lib().mimk_conv(C.byref(d), None) == 8) == (not fits)
