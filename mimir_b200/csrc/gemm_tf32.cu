@@ -420,6 +420,7 @@ int gemm_tf32_preferred(const mimk_gemm_desc& d, int sm_count, double pieces_us)
     if (d.m < 128 || d.n < 128 || d.batch > 16) return 0;
     if (d.m >= (int64_t(1) << 31) || d.n >= (int64_t(1) << 31) || d.k >= (int64_t(1) << 31)) return 0;
     if (!aligned16(d.c)) return 0;  // the operands are re-written as padded hi / lo copies; only the result is stored as is
+    if (d.batch > 1 && d.stride_c % (d.out_dtype == MIMK_BF16 ? 8 : 4) != 0) return 0;  // of every entry
     if (d.post_full && !aligned16(d.post_full)) return 0;
     if (d.b_layout != MIMK_B_NK && (d.k + 31) / 32 > 65535) return 0;  // grid of the transposing split
     const double m = double(d.m), n = double(d.n), k = double(d.k);

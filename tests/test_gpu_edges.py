@@ -189,6 +189,27 @@ def test_f32_products_with_many_tiles(T, batch, m, n, k, b_nk, offset, out):
     close_cells(got, want, scale, F32_CELL if out == F32 else BF16_ROUND)
 
 
+@pytest.mark.parametrize("out,gap", [(F32, 1), (F32, 4), (BF16, 4), (BF16, 8)])
+def test_batched_f32_results_at_any_stride(T, out, gap):
+    # entries of a result `gap` elements apart: 16-byte stores only where every entry starts on 16 bytes
+    from mimir_b200 import _lib as L
+    import ctypes as C
+    batch, m, n, k = 3, 1153, 1160, 515
+    a, b = rnd((batch, m, k), 1), rnd((batch, n, k), 2)
+    room = torch.full((batch * (m * n + gap),), 7.0, dtype=out, device="cuda")
+    d = L.GemmDesc()
+    d.batch, d.m, d.n, d.k = batch, m, n, k
+    d.a, d.b, d.c = a.data_ptr(), b.data_ptr(), room.data_ptr()
+    d.stride_a, d.stride_b, d.stride_c = m * k, n * k, m * n + gap
+    d.in_dtype, d.out_dtype, d.b_layout, d.post = L.F32, L.F32 if out == F32 else L.BF16, L.B_NK, L.POST_ID
+    L.check(L.lib().mimk_gemm(C.byref(d), T._stream()), "gemm")
+    T.device_status()
+    room = room.view(batch, m * n + gap)
+    assert (room[:, m * n:] == 7.0).all()
+    bt = b.transpose(1, 2)
+    close_cells(room[:, :m * n].reshape(batch, m, n), d64(a) @ d64(bt), d64(a).abs() @ d64(bt).abs(), TF32_CELL if out == F32 else BF16_ROUND)
+
+
 def test_f32_products_keep_infinities_and_extremes(T):
     a, b = rnd((200, 600), 1), rnd((600, 300), 2)
     a[3, 5], a[7, 0], b[9, 11] = math.inf, math.nan, -math.inf
