@@ -701,7 +701,7 @@ def _patches_pay(dtype, pixels, cout, k, window, padded) -> bool:
 
 def _conv_indexable(x, w, oh, ow, stride, dilation, padding) -> bool:
     """What mimk_conv takes (30-bit coordinates, windows of up to 31 x 31 whose last tap is less than 2^31 elements from the first);
-    anything larger (or cropped by a negative padding) stays on the per-cell kernel."""
+    anything larger goes through a patch matrix, or bf16 of ragged extents to the per-cell kernel."""
     n, cin, h, wd = x.shape
     cout, _, kh, kw = w.shape
     return (max(kh, kw) <= 31 and min(oh, ow) >= 1 and min(*stride, *dilation) >= 1 and min(padding) >= 0
@@ -721,6 +721,10 @@ def _conv_as_contraction(xp, w, n, cin, cout, kh, kw, oh, ow, stride, dilation) 
     per_image = oh * ow * k * esize
     step = max(1, min(n, _CONV_PATCH_BYTES // max(per_image, 1)))
     w2 = w.contiguous().view(cout, k)
+    # f32 products with a short K and rows that are no multiple of four stay on the CUDA cores: a few filters of zeros, dropped below
+    extra = -cout % 4 if xp.dtype == torch.float32 else 0
+    if extra:
+        w2 = torch.cat([w2, torch.zeros((extra, k), dtype=w2.dtype, device=w2.device)])
     out = torch.empty((n, cout, oh, ow), dtype=xp.dtype, device=xp.device)
     # loops: 0 n, 1 oh, 2 ow, 3 ci, 4 kh, 5 kw
     mi = [[0] * 7 for _ in range(4)]
@@ -733,7 +737,9 @@ def _conv_as_contraction(xp, w, n, cin, cout, kh, kw, oh, ow, stride, dilation) 
         shape = (nb, oh, ow, cin, kh, kw)
         patches = map_reduce_post(shape, shape, L.F_FIRST, 0.0, L.P_ID, id_map(6), [mi], [xp[n0:n0 + nb].contiguous()],
                                   acc_dtype=torch.float32, out_dtype=xp.dtype)
-        y = product_2d(patches.view(nb * oh * ow, k), transpose_2d(w2))          # [(n, oh, ow), cout]
+        y = product_2d(patches.view(nb * oh * ow, k), transpose_2d(w2))          # [(n, oh, ow), cout + extra]
+        if extra:
+            y = y[:, :cout].contiguous()
         out[n0:n0 + nb] = transpose(y.view(nb, oh, ow, cout), (0, 3, 1, 2))
     return out
 
@@ -750,15 +756,17 @@ def conv(x: torch.Tensor, w: torch.Tensor, stride=(1, 1), dilation=(1, 1), paddi
     oh = (h + 2 * padding[0] - dilation[0] * (kh - 1) - 1) // stride[0] + 1
     ow = (wd + 2 * padding[1] - dilation[1] * (kw - 1) - 1) // stride[1] + 1
     k = cin * kh * kw
-    contraction = _conv_on_tensor_cores(x.dtype, n, cin, cout, kh, kw, oh, ow) and _conv_indexable(x, w, oh, ow, stride, dilation, padding)
+    contraction = _conv_on_tensor_cores(x.dtype, n, cin, cout, kh, kw, oh, ow)
+    as_patches = contraction and (x.dtype == torch.float32 or _whole_tiles(k, cout))   # extents the patch matrix is made for
+    gathered = contraction and _conv_indexable(x, w, oh, ow, stride, dilation, padding)
     if contraction and x.dtype != w.dtype:
-        if x.dtype == torch.float32 or _whole_tiles(k, cout):
+        if as_patches:
             raise TypeError("conv: both operands share the ring's element type")
-        contraction = False   # the per-cell kernel takes operands of two element types
-    if contraction:
-        if _patches_pay(x.dtype, n * oh * ow, cout, k, kh * kw, any(padding)):
-            xp = pad(x, (0, 0, padding[0], padding[1]), (0, 0, padding[0], padding[1])) if any(padding) else x
-            return _conv_as_contraction(xp, w, n, cin, cout, kh, kw, oh, ow, stride, dilation)
+        gathered = False   # the per-cell kernel takes operands of two element types
+    if as_patches and not (gathered and not _patches_pay(x.dtype, n * oh * ow, cout, k, kh * kw, any(padding))):
+        xp = pad(x, (0, 0, padding[0], padding[1]), (0, 0, padding[0], padding[1])) if any(padding) else x
+        return _conv_as_contraction(xp, w, n, cin, cout, kh, kw, oh, ow, stride, dilation)
+    if gathered:
         x, w = x.contiguous(), w.contiguous()
         out = torch.empty((n, cout, oh, ow), dtype=x.dtype, device=x.device)
         d = L.ConvDesc()

@@ -249,6 +249,26 @@ def test_convolutions_with_and_without_a_patch_matrix(T, monkeypatch, n, cin, h,
         close_cells(got, want, scale + 1e-6, BF16_ROUND if dtype == BF16 else TF32_CELL)
 
 
+@pytest.mark.parametrize("n,cin,h,w,cout,kh,kw,stride,dil,pad,dtype", [
+    (2, 3, 256, 259, 40, 32, 32, (32, 32), (1, 1), (0, 0), F32), (2, 3, 96, 128, 40, 32, 32, (32, 32), (1, 1), (0, 0), BF16),
+    (3, 3, 1, 700, 33, 1, 64, (1, 2), (1, 1), (0, 5), F32), (3, 2, 1, 700, 64, 1, 64, (1, 1), (1, 1), (0, 0), BF16),
+    (1, 20, 80, 9, 130, 33, 1, (1, 1), (2, 1), (3, 0), F32)])
+def test_windows_too_wide_to_gather_go_through_patches(T, monkeypatch, n, cin, h, w, cout, kh, kw, stride, dil, pad, dtype):
+    monkeypatch.setattr(T, "CONV_CONTRACTION_MIN_WORK", 1)
+    calls, through = [], T._conv_as_contraction
+    monkeypatch.setattr(T, "_conv_as_contraction", lambda *a: calls.append(1) or through(*a))
+    x, f = rnd((n, cin, h, w), 1, dtype), rnd((cout, cin, kh, kw), 2, dtype)
+    got = T.conv(x, f, stride=stride, dilation=dil, padding=pad)
+    T.device_status()
+    conv = torch.nn.functional.conv2d
+    want, scale = (conv(u, v, stride=stride, dilation=dil, padding=pad) for u, v in ((d64(x), d64(f)), (d64(x).abs(), d64(f).abs())))
+    close_cells(got, want, scale + 1e-6, F32_CELL if dtype == F32 else BF16_ROUND)
+    assert calls and got.is_contiguous()
+    other = BF16 if dtype == F32 else F32
+    with pytest.raises(TypeError):
+        T.conv(x, f.to(other), stride=stride, dilation=dil, padding=pad)
+
+
 @pytest.mark.parametrize("m,n,k,b_nk,post,out,offset", [
     (2000, 1003, 520, True, "bias_relu", BF16, 0), (300, 257, 1031, True, None, BF16, 0), (129, 255, 1033, False, "bias", F32, 0),
     (640, 5003, 264, False, None, BF16, 0), (640, 5001, 257, True, "bias_tanh", F32, 1), (65, 2056, 512, True, None, BF16, 1),
