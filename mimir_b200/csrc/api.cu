@@ -112,7 +112,8 @@ int gemm_tc_any(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* 
         const char* e = getenv("MIMK_GEMM_2CTA");
         allow_pair    = (e && e[0] == '0') ? 0 : ((e && e[0] == '2') ? 2 : 1);
     }
-    if (allow_pair != 2 && !gather && a_panels == 1 && gemm_tc_split_preferred(d, gated)) return gemm_tc_split(d, s, gated, b2);
+    // (by the extents alone, so that a gathered product, and one given as panels, has the bits of the plain one)
+    if (allow_pair != 2 && gemm_tc_split_preferred(d, gated)) return gemm_tc_split(d, s, gated, b2, gather, a_panels);
     // the paired kernel takes one launch per batch entry; long batches go to the one-CTA kernel, which walks
     // (batch, tile) pairs in a single launch
     if (allow_pair == 2 && d.batch <= 64 && gemm_tc_supported(d)) return gemm_tc2(d, s, gated, b2, gather, a_panels);

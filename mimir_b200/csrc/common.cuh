@@ -70,9 +70,10 @@ struct GemmPitch {
 int gemm_tc(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, const mimk_gather_dst* gather = nullptr,
             int64_t a_panels = 1, const GemmPitch* pitch = nullptr);
 int gemm_tc_ragged(const mimk_gemm_desc& d, cudaStream_t s);  // bf16 with extents or pointers TMA cannot take as they are
-// few tiles: narrower ones, their k-blocks dealt out to a cluster (gemm_tc_split.cu); takes what gemm_tc takes, one destination
+// few tiles: narrower ones, their k-blocks dealt out to a cluster (gemm_tc_split.cu); takes what gemm_tc takes
 int gemm_tc_split_preferred(const mimk_gemm_desc& d, int gated);
-int gemm_tc_split(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, const GemmPitch* pitch = nullptr);
+int gemm_tc_split(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, const mimk_gather_dst* gather = nullptr,
+                  int64_t a_panels = 1, const GemmPitch* pitch = nullptr);
 int gemm_tc2_enough(int64_t m, int64_t n, int gated);        // the paired kernel has tiles for every pair of SMs
 int gemm_tc2_supported(const mimk_gemm_desc& d, int gated);  // the paired-SM (cta_group::2) form
 // scatter_rows > 0 (gemm_tc2 only): rows [t scatter_rows, (t + 1) scatter_rows) of the f32 result are added into gather->dst[t]

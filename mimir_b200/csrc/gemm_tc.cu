@@ -598,7 +598,7 @@ int gemm_tc_ragged(const mimk_gemm_desc& d, cudaStream_t s) {
     }
     const GemmPitch pitch{r.pitch_a, r.pitch_b};
     // (a few more tiles than the aligned rule allows: the plain stores of a narrow tile's cells are spread over all its threads)
-    if (((t.m + 127) / 128) * ((t.n + 255) / 256) * t.batch < 74) return gemm_tc_split(t, s, 0, nullptr, &pitch);
+    if (((t.m + 127) / 128) * ((t.n + 255) / 256) * t.batch < 74) return gemm_tc_split(t, s, 0, nullptr, nullptr, 1, &pitch);
     if (t.batch <= 64 && gemm_tc2_enough(t.m, t.n, 0)) return gemm_tc2(t, s, 0, nullptr, nullptr, 1, 0, &pitch);
     return gemm_tc(t, s, 0, nullptr, nullptr, 1, &pitch);
 }

@@ -11,7 +11,8 @@
 //   warp 0      TMA producer    warp 1   MMA issuer, one accumulator
 //   warps 2..5  accumulator -> f32 partial tile in shared memory, over the stages
 //   all         after a cluster barrier: the partial tiles are added in rank order through distributed shared memory, each CTA
-//               a share of the cells, `post`, and stored with neighbouring lanes on neighbouring columns (any pitch and alignment)
+//               a share of the cells, `post`, and stored with neighbouring lanes on neighbouring columns (any pitch and alignment,
+//               one destination or each of a gather's)
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -32,10 +33,12 @@ struct Bars {
 static_assert(sizeof(Bars) <= 256, "barrier block too large");
 
 struct Params {
-    int64_t M, N, K, stride_c;
+    int64_t M, N, K, stride_c, ldc, col_off;
     int64_t tiles_m, tiles_n;
     int a_batched, b_batched, a_rows, stages, split, vec_c;
-    void* C;
+    int a_panel_kb, a_panel_rows;  // A as panels one below the other: k-blocks of a panel, rows from one to the next
+    int n_dst;
+    void* dst[MIMK_MAX_GATHER];
     const float* post_row;
     const void* post_full;
     int post;
@@ -103,7 +106,8 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
                 if (!mbar_wait(smem_u32(&bars->empty[stage]), phase ^ 1u, abort_flag)) break;
                 const uint32_t full = smem_u32(&bars->full[stage]), sa = tiles_at + stage * a_bytes, sb = b_at + stage * B_BYTES;
                 mbar_expect_tx(full, a_bytes + B_BYTES);
-                tma_load_3d(sa, &tmA, kb * BK, int(m0), za, full);
+                const int panel = kb / p.a_panel_kb;
+                tma_load_3d(sa, &tmA, (kb - panel * p.a_panel_kb) * BK, int(m0) + panel * p.a_panel_rows, za, full);
                 if (!B_MN) {
                     tma_load_3d(sb, &tmB, kb * BK, int(n0), zb, full);
                     if (GATED) tma_load_3d(sb + B_BYTES / 2, &tmB2, kb * BK, int(n0), zb, full);
@@ -168,7 +172,6 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     if (p.split > 1) cluster_sync();
 
     const int rows = int(p.M - m0 < BM ? p.M - m0 : BM);
-    TOut* C               = static_cast<TOut*>(p.C) + bz * p.stride_c;
     const TOut* post_full = p.post_full ? static_cast<const TOut*>(p.post_full) + bz * p.stride_c : nullptr;
     for (int i = rank * NUM_THREADS + tid; i < rows * (BNO / 4); i += p.split * NUM_THREADS) {
         const int r = i / (BNO / 4), c = (i % (BNO / 4)) * 4;
@@ -192,16 +195,18 @@ gemm_tc_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
             const float full = post_full ? float(post_full[row * p.N + col + e]) : 0.f;
             v[e]             = apply_post(p.post, v[e], rowv, full);
         }
-        TOut* dst = C + row * p.N + col;
-        if (p.vec_c) {  // four results are one aligned store, and N is a multiple of 4
-            if (sizeof(TOut) == 4)
-                *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
-            else
-                *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
-        } else {
+        for (int t = 0; t < p.n_dst; ++t) {
+            TOut* dst = static_cast<TOut*>(p.dst[t]) + bz * p.stride_c + row * p.ldc + p.col_off + col;
+            if (p.vec_c) {  // four results are one aligned store, and N is a multiple of 4
+                if (sizeof(TOut) == 4)
+                    *reinterpret_cast<float4*>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+                else
+                    *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
+            } else {
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (col + e < p.N) dst[e] = TOut(v[e]);
+                for (int e = 0; e < 4; ++e)
+                    if (col + e < p.N) dst[e] = TOut(v[e]);
+            }
         }
     }
     if (p.split > 1) cluster_sync();  // no CTA of the cluster exits while another may read its partial tile
@@ -264,14 +269,17 @@ int gemm_tc_split_preferred(const mimk_gemm_desc& d, int gated) {
     return d.m <= 32 ? d.k >= 8 * BK && tiles <= 74 : d.k >= 16 * BK && tiles <= (gated ? 24 : 16);
 }
 
-int gemm_tc_split(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, const GemmPitch* pitch) {
+int gemm_tc_split(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, const mimk_gather_dst* gather, int64_t a_panels,
+                  const GemmPitch* pitch) {
+    if (a_panels < 1 || (a_panels > 1 && (d.batch != 1 || pitch || d.k % a_panels != 0 || (d.k / a_panels) % BK != 0)) || (gather && d.batch != 1))
+        return MIMK_E_UNSUPPORTED;
     int st          = MIMK_OK;
     DeviceInfo* dev = device_info(&st);
     if (!dev) return st;
     const bool b_mn = d.b_layout == MIMK_B_KN;
     const bool a_b = d.batch > 1 && d.stride_a != 0, b_b = d.batch > 1 && d.stride_b != 0;
     const uint64_t na = a_b ? uint64_t(d.batch) : 1, nb = b_b ? uint64_t(d.batch) : 1;
-    const uint64_t lda = pitch ? uint64_t(pitch->a) : uint64_t(d.k), ldb = pitch ? uint64_t(pitch->b) : uint64_t(b_mn ? d.n : d.k);
+    const uint64_t kp = uint64_t(d.k / a_panels), lda = pitch ? uint64_t(pitch->a) : kp, ldb = pitch ? uint64_t(pitch->b) : uint64_t(b_mn ? d.n : d.k);
     // (the outermost stride of a one-entry operand is never used; it only has to be a legal value)
     const uint64_t sa = a_b ? uint64_t(d.stride_a) * 2 : lda * 2, sb = b_b ? uint64_t(d.stride_b) * 2 : ldb * 2;
     const int64_t tiles_m = (d.m + BM - 1) / BM, kb = (d.k + BK - 1) / BK;
@@ -289,12 +297,19 @@ int gemm_tc_split(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void
     const int64_t items = p.tiles_m * p.tiles_n * d.batch;
     p.split = 1;
     while (p.split < 8 && items * p.split * 2 <= 2 * dev->sm_count && kb >= p.split * 8) p.split *= 2;
-    p.C = d.c, p.post_row = static_cast<const float*>(d.post_row), p.post_full = d.post_full, p.post = d.post;
-    p.vec_c  = d.n % 4 == 0 && aligned16(d.c) && p.stride_c % 4 == 0;
+    p.a_panel_kb = a_panels > 1 ? int(kp / BK) : int(kb), p.a_panel_rows = a_panels > 1 ? int(d.m) : 0;
+    p.n_dst = 1, p.dst[0] = d.c, p.ldc = d.n;
+    if (gather) {
+        p.n_dst = gather->n_dst, p.ldc = gather->ldc, p.col_off = gather->col_off;
+        for (int t = 0; t < gather->n_dst; ++t) p.dst[t] = gather->dst[t];
+    }
+    p.post_row = static_cast<const float*>(d.post_row), p.post_full = d.post_full, p.post = d.post;
+    p.vec_c = d.n % 4 == 0 && p.ldc % 4 == 0 && p.col_off % 4 == 0 && p.stride_c % 4 == 0;
+    for (int t = 0; t < p.n_dst; ++t) p.vec_c = p.vec_c && aligned16(p.dst[t]);
     p.status = dev->status_dev;
     const void* B2 = b2 ? b2 : d.b;
     CUtensorMap tA, tB, tB2;
-    MIMK_TRY(make_tmap_bf16_3d(&tA, d.a, uint64_t(d.k), uint64_t(d.m), na, lda * 2, sa, BK, uint32_t(p.a_rows)));
+    MIMK_TRY(make_tmap_bf16_3d(&tA, d.a, kp, uint64_t(d.m) * uint64_t(a_panels), na, lda * 2, sa, BK, uint32_t(p.a_rows)));
     if (b_mn) {
         MIMK_TRY(make_tmap_bf16_3d(&tB, d.b, uint64_t(d.n), uint64_t(d.k), nb, ldb * 2, sb, 64, BK));
         MIMK_TRY(make_tmap_bf16_3d(&tB2, B2, uint64_t(d.n), uint64_t(d.k), nb, ldb * 2, sb, 64, BK));

@@ -329,3 +329,34 @@ def test_gated_mlp_of_few_rows(T, m, k, f, n, b_nk):
     want, terms = h @ d64(w[2]), h.abs() @ d64(w[2]).abs()
     # the hidden layer is rounded to bf16: 2^-9 of every term, like the result itself
     assert ((d64(got) - want).abs() <= BF16_ROUND * (want.abs() + terms) + 1e-6).all()
+
+
+@pytest.mark.parametrize("m,panels,kp,n", [(300, 8, 256, 264), (16, 4, 512, 2048), (129, 2, 1024, 72), (5, 16, 64, 1000)])
+@pytest.mark.parametrize("b_nk", [True, False])
+def test_products_of_few_tiles_keep_their_bits_as_panels_and_gathered(T, m, panels, kp, n, b_nk):
+    from mimir_b200 import _lib as L
+    import ctypes as C
+    k = panels * kp
+    a, b, b2 = rnd((m, k), 1, BF16), rnd((n, k) if b_nk else (k, n), 2, BF16), rnd((n, k) if b_nk else (k, n), 3, BF16)
+    want = T.product_2d(a, b.t() if b_nk else b)
+    got = T.product_2d_panels(a.view(m, panels, kp).transpose(0, 1).contiguous(), b.t() if b_nk else b)
+    T.device_status()
+    assert torch.equal(got, want)
+    # the gated block's hidden layer, and both gathered into three copies of a wider matrix
+    hidden = torch.empty((m, n), dtype=BF16, device="cuda")
+    w2 = rnd((8, n) if b_nk else (n, 8), 4, BF16)
+    T.mlp_gated(a, *((w.t() if b_nk else w) for w in (b, b2, w2)), h=hidden)
+    for second, whole in ((None, want), (b2, hidden)):
+        copies = [torch.full((m, n + 24), 3.0, dtype=BF16, device="cuda") for _ in range(3)]
+        d = L.GemmDesc()
+        d.batch, d.m, d.n, d.k = 1, m, n, k
+        d.a, d.b = a.data_ptr(), b.data_ptr()
+        d.in_dtype, d.out_dtype, d.b_layout, d.post = L.BF16, L.BF16, L.B_NK if b_nk else L.B_KN, L.POST_ID
+        g = L.GatherDst()
+        g.n_dst, g.ldc, g.col_off = 3, n + 24, 8
+        for i, t in enumerate(copies):
+            g.dst[i] = t.data_ptr()
+        L.check(L.lib().mimk_gemm_gather(C.byref(d), second.data_ptr() if second is not None else None, C.byref(g), T._stream()), "gather")
+        T.device_status()
+        for t in copies:
+            assert torch.equal(t[:, 8:8 + n], whole) and (t[:, :8] == 3.0).all() and (t[:, 8 + n:] == 3.0).all()
