@@ -83,6 +83,7 @@ int gemm_tc_any(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* 
                 const mimk_gather_dst* gather = nullptr, int64_t a_panels = 1);  // picks between the two
 int gemm_f32_tc_supported(const mimk_gemm_desc& d);  // f32 operands on the tensor cores (three bf16 pieces each)
 int gemm_f32_tc(const mimk_gemm_desc& d, cudaStream_t s);
+double gemm_f32_tc_us(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count);  // its time estimate
 int gemm_bf16_chunked(const mimk_gemm_desc& d, cudaStream_t s);  // bf16 operands of any extent and alignment, f32 result
 // results with many tiles: the operands cut beforehand, three TF32 products (gemm_tf32.cu)
 int gemm_tf32_preferred(const mimk_gemm_desc& d, int sm_count, double pieces_us);

@@ -518,7 +518,8 @@ Plan make_plan(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count) {
     for (int wide = 0; wide < 2; ++wide)
         for (int split = 1; split <= 8 && split <= chunks; split *= 2) {
             const int64_t items = tiles_m * ((n + (wide ? 127 : 63)) / (wide ? 128 : 64)) * batch;
-            const int64_t room  = split == 1 ? sm_count : split == 2 ? sm_count / 2 - 4 : split == 4 ? sm_count / 4 - 5 : sm_count / 8 - 3;
+            int64_t room        = split == 1 ? sm_count : split == 2 ? sm_count / 2 - 4 : split == 4 ? sm_count / 4 - 5 : sm_count / 8 - 3;
+            if (room < 1) room = 1;  // (a slice of a GPU)
             const double rounds = double((items + room - 1) / room);
             const int per       = (chunks + split - 1) / split * CHUNK;
             const double time   = rounds * ((split > 1 ? 9.0 : 8.0) + (per < kb ? per : kb) * (wide ? 1.15 : 0.95));
@@ -543,6 +544,7 @@ static int extents_fit(const mimk_gemm_desc& d) {
     const int64_t tiles = ((d.m + BM - 1) / BM) * ((d.n + 63) / 64);
     return tiles < (int64_t(1) << 28) && d.batch < (int64_t(1) << 28) && tiles * d.batch < (int64_t(1) << 28);  // one grid
 }
+double gemm_f32_tc_us(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count) { return make_plan(m, n, k, batch, sm_count).us; }
 int gemm_f32_tc_supported(const mimk_gemm_desc& d) { return d.in_dtype == MIMK_F32 && extents_fit(d); }
 
 static Params product_params(const mimk_gemm_desc& d, const DeviceInfo& dev) {
@@ -563,7 +565,7 @@ int gemm_f32_tc(const mimk_gemm_desc& d, cudaStream_t s) {
     int st          = MIMK_OK;
     DeviceInfo* dev = device_info(&st);
     if (!dev) return st;
-    if (gemm_tf32_preferred(d, dev->sm_count, make_plan(d.m, d.n, d.k, d.batch, dev->sm_count).us)) {
+    if (gemm_tf32_preferred(d, dev->sm_count, gemm_f32_tc_us(d.m, d.n, d.k, d.batch, dev->sm_count))) {
         const int r = gemm_tf32(d, s);
         if (r != MIMK_E_UNSUPPORTED) return r;
     }

@@ -161,3 +161,13 @@ def test_convolution_offsets_fit_their_32_bits(lib, cin, h, w, kh, kw, dil, pad,
     assert T._conv_indexable(x, f, oh, ow, (1, 1), dil, pad) == fits
     # (no operands: a shape that is taken fails at the next check, for want of a device or of a pointer)
     assert (lib.lib().mimk_conv(C.byref(d), None) == 8) == (not fits)
+
+
+def test_f32_contraction_estimate_on_any_number_of_sms(lib):
+    """The kernel choice of f32 products divides by the clusters that fit on the device, also where none of eight does (a slice
+    of a GPU)."""
+    estimate = lib.lib()["_ZN4mimk14gemm_f32_tc_usElllli"]
+    estimate.restype, estimate.argtypes = C.c_double, [C.c_int64] * 4 + [C.c_int]
+    for sms in list(range(1, 60)) + [132, 148, 160]:
+        for m, n, k in ((256, 256, 256), (100, 3000, 4096), (1, 64, 100000)):
+            assert 0 < estimate(m, n, k, 1, sms) < 1e12
