@@ -260,8 +260,9 @@ extern "C" int mimk_attn_fwd(const mimk_attn_desc* d, void* stream) {
     if (!d) return MIMK_E_ARG;
     if (d->batch_heads < 0 || d->seq_q < 0 || d->seq_k < 0 || d->head_dim < 0) return MIMK_E_ARG;
     if (d->dtype != MIMK_F32 && d->dtype != MIMK_BF16) return MIMK_E_DTYPE;
-    int st = MIMK_OK;
-    if (!device_info(&st)) return st;
+    int st                = MIMK_OK;
+    const DeviceInfo* dev = device_info(&st);
+    if (!dev) return st;
     if (d->batch_heads == 0 || d->seq_q == 0 || d->head_dim == 0) return MIMK_OK;
     if (!d->q || !d->o || (d->seq_k > 0 && (!d->k || !d->v))) return MIMK_E_ARG;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -282,7 +283,7 @@ extern "C" int mimk_attn_fwd(const mimk_attn_desc* d, void* stream) {
         const char* e = getenv("MIMK_F32_TC");
         f32_tc        = (e && e[0] == '0') ? 0 : 1;
     }
-    if (f32_tc && attn_f32_tc_supported(*d)) return attn_f32_tc(*d, s);
+    if (f32_tc && attn_f32_tc_supported(*d)) return attn_simt_preferred(*d, dev->sm_count) ? attn_simt(*d, s) : attn_f32_tc(*d, s);
     if (composed < 0) {
         const char* e = getenv("MIMK_ATTN_COMPOSED");
         composed      = (e && e[0] == '0') ? 0 : 1;

@@ -123,6 +123,7 @@ MrpPlan mrp_plan(const mimk_mrp_desc& d);
 // axis permutation as a tiled copy (permute.cu); perm[j] = the output loop that indexes input axis j
 int permute_copy(const void* in, void* out, int esize, int rank, const int64_t* out_shape, const int* perm, cudaStream_t s);
 int attn_simt(const mimk_attn_desc& d, cudaStream_t s);
+int attn_simt_preferred(const mimk_attn_desc& d, int sm_count);  // f32 with so few keys that a warp per row is ahead
 // f32, head_dim up to 128: fused, on the tensor cores, three bf16 pieces per value (attn_f32_tc.cu)
 int attn_f32_tc_supported(const mimk_attn_desc& d);
 int attn_f32_tc(const mimk_attn_desc& d, cudaStream_t s);

@@ -86,6 +86,17 @@ def test_f32_attention_of_any_length(T, bh, sq, sk, d, causal):
     assert torch.equal(got, T.attention(q, k, v, scale=d ** -0.5, causal=causal))
 
 
+@pytest.mark.parametrize("d", [16, 64, 128])
+@pytest.mark.parametrize("bh,sq,sk", [(1, 3, 1), (1, 3, 24), (700, 2, 20), (700, 40, 20), (700, 2, 64)])
+def test_f32_attention_of_few_keys(T, bh, sq, sk, d):
+    # a warp per row up to some number of rows and keys, which lies between these
+    q, k, v = rnd((bh, sq, d), 1), rnd((bh, sk, d), 2), rnd((bh, sk, d), 3)
+    got, lse = T.attention(q, k, v, scale=d ** -0.5, return_lse=True)
+    T.device_status()
+    want, want_lse = attention_reference(q, k, v, d ** -0.5, False)
+    assert ((d64(got) - want).abs() <= 64 * F32_CELL).all() and ((d64(lse) - want_lse).abs() <= 64 * F32_CELL).all()
+
+
 def test_f32_attention_with_infinities_takes_the_general_path(T):
     q, k, v = rnd((2, 300, 64), 1), rnd((2, 200, 64), 2), rnd((2, 200, 64), 3)
     q[0, 5, 3], k[1, 7, 2], v[0, 9, 1], v[1, 8, 1] = math.inf, -math.inf, math.nan, math.inf
