@@ -385,41 +385,62 @@ __global__ void map_kernel(int op, const TIn* __restrict__ x, const TIn* __restr
 // divisible by 4, and a broadcast operand whose index is constant over the four elements (y_mode 1 with inner == 1 and
 // len % 4 == 0) or runs with them (y_mode 0; y_mode 2 with (len * inner) % 4 == 0; y_mode 1 with inner % 4 == 0).
 // Bound by memory: a [32, 2048, 512] f32 scaling with its activation took 164 us through the scalar form and takes 40 (6.7 TB/s).
-template <class TIn, class TOut>
+// WIDE: two accesses per thread and step, and the operator dispatched once for eight elements. For composed operators, whose two
+// dispatches cost more than the bytes (|x - y| of 2^23 bf16: 13.7 -> 8.4 us), and for operands that run with the innermost extents,
+// whose index costs divisions, and unary operators on bf16, where an access is 8 bytes, as soon as every thread has two of them (tanh of
+// 2^24: 20.1 -> 17.6). The other plain operators one access at a time: two took longer (x y of 2^26 bf16 83 against 93 us, tanh of
+// 2^26 f32 86 / 94, a row scaling of [32, 2048, 512] f32 43 / 49).
+template <bool WIDE, class TIn, class TOut>
 __global__ void __launch_bounds__(256) map_vec4_kernel(int op, const TIn* __restrict__ x, const TIn* __restrict__ y,
                                                       TOut* __restrict__ out, int64_t total4, int64_t len, int64_t inner,
                                                       int64_t period4, int y_mode) {
-    auto second = [&](int64_t t) {
-        if (y_mode == 0) return load4(y + 4 * t);
-        if (y_mode == 1 && inner == 1) {
-            const float v = ldf(y, (4 * t) / len);
-            return make_float4(v, v, v, v);
-        }
-        if (y_mode == 1) {
-            const int64_t in4 = inner >> 2;
-            int64_t o, i;
-            if (total4 <= 0xffffffffLL && len <= 0xffffffffLL) {  // 32-bit divisions, as above
-                const uint32_t row = uint32_t(t) / uint32_t(in4);
-                i = uint32_t(t) - row * uint32_t(in4), o = row / uint32_t(len);
-            } else {
-                const int64_t row = t / in4;
-                i = t - row * in4, o = row / len;
-            }
-            return load4_cached(y + 4 * (o * in4 + i));
-        }
-        if (y_mode == 2) return load4_cached(y + 4 * (t % period4));
-        return make_float4(0.f, 0.f, 0.f, 0.f);
-    };
-    // Two accesses per thread and step: twice the bytes on their way, and the operator is dispatched once for eight elements.
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < total4; t += 2 * stride) {
-        const int64_t u = t + stride < total4 ? t + stride : t;
-        const float4 a0 = load4(x + 4 * t), a1 = load4(x + 4 * u), b0 = second(t), b1 = second(u);
-        float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-        const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-        apply_op_n(op, a, b);
-        store4(out + 4 * t, make_float4(a[0], a[1], a[2], a[3]));
-        if (u != t) store4(out + 4 * u, make_float4(a[4], a[5], a[6], a[7]));
+    if constexpr (WIDE) {
+        auto second = [&](int64_t t) {
+            if (y_mode == 0) return load4(y + 4 * t);
+            if (y_mode == 1 && inner == 1) {
+                const float v = ldf(y, (4 * t) / len);
+                return make_float4(v, v, v, v);
+            }
+            if (y_mode == 1) {
+                const int64_t in4 = inner >> 2;
+                int64_t o, i;
+                if (total4 <= 0xffffffffLL && len <= 0xffffffffLL) {  // 32-bit divisions, as above
+                    const uint32_t row = uint32_t(t) / uint32_t(in4);
+                    i = uint32_t(t) - row * uint32_t(in4), o = row / uint32_t(len);
+                } else {
+                    const int64_t row = t / in4;
+                    i = t - row * in4, o = row / len;
+                }
+                return load4_cached(y + 4 * (o * in4 + i));
+            }
+            if (y_mode == 2) return load4_cached(y + 4 * (t % period4));
+            return make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < total4; t += 2 * stride) {
+            const int64_t u = t + stride < total4 ? t + stride : t;
+            const float4 a0 = load4(x + 4 * t), a1 = load4(x + 4 * u), b0 = second(t), b1 = second(u);
+            float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+            const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+            apply_op_n(op, a, b);
+            store4(out + 4 * t, make_float4(a[0], a[1], a[2], a[3]));
+            if (u != t) store4(out + 4 * u, make_float4(a[4], a[5], a[6], a[7]));
+        }
+        return;
+    }
+    for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < total4; t += stride) {
+        const float4 a = load4(x + 4 * t);
+        float4 b       = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (y_mode == 0) {
+            b = load4(y + 4 * t);
+        } else if (y_mode == 1) {
+            const float v = ldf(y, (4 * t) / len);
+            b             = make_float4(v, v, v, v);
+        } else if (y_mode == 2) {
+            b = load4_cached(y + 4 * (t % period4));
+        }
+        store4(out + 4 * t, make_float4(apply_op_plain(op, a.x, b.x), apply_op_plain(op, a.y, b.y), apply_op_plain(op, a.z, b.z),
+                                        apply_op_plain(op, a.w, b.w)));
     }
 }
 
@@ -780,10 +801,14 @@ int map_impl(int op, const TIn* x, const TIn* y, void* out, int out_dtype, int64
     if (total % 4 == 0 && al(x) && out_al && y_ok) {
         const int64_t total4 = total / 4, period4 = y_mode == 2 ? (len * inner) / 4 : 1;
         const int vgrid      = grid_for(total4, 256, dev.sm_count, 8);
-        if (out_dtype == MIMK_F32)
-            map_vec4_kernel<<<vgrid, 256, 0, s>>>(op, x, y, static_cast<float*>(out), total4, len, inner, period4, y_mode);
-        else
-            map_vec4_kernel<<<vgrid, 256, 0, s>>>(op, x, y, static_cast<__nv_bfloat16*>(out), total4, len, inner, period4, y_mode);
+        const bool wide      = (op & MIMK_OP_COMPOSED_BASE) || (y_mode == 1 && inner > 1) ||
+                          (sizeof(TIn) == 2 && y_mode == 3 && total4 >= 2 * 256 * int64_t(vgrid));
+        auto run             = [&](auto* dst) {
+            if (wide) map_vec4_kernel<true><<<vgrid, 256, 0, s>>>(op, x, y, dst, total4, len, inner, period4, y_mode);
+            else map_vec4_kernel<false><<<vgrid, 256, 0, s>>>(op, x, y, dst, total4, len, inner, period4, y_mode);
+        };
+        if (out_dtype == MIMK_F32) run(static_cast<float*>(out));
+        else run(static_cast<__nv_bfloat16*>(out));
         return launch_status();
     }
     const int grid = grid_for(total, 256, dev.sm_count, 8);
