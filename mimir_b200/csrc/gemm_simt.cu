@@ -256,15 +256,17 @@ int launch(const mimk_gemm_desc& d, cudaStream_t s) {
 // Where f32 products stay on the CUDA cores (times: CUDA-graph replays, warm, CUDA cores against tensor cores).
 //   batches below 2^25 multiply-adds      64 of 64^3: 4.5 / 8.4 us; above: 10 of 76 x 704 x 448, 33.6 / 19.1
 //   K <= 256: below 5 * 2^24 where the small-tile kernel applies (256^3: 6.2 / 7.8 us; 815 x 524 x 168: 13 / 15;
-//             784 x 1024 x 128: 13.9 / 10.7), else 2^24
-//             (245 x 674 x 146: 15.3 / 10.0); and a result whose rows are no multiple of four, so that any part of it has the
-//             bits of the small product of the same rows and columns
+//             784 x 1024 x 128: 13.9 / 10.7), else 2^24 (245 x 674 x 146: 15.3 / 10.0).
+//             Rows that are no multiple of four below 20 * 2^24: any part of such a product has the bits of the small product of the
+//             same rows and columns, which is worth more there than the time (1280 x 961 x 256: 60 / 25; x 128: 34 / 20; 4096 x 250 x
+//             17: 8.5 / 10.5). Above, K <= 32 only (4096 x 4001 x 17: 97 / 101; x 64: 144 / 112; x 256: 408 / 171)
 //   longer K: only what is hardly any work (the CUDA cores walk all of K in one CTA: 32 x 1024 x 1024, 19.0 / 11.2)
 int gemm_simt_preferred(const mimk_gemm_desc& d) {
     const double work = double(d.m) * double(d.n) * double(d.k);
     if (d.batch > 1) return work * double(d.batch) < double(1 << 25);
     if (d.k > 256) return d.k < 1024 && work < double(1 << 20);
-    return d.n % 4 != 0 || work < (small_tiles_apply(d) ? double(5 << 24) : double(1 << 24));
+    if (d.n % 4 != 0 && (d.k <= 32 || work < double(20 << 24))) return 1;
+    return work < (small_tiles_apply(d) ? double(5 << 24) : double(1 << 24));
 }
 
 int gemm_simt(const mimk_gemm_desc& d, cudaStream_t s) {

@@ -58,6 +58,17 @@ elif what == "gemm_f32":
     c = T.product_2d(a, b)
     T.device_status()
     assert nerr(f64(c), mo.gemm_truth(a.cpu().numpy(), b.cpu().numpy())) <= TOL_F32
+elif what == "gemm_f32_kernels":
+    # the small-tile kernel beyond the two stages that K = 256 fills, bit for bit against the 64 x 64 kernel
+    for m, n, K in ((96, 80, 520), (7, 260, 1028), (33, 64, 300)):
+        for nk in (False, True):
+            a, b = uniform((1280, K), 500 + K), uniform((961, K) if nk else (K, 961), 501 + K)
+            big = T.product_2d(a, T.transpose_2d(b) if nk else b)
+            bs = b[:n].contiguous() if nk else b[:, :n].contiguous()
+            small = T.product_2d(a[:m].contiguous(), T.transpose_2d(bs) if nk else bs)
+            T.device_status()
+            assert torch.equal(small, big[:m, :n])
+            assert nerr(f64(small), mo.gemm_truth(a[:m].cpu().numpy(), bs.cpu().numpy(), b_nk=nk)) <= TOL_F32
 elif what == "mrp":
     # instances the recognisers would hand to the contraction / fold kernels: here they stay on the per-cell kernel
     from mimir_b200 import _lib as L
@@ -77,6 +88,7 @@ CASES = [
     ("MIMK_GEMM_2CTA", "0", "gemm_bf16"),       # bf16 contraction on the one-CTA kernel only
     ("MIMK_GEMM_2CTA", "2", "gemm_bf16"),       # ... and on the paired kernel whenever it can run
     ("MIMK_F32_TC", "0", "gemm_f32"),           # f32 contraction on the CUDA cores
+    ("MIMK_F32_TC", "0", "gemm_f32_kernels"),   # ... and both of its kernels, the same bits
     ("MIMK_MRP_ROUTE", "0", "mrp"),             # every map_reduce_post instance on the per-cell kernel
 ]
 
