@@ -33,19 +33,34 @@ struct Chain {
 
 double lanes(double v, double vec) { return std::ceil(v / vec) * vec; }
 
-// Figures of this library's own kernels on one B200: bf16 contraction 1.45 PFLOP/s sustained (128 x 256 tiles, K-step
-// 64), f32 contraction as three TF32 products 0.21 PFLOP/s (128 x 128 tiles, K-step 32), 6.4 TB/s of HBM, 148 SMs.
+// Figures of this library's own kernels on one B200: 148 SMs, 6.4 TB/s of HBM, 4 us for a launch.
+// bf16: 1.45 PFLOP/s sustained in tiles of 128 x 256, K-step 64; with few tiles the time of gemm_tc_split.cu, which deals the k-blocks
+// of 128-column tiles out over the chip, up to eight CTAs to a tile: 8 us and 0.3 us per k-block of an SM's share (300 x 200 x 16000:
+// 17.4 us estimated, 16.7 measured; 256 x 4096 x 4096: 16.3 / 17.7; 5000 x 64 x 8192: 18.4 / 17.7; 16 x 14336 x 4096: 22.5 / 24.3).
+// f32: the least of the estimates that choose between its two tensor-core kernels, and the CUDA cores at 12 TFLOP/s for the
+// products that stay there (256^3: 6.8 us / 6.2).
 constexpr double SMS = 148.0, HBM_BPS = 6.4e12, LAUNCH_S = 4e-6;
 
 double b200_product(double m, double k, double n, int dtype) {
-    const bool half   = dtype == MIMK_BF16;
-    const double tm   = 128.0, tn = half ? 256.0 : 128.0, tk = half ? 64.0 : 32.0;
-    const double peak = half ? 1.45e15 : 0.21e15;
-    const double es   = half ? 2.0 : 4.0;
+    const double es    = dtype == MIMK_BF16 ? 2.0 : 4.0;
+    const double t_mem = (m * k + k * n + m * n) * es / HBM_BPS;
+    mimk_gemm_desc d   = {};
+    d.batch = 1, d.m = int64_t(m), d.n = int64_t(n), d.k = int64_t(k), d.b_layout = MIMK_B_KN;
+    d.in_dtype = d.out_dtype = dtype;
+    if (dtype == MIMK_F32) {
+        if (m * n * k == 0 || gemm_simt_preferred(d)) return std::fmax(2.0 * m * n * k / 12e12, t_mem) + LAUNCH_S;
+        double us = gemm_f32_tc_us(d.m, d.n, d.k, 1, int(SMS));
+        if (gemm_tf32_preferred(d, int(SMS), us)) us = gemm_tf32_us(d.m, d.n, d.k, 1, int(SMS));
+        return std::fmax(us * 1e-6, t_mem + LAUNCH_S);
+    }
+    const double tm = 128.0, tn = 256.0, tk = 64.0, peak = 1.45e15;
     const double tiles = std::ceil(m / tm) * std::ceil(n / tn);
     const double waves = std::ceil(tiles / SMS);
     const double t_tc  = waves * (2.0 * tm * tn * lanes(k, tk)) / (peak / SMS);
-    const double t_mem = (m * k + k * n + m * n) * es / HBM_BPS;
+    if (gemm_tc_split_preferred(d, 0)) {
+        const double share = std::fmax(std::ceil(m / tm) * std::ceil(n / 128.0) * std::ceil(k / tk) / SMS, std::ceil(k / tk) / 8.0);
+        return std::fmin(std::fmax(t_tc, t_mem) + LAUNCH_S, std::fmax(8e-6 + 0.3e-6 * share, t_mem + LAUNCH_S));
+    }
     return std::fmax(t_tc, t_mem) + LAUNCH_S;
 }
 

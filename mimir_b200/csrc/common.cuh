@@ -88,6 +88,7 @@ int gemm_bf16_chunked(const mimk_gemm_desc& d, cudaStream_t s);  // bf16 operand
 // results with many tiles: the operands cut beforehand, three TF32 products (gemm_tf32.cu)
 int gemm_tf32_preferred(const mimk_gemm_desc& d, int sm_count, double pieces_us);
 int gemm_tf32(const mimk_gemm_desc& d, cudaStream_t s);
+double gemm_tf32_us(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count);
 int conv_tc(const mimk_conv_desc& d, cudaStream_t s);  // the same kernel, its left operand gathered from an image
 // map_reduce_post instances that are a contraction, an axis fold or an elementwise map go to those kernels (mrp_route.cu)
 bool mrp_try_route(const mimk_mrp_desc& d, void* stream, int* status);

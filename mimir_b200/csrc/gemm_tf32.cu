@@ -409,10 +409,16 @@ int launch(const CUtensorMap& ah, const CUtensorMap& al, const CUtensorMap& bh, 
 
 }  // namespace
 
-// Many tiles of 128 x 128 and rows of 16-byte pieces, where the estimate is below that of gemm_f32_tc.cu (`pieces_us`):
-// per batch entry 5 us of launches, the operands read once and written twice (6 TB/s), and rounds of one tile per SM at 3.8 us
+// Per batch entry 5 us of launches, the operands read once and written twice (6 TB/s), and rounds of one tile per SM at 3.8 us
 // + 0.64 us per k-block. It lies within 10 % of the measured 50 us (1536^3), 37 (2048 x 2048 x 512), 65 (4096 x 4096 x 256),
 // 650 (4096^3), 101 (1024 x 1024 x 4096), 35 per entry of a batch of 1024^3.
+double gemm_tf32_us(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count) {
+    const int64_t tiles = ((m + BM - 1) / BM) * ((n + BN - 1) / BN);
+    const double rounds = double((tiles + sm_count - 1) / sm_count), kb = double((k + BK - 1) / BK);
+    return double(batch) * (5.0 + 12.0 * double(k) * double(m + n) / 6e6 + rounds * (3.8 + 0.64 * kb));
+}
+
+// Many tiles of 128 x 128 and rows of 16-byte pieces, where the estimate is below that of gemm_f32_tc.cu (`pieces_us`).
 // Below 2^27 multiply-adds the CUDA cores were ahead of the three launches, and are more accurate.
 int gemm_tf32_preferred(const mimk_gemm_desc& d, int sm_count, double pieces_us) {
     if (d.in_dtype != MIMK_F32 || d.k <= 0) return 0;
@@ -423,12 +429,8 @@ int gemm_tf32_preferred(const mimk_gemm_desc& d, int sm_count, double pieces_us)
     if (d.batch > 1 && d.stride_c % (d.out_dtype == MIMK_BF16 ? 8 : 4) != 0) return 0;  // of every entry
     if (d.post_full && !aligned16(d.post_full)) return 0;
     if (d.b_layout != MIMK_B_NK && (d.k + 31) / 32 > 65535) return 0;  // grid of the transposing split
-    const double m = double(d.m), n = double(d.n), k = double(d.k);
-    if (m * n * k * double(d.batch) < double(1 << 27)) return 0;
-    const int64_t tiles = ((d.m + BM - 1) / BM) * ((d.n + BN - 1) / BN);
-    const double rounds = double((tiles + sm_count - 1) / sm_count), kb = double((d.k + BK - 1) / BK);
-    const double us     = double(d.batch) * (5.0 + 12.0 * k * (m + n) / 6e6 + rounds * (3.8 + 0.64 * kb));
-    return us < pieces_us;
+    if (double(d.m) * double(d.n) * double(d.k) * double(d.batch) < double(1 << 27)) return 0;
+    return gemm_tf32_us(d.m, d.n, d.k, d.batch, sm_count) < pieces_us;
 }
 
 // MIMK_E_UNSUPPORTED, with nothing launched, where the copies' buffer cannot be had: under stream capture (a graph must not
