@@ -173,6 +173,15 @@ static int check_gemm(const mimk_gemm_desc* d) {
     return MIMK_OK;
 }
 
+// MIMK_F32_TC=0 keeps f32 contractions and attention on the CUDA cores (for A/B measurements)
+static bool f32_on_tensor_cores() {
+    static const bool on = [] {
+        const char* e = getenv("MIMK_F32_TC");
+        return !(e && e[0] == '0');
+    }();
+    return on;
+}
+
 extern "C" int mimk_gemm(const mimk_gemm_desc* d, void* stream) {
     MIMK_TRY(check_gemm(d));
     int st = MIMK_OK;
@@ -185,12 +194,7 @@ extern "C" int mimk_gemm(const mimk_gemm_desc* d, void* stream) {
         const int r = gemm_tc_ragged(*d, s);
         if (r != MIMK_E_UNSUPPORTED) return r;
     }
-    static int f32_tc = -1;  // MIMK_F32_TC=0 keeps f32 contractions on the CUDA cores (for A/B measurements)
-    if (f32_tc < 0) {
-        const char* e = getenv("MIMK_F32_TC");
-        f32_tc        = (e && e[0] == '0') ? 0 : 1;
-    }
-    if (f32_tc && gemm_f32_tc_supported(*d) && !gemm_simt_preferred(*d)) return gemm_f32_tc(*d, s);
+    if (f32_on_tensor_cores() && gemm_f32_tc_supported(*d) && !gemm_simt_preferred(*d)) return gemm_f32_tc(*d, s);
     return gemm_simt(*d, s);
 }
 
@@ -278,12 +282,7 @@ extern "C" int mimk_attn_fwd(const mimk_attn_desc* d, void* stream) {
     if (attn_few_supported(*d) && !(attn_tc_persistent_supported(*d) && attn_heads_fill(*d))) return attn_few(*d, s);
     if (attn_tc_persistent_supported(*d)) return attn_tc_persistent(*d, s);
     static int composed = -1;  // MIMK_ATTN_COMPOSED=0 keeps every such problem on the one-launch CUDA-core kernel
-    static int f32_tc = -1;
-    if (f32_tc < 0) {
-        const char* e = getenv("MIMK_F32_TC");
-        f32_tc        = (e && e[0] == '0') ? 0 : 1;
-    }
-    if (f32_tc && attn_f32_tc_supported(*d)) return attn_simt_preferred(*d, dev->sm_count) ? attn_simt(*d, s) : attn_f32_tc(*d, s);
+    if (f32_on_tensor_cores() && attn_f32_tc_supported(*d)) return attn_simt_preferred(*d, dev->sm_count) ? attn_simt(*d, s) : attn_f32_tc(*d, s);
     if (composed < 0) {
         const char* e = getenv("MIMK_ATTN_COMPOSED");
         composed      = (e && e[0] == '0') ? 0 : 1;

@@ -678,6 +678,11 @@ def _whole_tiles(k, cout) -> bool:
     return k % 8 == 0 and cout % 8 == 0
 
 
+@functools.lru_cache(maxsize=64)
+def _sm_count(device: int) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
+
+
 def _patches_pay(dtype, pixels, cout, k, window, padded) -> bool:
     """Whether a patch matrix and the full-rate contraction beat gathering the patches inside the contraction.
 
@@ -692,10 +697,10 @@ def _patches_pay(dtype, pixels, cout, k, window, padded) -> bool:
         return window == 1 and cout > 256 and cout % 4 == 0 and pixels * cout * k >= 1 << 33
     if not _whole_tiles(k, cout):
         return False
-    wide = cout > 64
-    rounds = -(-(-(-pixels // 128) * -(-cout // (128 if wide else 64))) // 148)
+    wide, sms = cout > 64, _sm_count(torch.cuda.current_device())
+    rounds = -(-(-(-pixels // 128) * -(-cout // (128 if wide else 64))) // sms)
     gathered = rounds * ((14 + 1.85 * -(-k // 32)) if wide else (7 + 1.25 * -(-k // 32)))
-    passes = (1.3 * k + 2.0 * cout) * pixels * 2e-6 + 3.3 * -(-(-(-pixels // 128) * -(-cout // 256)) // 148)
+    passes = (1.3 * k + 2.0 * cout) * pixels * 2e-6 + 3.3 * -(-(-(-pixels // 128) * -(-cout // 256)) // sms)
     return max(112 if padded else 85, passes) < gathered
 
 
