@@ -94,8 +94,16 @@ enum {
  * gpu::phase::LowerMapReduce::build_kernel generates for them (src/mim/plug/gpu/phase/lower_map_reduce.cpp:148-265).
  * in_dtype F32: f32-grade results -- small or oddly shaped problems fold each cell in ascending k on the CUDA cores,
  * larger ones run on the tensor cores, every value as the exact sum of three bf16 pieces (six products per term) or, with
- * many tiles, as three TF32 products per term (head/tail split, about 21 mantissa bits per product); f32 accumulation. in_dtype BF16: f32 accumulation on the tensor cores.
- * out_dtype F32 or BF16 (round to nearest even). batch strides are in elements; 0 re-uses the operand. */
+ * many tiles, as three TF32 products per term (head/tail split, about 21 mantissa bits per product); f32 accumulation.
+ * in_dtype BF16: f32 accumulation on the tensor cores.
+ * out_dtype F32 or BF16 (round to nearest even). batch strides are in elements; 0 re-uses the operand.
+ * Which calls share their bits: equal extents, strides, alignment, types and layouts do, call after call, and BF16 ones whether the
+ * product is plain, given as K panels (mimk_gemm_kpanels) or gathered (mimk_gemm_gather). A part of a product (fewer rows or columns,
+ * one entry of a batch) need not have the bits of the whole: F32 products change kernels with their size, and products with few
+ * tiles deal K out over the chip by their extents (BF16 from K = 512 on). F32 products with many tiles, and BF16 ones whose extents
+ * or alignment break 16-byte rows, need a buffer of the library; under stream capture, where a graph would hold on to it, they take a
+ * kernel that needs none (F32: bf16 pieces, more exact than the TF32 products, up to 1.7 times the time; BF16: the CUDA cores, if an
+ * operand has to be copied) and have other last bits. */
 typedef struct mimk_gemm_desc {
     int64_t batch, m, n, k;
     const void* a;

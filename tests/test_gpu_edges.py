@@ -371,3 +371,29 @@ def test_products_of_few_tiles_keep_their_bits_as_panels_and_gathered(T, m, pane
         T.device_status()
         for t in copies:
             assert torch.equal(t[:, 8:8 + n], whole) and (t[:, :8] == 3.0).all() and (t[:, 8 + n:] == 3.0).all()
+
+
+def test_two_streams_at_once_give_what_one_gives(T):
+    # kernels with clusters, with copies in the library's buffer (one per stream) and without, two callers beside one another
+    def work(i):
+        bf, f = (lambda *shape: rnd(shape, i, BF16)), (lambda *shape: rnd(shape, i + 50))
+        a, b, w = bf(300, 1031), bf(257, 1031), bf(2048, 16)
+        x, y, q, k = f(1280, 516), f(516, 1284), f(3, 130, 64), f(3, 200, 64)
+        few, keys, image, filters = bf(4, 3, 128), bf(4, 900, 128), f(12, 16, 40, 40), f(64, 16, 3, 3)
+        return lambda: [T.product_2d(a, b.t()), T.product_2d(w.t(), bf2), T.product_2d(x, y), T.attention(q, k, k, scale=0.1),
+                        T.attention(few, keys, keys, scale=0.1, causal=True), T.conv(image, filters, padding=(1, 1)),
+                        T.product_2d(x[:200], y[:, :300].contiguous())]
+    bf2 = rnd((2048, 1000), 7, BF16)
+    calls = [work(1), work(2)]
+    want = [c() for c in calls]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in calls]
+    for _ in range(4):
+        got = []
+        for c, s in zip(calls, streams):
+            with torch.cuda.stream(s):
+                got.append(c())
+        torch.cuda.synchronize()
+        for g, w in zip(got, want):
+            assert all(torch.equal(u, v) for u, v in zip(g, w))
+    T.device_status()
