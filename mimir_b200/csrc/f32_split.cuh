@@ -2,8 +2,8 @@
 // hold the pieces.
 //
 // An f32 significand has 24 bits and a bf16 one 8, so cutting x after its first 8 bits, and what is left after its next 8,
-// gives x = h + m + l exactly (below the bf16 range of small numbers the last bits are lost, as in any product that
-// underflows). Of the nine products of two such sums the six with at least 2^-16 of the value are taken,
+// gives x = h + m + l exactly, unless bits of l lie below 2^-133, where bf16 ends: from values below 2^-109 on. The cutting
+// says so (lost_bits), and what such values may have spoiled is computed again by the scalar fold. Of the nine products of two such sums the six with at least 2^-16 of the value are taken,
 //     h h,  h m + m h,  h l + m m + l h,
 // the three left out are below 2^-22 of it. An infinite or NaN operand leaves NaN in a piece, so every cell it reaches
 // comes out non-finite and is computed again by the scalar fold.
@@ -28,10 +28,16 @@ __device__ __forceinline__ void st_shared16(uint32_t a, uint32_t x, uint32_t y, 
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 
+// What the cutting returns has bits set here if a value was not the sum of its pieces (an infinite or NaN one included).
+constexpr uint32_t lost_bits = 0xffff;
+// A sum of |a b| over k terms is off by less than k (max |a| + max |b|) times this where values have lost bits.
+constexpr float LOST_ABS = 0x1p-133f;
+
 // Eight consecutive k of one row, cut into pieces and stored at `addr` of the three piece tiles (`piece_bytes` apart). Values
 // that are bf16 already are their own first piece (PIECES = 1).
 template <int PIECES = 3>
-__device__ __forceinline__ void split_store8(uint32_t addr, uint32_t piece_bytes, const float (&x)[8]) {
+__device__ __forceinline__ uint32_t split_store8(uint32_t addr, uint32_t piece_bytes, const float (&x)[8]) {
+    uint32_t lost = 0;
     st_shared16(addr, upper_halves(x[0], x[1]), upper_halves(x[2], x[3]), upper_halves(x[4], x[5]), upper_halves(x[6], x[7]));
     if constexpr (PIECES == 3) {
         float r[8];
@@ -40,22 +46,28 @@ __device__ __forceinline__ void split_store8(uint32_t addr, uint32_t piece_bytes
         st_shared16(addr + piece_bytes, upper_halves(r[0], r[1]), upper_halves(r[2], r[3]), upper_halves(r[4], r[5]),
                     upper_halves(r[6], r[7]));
 #pragma unroll
-        for (int i = 0; i < 8; ++i) r[i] = lower_part(r[i]);
+        for (int i = 0; i < 8; ++i) r[i] = lower_part(r[i]), lost |= __float_as_uint(r[i]);
         st_shared16(addr + 2 * piece_bytes, upper_halves(r[0], r[1]), upper_halves(r[2], r[3]), upper_halves(r[4], r[5]),
                     upper_halves(r[6], r[7]));
     }
+    return lost;
 }
 // Four consecutive k of a row, half a 16-byte unit.
 template <int PIECES = 3>
-__device__ __forceinline__ void split_store4(uint32_t addr, uint32_t piece_bytes, const float* x) {
-    float r[4] = {x[0], x[1], x[2], x[3]};
+__device__ __forceinline__ uint32_t split_store4(uint32_t addr, uint32_t piece_bytes, const float* x) {
+    float r[4]    = {x[0], x[1], x[2], x[3]};
+    uint32_t lost = 0;
 #pragma unroll
     for (int t = 0; t < PIECES; ++t) {
         asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr + t * piece_bytes), "r"(upper_halves(r[0], r[1])), "r"(upper_halves(r[2], r[3]))
                      : "memory");
 #pragma unroll
-        for (int i = 0; i < 4; ++i) r[i] = lower_part(r[i]);
+        for (int i = 0; i < 4; ++i) {
+            if (t == 2) lost |= __float_as_uint(r[i]);
+            r[i] = lower_part(r[i]);
+        }
     }
+    return lost;
 }
 __device__ __forceinline__ uint32_t half_unit_offset(int row, int half) {
     return uint32_t(row * 64 + (((half >> 1) ^ ((row >> 1) & 3)) << 4) + (half & 1) * 8);

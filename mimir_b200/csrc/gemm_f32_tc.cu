@@ -10,7 +10,8 @@
 //   warp 16       one thread issues the MMAs, 128 x BN x 32 per k-block; every two k-blocks go into a fresh accumulator
 // The tensor core does not round its accumulator updates to nearest; with four updates by full-size terms per accumulator (all
 // small terms first) and ordinary f32 adds between accumulators, the error stays below that of an f32 fold for any K.
-// The accumulators are added in order whatever the grid (up to K = 1536: beyond that a CTA of a cluster may first add its own).
+// The accumulators are added in order whatever the grid as long as each CTA of a cluster can hold its own to the end: K <= 64 * SLOTS
+// * split, at least 384 (128 columns, two CTAs). Beyond that a CTA adds its own first, and the bits follow the split.
 //
 // The operands are read as the caller has them: any extents, strides and alignment, no copies, no scratch. What bounds it:
 // shared-memory bandwidth (a k-block of 128 x 128 moves 96 KB into the MMA and 48 KB from the loaders; measured 100 clocks per
@@ -53,6 +54,10 @@ struct Bars {
     uint64_t full[STAGES], empty[STAGES], acc_full[8];
     uint32_t tmem_base;
     int abort_flag;
+    // not zero: a value of this CTA's k-blocks was not the sum of its pieces; then whether some values are below all their pieces, and
+    // what sums have to reach for all that not to matter (0: nothing lost)
+    uint32_t lost, deep;
+    float bound;
 };
 
 // A convolution as a contraction: row = output pixel (image, oh, ow), k = (input channel, kh, kw), column = filter. Rows of the
@@ -85,6 +90,12 @@ __device__ __forceinline__ float4 ld_cluster4(uint32_t saddr, uint32_t rank) {
     float4 v;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_cluster1(uint32_t saddr, uint32_t rank) {
+    uint32_t a, v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     return v;
 }
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld_32x32(taddr, r); }
@@ -123,7 +134,7 @@ __device__ __forceinline__ void store4(TOut* row, int64_t col, int64_t n, float4
 }
 
 // The scalar fold of one cell -- ascending k, one fma per step, what the CUDA-core kernel computes -- for cells the pieces make
-// non-finite: an operand of the fold was inf / NaN, or the sum overflowed.
+// non-finite (an operand of the fold was inf / NaN, or the sum overflowed), and for cells as small as the bits lost in cutting.
 template <class TIn, bool CONV>
 __device__ __noinline__ float scalar_fold(const Params& p, int64_t bz, int64_t row, int64_t col) {
     const TIn* A = static_cast<const TIn*>(p.A) + bz * p.sa;
@@ -154,15 +165,35 @@ __device__ __noinline__ float scalar_fold(const Params& p, int64_t bz, int64_t r
     return v;
 }
 
-// Four neighbouring sums of one row: non-finite ones folded again, `post`, stored.
+// What a CTA works on: a tile of a batch entry, and of its k-blocks the accumulators [ch0, ch1).
+template <int BN> struct Place {
+    int rank, ch0, ch1, kb0, kb1, per, chunks;
+    int64_t bz, m0, n0;
+    __device__ __forceinline__ explicit Place(const Params& p) {
+        const int64_t tiles = p.tiles_m * p.tiles_n;
+        rank                = int(blockIdx.x % unsigned(p.split));  // a cluster is `split` consecutive CTAs
+        const int64_t item  = blockIdx.x / unsigned(p.split);
+        bz                  = item / tiles;
+        int64_t tm, tn;
+        tile_coords(item - bz * tiles, p.tiles_m, p.tiles_n, tm, tn);
+        m0 = tm * BM, n0 = tn * BN;
+        const int all_kb = int((p.K + BK - 1) / BK);
+        chunks = (all_kb + CHUNK - 1) / CHUNK, per = (chunks + p.split - 1) / p.split;
+        ch0 = rank * per < chunks ? rank * per : chunks, ch1 = ch0 + per < chunks ? ch0 + per : chunks;
+        kb0 = ch0 * CHUNK, kb1 = ch1 * CHUNK < all_kb ? ch1 * CHUNK : all_kb;
+    }
+};
+
+// Four neighbouring sums of one row: non-finite ones and those below `bound` (zeros, if so said) folded again, `post`, stored.
 template <class TIn, class TOut>
-__device__ __forceinline__ void finish4(const Params& p, TOut* out, const TOut* post_full, int64_t bz, int64_t row, int64_t col, float4 q) {
+__device__ __forceinline__ void finish4(const Params& p, TOut* out, const TOut* post_full, int64_t bz, int64_t row, int64_t col, float4 q, float bound,
+                                        bool zeros) {
     if (row >= p.M || col >= p.N) return;
     float v[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         if (col + e >= p.N) break;
-        if (!isfinite(v[e])) v[e] = scalar_fold<TIn, false>(p, bz, row, col + e);
+        if (!isfinite(v[e]) || (fabsf(v[e]) < bound && (v[e] != 0.f || zeros))) v[e] = scalar_fold<TIn, false>(p, bz, row, col + e);
         const float rowv = p.post_row ? __ldg(p.post_row + col + e) : 0.f;
         const float full = post_full ? float(post_full[row * p.N + col + e]) : 0.f;
         v[e]             = apply_post(p.post, v[e], rowv, full);
@@ -170,10 +201,90 @@ __device__ __forceinline__ void finish4(const Params& p, TOut* out, const TOut* 
     store4(out + row * p.N, col, p.N, make_float4(v[0], v[1], v[2], v[3]), p.vec_c);
 }
 
+// The accumulators of a tile in order, each CTA of the cluster a share of the rows. hold: every accumulator has a partial tile of its
+// own, else each CTA has one.
+template <int BN, class TIn, class TOut, bool CONV>
+__device__ __forceinline__ void store_tile(const Params& p, const Place<BN>& at, uint32_t base, bool hold, float bound, bool zeros) {
+    using C = Cfg<BN, TIn>;
+    const int rows = BM / p.split, held = hold ? at.per : 1, used = hold ? at.chunks : (at.chunks + at.per - 1) / at.per;
+    TOut* out             = static_cast<TOut*>(p.C) + at.bz * p.sc;
+    const TOut* post_full = p.post_full ? static_cast<const TOut*>(p.post_full) + at.bz * p.sc : nullptr;
+    for (int i = threadIdx.x; i < rows * (BN / 4); i += NUM_THREADS) {
+        // CONV: neighbouring threads take neighbouring pixels, else neighbouring columns
+        const int r = at.rank * rows + (CONV ? i % rows : i / (BN / 4)), col = (CONV ? i / rows : i % (BN / 4)) * 4;
+        const int64_t row = at.m0 + r, gcol = at.n0 + col;
+        if (row >= p.M || gcol >= p.N) continue;
+        const uint32_t a = base + uint32_t(r * C::PITCH + col) * 4;
+        float4 q         = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int t0 = 0; t0 < used; t0 += 4) {  // four on their way at a time, added in order
+            float4 w[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                w[t] = t0 + t < used ? ld_cluster4(a + ((t0 + t) % held) * C::PART_BYTES, uint32_t((t0 + t) / held)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) q.x += w[t].x, q.y += w[t].y, q.z += w[t].z, q.w += w[t].w;
+        }
+        if (CONV) {
+            const int pixels  = cv_pixels(p);
+            const int64_t img = row / pixels;
+            TOut* plane       = out + (img * p.N + gcol) * pixels + (row - img * pixels);
+            const float v[4]  = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (gcol + e < p.N) plane[int64_t(e) * pixels] = TOut(isfinite(v[e]) ? v[e] : scalar_fold<TIn, CONV>(p, at.bz, row, gcol + e));
+        } else {
+            finish4<TIn, TOut>(p, out, post_full, at.bz, row, gcol, q, bound, zeros);
+        }
+    }
+}
+
+template <int BN, class TIn> __device__ __forceinline__ bool holds(const Params& p, const Place<BN>& at) { return p.split > 1 && at.per <= Cfg<BN, TIn>::SLOTS; }
+
+// Bits were lost in cutting this CTA's part of the operands: what a sum has to reach for that not to matter, 22 bits above the loss,
+// from the largest finite magnitudes among the CTA's rows, columns and k; a sum of exactly zero can be short of something only if there
+// are values below 2^-133. By the MMA warp, which has nothing else to do by then: anywhere in the loaders' code it costs their loop
+// registers (1000^3 30 -> 35 us), and so it finds its place again.
+template <class TIn, int BN>
+__device__ __noinline__ void find_bound(const Params& p, Bars* bars) {
+    const Place<BN> at(p);
+    const TIn* A = static_cast<const TIn*>(p.A) + at.bz * p.sa;
+    const TIn* B = static_cast<const TIn*>(p.B) + at.bz * p.sb;
+    const int lane   = threadIdx.x & 31;
+    const int64_t k0 = int64_t(at.kb0) * BK, k1 = int64_t(at.kb1) * BK < p.K ? int64_t(at.kb1) * BK : p.K;
+    const int64_t rows = p.M - at.m0 < BM ? p.M - at.m0 : BM, cols = p.N - at.n0 < BN ? p.N - at.n0 : BN;
+    uint32_t deep = 0;
+    // the largest of `n` rows of `len` elements, `pitch` apart; four rows of 128 elements on their way at a time
+    auto largest = [&](const TIn* first, int64_t n, int64_t pitch, int64_t len, bool vec) {
+        uint32_t most = 0;
+        for (int64_t r = 0; r < n; r += 4)
+            for (int64_t c = lane * 4; c < len; c += 128) {
+                float x[4][4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) load4(x[j], first + (r + j) * pitch + c, r + j < n, int(len - c < 4 ? len - c : 4), vec);
+#pragma unroll
+                for (int j = 0; j < 4 * 4; ++j) {
+                    const uint32_t u = __float_as_uint(x[j >> 2][j & 3]) & 0x7fffffffu;
+                    if (u < 0x7f800000u) most = max(most, u), deep |= u > 0u && u < __float_as_uint(LOST_ABS);
+                }
+            }
+        return __reduce_max_sync(0xffffffffu, most);
+    };
+    const uint32_t a = largest(A + at.m0 * p.K + k0, rows, p.K, k1 - k0, p.vec_a);
+    const TIn* b0    = p.b_nk ? B + at.n0 * p.K + k0 : B + k0 * p.N + at.n0;
+    const uint32_t b = p.b_nk ? largest(b0, cols, p.K, k1 - k0, p.vec_b)
+                              : largest(b0, k1 - k0, p.N, cols, p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(b0) & 15) == 0);
+    deep             = __reduce_or_sync(0xffffffffu, deep);
+    if (lane == 0) {
+        bars->bound = float(k1 - k0) * (0x1p22f * LOST_ABS) * (__uint_as_float(a) + __uint_as_float(b));
+        bars->deep  = deep;
+    }
+}
+
 template <int BN, class TIn, class TOut, bool CONV>
 __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __grid_constant__ Params p) {
     using C = Cfg<BN, TIn>;
     constexpr int PIECES = C::PIECES;
+    constexpr bool LOSES = PIECES == 3 && !CONV;  // (large convolutions always cut their values, into heads and tails before)
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
     const uint32_t base     = (raw_addr + 1023u) & ~1023u;
@@ -181,19 +292,13 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
     volatile int* abort_flag = &bars->abort_flag;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-    const int64_t tiles = p.tiles_m * p.tiles_n;
-    const int rank      = int(blockIdx.x % unsigned(p.split));  // a cluster is `split` consecutive CTAs
-    const int64_t item  = blockIdx.x / unsigned(p.split), bz = item / tiles;
-    int64_t tm, tn;
-    tile_coords(item - bz * tiles, p.tiles_m, p.tiles_n, tm, tn);
-    const int64_t m0 = tm * BM, n0 = tn * BN;
+    const Place<BN> place(p);
+    const int rank = place.rank, ch0 = place.ch0, ch1 = place.ch1, kb0 = place.kb0, kb1 = place.kb1, per = place.per, chunks = place.chunks;
+    const int64_t bz = place.bz, m0 = place.m0, n0 = place.n0;
     const TIn* A = static_cast<const TIn*>(p.A) + bz * p.sa;
     const TIn* B = static_cast<const TIn*>(p.B) + bz * p.sb;
-    const int all_kb = int((p.K + BK - 1) / BK), chunks = (all_kb + CHUNK - 1) / CHUNK, per = (chunks + p.split - 1) / p.split;
-    const int ch0 = rank * per < chunks ? rank * per : chunks, ch1 = ch0 + per < chunks ? ch0 + per : chunks;
-    const int kb0 = ch0 * CHUNK, kb1 = ch1 * CHUNK < all_kb ? ch1 * CHUNK : all_kb;
     // this CTA's accumulators stay in tensor memory to the end and leave one by one, or are added up as they are finished
-    const bool hold = p.split > 1 && per <= C::SLOTS;
+    const bool hold = holds<BN, TIn>(p, place);
 
     // A thread's part of a k-block. Where memory runs along k: four k of one or two rows 64 apart, eight lanes to a row's 128
     // bytes. Where it runs along the rows (B stored [K, N], the pixels of an image): eight k of one row, a warp's lanes on
@@ -270,20 +375,21 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
             for (int j = 0; j < 8; ++j) fb[j] = in && j < left ? load1(at + j * p.N) : 0.f;
         }
     };
+    uint32_t lost = 0;
     auto store_a = [&](uint32_t at) {
         if (CONV) {
             split_store8<PIECES>(at + unit_offset(across, unit), A_PIECE, fa);
         } else {
-            split_store4<PIECES>(at + half_unit_offset(along, half), A_PIECE, fa);
-            split_store4<PIECES>(at + half_unit_offset(along + 64, half), A_PIECE, fa + 4);
+            lost |= split_store4<PIECES>(at + half_unit_offset(along, half), A_PIECE, fa);
+            lost |= split_store4<PIECES>(at + half_unit_offset(along + 64, half), A_PIECE, fa + 4);
         }
     };
     auto store_b = [&](uint32_t at) {
         if (p.b_nk) {
-            split_store4<PIECES>(at + half_unit_offset(along, half), C::B_PIECE, fb);
-            if (NB == 2) split_store4<PIECES>(at + half_unit_offset(along + 64, half), C::B_PIECE, fb + 4);
+            lost |= split_store4<PIECES>(at + half_unit_offset(along, half), C::B_PIECE, fb);
+            if (NB == 2) lost |= split_store4<PIECES>(at + half_unit_offset(along + 64, half), C::B_PIECE, fb + 4);
         } else if (has_b) {
-            split_store8<PIECES>(at + unit_offset(across, unit), C::B_PIECE, fb);
+            lost |= split_store8<PIECES>(at + unit_offset(across, unit), C::B_PIECE, fb);
         }
     };
     if (warp < MMA_WARP && kb0 < kb1) {  // on their way while the barriers and the tensor memory are set up
@@ -298,6 +404,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
         }
         for (int b = 0; b < C::NACC; ++b) mbar_init(smem_u32(&bars->acc_full[b]), 1);
         bars->abort_flag = 0;
+        bars->lost = bars->deep = 0, bars->bound = 0.f;
         fence_barrier_init();
     }
     if (warp == MMA_WARP) {
@@ -336,6 +443,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
             }
         }
         __syncwarp();
+        // (every full stage is noted; the whole warp goes, whatever its lanes see after an abandoned wait)
+        if (LOSES && __any_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(&bars->lost) != 0)) find_bound<TIn, BN>(p, bars);
     } else {
         static_assert(CHUNK == 2 && STAGES == 2 * CHUNK && C::NACC >= 4, "see the waits of the MMA warp");
         constexpr int COLS = BN / 4;  // accumulator columns per warp
@@ -366,6 +475,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
             if (kb + 1 < kb1) fetch_a(kb + 1);
             store_b(s0 + PIECES * A_PIECE);
             if (kb + 1 < kb1) fetch_b(kb + 1);
+            else if (LOSES && (lost & lost_bits)) bars->lost = 1;
             fence_proxy_async_smem();  // the MMA reads shared memory through the async proxy
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bars->full[stage]));
@@ -439,46 +549,20 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
     __syncthreads();
     // (an abandoned wait leaves MMAs that read the stages; their results are marked invalid by the status word)
     if (p.split > 1) cluster_sync();
-    {
-        // the accumulators in order, each CTA a share of the rows
-        const int rows = BM / p.split, held = hold ? per : 1, used = hold ? chunks : (chunks + per - 1) / per;
-        TOut* out             = static_cast<TOut*>(p.C) + bz * p.sc;
-        const TOut* post_full = p.post_full ? static_cast<const TOut*>(p.post_full) + bz * p.sc : nullptr;
-        for (int i = tid; i < rows * (BN / 4); i += NUM_THREADS) {
-            // CONV: neighbouring threads take neighbouring pixels, else neighbouring columns
-            const int r = rank * rows + (CONV ? i % rows : i / (BN / 4)), col = (CONV ? i / rows : i % (BN / 4)) * 4;
-            const int64_t row = m0 + r, gcol = n0 + col;
-            if (row >= p.M || gcol >= p.N) continue;
-            const uint32_t a = base + uint32_t(r * C::PITCH + col) * 4;
-            float4 q         = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int t0 = 0; t0 < used; t0 += 4) {  // four on their way at a time, added in order
-                float4 w[4];
-#pragma unroll
-                for (int t = 0; t < 4; ++t)
-                    w[t] = t0 + t < used ? ld_cluster4(a + ((t0 + t) % held) * C::PART_BYTES, uint32_t((t0 + t) / held)) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-                for (int t = 0; t < 4; ++t) q.x += w[t].x, q.y += w[t].y, q.z += w[t].z, q.w += w[t].w;
-            }
-            if (CONV) {
-                const int pixels  = cv_pixels(p);
-                const int64_t img = row / pixels;
-                TOut* plane       = out + (img * p.N + gcol) * pixels + (row - img * pixels);
-                const float v[4]  = {q.x, q.y, q.z, q.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (gcol + e < p.N) plane[int64_t(e) * pixels] = TOut(isfinite(v[e]) ? v[e] : scalar_fold<TIn, CONV>(p, bz, row, gcol + e));
-            } else {
-                finish4<TIn, TOut>(p, out, post_full, bz, row, gcol, q);
-            }
-        }
+    float bound   = 0.f;
+    uint32_t deep = 0;
+    for (int r = 0; LOSES && r < p.split; ++r) {
+        bound += __uint_as_float(ld_cluster1(smem_u32(&bars->bound), uint32_t(r)));
+        deep |= ld_cluster1(smem_u32(&bars->deep), uint32_t(r));
     }
+    store_tile<BN, TIn, TOut, CONV>(p, place, base, hold, bound, deep != 0);
     if (p.split > 1) cluster_sync();  // no CTA of the cluster exits while another may read its partial tiles
 
     tc_fence_before();
     __syncthreads();
     if (warp == MMA_WARP) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, 512);
+        tmem_dealloc(*reinterpret_cast<volatile uint32_t*>(&bars->tmem_base), 512);
     }
     if (tid == 0 && *abort_flag) *p.status = MIMK_E_DEVICE_WAIT;
 }

@@ -229,6 +229,24 @@ def test_f32_products_keep_infinities_and_extremes(T):
     close_cells(T.product_2d(a, b), d64(a) @ d64(b), d64(a).abs() @ d64(b).abs(), F32_CELL)
 
 
+@pytest.mark.parametrize("batch,m,n,k,b_nk,out", [
+    (1, 100, 130, 300, True, F32), (1, 129, 70, 5000, False, F32), (1, 300, 200, 1000, True, BF16), (1, 40, 1301, 2000, False, F32), (20, 65, 100, 700, True, F32)])
+@pytest.mark.parametrize("low,high", [(1e-36, 1.0), (1e-38, 1e30), (1.0, 1e-37), (3e-42, 1e10)])
+def test_f32_products_of_tiny_values(T, batch, m, n, k, b_nk, out, low, high):
+    # values below 2^-109 do not fit three bf16 pieces; a third of the rows of A and of the columns of B are left as they are
+    lead = (batch,) if batch > 1 else ()
+    a, b = rnd(lead + (m, k), 1), rnd(lead + ((n, k) if b_nk else (k, n)), 2)
+    b = b.transpose(-1, -2) if b_nk else b
+    a[..., m // 3:, :] *= low
+    b[..., n // 3:] *= high
+    b[..., n // 2] = 0.0
+    got = T.bmm(a, b, out_dtype=out) if batch > 1 else T.product_2d(a, b, out_dtype=out)
+    T.device_status()
+    # (near the end of its range an f32 sum is rounded to multiples of 2^-149, a bf16 result to multiples of 2^-133)
+    cell, end = (F32_CELL, k * 2.0 ** -149) if out == F32 else (BF16_ROUND, 2.0 ** -133)
+    close_cells(got, d64(a) @ d64(b), d64(a).abs() @ d64(b).abs() + end / cell, cell)
+
+
 @pytest.mark.parametrize("n,cin,h,w,cout,kh,kw,stride,dil,pad,dtype", [
     (2, 5, 17, 23, 16, 3, 3, (1, 1), (1, 1), (1, 1), F32), (1, 33, 30, 31, 65, 3, 2, (2, 1), (1, 2), (0, 1), F32),
     (3, 16, 40, 40, 130, 1, 1, (1, 1), (1, 1), (0, 0), F32), (2, 3, 50, 41, 40, 7, 5, (2, 2), (1, 1), (3, 2), BF16),
