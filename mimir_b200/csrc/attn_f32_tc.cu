@@ -13,7 +13,8 @@
 // Measured: 32 heads x 1000 x 64, 112 us (73 TFLOP/s; 906 us as three passes over a score matrix); 127 heads x 215 x 64, 35 us,
 // and causal 11 x 1047 x 128, 91 us (1776 and 4021 us with a warp per row). 2-norm error 1.7e-7 to 3.8e-7.
 //
-// Rows whose result is not finite (an infinite or NaN operand, an overflow) are computed again by the general path.
+// Rows whose result is not finite (an infinite or NaN operand, an overflow), or so small that bits lost in the cutting of tiny
+// values (and weights) would show, are computed again by the general path.
 #include "attn_row.cuh"
 #include "common.cuh"
 #include "f32_split.cuh"
@@ -38,9 +39,11 @@ template <int DP> struct Cfg {
 };
 
 struct Bars {
-    uint64_t k_full, v_full, p_full, s_full, o_full, pair[4];
+    uint64_t k_full, v_full, p_full, s_full, o_full, pair[4], all;
     uint32_t tmem_base;
     int abort_flag;
+    uint32_t max_qk, max_v;  // the largest magnitudes that were cut
+    uint32_t zeros, deep;    // a result is exactly zero; then: V has values below all their pieces
 };
 
 struct Params {
@@ -56,7 +59,7 @@ struct Params {
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
-// The two warps that share 32 rows meet (a bounded wait like any other: a named barrier would keep one of them for good once
+// The warps that share a barrier meet: the two of 32 rows, or all eight (a bounded wait like any other: a named barrier would keep one of them for good once
 // the other has given up).
 __device__ __forceinline__ bool pair_meet(uint64_t* bar, uint32_t& parity, volatile int* abort_flag) {
     __syncwarp();
@@ -93,6 +96,8 @@ __global__ void __launch_bounds__(NUM_THREADS, DP <= 64 ? 2 : 1) attn_f32_tc_ker
         mbar_init(smem_u32(&bars->v_full), WORKERS / 32);
         mbar_init(smem_u32(&bars->p_full), WORKERS / 32);
         for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&bars->pair[i]), 2);
+        mbar_init(smem_u32(&bars->all), WORKERS / 32);
+        bars->max_qk = bars->max_v = bars->zeros = bars->deep = 0;
         mbar_init(smem_u32(&bars->s_full), 1);
         mbar_init(smem_u32(&bars->o_full), 1);
         bars->abort_flag = 0;
@@ -147,6 +152,11 @@ __global__ void __launch_bounds__(NUM_THREADS, DP <= 64 ? 2 : 1) attn_f32_tc_ker
         const int r       = quarter * 32 + lane;  // this thread's row of the tile: tensor-memory lane r
         const uint32_t lanes = uint32_t(quarter * 32) << 16;
         float o[HALF], m = -CUDART_INF_F, l = 0.f;
+        float most_qk = 0.f, most_v = 0.f;
+        auto see = [](float& most, const float (&x)[8]) {
+#pragma unroll
+            for (int i = 0; i < 8; i += 2) most = fmaxf(fmaxf(most, fabsf(x[i])), fabsf(x[i + 1]));
+        };
 #pragma unroll
         for (int i = 0; i < HALF; ++i) o[i] = 0.f;
 
@@ -159,7 +169,7 @@ __global__ void __launch_bounds__(NUM_THREADS, DP <= 64 ? 2 : 1) attn_f32_tc_ker
         auto store_k = [&](const float (&x)[C::TILES][8]) {
 #pragma unroll
             for (int t = 0; t < C::TILES; ++t)
-                split_store8(base + C::K_AT + t * (BKEYS * 64) + unit_offset(tid >> 2, tid & 3), C::K_PIECE, x[t]);
+                see(most_qk, x[t]), split_store8(base + C::K_AT + t * (BKEYS * 64) + unit_offset(tid >> 2, tid & 3), C::K_PIECE, x[t]);
         };
         auto fetch_v = [&](float (&x)[C::TILES][8], int j) {  // eight keys of one column; neighbouring lanes, neighbouring columns
             const int64_t key = int64_t(j) * BKEYS + warp * 8;
@@ -172,7 +182,7 @@ __global__ void __launch_bounds__(NUM_THREADS, DP <= 64 ? 2 : 1) attn_f32_tc_ker
         auto store_v = [&](const float (&x)[C::TILES][8]) {
 #pragma unroll
             for (int t = 0; t < C::TILES; ++t)
-                split_store8(base + C::V_AT + (warp >> 2) * (DP * 64) + unit_offset(t * 32 + lane, warp & 3), C::V_PIECE, x[t]);
+                see(most_v, x[t]), split_store8(base + C::V_AT + (warp >> 2) * (DP * 64) + unit_offset(t * 32 + lane, warp & 3), C::V_PIECE, x[t]);
         };
         auto publish = [&](uint64_t* bar) {  // this warp's shared-memory stores are ready for the MMA
             fence_proxy_async_smem();
@@ -187,6 +197,7 @@ __global__ void __launch_bounds__(NUM_THREADS, DP <= 64 ? 2 : 1) attn_f32_tc_ker
                     const int row = (tid >> 2) + i * 64;
                     float x[8];
                     load8(x, Q + (q0 + row) * p.d + t * 32 + (tid & 3) * 8, q0 + row < p.sq, p.d - t * 32 - (tid & 3) * 8, p.vec_q);
+                    see(most_qk, x);
                     split_store8(base + t * (BQ * 64) + unit_offset(row, tid & 3), C::Q_PIECE, x);
                 }
             float x[C::TILES][8];
@@ -275,15 +286,38 @@ __global__ void __launch_bounds__(NUM_THREADS, DP <= 64 ? 2 : 1) attn_f32_tc_ker
             }
         }
         pair_sum[half * 128 + r] = l;
-        ok = ok && pair_meet(&bars->pair[quarter], meeting, abort_flag);
+        // What the cutting may have lost: a value below 2^-109 the bits under 2^-133. Scores are off by less than d (max |q| + max |k|)
+        // 2^-133, a result by 2^-133 for V, whose weights sum to at least one, and by keys * max |v| * 2^-133 for the weights.
+        const uint32_t mqk = __reduce_max_sync(0xffffffffu, __float_as_uint(most_qk)), mv = __reduce_max_sync(0xffffffffu, __float_as_uint(most_v));
+        if (lane == 0) atomicMax(&bars->max_qk, mqk), atomicMax(&bars->max_v, mv);
+        uint32_t together = 0;
+        ok = ok && pair_meet(&bars->all, together, abort_flag);
         l += pair_sum[(half ^ 1) * 128 + r];
-        // a row both of whose threads saw only finite results is written here, any other one below
+        auto shared          = [](const uint32_t* word) { return *reinterpret_cast<const volatile uint32_t*>(word); };
+        const bool spoiled   = fabsf(p.scale) * p.d * 2.f * LOST_ABS * __uint_as_float(shared(&bars->max_qk)) > 0x1p-24f;
+        const float small    = 0x1p22f * LOST_ABS * (1.f + float(visible) * __uint_as_float(shared(&bars->max_v)));  // 22 bits above the loss
+        // a row both of whose threads saw only finite results that are large enough is written here, any other one below
         const float inv = l > 0.f ? 1.f / l : 0.f;
-        bool finite     = isfinite(l) && (l > 0.f || limit <= 0);  // (keys seen and no weight: the general path knows the answer)
+        bool finite     = isfinite(l) && (l > 0.f || limit <= 0) && !spoiled, zero = false;  // (keys seen and no weight: the general path)
 #pragma unroll
         for (int i = 0; i < HALF; ++i) {
             o[i] *= inv;
-            finite = finite && isfinite(o[i]);
+            finite = finite && isfinite(o[i]) && (fabsf(o[i]) >= small || o[i] == 0.f);
+            zero   = zero || (o[i] == 0.f && half * HALF + i < p.d);
+        }
+        // A zero is short of something only if V has values below all their pieces.
+        zero = zero && q0 + r < p.sq && limit > 0;
+        if (__any_sync(0xffffffffu, zero) && lane == 0) bars->zeros = 1;
+        ok = ok && pair_meet(&bars->all, together, abort_flag);
+        if (__any_sync(0xffffffffu, shared(&bars->zeros) != 0)) {
+            bool deep = false;
+            for (int64_t i = tid; i < visible * p.d; i += WORKERS) {
+                const float v = fabsf(__ldg(V + i));
+                deep          = deep || (v > 0.f && v < LOST_ABS);
+            }
+            if (__any_sync(0xffffffffu, deep) && lane == 0) bars->deep = 1;
+            ok     = ok && pair_meet(&bars->all, together, abort_flag);
+            finite = finite && !(zero && shared(&bars->deep));
         }
         pair_max[half * 128 + r] = finite ? 0.f : 1.f;  // (its last reads as a maximum lie before the exchange of sums)
         ok = ok && pair_meet(&bars->pair[quarter], meeting, abort_flag);

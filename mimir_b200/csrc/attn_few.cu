@@ -10,8 +10,9 @@
 //   K   a lane takes 16 consecutive bytes of a key (head_dim 8c .. 8c+7 of each 32), which are the fragments of two k-steps
 //   V   a lane takes 16 consecutive bytes of four keys; pairs of keys are interleaved by byte permutes, and the eight elements
 //       belong to eight different column tiles of the result
-// Measured: 128 heads x 1 x 4096 x 128, 61 us (4.4 TB/s, as the 128-row kernel); 8 x 1 x 8192 x 128, 22 us; causal 32 x 11 x 5000
-// x 128, 26 us. One bulk copy per key instead of 16 lanes' copies was slower (69, 32 and 29 us), registers instead of the ring too.
+// Measured: 128 heads x 1 x 4096 x 128, 61 us (4.4 TB/s, as the 128-row kernel); 8 x 1 x 8192 x 128, 22 us; causal, with f32 weights,
+// 32 x 11 x 5000 x 128, 32 us (26 with weights rounded to bf16: the products of two more pieces are no longer hidden). One bulk copy per
+// key instead of 16 lanes' copies was slower (69 and 32 us for the first two), registers instead of the ring too.
 // Each warp keeps its own running maximum, sum and output; they are merged through (distributed) shared memory in a fixed order.
 #include <math_constants.h>
 

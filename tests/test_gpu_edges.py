@@ -86,6 +86,26 @@ def test_f32_attention_of_any_length(T, bh, sq, sk, d, causal):
     assert torch.equal(got, T.attention(q, k, v, scale=d ** -0.5, causal=causal))
 
 
+@pytest.mark.parametrize("sq,sk,d,causal", [(50, 60, 33, False), (200, 130, 128, True), (130, 300, 64, False)])
+@pytest.mark.parametrize("qs,ks,vs", [(1.0, 1.0, 1e-36), (1.0, 1.0, 1e-38), (1.0, 1.0, 1e-41), (1e-37, 1e37, 1.0), (30.0, 30.0, 1.0)])
+def test_f32_attention_of_tiny_values(T, sq, sk, d, causal, qs, ks, vs):
+    # values below 2^-109, and weights (the last case), do not fit three bf16 pieces
+    q, k, v = rnd((2, sq, d), 1) * qs, rnd((2, sk, d), 2) * ks, rnd((2, sk, d), 3)
+    v[:, :, d // 2:] *= vs
+    if qs > 1:  # the key with nearly all the weight holds nothing: the rest of the row is what the smallest weights bring
+        k[:, 7, 0], q[..., 0] = 5000.0, 1.0
+        k[:, 7, 1:] = k[:, 7, 1:] * 0.01
+        q[..., 0] *= 1.0 / (5000.0 * 0.1) * 80.0
+        q[..., 1:] *= 0.01
+        v[:, 7] = 0.0
+    got = T.attention(q, k, v, scale=0.1, causal=causal)
+    T.device_status()
+    want, _ = attention_reference(q, k, v, 0.1, causal)
+    weights = attention_reference(q, k, v.abs(), 0.1, causal)[0]
+    # scores of up to 100, off by F32_CELL of their terms and by the rounding of the exponential's argument
+    assert ((d64(got) - want).abs() <= 200 * F32_CELL * weights + 1e-43).all()
+
+
 @pytest.mark.parametrize("d", [16, 64, 128])
 @pytest.mark.parametrize("bh,sq,sk", [(1, 3, 1), (1, 3, 24), (700, 2, 20), (700, 40, 20), (700, 2, 64)])
 def test_f32_attention_of_few_keys(T, bh, sq, sk, d):
