@@ -10,8 +10,8 @@
 // P V of a block runs while K of the next is read and cut, the next scores while V is; only the softmax leaves the tensor
 // cores idle, and head_dim <= 64 has a second CTA on the SM for that. What bounds it: the shared-memory reads of S (A 4 KB and
 // B 2 KB per instruction, 48 clocks against 32 of arithmetic) and the serial chain score -> softmax -> P V.
-// Measured: 32 heads x 1000 x 64, 112 us (73 TFLOP/s; 906 us as three passes over a score matrix); 127 heads x 215 x 64, 35 us,
-// and causal 11 x 1047 x 128, 91 us (1776 and 4021 us with a warp per row). 2-norm error 1.7e-7 to 3.8e-7.
+// Measured: 32 heads x 1000 x 64, 116 us (71 TFLOP/s; 771 us as three passes over a score matrix); 127 heads x 215 x 64, 36 us, and
+// 11 x 1047 x 128, 97 us (1760 and 7710 us with a warp per row). 2-norm error 1.7e-7 to 3.8e-7.
 //
 // Rows whose result is not finite (an infinite or NaN operand, an overflow), or so small that bits lost in the cutting of tiny
 // values (and weights) would show, are computed again by the general path.
@@ -59,8 +59,8 @@ struct Params {
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
-// The warps that share a barrier meet: the two of 32 rows, or all eight (a bounded wait like any other: a named barrier would keep one of them for good once
-// the other has given up).
+// The warps that share a barrier meet: the two of 32 rows, or all eight (a bounded wait like any other: a named barrier would keep one
+// of them for good once another has given up).
 __device__ __forceinline__ bool pair_meet(uint64_t* bar, uint32_t& parity, volatile int* abort_flag) {
     __syncwarp();
     if ((threadIdx.x & 31) == 0) mbar_arrive(smem_u32(bar));
