@@ -17,8 +17,8 @@
 // shared-memory bandwidth (a k-block of 128 x 128 moves 96 KB into the MMA and 48 KB from the loaders; measured 100 clocks per
 // instruction of 64 clocks' arithmetic) next to the loaders' instructions. Too few tiles for the chip: the accumulators of one
 // tile are dealt out to a cluster of two, four or eight CTAs, which exchange them through distributed shared memory. Many tiles: the operands
-// are cut beforehand instead (gemm_tf32.cu). Measured: 1000^3 28 us (34 as three TF32 products, 2e-6 off; here 1.3e-7), 4096 x 128 x
-// 4096 45 (121), 64 of 512^3 220 (830 on the CUDA cores), 24 of 503 x 2052 x 407 342 (1062).
+// are cut beforehand instead (gemm_tf32.cu). Measured: 1000^3 29 us (30 as three TF32 products, 2e-6 off; here 1.3e-7), 4096 x 128 x
+// 4096 45 (112), 64 of 512^3 220 (830 on the CUDA cores), 24 of 503 x 2052 x 407 342 (1062).
 #include <type_traits>
 
 #include "common.cuh"
@@ -56,7 +56,7 @@ struct Bars {
     int abort_flag;
     // not zero: a value of this CTA's k-blocks was not the sum of its pieces; then whether some values are below all their pieces, and
     // what sums have to reach for all that not to matter (0: nothing lost)
-    uint32_t lost, deep;
+    uint32_t lost, deep, max_a, max_b;
     float bound;
 };
 
@@ -242,21 +242,21 @@ template <int BN, class TIn> __device__ __forceinline__ bool holds(const Params&
 
 // Bits were lost in cutting this CTA's part of the operands: what a sum has to reach for that not to matter, 22 bits above the loss,
 // from the largest finite magnitudes among the CTA's rows, columns and k; a sum of exactly zero can be short of something only if there
-// are values below 2^-133. By the MMA warp, which has nothing else to do by then: anywhere in the loaders' code it costs their loop
-// registers (1000^3 30 -> 35 us), and so it finds its place again.
+// are values below 2^-133. (It finds its place again, and loads four rows at a time: kept for it, or with eight, registers are spilled
+// by the loaders' loop, 1000^3 31 -> 35 us.) By all warps: 16 of 1000 x 1000 x 64 with softmax weights of 1e-38 67 us, 264 by one.
 template <class TIn, int BN>
 __device__ __noinline__ void find_bound(const Params& p, Bars* bars) {
     const Place<BN> at(p);
     const TIn* A = static_cast<const TIn*>(p.A) + at.bz * p.sa;
     const TIn* B = static_cast<const TIn*>(p.B) + at.bz * p.sb;
-    const int lane   = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t k0 = int64_t(at.kb0) * BK, k1 = int64_t(at.kb1) * BK < p.K ? int64_t(at.kb1) * BK : p.K;
     const int64_t rows = p.M - at.m0 < BM ? p.M - at.m0 : BM, cols = p.N - at.n0 < BN ? p.N - at.n0 : BN;
     uint32_t deep = 0;
     // the largest of `n` rows of `len` elements, `pitch` apart; four rows of 128 elements on their way at a time
     auto largest = [&](const TIn* first, int64_t n, int64_t pitch, int64_t len, bool vec) {
         uint32_t most = 0;
-        for (int64_t r = 0; r < n; r += 4)
+        for (int64_t r = warp * 4; r < n; r += NUM_THREADS / 32 * 4)
             for (int64_t c = lane * 4; c < len; c += 128) {
                 float x[4][4];
 #pragma unroll
@@ -274,10 +274,10 @@ __device__ __noinline__ void find_bound(const Params& p, Bars* bars) {
     const uint32_t b = p.b_nk ? largest(b0, cols, p.K, k1 - k0, p.vec_b)
                               : largest(b0, k1 - k0, p.N, cols, p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(b0) & 15) == 0);
     deep             = __reduce_or_sync(0xffffffffu, deep);
-    if (lane == 0) {
-        bars->bound = float(k1 - k0) * (0x1p22f * LOST_ABS) * (__uint_as_float(a) + __uint_as_float(b));
-        bars->deep  = deep;
-    }
+    if (lane == 0) atomicMax(&bars->max_a, a), atomicMax(&bars->max_b, b), atomicOr(&bars->deep, deep);
+    __syncthreads();
+    if (threadIdx.x == 0) bars->bound = float(k1 - k0) * (0x1p22f * LOST_ABS) * (__uint_as_float(bars->max_a) + __uint_as_float(bars->max_b));
+    __syncthreads();
 }
 
 template <int BN, class TIn, class TOut, bool CONV>
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
         }
         for (int b = 0; b < C::NACC; ++b) mbar_init(smem_u32(&bars->acc_full[b]), 1);
         bars->abort_flag = 0;
-        bars->lost = bars->deep = 0, bars->bound = 0.f;
+        bars->lost = bars->deep = bars->max_a = bars->max_b = 0, bars->bound = 0.f;
         fence_barrier_init();
     }
     if (warp == MMA_WARP) {
@@ -443,8 +443,6 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
             }
         }
         __syncwarp();
-        // (every full stage is noted; the whole warp goes, whatever its lanes see after an abandoned wait)
-        if (LOSES && __any_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(&bars->lost) != 0)) find_bound<TIn, BN>(p, bars);
     } else {
         static_assert(CHUNK == 2 && STAGES == 2 * CHUNK && C::NACC >= 4, "see the waits of the MMA warp");
         constexpr int COLS = BN / 4;  // accumulator columns per warp
@@ -547,6 +545,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
         }
     }
     __syncthreads();
+    if (LOSES && bars->lost) find_bound<TIn, BN>(p, bars);
     // (an abandoned wait leaves MMAs that read the stages; their results are marked invalid by the status word)
     if (p.split > 1) cluster_sync();
     float bound   = 0.f;
