@@ -292,7 +292,10 @@ int mimk_attn_fwd(const mimk_attn_desc* desc, void* stream);
  * outside it read as zeros: tensor.conv (tensor.mim:434-438) with its padding, as one contraction on the tensor cores whose left
  * operand is gathered from the image. dtype F32 or BF16 (out the same); any extents and alignment, windows up to 31 x 31.
  * by_tap: the filters are given as [co, kh, kw, ci], ci a multiple of 8; then each load's place in the window is tested once for
- * eight channels. */
+ * eight channels.
+ * Where an estimate says so, the image is laid out for the tensor cores first, in the library's cached buffer (not under stream
+ * capture); mimk_conv_laid_out tells (1 / 0) whether a call with these sizes on this stream would do that, when the order of the
+ * filters makes no difference. */
 typedef struct mimk_conv_desc {
     int64_t n, cin, h, w, cout, kh, kw;
     int64_t stride_h, stride_w, dil_h, dil_w, pad_h, pad_w;
@@ -302,6 +305,7 @@ typedef struct mimk_conv_desc {
     int32_t dtype, by_tap;
 } mimk_conv_desc;
 int mimk_conv(const mimk_conv_desc* desc, void* stream);
+int mimk_conv_laid_out(const mimk_conv_desc* desc, void* stream);
 
 /* Y = (silu(X W1) * (X W3)) W2 with the gated product H kept in `dtype`.
  * Replaces: two product_2d + math.slf + binary mul (epilogue-fused into one contraction) + product_2d.

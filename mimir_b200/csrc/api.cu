@@ -291,7 +291,7 @@ extern "C" int mimk_attn_fwd(const mimk_attn_desc* d, void* stream) {
     return attn_simt(*d, s);
 }
 
-extern "C" int mimk_conv(const mimk_conv_desc* d, void* stream) {
+static int check_conv(const mimk_conv_desc* d) {
     if (!d) return MIMK_E_ARG;
     if (d->n < 0 || d->cin < 1 || d->h < 1 || d->w < 1 || d->cout < 0 || d->kh < 1 || d->kw < 1) return MIMK_E_ARG;
     if (d->stride_h < 1 || d->stride_w < 1 || d->dil_h < 1 || d->dil_w < 1 || d->pad_h < 0 || d->pad_w < 0) return MIMK_E_ARG;
@@ -312,11 +312,31 @@ extern "C" int mimk_conv(const mimk_conv_desc* d, void* stream) {
     if (span_h < 0 || span_w < 0) return MIMK_E_SHAPE;
     const double pixels = double(span_h / d->stride_h + 1) * double(span_w / d->stride_w + 1);
     if (pixels >= LIM || double(d->n) * pixels * double(d->cout) >= double(int64_t(1) << 40)) return MIMK_E_UNSUPPORTED;
-    int st = MIMK_OK;
-    if (!device_info(&st)) return st;
+    return MIMK_OK;
+}
+
+extern "C" int mimk_conv(const mimk_conv_desc* d, void* stream) {
+    MIMK_TRY(check_conv(d));
+    int st                = MIMK_OK;
+    const DeviceInfo* dev = device_info(&st);
+    if (!dev) return st;
     if (d->n == 0 || d->cout == 0) return MIMK_OK;
     if (!d->x || !d->filters || !d->out) return MIMK_E_ARG;
-    return conv_tc(*d, static_cast<cudaStream_t>(stream));
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (!conv_tc_preferred(*d, dev->sm_count)) {
+        const int r = conv_pieces(*d, s);
+        if (r != MIMK_E_UNSUPPORTED) return r;
+    }
+    return conv_tc(*d, s);
+}
+
+extern "C" int mimk_conv_laid_out(const mimk_conv_desc* d, void* stream) {
+    if (check_conv(d) != MIMK_OK) return 0;
+    int st                = MIMK_OK;
+    const DeviceInfo* dev = device_info(&st);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (!dev || cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &cap) != cudaSuccess) return 0;
+    return cap == cudaStreamCaptureStatusNone && !conv_tc_preferred(*d, dev->sm_count);
 }
 
 extern "C" int mimk_mlp_gated(const mimk_mlp_desc* d, void* stream) {

@@ -90,6 +90,9 @@ int gemm_tf32_preferred(const mimk_gemm_desc& d, int sm_count, double pieces_us)
 int gemm_tf32(const mimk_gemm_desc& d, cudaStream_t s);
 double gemm_tf32_us(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count);
 int conv_tc(const mimk_conv_desc& d, cudaStream_t s);  // the same kernel, its left operand gathered from an image
+int conv_tc_preferred(const mimk_conv_desc& d, int sm_count);  // ... where conv_pieces is not ahead
+int conv_pieces(const mimk_conv_desc& d, cudaStream_t s);      // image laid out once, then shifted products (conv_pieces.cu)
+int conv_pieces_preferred(const mimk_conv_desc& d, int sm_count, double other_us);
 // map_reduce_post instances that are a contraction, an axis fold or an elementwise map go to those kernels (mrp_route.cu)
 bool mrp_try_route(const mimk_mrp_desc& d, void* stream, int* status);
 // What a descriptor's access maps spell, whatever its size (the router itself leaves small instances on the per-cell

@@ -1,0 +1,509 @@
+// Convolution as shifted products over an image that is laid out for the tensor cores once.
+//
+//   cut kernel    one pass over image and filters: channels last, the padding written as zeros, f32 values cut into three bf16 pieces
+//                 (f32_split.cuh). With strides the pixels are dealt out to one grid per remainder of their coordinates, so that
+//                 whatever the stride, window and dilation, the pixels that one tap reads for consecutive output positions are
+//                 consecutive rows: tap (r, q) of output row v is row v + shift(r, q).
+//   conv kernel   D[filter, position] over (tap, channel block of 32): both operands come by TMA (box of 32 channels x rows x pieces),
+//                 no address arithmetic, tests or cutting in the loop. Positions run over the padded width (a window that crosses
+//                 the edge of an image gives a column that is not stored: 7 % at 56 x 56 with a 3 x 3 window).
+//     warps 0..7  add finished accumulators to sums in registers, store the tile by pixels (NCHW)
+//     warp 8      TMA, warp 9 one thread issues the MMAs, 128 x BN x 16
+// f32: every block of 64 channels goes into a fresh accumulator, the products of small pieces first, and accumulators are added with
+// ordinary f32 adds (the tensor core does not round its updates to nearest); non-finite cells are folded again by the scalar code.
+// bf16: one accumulator.
+//
+// Against gathering the image by the contraction's own loaders (gemm_f32_tc.cu), where every value is fetched, tested and cut again
+// for each tap that reads it: 16 x 128 x 56 x 56, 128 filters of 3 x 3, f32 214 -> 95 us (cut 16, conv 75), bf16 247 -> 45;
+// 32 x 256 x 28 x 28, 256 of 3 x 3: f32 380 -> 214, bf16 462 -> 71. What bounds the f32 form: shared memory, 142 clocks per MMA of 96 (its
+// operands 10 KB and 5 KB of TMA writes). Also measured: blocks of 32 channels in 64-byte rows, 105 us (TMA takes as long for a row of 64
+// bytes as for one of 128); four accumulators of 128 columns, 114.
+#include "common.cuh"
+#include "f32_split.cuh"
+#include "sm100.cuh"
+
+namespace mimk {
+
+using namespace sm100;
+using namespace f32split;
+
+namespace {
+
+constexpr int BM = 128, BKC = 64, NUM_THREADS = 384, TMA_WARP = 8, MMA_WARP = 9;
+constexpr int STORE_REGS = 224, ISSUE_REGS = 56;  // two warpgroups and one, of 168 a thread at launch
+static_assert(2 * STORE_REGS + ISSUE_REGS <= 3 * 168, "setmaxnreg waits for ever for more than the launch was given");
+constexpr int A_BYTES = BM * BKC * 2;
+constexpr int PITCH = 33, STAGING = 8 * 32 * PITCH * 4;  // a 32 x 32 block per storing warp
+
+// A slot holds one piece of both operands, 64 channels. The pieces l, h of a block go through one ring and m through another, in the
+// order the products need them, and leave as soon as their last product is done: l after two of six, m after five, h at the end.
+template <int BN, int PIECES> struct Cfg {
+    static constexpr int SLOT_BYTES = A_BYTES + BN * BKC * 2;
+    static constexpr int ROOM  = (232448 - STAGING - 1024 - 512) / SLOT_BYTES;
+    static constexpr int M_SLOTS = PIECES == 3 ? (ROOM >= 6 ? 2 : 1) : 0, X_SLOTS = ROOM - M_SLOTS;
+    static constexpr int SMEM_BYTES = ROOM * SLOT_BYTES + STAGING + 1024 + 512;
+    static constexpr int NACC = 512 / BN;  // accumulators in tensor memory
+    static_assert(X_SLOTS >= 3 && X_SLOTS <= 6, "a block's l and h, and the next block's l on its way");
+};
+
+struct Bars {
+    uint64_t full[6], empty[6], m_full[2], m_empty[2], acc_full[4], acc_empty[4];
+    uint32_t tmem_base;
+    int abort_flag;
+};
+struct Ring {  // a place in a ring of N slots
+    uint32_t slot = 0, phase = 0;
+    template <int N> __device__ __forceinline__ void step() {
+        if (++slot == N) slot = 0, phase ^= 1u;
+    }
+};
+
+// the image laid out: grids of [n, hq, wq] rows of `pitch` channels, one per remainder of the padded coordinates by the strides
+// (one in all where the window is one pixel high / wide)
+struct Shape {
+    int n, cin, h, w, cout, kh, kw, oh, ow, stride_h, stride_w, dil_h, dil_w, pad_h, pad_w, by_tap;
+    int hp, wp, hq, wq, grids_h, grids_w, pitch;
+};
+struct Params {
+    Shape c;
+    const void* x;
+    const void* filters;
+    void* out;
+    int64_t tiles_m, tiles_n;
+    int* status;
+};
+
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
+
+template <class TIn>
+__device__ __forceinline__ const TIn* filter_at(const Shape& c, const void* filters, int co, int ci, int tap) {
+    const int taps = c.kh * c.kw;
+    return static_cast<const TIn*>(filters) + int64_t(co) * c.cin * taps + (c.by_tap ? tap * c.cin + ci : ci * taps + tap);
+}
+
+// neighbouring channels cut and stored, the pieces `piece` elements apart
+template <int PIECES>
+__device__ __forceinline__ void store_pieces(__nv_bfloat16* dst, int64_t piece, float a, float b) {
+#pragma unroll
+    for (int t = 0; t < PIECES; ++t) {
+        *reinterpret_cast<uint32_t*>(dst + t * piece) = upper_halves(a, b);
+        a = lower_part(a), b = lower_part(b);
+    }
+}
+template <int PIECES>
+__device__ __forceinline__ void store_pieces4(__nv_bfloat16* dst, int64_t piece, float (&v)[4]) {
+#pragma unroll
+    for (int t = 0; t < PIECES; ++t) {
+        *reinterpret_cast<uint2*>(dst + t * piece) = make_uint2(upper_halves(v[0], v[1]), upper_halves(v[2], v[3]));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = lower_part(v[i]);
+    }
+}
+
+// Blocks [0, n hp groups): one padded image row and 64 channels, turned in shared memory; the others: 2048 filter elements each.
+template <class TIn, int PIECES>
+__global__ void __launch_bounds__(256) conv_cut_kernel(const Params p, __nv_bfloat16* __restrict__ image, __nv_bfloat16* __restrict__ filters,
+                                                       int64_t image_piece, int64_t filter_piece) {
+    __shared__ float tile[64][65];
+    const Shape& c   = p.c;
+    const int groups = (c.pitch + 63) / 64, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int64_t rows = int64_t(c.n) * c.hp * groups;
+    if (blockIdx.x >= rows) {
+        const int taps = c.kh * c.kw;
+        int64_t i      = ((blockIdx.x - rows) * 256 + threadIdx.x) * 2;
+        const int64_t n = int64_t(c.cout) * taps * c.pitch, step = (gridDim.x - rows) * 512;
+        for (; i < n; i += step) {
+            const int64_t t = i / c.pitch;
+            const int ci = int(i - t * c.pitch), co = int(t / taps), tap = int(t - int64_t(co) * taps);
+            const float a = ci < c.cin ? load1(filter_at<TIn>(c, p.filters, co, ci, tap)) : 0.f;
+            const float b = ci + 1 < c.cin ? load1(filter_at<TIn>(c, p.filters, co, ci + 1, tap)) : 0.f;
+            store_pieces<PIECES>(filters + i, filter_piece, a, b);
+        }
+        return;
+    }
+    const int64_t line = blockIdx.x / groups;
+    const int c0 = int(blockIdx.x - line * groups) * 64, img = int(line / c.hp), y = int(line - int64_t(img) * c.hp);
+    const int yi = y - c.pad_h, yg = y % c.stride_h, yq = y / c.stride_h;
+    if (yg >= c.grids_h) return;  // no tap reads the row
+    const bool inside = unsigned(yi) < unsigned(c.h);
+    const int64_t plane = int64_t(c.h) * c.w, grid_rows = int64_t(c.n) * c.hq * c.wq;
+    __nv_bfloat16* line_out = image + (int64_t(yg) * c.grids_w * grid_rows + (int64_t(img) * c.hq + yq) * c.wq) * c.pitch + c0;
+    const TIn* src = static_cast<const TIn*>(p.x) + (int64_t(img) * c.cin + c0) * plane + int64_t(inside ? yi : 0) * c.w;
+    for (int x0 = 0; x0 < c.wp; x0 += 64) {
+        const int xi  = x0 + tx - c.pad_w;
+        const bool in0 = inside && unsigned(xi) < unsigned(c.w), in1 = inside && unsigned(xi + 32) < unsigned(c.w);
+        float v[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const int ch = ty + 8 * (j >> 1);
+            v[j]         = ((j & 1) ? in1 : in0) && c0 + ch < c.cin ? load1(src + ch * plane + xi + (j & 1) * 32) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) tile[tx + (j & 1) * 32][ty + 8 * (j >> 1)] = v[j];
+        __syncthreads();
+        const int ch = (tx & 15) * 4;  // four channels of every sixteenth pixel: half a warp writes 128 bytes of each piece
+        if (c0 + ch < c.pitch) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int px = j * 16 + ty * 2 + (tx >> 4), x = x0 + px;
+                const int xg = c.stride_w == 1 ? 0 : x % c.stride_w, xq = c.stride_w == 1 ? x : x / c.stride_w;
+                if (x >= c.wp || xg >= c.grids_w) continue;
+                float w[4] = {tile[px][ch], tile[px][ch + 1], tile[px][ch + 2], tile[px][ch + 3]};
+                store_pieces4<PIECES>(line_out + (xg * grid_rows + xq) * c.pitch + ch, image_piece, w);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// The scalar fold of one cell, ascending (channel, kh, kw), one fma per step, padding read as zeros: for cells the pieces make
+// non-finite (an operand was inf / NaN, or the sum overflowed).
+template <class TIn>
+__device__ __noinline__ float scalar_fold(const Params& p, int img, int co, int y, int x) {
+    const Shape& c = p.c;
+    const TIn* im  = static_cast<const TIn*>(p.x) + int64_t(img) * c.cin * c.h * c.w;
+    float v        = 0.f;
+    for (int ci = 0; ci < c.cin; ++ci)
+        for (int r = 0; r < c.kh; ++r)
+            for (int q = 0; q < c.kw; ++q) {
+                const int iy = y * c.stride_h - c.pad_h + r * c.dil_h, ix = x * c.stride_w - c.pad_w + q * c.dil_w;
+                const bool in = unsigned(iy) < unsigned(c.h) && unsigned(ix) < unsigned(c.w);
+                v = fmaf(in ? load1(im + (int64_t(ci) * c.h + iy) * c.w + ix) : 0.f, load1(filter_at<TIn>(c, p.filters, co, ci, r * c.kw + q)), v);
+            }
+    return v;
+}
+
+template <int BN, int PIECES, class T>
+__global__ void __launch_bounds__(NUM_THREADS, 1)
+conv_pieces_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ Params p) {
+    using C = Cfg<BN, PIECES>;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw_addr = smem_u32(smem_raw), base = (raw_addr + 1023u) & ~1023u;
+    uint8_t* after           = smem_raw + (base - raw_addr) + C::ROOM * C::SLOT_BYTES;
+    Bars* bars               = reinterpret_cast<Bars*>(after + STAGING);
+    volatile int* abort_flag = &bars->abort_flag;
+    const Shape& c           = p.c;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t num_tiles = p.tiles_m * p.tiles_n;
+    const int taps = c.kh * c.kw, cblocks = (c.cin + BKC - 1) / BKC, num_kb = taps * cblocks;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < C::X_SLOTS; ++i) {
+            mbar_init(smem_u32(&bars->full[i]), 1);
+            mbar_init(smem_u32(&bars->empty[i]), 1);
+        }
+        for (int i = 0; i < C::M_SLOTS; ++i) {
+            mbar_init(smem_u32(&bars->m_full[i]), 1);
+            mbar_init(smem_u32(&bars->m_empty[i]), 1);
+        }
+        for (int b = 0; b < C::NACC; ++b) {
+            mbar_init(smem_u32(&bars->acc_full[b]), 1);
+            mbar_init(smem_u32(&bars->acc_empty[b]), 8);
+        }
+        bars->abort_flag = 0;
+        fence_barrier_init();
+        tma_prefetch_desc(&tmA);
+        tma_prefetch_desc(&tmB);
+    }
+    if (warp == MMA_WARP) {
+        tmem_alloc(smem_u32(&bars->tmem_base), 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
+
+    const uint32_t m_base = base + C::X_SLOTS * C::SLOT_BYTES;
+
+    if (warp >= 8) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(ISSUE_REGS));
+    if (warp == TMA_WARP) {
+        if (lane == 0) {
+            Ring x, m;
+            bool ok = true;
+            const int grid_rows = c.n * c.hq * c.wq;
+            auto load = [&](uint32_t full, uint32_t empty, uint32_t phase, uint32_t at, int ax, int bx, int m0, int row, int piece) {
+                if (!(ok = mbar_wait(empty, phase ^ 1u, abort_flag))) return;
+                mbar_expect_tx(full, C::SLOT_BYTES);
+                tma_load_3d(at, &tmA, ax, m0, piece, full);
+                tma_load_3d(at + A_BYTES, &tmB, bx, row, piece, full);
+            };
+            for (int64_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+                const int m0 = int(tile % p.tiles_m) * BM, n0 = int(tile / p.tiles_m) * BN;
+                for (int r = 0, tap = 0; r < c.kh && ok; ++r)
+                    for (int q = 0; q < c.kw && ok; ++q, ++tap) {
+                        const int dy = r * c.dil_h, dx = q * c.dil_w;
+                        const int grid = (dy % c.stride_h) * c.grids_w + dx % c.stride_w;
+                        const int row  = n0 + grid * grid_rows + dy / c.stride_h * c.wq + dx / c.stride_w;
+                        for (int cb = 0; cb < cblocks && ok; ++cb) {
+                            const int ax = tap * c.pitch + cb * BKC, bx = cb * BKC;
+                            for (int t = PIECES == 3 ? 2 : 0; t >= 0 && ok; t -= 2) {  // l, h
+                                load(smem_u32(&bars->full[x.slot]), smem_u32(&bars->empty[x.slot]), x.phase, base + x.slot * C::SLOT_BYTES, ax, bx, m0, row, t);
+                                x.step<C::X_SLOTS>();
+                            }
+                            if constexpr (PIECES == 3) {
+                                if (!ok) break;
+                                load(smem_u32(&bars->m_full[m.slot]), smem_u32(&bars->m_empty[m.slot]), m.phase, m_base + m.slot * C::SLOT_BYTES, ax, bx, m0, row, 1);
+                                m.step<C::M_SLOTS>();
+                            }
+                        }
+                    }
+            }
+        }
+        __syncwarp();
+    } else if (warp == MMA_WARP) {
+        if (lane == 0) {
+            const uint32_t idesc = idesc_bf16_f32(BM, BN, 0, 0);
+            Ring x, m;
+            Ring acc;
+            bool ok = true;
+            // the product of two pieces over `steps` times 16 channels; first: into a fresh accumulator
+            auto product = [&](uint32_t d, uint32_t a, uint32_t b, int steps, bool first) {
+#pragma unroll
+                for (int k = 0; k < BKC / 16; ++k)
+                    if (k < steps)
+                        mma_f16_ss(d, smem_desc_sw128(a + k * 32, 16, 1024), smem_desc_sw128(b + A_BYTES + k * 32, 16, 1024), idesc, (!first || k > 0) ? 1u : 0u);
+            };
+            auto wait = [&](uint64_t& bar, uint32_t phase) { return ok = mbar_wait(smem_u32(&bar), phase, abort_flag); };
+            for (int64_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+                for (int kb = 0, cb = 0; kb < num_kb; ++kb) {
+                    const int left = c.cin - cb * BKC, steps = left >= BKC ? BKC / 16 : (left + 15) / 16;
+                    if (++cb == cblocks) cb = 0;
+                    if ((PIECES == 3 || kb == 0) && !wait(bars->acc_empty[acc.slot], acc.phase ^ 1u)) break;
+                    const uint32_t d = tmem_base + acc.slot * BN;
+                    if constexpr (PIECES == 3) {
+                        const uint32_t lo = base + x.slot * C::SLOT_BYTES;
+                        const uint32_t lo_empty = smem_u32(&bars->empty[x.slot]);
+                        if (!wait(bars->full[x.slot], x.phase)) break;
+                        x.step<C::X_SLOTS>();
+                        const uint32_t hi = base + x.slot * C::SLOT_BYTES;
+                        const uint32_t hi_empty = smem_u32(&bars->empty[x.slot]);
+                        if (!wait(bars->full[x.slot], x.phase)) break;
+                        x.step<C::X_SLOTS>();
+                        tc_fence_after();
+                        product(d, lo, hi, steps, true);
+                        product(d, hi, lo, steps, false);
+                        mma_commit(lo_empty);
+                        const uint32_t mid = m_base + m.slot * C::SLOT_BYTES;
+                        if (!wait(bars->m_full[m.slot], m.phase)) break;
+                        tc_fence_after();
+                        product(d, mid, mid, steps, false);
+                        product(d, mid, hi, steps, false);
+                        product(d, hi, mid, steps, false);
+                        mma_commit(smem_u32(&bars->m_empty[m.slot]));
+                        m.step<C::M_SLOTS>();
+                        product(d, hi, hi, steps, false);
+                        mma_commit(hi_empty);
+                    } else {
+                        if (!wait(bars->full[x.slot], x.phase)) break;
+                        tc_fence_after();
+                        product(d, base + x.slot * C::SLOT_BYTES, base + x.slot * C::SLOT_BYTES, steps, kb == 0);
+                        mma_commit(smem_u32(&bars->empty[x.slot]));
+                        x.step<C::X_SLOTS>();
+                    }
+                    if (PIECES == 3 || kb + 1 == num_kb) {
+                        mma_commit(smem_u32(&bars->acc_full[acc.slot]));
+                        acc.step<C::NACC>();
+                    }
+                }
+            }
+        }
+        __syncwarp();
+    }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(STORE_REGS));
+        constexpr int HALF = BN / 2;
+        static_assert(HALF % 32 == 0, "blocks of 32 columns");
+        const uint32_t quarter = uint32_t(warp & 3), col0 = uint32_t(warp >> 2) * HALF;
+        float* block = reinterpret_cast<float*>(after) + warp * (32 * PITCH);
+        Ring acc;
+        bool ok      = true;
+        const int chunks = PIECES == 3 ? num_kb : 1, per_image = c.hq * c.wq;
+        const int64_t pixels = int64_t(c.oh) * c.ow;
+        for (int64_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+            const int m0 = int(tile % p.tiles_m) * BM, n0 = int(tile / p.tiles_m) * BN;
+            float sum[HALF];
+#pragma unroll
+            for (int i = 0; i < HALF; ++i) sum[i] = 0.f;
+            for (int ch = 0; ch < chunks; ++ch) {
+                if (!(ok = warp_wait(smem_u32(&bars->acc_full[acc.slot]), acc.phase, abort_flag))) break;
+                tc_fence_after();
+                // all columns requested, then one wait: a read of tensor memory stands in line behind the MMAs that are queued
+                const uint32_t t0 = tmem_base + acc.slot * BN + col0 + ((quarter * 32u) << 16);
+                uint32_t r[HALF / 32][32];
+#pragma unroll
+                for (int i = 0; i < HALF / 32; ++i) tmem_ld_32x32(t0 + i * 32, r[i]);
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < HALF; ++i) sum[i] = PIECES == 3 ? sum[i] + __uint_as_float(r[i / 32][i % 32]) : __uint_as_float(r[i / 32][i % 32]);
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&bars->acc_empty[acc.slot]));
+                acc.step<C::NACC>();
+            }
+            if (!ok) break;
+            const int rows = c.cout - (m0 + int(quarter) * 32);
+#pragma unroll
+            for (int i = 0; i < HALF; i += 32) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) block[lane * PITCH + j] = sum[i + j];
+                __syncwarp();
+                const int v = n0 + int(col0) + i + lane, img = v / per_image, in = v - img * per_image, y = in / c.wq, x = in - y * c.wq;
+                const bool there = img < c.n && y < c.oh && x < c.ow;
+                const int co     = m0 + int(quarter) * 32;
+                T* dst           = static_cast<T*>(p.out) + (int64_t(img) * c.cout + co) * pixels + (int64_t(y) * c.ow + x);
+                float value[32], probe = 0.f;  // (a sum of v * 0 is zero where all are finite)
+#pragma unroll
+                for (int r = 0; r < 32; ++r) value[r] = block[r * PITCH + lane], probe = fmaf(value[r], 0.f, probe);
+                if (there) {
+#pragma unroll
+                    for (int r = 0; r < 32; ++r)
+                        if (r < rows) dst[r * pixels] = T(value[r]);
+                    if (probe != 0.f)
+                        for (int r = 0; r < 32 && r < rows; ++r)
+                            if (!isfinite(block[r * PITCH + lane])) dst[r * pixels] = T(scalar_fold<T>(p, img, co + r, y, x));
+                }
+                __syncwarp();
+            }
+        }
+    }
+
+    tc_fence_before();
+    __syncthreads();
+    if (warp == MMA_WARP) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, 512);
+    }
+    if (threadIdx.x == 0 && *abort_flag) *p.status = MIMK_E_DEVICE_WAIT;
+}
+
+Shape make_shape(const mimk_conv_desc& d) {
+    Shape c{};
+    c.n = int(d.n), c.cin = int(d.cin), c.h = int(d.h), c.w = int(d.w), c.cout = int(d.cout), c.kh = int(d.kh), c.kw = int(d.kw);
+    c.stride_h = int(d.stride_h), c.stride_w = int(d.stride_w), c.dil_h = int(d.dil_h), c.dil_w = int(d.dil_w);
+    c.pad_h = int(d.pad_h), c.pad_w = int(d.pad_w), c.by_tap = d.by_tap;
+    c.hp = c.h + 2 * c.pad_h, c.wp = c.w + 2 * c.pad_w;
+    c.oh = (c.hp - c.dil_h * (c.kh - 1) - 1) / c.stride_h + 1, c.ow = (c.wp - c.dil_w * (c.kw - 1) - 1) / c.stride_w + 1;
+    c.hq = (c.hp + c.stride_h - 1) / c.stride_h, c.wq = (c.wp + c.stride_w - 1) / c.stride_w;
+    c.grids_h = c.kh == 1 ? 1 : c.stride_h, c.grids_w = c.kw == 1 ? 1 : c.stride_w;
+    c.pitch = (c.cin + 7) & ~7;
+    return c;
+}
+
+struct Sizes {
+    int64_t image, filters;  // elements of one piece
+    size_t bytes(int pieces) const { return size_t(pieces) * size_t(image + filters) * 2 + 512; }
+};
+Sizes make_sizes(const Shape& c) {
+    return Sizes{int64_t(c.grids_h) * c.grids_w * c.n * c.hq * c.wq * c.pitch, int64_t(c.cout) * c.kh * c.kw * c.pitch};
+}
+
+// Tile width: the one with the least estimated time: launches, a pass over the image at 4.1 TB/s, and rounds of a tile per SM. Measured
+// per block of 64 channels, f32: 1.52 us (128 wide) and 1.85 (192), what the tile's shared-memory traffic takes at 106 bytes a clock
+// (of 288 and 360 KB, a third of it written by TMA); bf16 0.45, 0.55 and 0.7 (256), the loads.
+struct Plan {
+    int bn;
+    double us;
+};
+Plan make_plan(const Shape& c, int pieces, int sm_count) {
+    const int64_t positions = int64_t(c.n) * c.hq * c.wq, tiles_m = (c.cout + BM - 1) / BM;
+    const double kb = double(c.kh) * c.kw * ((c.cin + BKC - 1) / BKC);
+    const Sizes s   = make_sizes(c);
+    const double bytes = double(c.n) * c.cin * c.h * c.w * (pieces == 3 ? 4 : 2) + double(s.bytes(pieces));
+    const double part  = double((c.cin < BKC ? c.cin : BKC) + 15) / 16 / 4;  // of a block's MMAs that are issued
+    Plan best{128, 1e300};
+    for (int bn : {128, 192, 256}) {
+        if (pieces == 3 && bn == 256) continue;
+        const double rounds = double((tiles_m * ((positions + bn - 1) / bn) + sm_count - 1) / sm_count);
+        const double loads = pieces == 3 ? (bn == 128 ? 0.95 : 1.2) : (bn == 128 ? 0.45 : bn == 192 ? 0.55 : 0.7);
+        const double mmas  = (pieces == 3 ? (bn == 128 ? 1.52 : 1.85) : 0.0) * part;
+        const double us    = 11.0 + bytes / 4.1e6 + rounds * (4.0 + kb * (mmas > loads ? mmas : loads));
+        if (us < best.us) best = Plan{bn, us};
+    }
+    return best;
+}
+
+int make_tmap(CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows, uint64_t pieces, uint64_t piece_elems, uint32_t box_rows) {
+    cuuint64_t dims[3]    = {inner, rows, pieces};
+    cuuint64_t strides[2] = {inner * 2, piece_elems * 2};
+    cuuint32_t box[3]     = {BKC, box_rows, 1};
+    return encode_tmap_bf16_3d(out, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+template <int BN, int PIECES, class T>
+int launch(Params& p, __nv_bfloat16* image, __nv_bfloat16* filters, const Sizes& sizes, int sm_count, cudaStream_t s) {
+    const Shape& c = p.c;
+    auto kern      = conv_pieces_kernel<BN, PIECES, T>;
+    constexpr int SMEM = Cfg<BN, PIECES>::SMEM_BYTES;
+    static bool configured[64] = {};  // per template instance and device: the attribute is a per-device setting
+    int dev = 0;
+    MIMK_CUDA_TRY(cudaGetDevice(&dev));
+    if (!configured[dev & 63]) {
+        MIMK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        configured[dev & 63] = true;
+    }
+    const int64_t positions = int64_t(c.n) * c.hq * c.wq;
+    CUtensorMap tmA, tmB;
+    MIMK_TRY(make_tmap(&tmA, filters, uint64_t(c.kh) * c.kw * c.pitch, uint64_t(c.cout), PIECES, uint64_t(sizes.filters), BM));
+    MIMK_TRY(make_tmap(&tmB, image, uint64_t(c.pitch), uint64_t(positions) * c.grids_h * c.grids_w, PIECES, uint64_t(sizes.image), BN));
+    p.tiles_m = (c.cout + BM - 1) / BM, p.tiles_n = (positions + BN - 1) / BN;
+    const int64_t tiles = p.tiles_m * p.tiles_n;
+    kern<<<unsigned(tiles < sm_count ? tiles : sm_count), NUM_THREADS, SMEM, s>>>(tmA, tmB, p);
+    return launch_status();
+}
+
+}  // namespace
+
+// Whether this route takes the convolution: 31-bit rows, a buffer of at most 1 GiB, an estimate below `other_us`, and f32 only where
+// the accumulators are not many more than one per 64 k, whose sums are what the error comes from (channels in whole blocks; 32 in 25 taps 1.41e-7
+// on either route, but 16 in 25 taps 1.35e-7 against 1.33e-7, 96 in 25 taps 1.75e-7 against 1.68e-7).
+int conv_pieces_preferred(const mimk_conv_desc& d, int sm_count, double other_us) {
+    if (d.n < 1 || d.cout < 1 || d.n >= (1 << 30) || d.cout >= (1 << 30)) return 0;
+    const double rows = double(d.n) * (double(d.h) + 2.0 * double(d.pad_h) + double(d.stride_h)) * (double(d.w) + 2.0 * double(d.pad_w) + double(d.stride_w));
+    if (rows >= double(1 << 30) || double(d.cin + 8) * double(d.kh) * double(d.kw) >= double(1 << 30)) return 0;
+    const Shape c    = make_shape(d);
+    const int pieces = d.dtype == MIMK_F32 ? 3 : 1;
+    if (pieces == 3 && c.cin % BKC != 0 && (c.cin <= 16 || c.cin > 32) && c.kh * c.kw * ((c.cin + BKC - 1) / BKC) > 10) return 0;
+    if (make_sizes(c).bytes(pieces) > (size_t(1) << 30)) return 0;
+    return make_plan(c, pieces, sm_count).us < other_us;
+}
+
+// MIMK_E_UNSUPPORTED, with nothing launched, where the buffer cannot be had: under stream capture (a graph must not hold on to the
+// cached buffer) and when there is no memory for it.
+int conv_pieces(const mimk_conv_desc& d, cudaStream_t s) {
+    int st          = MIMK_OK;
+    DeviceInfo* dev = device_info(&st);
+    if (!dev) return st;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    MIMK_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return MIMK_E_UNSUPPORTED;
+    Params p{};
+    p.c = make_shape(d);
+    const int pieces  = d.dtype == MIMK_F32 ? 3 : 1;
+    const Sizes sizes = make_sizes(p.c);
+    void* scratch     = nullptr;
+    if (get_scratch(sizes.bytes(pieces), &scratch, s) != MIMK_OK) {
+        cudaGetLastError();
+        return MIMK_E_UNSUPPORTED;
+    }
+    auto* image   = static_cast<__nv_bfloat16*>(scratch);
+    auto* filters = reinterpret_cast<__nv_bfloat16*>((reinterpret_cast<uintptr_t>(image + pieces * sizes.image) + 255) & ~uintptr_t(255));
+    p.x = d.x, p.filters = d.filters, p.out = d.out, p.status = dev->status_dev;
+    const Shape& c = p.c;
+    const int64_t rows = int64_t(c.n) * c.hp * ((c.pitch + 63) / 64), extra = (sizes.filters + 2047) / 2048;
+    const unsigned blocks = unsigned(rows + (extra < 1024 ? extra : 1024));
+    if (pieces == 3) conv_cut_kernel<float, 3><<<blocks, 256, 0, s>>>(p, image, filters, sizes.image, sizes.filters);
+    else conv_cut_kernel<__nv_bfloat16, 1><<<blocks, 256, 0, s>>>(p, image, filters, sizes.image, sizes.filters);
+    MIMK_TRY(launch_status());
+    const int bn = make_plan(c, pieces, dev->sm_count).bn;
+    if (pieces == 3)
+        return bn == 128 ? launch<128, 3, float>(p, image, filters, sizes, dev->sm_count, s) : launch<192, 3, float>(p, image, filters, sizes, dev->sm_count, s);
+    return bn == 128   ? launch<128, 1, __nv_bfloat16>(p, image, filters, sizes, dev->sm_count, s)
+           : bn == 192 ? launch<192, 1, __nv_bfloat16>(p, image, filters, sizes, dev->sm_count, s)
+                       : launch<256, 1, __nv_bfloat16>(p, image, filters, sizes, dev->sm_count, s);
+}
+
+}  // namespace mimk

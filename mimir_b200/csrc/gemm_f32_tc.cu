@@ -669,12 +669,28 @@ int gemm_bf16_chunked(const mimk_gemm_desc& d, cudaStream_t s) {
     return plan_and_launch<__nv_bfloat16, float, false>(p, d.batch, dev->sm_count, s);
 }
 
+static int64_t conv_oh(const mimk_conv_desc& d) { return (d.h + 2 * d.pad_h - d.dil_h * (d.kh - 1) - 1) / d.stride_h + 1; }
+static int64_t conv_ow(const mimk_conv_desc& d) { return (d.w + 2 * d.pad_w - d.dil_w * (d.kw - 1) - 1) / d.stride_w + 1; }
+
+// Gathering costs more than the plan's k-blocks: rounds * (14 + 1.75 us per k-block), 7 + 1.25 up to 64 filters, within 15 % of the
+// measured 214 us (16 x 128 x 56 x 56, 128 filters of 3 x 3), 69 (of 1 x 1), 79 (6 images), 380 (32 x 256 x 28 x 28, 256 of 3 x 3),
+// 161 (64 filters). f32 over a cluster stays here: each CTA adds its own accumulators first, which leaves less rounding than one long
+// sum (4 x 256 x 28 x 28, 256 filters of 3 x 3, 77 us and 1.50e-7 against 73 and 1.65e-7).
+int conv_tc_preferred(const mimk_conv_desc& d, int sm_count) {
+    const int64_t pixels = d.n * conv_oh(d) * conv_ow(d), k = d.cin * d.kh * d.kw;
+    const Plan plan = make_plan(pixels, d.cout, k, 1, sm_count);
+    if (d.dtype == MIMK_F32 && plan.split > 1) return 1;
+    const int64_t tiles = ((pixels + BM - 1) / BM) * ((d.cout + plan.bn - 1) / plan.bn);
+    const double kb = double((k + BK - 1) / BK), round = plan.bn == 128 ? 14.0 + 1.75 * kb : 7.0 + 1.25 * kb;
+    return !conv_pieces_preferred(d, sm_count, plan.split > 1 ? plan.us : double((tiles + sm_count - 1) / sm_count) * round);
+}
+
 int conv_tc(const mimk_conv_desc& d, cudaStream_t s) {
     int st          = MIMK_OK;
     DeviceInfo* dev = device_info(&st);
     if (!dev) return st;
     Params p{};
-    const int64_t oh = (d.h + 2 * d.pad_h - d.dil_h * (d.kh - 1) - 1) / d.stride_h + 1, ow = (d.w + 2 * d.pad_w - d.dil_w * (d.kw - 1) - 1) / d.stride_w + 1;
+    const int64_t oh = conv_oh(d), ow = conv_ow(d);
     p.A = d.x, p.B = d.filters, p.C = d.out;
     p.M = d.n * oh * ow, p.N = d.cout, p.K = d.cin * d.kh * d.kw;
     p.conv = ConvShape{int(d.cin), int(d.h), int(d.w), int(d.kh), int(d.kw), int(oh), int(ow), int(d.stride_h), int(d.stride_w),

@@ -225,5 +225,8 @@ int make_tmap_bf16_3d(CUtensorMap* out, const void* base, uint64_t inner, uint64
                       uint64_t mid_stride_bytes, uint64_t outer_stride_bytes, uint32_t box_inner, uint32_t box_mid);
 int make_tmap_3d(CUtensorMap* out, bool f32, const void* base, uint64_t inner, uint64_t mid, uint64_t outer,
                  uint64_t mid_stride_bytes, uint64_t outer_stride_bytes, uint32_t box_inner, uint32_t box_mid);
+// any 3-D bf16 map: dims and box innermost first, strides in bytes (multiples of 16)
+int encode_tmap_bf16_3d(CUtensorMap* out, const void* base, const cuuint64_t (&dims)[3], const cuuint64_t (&strides)[2], const cuuint32_t (&box)[3],
+                        CUtensorMapSwizzle swizzle);
 
 }  // namespace mimk

@@ -683,8 +683,9 @@ def _sm_count(device: int) -> int:
     return torch.cuda.get_device_properties(device).multi_processor_count
 
 
-def _patches_pay(dtype, pixels, cout, k, window, padded) -> bool:
-    """Whether a patch matrix and the full-rate contraction beat gathering the patches inside the contraction.
+def _patches_pay(dtype, pixels, cout, k, window, padded, laid_out) -> bool:
+    """Whether a patch matrix and the full-rate contraction beat gathering the patches inside the contraction. They never do where
+    the contraction lays the image out first and reads it in place of patches (mimk_conv_laid_out).
 
     bf16: both estimated, in us. Gathered: rounds of a tile per SM, 14 + 1.85 per k-block of 32 (7 + 1.25 for up to 64 filters).
     Patches: three or four operators' host time, 85 or 112, or where it is more the matrix at 1.3 per MB, the result at 2 (written
@@ -693,6 +694,8 @@ def _patches_pay(dtype, pixels, cout, k, window, padded) -> bool:
     1 x 1, 45 / 83.
     f32: the contraction that takes the patches writes two copies of them; only where each pixel is gathered again for many filters
     without a window to blow it up: 32 x 256 x 56 x 56, 512 of 1 x 1, 595 / 536; 256 of them, 307 / 371."""
+    if laid_out:
+        return False
     if dtype == torch.float32:
         return window == 1 and cout > 256 and cout % 4 == 0 and pixels * cout * k >= 1 << 33
     if not _whole_tiles(k, cout):
@@ -768,19 +771,23 @@ def conv(x: torch.Tensor, w: torch.Tensor, stride=(1, 1), dilation=(1, 1), paddi
         if as_patches:
             raise TypeError("conv: both operands share the ring's element type")
         gathered = False   # the per-cell kernel takes operands of two element types
-    if as_patches and not (gathered and not _patches_pay(x.dtype, n * oh * ow, cout, k, kh * kw, any(padding))):
+    laid_out = False
+    if gathered:
+        d = L.ConvDesc()
+        d.n, d.cin, d.h, d.w, d.cout, d.kh, d.kw = n, cin, h, wd, cout, kh, kw
+        d.stride_h, d.stride_w, d.dil_h, d.dil_w, d.pad_h, d.pad_w = *stride, *dilation, *padding
+        d.dtype = _dt(x)
+        laid_out = bool(L.lib().mimk_conv_laid_out(C.byref(d), _stream()))
+    if as_patches and not (gathered and not _patches_pay(x.dtype, n * oh * ow, cout, k, kh * kw, any(padding), laid_out)):
         xp = pad(x, (0, 0, padding[0], padding[1]), (0, 0, padding[0], padding[1])) if any(padding) else x
         return _conv_as_contraction(xp, w, n, cin, cout, kh, kw, oh, ow, stride, dilation)
     if gathered:
         x, w = x.contiguous(), w.contiguous()
         out = torch.empty((n, cout, oh, ow), dtype=x.dtype, device=x.device)
-        d = L.ConvDesc()
-        d.by_tap = cin % 8 == 0 and kh * kw > 1
+        d.by_tap = not laid_out and cin % 8 == 0 and kh * kw > 1
         if d.by_tap:
             w = transpose(w.view(cout, cin, kh * kw), (0, 2, 1))
-        d.n, d.cin, d.h, d.w, d.cout, d.kh, d.kw = n, cin, h, wd, cout, kh, kw
-        d.stride_h, d.stride_w, d.dil_h, d.dil_w, d.pad_h, d.pad_w = *stride, *dilation, *padding
-        d.x, d.filters, d.out, d.dtype = x.data_ptr(), w.data_ptr(), out.data_ptr(), _dt(x)
+        d.x, d.filters, d.out = x.data_ptr(), w.data_ptr(), out.data_ptr()
         L.check(L.lib().mimk_conv(C.byref(d), _stream()), "conv")
         return out
     xp = pad(x, (0, 0, padding[0], padding[1]), (0, 0, padding[0], padding[1])) if any(padding) else x

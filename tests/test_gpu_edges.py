@@ -1,6 +1,7 @@
 """GPU parity at the edges of tiles, alignments and splits: contractions with ragged extents and with few tiles, f32 products and
 attention on the tensor cores, attention of a few queries, convolutions gathered from the image, folds and maps with remainders.
 References are float64 on the CPU."""
+import ctypes as C
 import math
 
 import pytest
@@ -316,6 +317,38 @@ def test_windows_too_wide_to_gather_go_through_patches(T, monkeypatch, n, cin, h
     other = BF16 if dtype == F32 else F32
     with pytest.raises(TypeError):
         T.conv(x, f.to(other), stride=stride, dilation=dil, padding=pad)
+
+
+@pytest.mark.parametrize("n,cin,h,w,cout,kh,kw,stride,dil,pad", [
+    (1, 1, 5, 7, 1, 1, 1, (1, 1), (1, 1), (0, 0)), (2, 5, 17, 23, 16, 3, 3, (1, 1), (1, 1), (1, 1)),
+    (3, 33, 30, 31, 65, 3, 2, (2, 1), (1, 2), (0, 1)), (2, 64, 15, 66, 130, 3, 3, (2, 2), (1, 1), (1, 1)),
+    (5, 72, 20, 70, 128, 1, 1, (2, 2), (1, 1), (0, 0)), (2, 130, 13, 9, 257, 5, 5, (3, 2), (2, 3), (4, 6)),
+    (1, 64, 65, 130, 129, 1, 4, (1, 3), (1, 1), (0, 2)), (40, 16, 28, 28, 96, 3, 3, (1, 1), (1, 1), (1, 1))])
+@pytest.mark.parametrize("by_tap", [0, 1])
+@pytest.mark.parametrize("dtype", [F32, BF16])
+def test_convolutions_over_an_image_laid_out_once(T, n, cin, h, w, cout, kh, kw, stride, dil, pad, by_tap, dtype):
+    # the kernel itself, whatever the estimate says: ragged channels and filters, strided and dilated windows, tiles across images
+    L = T.L
+    run = L.lib()["_ZN4mimk11conv_piecesERK14mimk_conv_descP11CUstream_st"]
+    run.restype, run.argtypes = C.c_int, [C.POINTER(L.ConvDesc), C.c_void_p]
+    x, f = rnd((n, cin, h, w), 1, dtype), rnd((cout, cin, kh, kw), 2, dtype)
+    stored = f.flatten(2).transpose(1, 2).contiguous() if by_tap else f
+    oh, ow = ((e + 2 * p - d * (k - 1) - 1) // s + 1 for e, p, d, k, s in zip((h, w), pad, dil, (kh, kw), stride))
+    d = L.ConvDesc()
+    d.n, d.cin, d.h, d.w, d.cout, d.kh, d.kw = n, cin, h, w, cout, kh, kw
+    d.stride_h, d.stride_w, d.dil_h, d.dil_w, d.pad_h, d.pad_w = *stride, *dil, *pad
+    d.dtype, d.by_tap, d.x, d.filters = T._dt(x), by_tap, x.data_ptr(), stored.data_ptr()
+
+    def conv():
+        out = torch.full((n, cout, oh, ow), 7.0, dtype=dtype, device="cuda")
+        d.out = out.data_ptr()
+        L.check(run(C.byref(d), T._stream()), "conv")
+        T.device_status()
+        return out
+    ref = lambda u, v: torch.nn.functional.conv2d(u, v, stride=stride, dilation=dil, padding=pad)
+    close_cells(conv(), ref(d64(x), d64(f)), ref(d64(x).abs(), d64(f).abs()) + 1e-6, F32_CELL if dtype == F32 else BF16_ROUND)
+    x[0, 0, h // 2, w // 2] = math.inf   # it reaches the cells whose window holds it, and no other
+    assert torch.equal(d64(conv()).isfinite(), ref(d64(x), d64(f)).isfinite())
 
 
 @pytest.mark.parametrize("m,n,k,b_nk,post,out,offset", [
