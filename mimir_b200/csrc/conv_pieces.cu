@@ -14,10 +14,10 @@
 // bf16: one accumulator.
 //
 // Against gathering the image by the contraction's own loaders (gemm_f32_tc.cu), where every value is fetched, tested and cut again
-// for each tap that reads it: 16 x 128 x 56 x 56, 128 filters of 3 x 3, f32 214 -> 95 us (cut 16, conv 75), bf16 247 -> 45;
-// 32 x 256 x 28 x 28, 256 of 3 x 3: f32 380 -> 214, bf16 462 -> 71. What bounds the f32 form: shared memory, 142 clocks per MMA of 96 (its
+// for each tap that reads it: 16 x 128 x 56 x 56, 128 filters of 3 x 3, f32 214 -> 83 us (cut 16, conv 61), bf16 247 -> 42;
+// 32 x 256 x 28 x 28, 256 of 3 x 3: f32 380 -> 175, bf16 462 -> 68. What bounds the f32 form: shared memory, 116 clocks per MMA of 96 (its
 // operands 10 KB and 5 KB of TMA writes). Also measured: blocks of 32 channels in 64-byte rows, 105 us (TMA takes as long for a row of 64
-// bytes as for one of 128); four accumulators of 128 columns, 114.
+// bytes as for one of 128); four accumulators of 128 columns, 114; MMAs issued by lane 0 in a branch of its own, 95.
 #include "common.cuh"
 #include "f32_split.cuh"
 #include "sm100.cuh"
@@ -255,19 +255,25 @@ conv_pieces_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         }
         __syncwarp();
     } else if (warp == MMA_WARP) {
-        if (lane == 0) {
+        {
+            // (the whole warp runs, one lane issues: with lane 0 alone in the branch the descriptors are not known to be uniform, and moving them
+            // costs about 50 clocks per MMA)
+            const bool leader = elect_one();
             const uint32_t idesc = idesc_bf16_f32(BM, BN, 0, 0);
             Ring x, m;
             Ring acc;
             bool ok = true;
-            // the product of two pieces over `steps` times 16 channels; first: into a fresh accumulator
+            const uint64_t desc0 = smem_desc_sw128(base, 16, 1024);
+            // the product of the pieces in two places over `steps` times 16 channels; first: into a fresh accumulator
             auto product = [&](uint32_t d, uint32_t a, uint32_t b, int steps, bool first) {
+                const uint64_t da = desc0 + a * (C::SLOT_BYTES >> 4), db = desc0 + b * (C::SLOT_BYTES >> 4) + (A_BYTES >> 4);
+                if (leader)
 #pragma unroll
-                for (int k = 0; k < BKC / 16; ++k)
-                    if (k < steps)
-                        mma_f16_ss(d, smem_desc_sw128(a + k * 32, 16, 1024), smem_desc_sw128(b + A_BYTES + k * 32, 16, 1024), idesc, (!first || k > 0) ? 1u : 0u);
+                    for (int k = 0; k < BKC / 16; ++k)
+                        if (k < steps) mma_f16_ss(d, da + k * 2, db + k * 2, idesc, (!first || k > 0) ? 1u : 0u);
             };
-            auto wait = [&](uint64_t& bar, uint32_t phase) { return ok = mbar_wait(smem_u32(&bar), phase, abort_flag); };
+            auto commit = [&](uint32_t bar) { if (leader) mma_commit(bar); };
+            auto wait = [&](uint64_t& bar, uint32_t phase) { return ok = warp_wait(smem_u32(&bar), phase, abort_flag); };
             for (int64_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
                 for (int kb = 0, cb = 0; kb < num_kb; ++kb) {
                     const int left = c.cin - cb * BKC, steps = left >= BKC ? BKC / 16 : (left + 15) / 16;
@@ -275,37 +281,37 @@ conv_pieces_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                     if ((PIECES == 3 || kb == 0) && !wait(bars->acc_empty[acc.slot], acc.phase ^ 1u)) break;
                     const uint32_t d = tmem_base + acc.slot * BN;
                     if constexpr (PIECES == 3) {
-                        const uint32_t lo = base + x.slot * C::SLOT_BYTES;
+                        const uint32_t lo = x.slot;
                         const uint32_t lo_empty = smem_u32(&bars->empty[x.slot]);
                         if (!wait(bars->full[x.slot], x.phase)) break;
                         x.step<C::X_SLOTS>();
-                        const uint32_t hi = base + x.slot * C::SLOT_BYTES;
+                        const uint32_t hi = x.slot;
                         const uint32_t hi_empty = smem_u32(&bars->empty[x.slot]);
                         if (!wait(bars->full[x.slot], x.phase)) break;
                         x.step<C::X_SLOTS>();
                         tc_fence_after();
                         product(d, lo, hi, steps, true);
                         product(d, hi, lo, steps, false);
-                        mma_commit(lo_empty);
-                        const uint32_t mid = m_base + m.slot * C::SLOT_BYTES;
+                        commit(lo_empty);
+                        const uint32_t mid = C::X_SLOTS + m.slot;
                         if (!wait(bars->m_full[m.slot], m.phase)) break;
                         tc_fence_after();
                         product(d, mid, mid, steps, false);
                         product(d, mid, hi, steps, false);
                         product(d, hi, mid, steps, false);
-                        mma_commit(smem_u32(&bars->m_empty[m.slot]));
+                        commit(smem_u32(&bars->m_empty[m.slot]));
                         m.step<C::M_SLOTS>();
                         product(d, hi, hi, steps, false);
-                        mma_commit(hi_empty);
+                        commit(hi_empty);
                     } else {
                         if (!wait(bars->full[x.slot], x.phase)) break;
                         tc_fence_after();
-                        product(d, base + x.slot * C::SLOT_BYTES, base + x.slot * C::SLOT_BYTES, steps, kb == 0);
-                        mma_commit(smem_u32(&bars->empty[x.slot]));
+                        product(d, x.slot, x.slot, steps, kb == 0);
+                        commit(smem_u32(&bars->empty[x.slot]));
                         x.step<C::X_SLOTS>();
                     }
                     if (PIECES == 3 || kb + 1 == num_kb) {
-                        mma_commit(smem_u32(&bars->acc_full[acc.slot]));
+                        commit(smem_u32(&bars->acc_full[acc.slot]));
                         acc.step<C::NACC>();
                     }
                 }
@@ -430,7 +436,7 @@ int make_tmap(CUtensorMap* out, const void* base, uint64_t inner, uint64_t rows,
     cuuint64_t dims[3]    = {inner, rows, pieces};
     cuuint64_t strides[2] = {inner * 2, piece_elems * 2};
     cuuint32_t box[3]     = {BKC, box_rows, 1};
-    return encode_tmap_bf16_3d(out, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+    return encode_tmap_bf16(out, base, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 template <int BN, int PIECES, class T>
