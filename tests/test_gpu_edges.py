@@ -107,6 +107,30 @@ def test_f32_attention_of_tiny_values(T, sq, sk, d, causal, qs, ks, vs):
     assert ((d64(got) - want).abs() <= 200 * F32_CELL * weights + 1e-43).all()
 
 
+@pytest.mark.parametrize("bh,sq,sk,d,causal", [
+    (2, 129, 384, 64, False), (90, 300, 449, 64, True), (90, 257, 400, 30, False), (3, 200, 513, 97, True), (2, 500, 385, 128, True), (2, 1000, 450, 33, True)])
+@pytest.mark.parametrize("vs", [1.0, 1e-38, 1e-41, math.inf])
+def test_f32_attention_with_keys_cut_beforehand(T, bh, sq, sk, d, causal, vs):
+    # one and two query tiles to an SM, tiles without a partner and of different lengths, values that do not fit the pieces, infinities
+    q, k, v = rnd((bh, sq, d), 1), rnd((bh, sk, d), 2), rnd((bh, sk, d), 3)
+    if vs == math.inf:
+        q[0, 5, 3], k[1, 7, 2] = math.inf, -math.inf
+        if not causal:   # (a hidden key's value is not read; the reference would multiply it by zero)
+            v[0, 9, 1], v[1, 300, 1] = math.nan, math.inf
+    else:
+        v[:, :, d // 2:] *= vs
+    got, lse = T.attention(q, k, v, scale=d ** -0.5, causal=causal, return_lse=True)
+    T.device_status()
+    want, want_lse = attention_reference(q, k, v, d ** -0.5, causal)
+    g, w = d64(got), want
+    assert torch.equal(g.isnan(), w.isnan()) and torch.equal(g.isinf(), w.isinf())
+    weights = attention_reference(q, k, v.abs().nan_to_num(1, 1, 1), d ** -0.5, causal)[0].nan_to_num(1)
+    ok = w.isfinite()
+    assert ((g - w).abs() <= 64 * F32_CELL * weights + 1e-43)[ok].all()
+    seen = want_lse.isfinite()
+    assert ((d64(lse) - want_lse).abs()[seen] <= 64 * F32_CELL).all()
+
+
 @pytest.mark.parametrize("d", [16, 64, 128])
 @pytest.mark.parametrize("bh,sq,sk", [(1, 3, 1), (1, 3, 24), (700, 2, 20), (700, 40, 20), (700, 2, 64)])
 def test_f32_attention_of_few_keys(T, bh, sq, sk, d):
