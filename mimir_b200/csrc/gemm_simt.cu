@@ -95,68 +95,81 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const TIn* __restrict__ 
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// Small f32 products: 32 x 32 tiles, the K extent staged in 128-wide chunks by asynchronous 16-byte copies.
+// Small f32 products: 32 x 32 tiles, or 16 x 32 where those leave most SMs without one, the K extent staged in 128-wide chunks by
+// asynchronous copies.
 //
 // A product like 256^3 has 16 tiles of 64 x 64: sixteen CTAs on 148 SMs, each walking K in sixteen steps that every one
-// pay a global-memory latency. Here the same product is 64 CTAs, and both chunks of a K <= 256 are in flight from the
+// pay a global-memory latency. Here the same product is 128 CTAs, and both chunks of a K <= 256 are in flight from the
 // first instruction (two stages; longer K streams through them), so a CTA waits for memory once. The fold per cell is
 // the one above -- ascending k, one fma per step -- so the two kernels agree bit for bit.
-// Thread (tx, ty) of the 16 x 16 block owns rows ty, ty + 16 and, for B stored [N, K], columns tx, tx + 16 (both operands
+// Copies of 16 bytes where an operand's rows allow them, of 4 else (1024 x 10 x 128: 10.8 us on the kernel above, 3.7 here; 1000 x 61 x 250 stored [N, K] 17 and 5).
+// Thread (tx, ty) of the 16 x 16 block owns rows ty (and ty + 16) and, for B stored [N, K], columns tx, tx + 16 (both operands
 // K-major in shared memory, read four k at a time: a quarter-warp reads one A address and eight B rows whose pitch of
 // KC + 4 floats spreads them over all banks); for B stored [K, N], columns 2 tx, 2 tx + 1 (one 8-byte read per k).
+// What bounds it: the launch, one trip to memory and the issue of 13 instructions per 4 k and cell pair. 256^3: 5.7 us (6.4 with
+// 32-row tiles on 64 CTAs).
 // ---------------------------------------------------------------------------------------------------------------------
-constexpr int ST = 32, KC = 128, KP = KC + 4, NP = ST + 4;
+constexpr int SN = 32, KC = 128, KP = KC + 4, NP = SN + 4;
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
     const uint32_t d = uint32_t(__cvta_generic_to_shared(dst));
     const int sz     = valid ? 16 : 0;  // 0: nothing is read, the 16 bytes are filled with zeros
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(sz) : "memory");
 }
+__device__ __forceinline__ void cp_async4(void* dst, const void* src, bool valid) {
+    const uint32_t d = uint32_t(__cvta_generic_to_shared(dst));
+    const int sz     = valid ? 4 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(sz) : "memory");
+}
 
-template <bool B_NK>
+// A [rows x width] part of a row-major matrix, `pitch` elements a row in memory and `to_pitch` in shared memory; zeros outside.
+template <int ROWS, int WIDTH>
+__device__ __forceinline__ void stage_part(float* to, int to_pitch, const float* from, int64_t pitch, int64_t rows, int64_t cols, bool vec) {
+    if (vec) {
+        constexpr int PER_ROW = WIDTH / 4;
+#pragma unroll
+        for (int r = 0; r < ROWS * PER_ROW / 256; ++r) {
+            const int g = threadIdx.x + r * 256, row = g / PER_ROW, col = g % PER_ROW * 4;
+            const bool ok = row < rows && col < cols;
+            cp_async16(to + row * to_pitch + col, ok ? from + row * pitch + col : from, ok);
+        }
+    } else {
+#pragma unroll 4
+        for (int r = 0; r < ROWS * WIDTH / 256; ++r) {
+            const int g = threadIdx.x + r * 256, row = g / WIDTH, col = g % WIDTH;
+            const bool ok = row < rows && col < cols;
+            cp_async4(to + row * to_pitch + col, ok ? from + row * pitch + col : from, ok);
+        }
+    }
+}
+
+// RT: rows of a thread
+template <bool B_NK, int RT>
 __global__ void __launch_bounds__(256) gemm_simt_small_kernel(const float* __restrict__ A, const float* __restrict__ B,
                                                              float* __restrict__ C, int64_t M, int64_t N, int64_t K,
-                                                             int64_t sa, int64_t sb, int64_t sc, int post,
+                                                             int64_t sa, int64_t sb, int64_t sc, int post, int vec_a, int vec_b,
                                                              const float* __restrict__ post_row,
                                                              const float* __restrict__ post_full) {
     extern __shared__ __align__(16) float smem[];
-    constexpr int A_FLOATS = ST * KP, B_FLOATS = B_NK ? ST * KP : KC * NP;
+    constexpr int SM = 16 * RT, A_FLOATS = SM * KP, B_FLOATS = B_NK ? SN * KP : KC * NP;
     const int64_t batch = blockIdx.z;
     A += batch * sa;
     B += batch * sb;
     C += batch * sc;
     if (post_full) post_full += batch * sc;
-    const int64_t m0 = int64_t(blockIdx.y) * ST, n0 = int64_t(blockIdx.x) * ST;
+    const int64_t m0 = int64_t(blockIdx.y) * SM, n0 = int64_t(blockIdx.x) * SN;
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
 
     auto stage = [&](int buf, int64_t k0) {
         float* As = smem + buf * (A_FLOATS + B_FLOATS);
         float* Bs = As + A_FLOATS;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int g = tid + r * 256, row = g >> 5, kq = (g & 31) * 4;  // 32 rows x 32 pieces of four k
-            const bool ok = m0 + row < M && k0 + kq < K;
-            cp_async16(As + row * KP + kq, ok ? A + (m0 + row) * K + k0 + kq : A, ok);
-        }
-        if (B_NK) {
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int g = tid + r * 256, row = g >> 5, kq = (g & 31) * 4;
-                const bool ok = n0 + row < N && k0 + kq < K;
-                cp_async16(Bs + row * KP + kq, ok ? B + (n0 + row) * K + k0 + kq : B, ok);
-            }
-        } else {
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int g = tid + r * 256, row = g >> 3, nq = (g & 7) * 4;  // 128 k-rows x 8 pieces of four columns
-                const bool ok = k0 + row < K && n0 + nq < N;
-                cp_async16(Bs + row * NP + nq, ok ? B + (k0 + row) * N + n0 + nq : B, ok);
-            }
-        }
+        stage_part<SM, KC>(As, KP, A + m0 * K + k0, K, M - m0, K - k0, vec_a);
+        if (B_NK) stage_part<SN, KC>(Bs, KP, B + n0 * K + k0, K, N - n0, K - k0, vec_b);
+        else stage_part<KC, SN>(Bs, NP, B + k0 * N + n0, N, K - k0, N - n0, vec_b);
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
-    float acc[2][2] = {};
+    float acc[RT][2] = {};
     const int64_t chunks = (K + KC - 1) / KC;
     if (chunks > 0) stage(0, 0);
     if (chunks > 1) stage(1, KC);
@@ -166,39 +179,46 @@ __global__ void __launch_bounds__(256) gemm_simt_small_kernel(const float* __res
         __syncthreads();
         const float* As = smem + int(c & 1) * (A_FLOATS + B_FLOATS);
         const float* Bs = As + A_FLOATS;
-        const int kn    = int(K - c * KC < KC ? K - c * KC : KC);  // a multiple of 4
+        const int kn    = int(K - c * KC < KC ? K - c * KC : KC);
+        int k           = 0;
 #pragma unroll 4
-        for (int k = 0; k < kn; k += 4) {
-            const float4 a0 = *reinterpret_cast<const float4*>(As + ty * KP + k);
-            const float4 a1 = *reinterpret_cast<const float4*>(As + (ty + 16) * KP + k);
-            const float av0[4] = {a0.x, a0.y, a0.z, a0.w}, av1[4] = {a1.x, a1.y, a1.z, a1.w};
+        for (; k + 4 <= kn; k += 4) {
+            float av[RT][4];
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+                const float4 a = *reinterpret_cast<const float4*>(As + (ty + 16 * i) * KP + k);
+                av[i][0] = a.x, av[i][1] = a.y, av[i][2] = a.z, av[i][3] = a.w;
+            }
             if (B_NK) {
                 const float4 b0 = *reinterpret_cast<const float4*>(Bs + tx * KP + k);
                 const float4 b1 = *reinterpret_cast<const float4*>(Bs + (tx + 16) * KP + k);
                 const float bv0[4] = {b0.x, b0.y, b0.z, b0.w}, bv1[4] = {b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    acc[0][0] = fmaf(av0[q], bv0[q], acc[0][0]);
-                    acc[0][1] = fmaf(av0[q], bv1[q], acc[0][1]);
-                    acc[1][0] = fmaf(av1[q], bv0[q], acc[1][0]);
-                    acc[1][1] = fmaf(av1[q], bv1[q], acc[1][1]);
-                }
+                for (int q = 0; q < 4; ++q)
+#pragma unroll
+                    for (int i = 0; i < RT; ++i) acc[i][0] = fmaf(av[i][q], bv0[q], acc[i][0]), acc[i][1] = fmaf(av[i][q], bv1[q], acc[i][1]);
             } else {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const float2 b = *reinterpret_cast<const float2*>(Bs + (k + q) * NP + tx * 2);
-                    acc[0][0]      = fmaf(av0[q], b.x, acc[0][0]);
-                    acc[0][1]      = fmaf(av0[q], b.y, acc[0][1]);
-                    acc[1][0]      = fmaf(av1[q], b.x, acc[1][0]);
-                    acc[1][1]      = fmaf(av1[q], b.y, acc[1][1]);
+#pragma unroll
+                    for (int i = 0; i < RT; ++i) acc[i][0] = fmaf(av[i][q], b.x, acc[i][0]), acc[i][1] = fmaf(av[i][q], b.y, acc[i][1]);
                 }
+            }
+        }
+        for (; k < kn; ++k) {
+            const float b0 = B_NK ? Bs[tx * KP + k] : Bs[k * NP + tx * 2], b1 = B_NK ? Bs[(tx + 16) * KP + k] : Bs[k * NP + tx * 2 + 1];
+#pragma unroll
+            for (int i = 0; i < RT; ++i) {
+                const float a = As[(ty + 16 * i) * KP + k];
+                acc[i][0] = fmaf(a, b0, acc[i][0]), acc[i][1] = fmaf(a, b1, acc[i][1]);
             }
         }
         __syncthreads();
         if (c + 2 < chunks) stage(int(c & 1), (c + 2) * KC);
     }
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < RT; ++i) {
         const int64_t m = m0 + ty + 16 * i;
         if (m >= M) continue;
 #pragma unroll
@@ -212,32 +232,38 @@ __global__ void __launch_bounds__(256) gemm_simt_small_kernel(const float* __res
     }
 }
 
-// Worth it while the 64 x 64 tiling leaves most SMs without a tile; needs 16-byte pieces along the operands' rows.
+bool vec_a(const mimk_gemm_desc& d) { return d.k % 4 == 0 && aligned16(d.a) && d.stride_a % 4 == 0; }
+bool vec_b(const mimk_gemm_desc& d) { return (d.b_layout == MIMK_B_NK ? d.k : d.n) % 4 == 0 && aligned16(d.b) && d.stride_b % 4 == 0; }
+
+// Worth it while the 64 x 64 tiling leaves most SMs without a tile.
 bool small_tiles_apply(const mimk_gemm_desc& d) {
-    if (d.in_dtype != MIMK_F32 || d.out_dtype != MIMK_F32 || d.k < 4 || d.k % 4 != 0) return false;
-    const bool b_nk = d.b_layout == MIMK_B_NK;
-    if (!b_nk && d.n % 4 != 0) return false;
-    if (!aligned16(d.a) || !aligned16(d.b) || d.stride_a % 4 != 0 || d.stride_b % 4 != 0) return false;
+    if (d.in_dtype != MIMK_F32 || d.out_dtype != MIMK_F32 || d.k < 1) return false;
     const int64_t big = ((d.m + TM - 1) / TM) * ((d.n + TN - 1) / TN) * d.batch;
-    return big < 2 * 148 && (d.m + ST - 1) / ST <= 65535 && d.batch <= 65535;
+    return big < 2 * 148 && (d.m + 31) / 32 <= 65535 && d.batch <= 65535;
 }
 
+template <bool B_NK, int RT>
 int launch_small(const mimk_gemm_desc& d, cudaStream_t s) {
-    const bool b_nk = d.b_layout == MIMK_B_NK;
-    const int smem  = 2 * (ST * KP + (b_nk ? ST * KP : KC * NP)) * int(sizeof(float));
-    auto kern       = b_nk ? gemm_simt_small_kernel<true> : gemm_simt_small_kernel<false>;
-    static bool configured[2][64] = {};  // per instance and device: the attribute is a per-device setting
+    constexpr int SMEM = 2 * (16 * RT * KP + (B_NK ? SN * KP : KC * NP)) * int(sizeof(float));
+    auto kern          = gemm_simt_small_kernel<B_NK, RT>;
+    static bool configured[64] = {};  // per instance and device: the attribute is a per-device setting
     int dev = 0;
     MIMK_CUDA_TRY(cudaGetDevice(&dev));
-    if (!configured[b_nk][dev & 63]) {
-        MIMK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        configured[b_nk][dev & 63] = true;
+    if (!configured[dev & 63]) {
+        MIMK_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        configured[dev & 63] = true;
     }
-    dim3 grid((unsigned)((d.n + ST - 1) / ST), (unsigned)((d.m + ST - 1) / ST), (unsigned)d.batch);
-    kern<<<grid, 256, smem, s>>>(static_cast<const float*>(d.a), static_cast<const float*>(d.b), static_cast<float*>(d.c),
-                                 d.m, d.n, d.k, d.stride_a, d.stride_b, d.stride_c, d.post,
+    dim3 grid((unsigned)((d.n + SN - 1) / SN), (unsigned)((d.m + 16 * RT - 1) / (16 * RT)), (unsigned)d.batch);
+    kern<<<grid, 256, SMEM, s>>>(static_cast<const float*>(d.a), static_cast<const float*>(d.b), static_cast<float*>(d.c),
+                                 d.m, d.n, d.k, d.stride_a, d.stride_b, d.stride_c, d.post, vec_a(d), vec_b(d),
                                  static_cast<const float*>(d.post_row), static_cast<const float*>(d.post_full));
     return launch_status();
+}
+int launch_small(const mimk_gemm_desc& d, cudaStream_t s) {
+    // 16 rows while the device has an SM for each such tile
+    const bool narrow = ((d.m + 15) / 16) * ((d.n + SN - 1) / SN) * d.batch <= 148;
+    if (d.b_layout == MIMK_B_NK) return narrow ? launch_small<true, 1>(d, s) : launch_small<true, 2>(d, s);
+    return narrow ? launch_small<false, 1>(d, s) : launch_small<false, 2>(d, s);
 }
 
 template <class TIn, class TOut>
@@ -255,7 +281,7 @@ int launch(const mimk_gemm_desc& d, cudaStream_t s) {
 
 // Where f32 products stay on the CUDA cores (times: CUDA-graph replays, warm, CUDA cores against tensor cores).
 //   batches below 2^25 multiply-adds      64 of 64^3: 4.5 / 8.4 us; above: 10 of 76 x 704 x 448, 33.6 / 19.1
-//   K <= 256: below 5 * 2^24 where the small-tile kernel applies (256^3: 6.2 / 7.8 us; 815 x 524 x 168: 13 / 15;
+//   K <= 256: below 5 * 2^24 where the small-tile kernel applies and copies 16 bytes at a time (256^3: 5.7 / 7.8 us; 815 x 524 x 168: 13 / 15;
 //             784 x 1024 x 128: 13.9 / 10.7), else 2^24 (245 x 674 x 146: 15.3 / 10.0).
 //             Rows that are no multiple of four below 20 * 2^24: any part of such a product has the bits of the small product of the
 //             same rows and columns, which is worth more there than the time (1280 x 961 x 256: 60 / 25; x 128: 34 / 20; 4096 x 250 x
@@ -266,7 +292,7 @@ int gemm_simt_preferred(const mimk_gemm_desc& d) {
     if (d.batch > 1) return work * double(d.batch) < double(1 << 25);
     if (d.k > 256) return d.k < 1024 && work < double(1 << 20);
     if (d.n % 4 != 0 && (d.k <= 32 || work < double(20 << 24))) return 1;
-    return work < (small_tiles_apply(d) ? double(5 << 24) : double(1 << 24));
+    return work < (small_tiles_apply(d) && vec_a(d) && vec_b(d) ? double(5 << 24) : double(1 << 24));
 }
 
 int gemm_simt(const mimk_gemm_desc& d, cudaStream_t s) {

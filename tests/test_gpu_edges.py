@@ -266,6 +266,23 @@ def test_batched_f32_results_at_any_stride(T, out, gap):
     close_cells(room[:, :m * n].reshape(batch, m, n), d64(a) @ d64(bt), d64(a).abs() @ d64(bt).abs(), TF32_CELL if out == F32 else BF16_ROUND)
 
 
+@pytest.mark.parametrize("nk", [False, True])
+@pytest.mark.parametrize("m,n,k,offset", [(1, 1, 1, 0), (17, 31, 77, 1), (1024, 10, 128, 0), (100, 130, 70, 3), (33, 100, 3, 1), (128, 257, 250, 2), (1200, 62, 129, 0)])
+def test_small_f32_products_of_any_alignment(T, m, n, k, offset, nk):
+    # tiles of 16 and of 32 rows, copies of 4 and of 16 bytes: one ascending fold per cell, so a corner of a product on the 64 x 64 kernel
+    # (several hundred of its tiles) has the same bits
+    M, N = 1280, 961
+    a, b = rnd((M, k), 1, F32, offset), rnd((N, k) if nk else (k, N), 2, F32, offset)
+    big = T.product_2d(a, b.t() if nk else b)
+    bs = b[:n].contiguous() if nk else b[:, :n].contiguous()
+    got = T.product_2d(a[:m].contiguous(), bs.t() if nk else bs)
+    T.device_status()
+    assert torch.equal(got, big[:m, :n])
+    bd = d64(bs).t() if nk else d64(bs)
+    # k roundings of an f32 sum at most
+    close_cells(got, d64(a[:m]) @ bd, d64(a[:m]).abs() @ bd.abs(), k * 2.0 ** -24)
+
+
 def test_f32_products_keep_infinities_and_extremes(T):
     a, b = rnd((200, 600), 1), rnd((600, 300), 2)
     a[3, 5], a[7, 0], b[9, 11] = math.inf, math.nan, -math.inf
