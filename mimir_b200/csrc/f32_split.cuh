@@ -87,11 +87,13 @@ __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t saddr) {
 
 // D = A B^T over `blocks` 32-wide k-blocks, the products smallest first over all of them: the tensor core cuts off what its
 // accumulator update cannot hold, which costs least while the accumulator is small (and so only 2 x blocks updates by full-size
-// terms count). stage[b]: block b's A tiles, its B tiles `b_off` behind; the h piece first. PIECES = 1: the product of the h pieces
+// terms count). stage[b]: descriptor of block b's A tiles, its B tiles behind them; the h piece first. PIECES = 1: the product of the h pieces
 // alone.
-template <int PIECES>
-__device__ __forceinline__ void mma_six(uint32_t d, const uint32_t (&stage)[2], int blocks, uint32_t a_piece, uint32_t b_off,
-                                        uint32_t b_piece, uint32_t idesc) {
+// Called by the lane that issues, from descriptors that the whole warp has made: made by lane 0 in a branch of its own they are not known to be
+// uniform, and moving them costs about 50 clocks per MMA.
+template <int PIECES, int A_PIECE, int B_PIECE>
+__device__ __forceinline__ void mma_six(uint32_t d, const uint64_t (&stage)[2], int blocks, uint32_t idesc) {
+    constexpr int B_OFF = PIECES * A_PIECE;
     constexpr int PA[6] = {2, 0, 1, 1, 0, 0}, PB[6] = {0, 2, 1, 0, 1, 0}, FIRST = PIECES == 1 ? 5 : 0;
 #pragma unroll
     for (int t = FIRST; t < 6; ++t)
@@ -100,8 +102,8 @@ __device__ __forceinline__ void mma_six(uint32_t d, const uint32_t (&stage)[2], 
             if (b < blocks)
 #pragma unroll
                 for (int k = 0; k < 2; ++k)
-                    sm100::mma_f16_ss(d, smem_desc_sw64(stage[b] + PA[t] * a_piece + k * 32),
-                                      smem_desc_sw64(stage[b] + b_off + PB[t] * b_piece + k * 32), idesc, (t > FIRST || b > 0 || k > 0) ? 1u : 0u);
+                    sm100::mma_f16_ss(d, stage[b] + ((PA[t] * A_PIECE + k * 32) >> 4), stage[b] + ((B_OFF + PB[t] * B_PIECE + k * 32) >> 4), idesc,
+                                      (t > FIRST || b > 0 || k > 0) ? 1u : 0u);
 }
 
 __device__ __forceinline__ float load1(const float* p) { return __ldg(p); }

@@ -10,13 +10,15 @@
 //   warp 16       one thread issues the MMAs, 128 x BN x 32 per k-block; every two k-blocks go into a fresh accumulator
 // The tensor core does not round its accumulator updates to nearest; with four updates by full-size terms per accumulator (all
 // small terms first) and ordinary f32 adds between accumulators, the error stays below that of an f32 fold for any K.
-// The accumulators are added in order whatever the grid as long as each CTA of a cluster can hold its own to the end: K <= 64 * SLOTS
-// * split, at least 384 (128 columns, two CTAs). Beyond that a CTA adds its own first, and the bits follow the split.
+// Accumulators are added in pairs. Few tiles: the pairs of one tile are dealt out to a cluster of two, four or eight CTAs, which exchange
+// them through distributed shared memory (about 14 bytes a clock per SM, what bounds such products: by single accumulators 128 x 1024 x
+// 784 took 17 us). They are added in order whatever the grid as long as each CTA can hold its own to the end and they are at most nine:
+// K <= 1152, with 128 columns K <= 256 * split. Beyond that a CTA adds its own first, and the bits follow the split (300 x 300 x 3000: 24
+// pairs held 31.6 us, eight sums 27).
 //
 // The operands are read as the caller has them: any extents, strides and alignment, no copies, no scratch. What bounds it:
 // shared-memory bandwidth (a k-block of 128 x 128 moves 96 KB into the MMA and 48 KB from the loaders; measured 100 clocks per
-// instruction of 64 clocks' arithmetic) next to the loaders' instructions. Too few tiles for the chip: the accumulators of one
-// tile are dealt out to a cluster of two, four or eight CTAs, which exchange them through distributed shared memory. Many tiles: the operands
+// instruction of 64 clocks' arithmetic) next to the loaders' instructions. Many tiles: the operands
 // are cut beforehand instead (gemm_tf32.cu). Measured: 1000^3 29 us (30 as three TF32 products, 2e-6 off; here 1.3e-7), 4096 x 128 x
 // 4096 45 (112), 64 of 512^3 220 (830 on the CUDA cores), 24 of 503 x 2052 x 407 342 (1062).
 #include <type_traits>
@@ -35,7 +37,7 @@ namespace {
 constexpr int BM = 128;
 constexpr int CHUNK = 2;        // k-blocks per accumulator
 constexpr int LOADERS = 512, NUM_THREADS = LOADERS + 32, MMA_WARP = LOADERS / 32;
-constexpr int STAGES = 4, GROUP_M = 16;
+constexpr int STAGES = 4, GROUP_M = 16, HELD_PAIRS = 9;
 constexpr int A_PIECE = BM * BK * 2;
 
 template <int BN, class TIn> struct Cfg {
@@ -44,7 +46,7 @@ template <int BN, class TIn> struct Cfg {
     static constexpr int STAGE_BYTES = PIECES * (A_PIECE + B_PIECE);
     static constexpr int PITCH = BN + 4, PART_BYTES = BM * PITCH * 4;  // a partial tile; they lie over the stages
     static constexpr int NACC  = 512 / BN;                             // accumulators in tensor memory
-    static constexpr int SLOTS = BN == 128 ? 3 : 4;                    // of them, what a CTA of a cluster may hold to the end
+    static constexpr int SLOTS = BN == 128 ? 2 : 4;                    // pairs of them that a CTA of a cluster may hold to the end
     static constexpr int TILE_BYTES = STAGES * STAGE_BYTES > SLOTS * PART_BYTES ? STAGES * STAGE_BYTES : SLOTS * PART_BYTES;
     static constexpr int SMEM_BYTES = TILE_BYTES + 1024 + 256;
     static_assert(SMEM_BYTES <= 232448, "more shared memory than a CTA can have");
@@ -98,8 +100,6 @@ __device__ __forceinline__ uint32_t ld_cluster1(uint32_t saddr, uint32_t rank) {
     asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
     return v;
 }
-__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld_32x32(taddr, r); }
-__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[16]) { tmem_ld_32x16(taddr, r); }
 
 // A wait of a whole warp, with one outcome for all its lanes.
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
@@ -178,7 +178,8 @@ template <int BN> struct Place {
         tile_coords(item - bz * tiles, p.tiles_m, p.tiles_n, tm, tn);
         m0 = tm * BM, n0 = tn * BN;
         const int all_kb = int((p.K + BK - 1) / BK);
-        chunks = (all_kb + CHUNK - 1) / CHUNK, per = (chunks + p.split - 1) / p.split;
+        // (whole pairs of accumulators to a CTA)
+        chunks = (all_kb + CHUNK - 1) / CHUNK, per = ((chunks + 1) / 2 + p.split - 1) / p.split * 2;
         ch0 = rank * per < chunks ? rank * per : chunks, ch1 = ch0 + per < chunks ? ch0 + per : chunks;
         kb0 = ch0 * CHUNK, kb1 = ch1 * CHUNK < all_kb ? ch1 * CHUNK : all_kb;
     }
@@ -201,12 +202,12 @@ __device__ __forceinline__ void finish4(const Params& p, TOut* out, const TOut* 
     store4(out + row * p.N, col, p.N, make_float4(v[0], v[1], v[2], v[3]), p.vec_c);
 }
 
-// The accumulators of a tile in order, each CTA of the cluster a share of the rows. hold: every accumulator has a partial tile of its
+// The accumulators of a tile in order, each CTA of the cluster a share of the rows. hold: every pair of them has a partial tile of its
 // own, else each CTA has one.
 template <int BN, class TIn, class TOut, bool CONV>
 __device__ __forceinline__ void store_tile(const Params& p, const Place<BN>& at, uint32_t base, bool hold, float bound, bool zeros) {
     using C = Cfg<BN, TIn>;
-    const int rows = BM / p.split, held = hold ? at.per : 1, used = hold ? at.chunks : (at.chunks + at.per - 1) / at.per;
+    const int rows = BM / p.split, held = hold ? at.per / 2 : 1, used = hold ? (at.chunks + 1) / 2 : (at.chunks + at.per - 1) / at.per;
     TOut* out             = static_cast<TOut*>(p.C) + at.bz * p.sc;
     const TOut* post_full = p.post_full ? static_cast<const TOut*>(p.post_full) + at.bz * p.sc : nullptr;
     for (int i = threadIdx.x; i < rows * (BN / 4); i += NUM_THREADS) {
@@ -238,7 +239,7 @@ __device__ __forceinline__ void store_tile(const Params& p, const Place<BN>& at,
     }
 }
 
-template <int BN, class TIn> __device__ __forceinline__ bool holds(const Params& p, const Place<BN>& at) { return p.split > 1 && at.per <= Cfg<BN, TIn>::SLOTS; }
+template <int BN, class TIn> __device__ __forceinline__ bool holds(const Params& p, const Place<BN>& at) { return p.split > 1 && at.chunks <= 2 * HELD_PAIRS && at.per <= 2 * Cfg<BN, TIn>::SLOTS; }
 
 // Bits were lost in cutting this CTA's part of the operands: what a sum has to reach for that not to matter, 22 bits above the loss,
 // from the largest finite magnitudes among the CTA's rows, columns and k; a sum of exactly zero can be short of something only if there
@@ -417,29 +418,34 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&bars->tmem_base);
 
     if (warp == MMA_WARP) {
-        if (lane == 0) {
+        {
+            const bool leader    = elect_one();
+            const uint64_t desc0 = smem_desc_sw64(base);
             const uint32_t idesc = idesc_bf16_f32(BM, BN, 0, 0);
             uint32_t stage = 0, phase = 0;
             for (int kb = kb0, c = 0; kb < kb1; kb += CHUNK, ++c) {
                 // A full stage also says that every warp has added up the chunk four before this one, so an accumulator is free
                 // when its turn comes again.
-                uint32_t at[CHUNK], empty[CHUNK];
+                uint64_t at[CHUNK];
+                uint32_t empty[CHUNK];
                 const int n = kb1 - kb < CHUNK ? kb1 - kb : CHUNK;
                 bool ok = true;
 #pragma unroll
                 for (int b = 0; b < CHUNK; ++b) {
-                    if (b < n && ok) ok = mbar_wait(smem_u32(&bars->full[stage]), phase, abort_flag);
-                    at[b] = base + stage * C::STAGE_BYTES, empty[b] = smem_u32(&bars->empty[stage]);
+                    if (b < n && ok) ok = warp_wait(smem_u32(&bars->full[stage]), phase, abort_flag);
+                    at[b] = desc0 + stage * (C::STAGE_BYTES >> 4), empty[b] = smem_u32(&bars->empty[stage]);
                     if (b < n && ++stage == STAGES) stage = 0, phase ^= 1u;
                 }
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t acc = uint32_t(c) % C::NACC;
-                mma_six<PIECES>(tmem_base + acc * BN, at, n, A_PIECE, PIECES * A_PIECE, C::B_PIECE, idesc);
+                if (leader) {
+                    mma_six<PIECES, A_PIECE, C::B_PIECE>(tmem_base + acc * BN, at, n, idesc);
 #pragma unroll
-                for (int b = 0; b < CHUNK; ++b)
-                    if (b < n) mma_commit(empty[b]);
-                mma_commit(smem_u32(&bars->acc_full[acc]));
+                    for (int b = 0; b < CHUNK; ++b)
+                        if (b < n) mma_commit(empty[b]);
+                    mma_commit(smem_u32(&bars->acc_full[acc]));
+                }
             }
         }
         __syncwarp();
@@ -461,6 +467,24 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
             tmem_ld_wait();
 #pragma unroll
             for (int i = 0; i < 16; ++i) sum[decltype(h)::value + i] += __uint_as_float(r[i]);
+            tc_fence_before();
+        };
+        // chunks c and c + 1 (or c alone) added up and to the sums
+        auto pair = [&](int c) {
+#pragma unroll
+            for (int h = 0; h < COLS; h += 16) {
+                uint32_t r[16], second[16];
+                request(c, h, r);
+                if (c + 1 < ch1 - ch0) {
+                    request(c + 1, h, second);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) second[i] = 0;
+                }
+                tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 16; ++i) sum[h + i] += __uint_as_float(r[i]) + __uint_as_float(second[i]);
+            }
             tc_fence_before();
         };
         using First  = std::integral_constant<int, 0>;
@@ -488,8 +512,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
             // 3 x 3: 241 -> 201 us; bf16 248 -> 279, 2048^3 163 -> 170, so not there). The chunk read is complete: its stages are in use again.
             constexpr bool EARLY = CONV && PIECES == 3;
             const int kb = kb0 + c * CHUNK;
-            const bool due = !hold && c >= (EARLY ? 3 : 2), second = kb + 1 < kb1;
+            const bool second = kb + 1 < kb1;
             if constexpr (EARLY) {
+                const bool due = !hold && c >= 3;
                 uint32_t r[16];
                 if (!(ok = !due || ready(added))) break;
                 if (due) request(added, 0, r);
@@ -498,19 +523,15 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
                 if (COLS == 32 && due) request(added, 16, r);
                 if (second && !(ok = load_block(kb + 1))) break;
                 if (COLS == 32 && due) add(Second{}, r);
+                added += due;
             } else {
                 if (!(ok = load_block(kb) && (!second || load_block(kb + 1)))) break;
-                if (due) {
-                    uint32_t r[COLS];
-                    if (!(ok = ready(added))) break;
-                    tmem_ld_cols(tmem_base + uint32_t(added) % C::NACC * BN + col0 + lanes, r);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int i = 0; i < COLS; ++i) sum[i] += __uint_as_float(r[i]);
-                    tc_fence_before();
+                if (!hold && c >= 3 && (c & 1)) {
+                    if (!(ok = ready(added) && ready(added + 1))) break;
+                    pair(added);
+                    added += 2;
                 }
             }
-            added += due;
         }
         auto part = [&](int slot, const float (&x)[COLS]) {
             const uint32_t a = base + slot * C::PART_BYTES + (uint32_t(quarter * 32 + lane) * C::PITCH + col0) * 4;
@@ -521,25 +542,26 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
         // Once the last chunk is finished every MMA of this CTA is complete, and the stages become its partial tiles.
         if (hold) {
             if (ok && ch1 > ch0) ok = ready(ch1 - ch0 - 1);
-            for (int c = 0; c < ch1 - ch0 && ok; ++c) {
-                if (!(ok = ready(c))) break;
-                uint32_t r[COLS];
-                tmem_ld_cols(tmem_base + uint32_t(c) % C::NACC * BN + col0 + lanes, r);
-                tmem_ld_wait();
+            for (int c = 0; c < ch1 - ch0 && ok; c += 2) {  // (the last being ready, all are)
 #pragma unroll
-                for (int i = 0; i < COLS; ++i) sum[i] = __uint_as_float(r[i]);
-                part(c, sum);
+                for (int i = 0; i < COLS; ++i) sum[i] = 0.f;
+                pair(c);
+                part(c / 2, sum);
             }
         } else {
-            for (; added < ch1 - ch0 && ok; ++added) {
-                if (!(ok = ready(added))) break;
-                uint32_t r[16];
-                request(added, 0, r);
-                add(First{}, r);
-                if (COLS == 32) {
-                    request(added, 16, r);
-                    add(Second{}, r);
+            if (ok && added < ch1 - ch0) ok = ready(ch1 - ch0 - 1);
+            if constexpr (CONV && PIECES == 3) {
+                for (; added < ch1 - ch0 && ok; ++added) {
+                    uint32_t r[16];
+                    request(added, 0, r);
+                    add(First{}, r);
+                    if (COLS == 32) {
+                        request(added, 16, r);
+                        add(Second{}, r);
+                    }
                 }
+            } else {
+                for (; added < ch1 - ch0 && ok; added += 2) pair(added);
             }
             part(0, sum);
         }
@@ -550,9 +572,9 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
     if (p.split > 1) cluster_sync();
     float bound   = 0.f;
     uint32_t deep = 0;
-    for (int r = 0; LOSES && r < p.split; ++r) {
-        bound += __uint_as_float(ld_cluster1(smem_u32(&bars->bound), uint32_t(r)));
-        deep |= ld_cluster1(smem_u32(&bars->deep), uint32_t(r));
+    if (LOSES) {  // (a lane asks a CTA each: one after the other the answers take 2000 clocks)
+        if (lane < p.split) bound = __uint_as_float(ld_cluster1(smem_u32(&bars->bound), uint32_t(lane))), deep = ld_cluster1(smem_u32(&bars->deep), uint32_t(lane));
+        bound = warp_sum(bound), deep = __reduce_or_sync(0xffffffffu, deep);
     }
     store_tile<BN, TIn, TOut, CONV>(p, place, base, hold, bound, deep != 0);
     if (p.split > 1) cluster_sync();  // no CTA of the cluster exits while another may read its partial tiles
@@ -596,15 +618,16 @@ struct Plan {
 };
 Plan make_plan(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count) {
     const int64_t tiles_m = (m + BM - 1) / BM;
-    const int kb = int((k + BK - 1) / BK), chunks = (kb + CHUNK - 1) / CHUNK;
+    const int kb = int((k + BK - 1) / BK), pairs = (kb + 2 * CHUNK - 1) / (2 * CHUNK);
     Plan best{64, 1, 1e300};
     for (int wide = 0; wide < 2; ++wide)
-        for (int split = 1; split <= 8 && split <= chunks; split *= 2) {
+        for (int split = 1; split <= 8; split *= 2) {
+            if (split > 1 && (pairs + split - 1) / split == (2 * pairs + split - 1) / split) break;  // no fewer for a CTA than with half the CTAs
             const int64_t items = tiles_m * ((n + (wide ? 127 : 63)) / (wide ? 128 : 64)) * batch;
             int64_t room        = split == 1 ? sm_count : split == 2 ? sm_count / 2 - 4 : split == 4 ? sm_count / 4 - 5 : sm_count / 8 - 3;
             if (room < 1) room = 1;  // (a slice of a GPU)
             const double rounds = double((items + room - 1) / room);
-            const int per       = (chunks + split - 1) / split * CHUNK;
+            const int per       = (pairs + split - 1) / split * 2 * CHUNK;
             const double time   = rounds * ((split > 1 ? 9.0 : 8.0) + (per < kb ? per : kb) * (wide ? 1.15 : 0.95));
             if (time < best.us) best = Plan{wide ? 128 : 64, split, time};
         }

@@ -202,39 +202,41 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap tmAh, const __grid_constant
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {
+            // (the whole warp runs and one lane issues: in a branch of lane 0 alone the descriptors are not known to be uniform, and moving them
+            // costs about 50 clocks per MMA: 2048^3 118 -> 112 us)
+            const bool leader    = elect_one();
             const uint32_t idesc = idesc_tf32(BM, BN);
             uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
             bool ok = true;
             for (int64_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
                 for (int kb0 = 0; kb0 < num_kb && ok; kb0 += CHUNK_KB) {
                     // one chunk: a fresh accumulator buffer, handed to the epilogue warps when the chunk is complete
-                    if (!(ok = mbar_wait(smem_u32(&bars->acc_empty[acc]), acc_phase ^ 1u, abort_flag))) break;
+                    if (!(ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->acc_empty[acc]), acc_phase ^ 1u, abort_flag)))) break;
                     tc_fence_after();
                     const uint32_t d0 = tmem_base + acc * BN;
                     const int kb1     = kb0 + CHUNK_KB < num_kb ? kb0 + CHUNK_KB : num_kb;
                     for (int kb = kb0; kb < kb1; ++kb) {
-                        if (!(ok = mbar_wait(smem_u32(&bars->full[stage]), phase, abort_flag))) break;
+                        if (!(ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->full[stage]), phase, abort_flag)))) break;
                         tc_fence_after();
-                        const uint32_t s0 = tile_base + stage * STAGE_BYTES;
+                        const uint64_t s0 = smem_desc_sw128(tile_base, 16, 1024) + stage * (STAGE_BYTES >> 4);
+                        if (leader) {
 #pragma unroll
-                        for (int k = 0; k < BK / 8; ++k) {  // 8 f32 = 32 bytes per k-step inside the 128-byte swizzle row
-                            const uint64_t ah = smem_desc_sw128(s0 + k * 32, 16, 1024);
-                            const uint64_t al = smem_desc_sw128(s0 + A_BYTES + k * 32, 16, 1024);
-                            const uint64_t bh = smem_desc_sw128(s0 + 2 * A_BYTES + k * 32, 16, 1024);
-                            const uint64_t bl = smem_desc_sw128(s0 + 2 * A_BYTES + B_BYTES + k * 32, 16, 1024);
-                            mma_tf32_ss(d0, al, bh, idesc, (kb > kb0 || k > 0) ? 1u : 0u);  // the small terms first
-                            mma_tf32_ss(d0, ah, bl, idesc, 1u);
-                            mma_tf32_ss(d0, ah, bh, idesc, 1u);
+                            for (int k = 0; k < BK / 8; ++k) {  // 8 f32 = 32 bytes per k-step inside the 128-byte swizzle row
+                                const uint64_t ah = s0 + k * 2, al = ah + (A_BYTES >> 4), bh = ah + (2 * A_BYTES >> 4), bl = bh + (B_BYTES >> 4);
+                                mma_tf32_ss(d0, al, bh, idesc, (kb > kb0 || k > 0) ? 1u : 0u);  // the small terms first
+                                mma_tf32_ss(d0, ah, bl, idesc, 1u);
+                                mma_tf32_ss(d0, ah, bh, idesc, 1u);
+                            }
+                            mma_commit(smem_u32(&bars->empty[stage]));
                         }
-                        mma_commit(smem_u32(&bars->empty[stage]));
                         if (++stage == STAGES) {
                             stage = 0;
                             phase ^= 1u;
                         }
                     }
                     if (!ok) break;
-                    mma_commit(smem_u32(&bars->acc_full[acc]));
+                    if (leader) mma_commit(smem_u32(&bars->acc_full[acc]));
                     if (++acc == 2) {
                         acc = 0;
                         acc_phase ^= 1u;
