@@ -1,4 +1,4 @@
-"""Builds libmimk.so (the C-ABI kernel library) in-tree with nvcc for sm_100a.
+"""Builds libmimk.so (the C-ABI kernel library) in-tree with nvcc for sm_100a, and _native.so (the operators' calls from Python) with g++.
 
     python -m mimir_b200.build [--force] [--verbose]
 
@@ -18,6 +18,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libmimk.so")
+NATIVE = os.path.join(HERE, "_native.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -41,6 +42,28 @@ def _stale(target: str, deps) -> bool:
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def _build_native(force: bool, verbose: bool) -> None:
+    """The extension module, against this interpreter's torch; it finds libmimk.so beside itself."""
+    src = os.path.join(CSRC, "py_ops.cpp")
+    if not force and not _stale(NATIVE, [src, os.path.join(ROOT, "include", "mimk.h")]):
+        return
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    includes = cpp_extension.include_paths() + [sysconfig.get_paths()["include"], os.path.join(cuda, "include"), os.path.join(ROOT, "include")]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           src, "-o", NATIVE, *(f"-I{i}" for i in includes), f"-L{lib}", f"-L{HERE}", "-l:libmimk.so", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu",
+           "-ltorch", "-lc10_cuda", "-lc10", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{lib}"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode != 0:
+        sys.stderr.write(f"--- py_ops.cpp\n{r.stdout}{r.stderr}\n")
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed on py_ops.cpp")
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -72,6 +95,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if r.returncode != 0:
             sys.stderr.write(r.stdout + r.stderr)
             raise RuntimeError("link failed")
+    _build_native(force, verbose)
     return LIB
 
 

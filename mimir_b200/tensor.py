@@ -3,7 +3,9 @@
 Names and argument meaning follow MimIR's src/mim/plug/tensor/tensor.mim (product_2d 510-513, bmm 404-407,
 transpose_2d, reduce 1151-1157, binary_ax 1162-1167, softmax 1172-1176, unary/binary 361-394); a dense row-major
 tensor is what `tensor.Tensor r s T` bufferises to (tensor.mim:48-50, buffer/phase/lower_ptr.cpp:16-20).
-torch is used for device memory and streams only; every operator is one call into the C ABI (include/mimk.h).
+torch is used for device memory and streams only; every operator is one call into the C ABI (include/mimk.h). The operators that most
+programs consist of try `_native` first, which makes that call without ctypes where the arguments are plain (about 3 us of host time
+instead of 9) and otherwise answers None.
 Shape errors the reference reports at compile time ("contracting dims don't match", tensor.mim:1393) are raised
 as ValueError before anything is launched; kernel-side failures raise MimkError.
 """
@@ -16,6 +18,7 @@ import math
 import torch
 
 from . import _lib as L
+from . import _native
 
 _DT = {torch.float32: L.F32, torch.bfloat16: L.BF16, torch.int32: L.I32, torch.int64: L.I64}
 _TORCH = {v: k for k, v in _DT.items()}
@@ -81,6 +84,8 @@ def _gemm(a, b_store, layout, batch, m, n, k, sa, sb, out, post, bias, full):
 
 def product_2d(a: torch.Tensor, b: torch.Tensor, *, post=None, bias=None, full=None, out_dtype=None) -> torch.Tensor:
     """C[m,l] = post(sum_k a[m,k] * b[k,l]).  `b` may be a transpose_2d view of a [l,k] tensor."""
+    if full is None and (out := _native.product_2d(a, b, _POST.get(post), bias, out_dtype)) is not None:
+        return out
     _dev(a, b, bias, full)
     if a.dim() != 2 or b.dim() != 2:
         raise ValueError("product_2d expects rank-2 tensors")
@@ -131,6 +136,8 @@ def product_2d_panels(a_panels: torch.Tensor, b: torch.Tensor, *, out_dtype=None
 
 def bmm(a: torch.Tensor, b: torch.Tensor, *, out_dtype=None) -> torch.Tensor:
     """C[B,m,n] = sum_k a[B,m,k] * b[B,k,n] (tensor.mim:404-407, batching axis 0)."""
+    if (out := _native.bmm(a, b, out_dtype)) is not None:
+        return out
     _dev(a, b)
     if a.dim() != 3 or b.dim() != 3:
         raise ValueError("bmm expects rank-3 tensors")
@@ -156,6 +163,8 @@ def _view3(x: torch.Tensor, ax: int):
 
 def reduce(monoid: str, ax: int, x: torch.Tensor) -> torch.Tensor:
     """`reduce (g, init) ax x`: folds axis `ax` away; monoid names the (g, init) pair (sum/max/min)."""
+    if (out := _native.reduce(_MONOID.get(monoid), ax, x)) is not None:
+        return out
     _dev(x)
     x = x.contiguous()
     ax, outer, ln, inner = _view3(x, ax)
@@ -170,6 +179,8 @@ def reduce_fused(monoid: str, ax: int, x: torch.Tensor, inner: str, y: torch.Ten
     outer(inner(v, y)) as the fold reads it -- what `fuse_tensor` makes of a map feeding a reduce (phase/fuse.cpp:183-358).
     `inner` is a binary operator name with `y` of x's shape, of x's shape without axis `ax` (binary_ax), or of x's trailing
     axes from `ax` on; or a unary name with y = None. `outer` is a unary name."""
+    if y is None and (out := _native.reduce_of_unary(_MONOID.get(monoid), ax, x, _UNOP.get(inner), _UNOP.get(outer))) is not None:
+        return out
     _dev(x)
     _same_float(x)
     x = x.contiguous()
@@ -199,6 +210,8 @@ def reduce_fused(monoid: str, ax: int, x: torch.Tensor, inner: str, y: torch.Ten
 
 def softmax(ax: int, x: torch.Tensor, *, out_dtype=None) -> torch.Tensor:
     """`softmax m ax x`: exp(x - max) / sum exp(x - max) along `ax`, one pass over memory."""
+    if (out := _native.softmax(ax, x, out_dtype)) is not None:
+        return out
     _dev(x)
     x = x.contiguous()
     ax, outer, ln, inner = _view3(x, ax)
@@ -209,6 +222,8 @@ def softmax(ax: int, x: torch.Tensor, *, out_dtype=None) -> torch.Tensor:
 
 def rmsnorm(x: torch.Tensor, gamma: torch.Tensor, eps: float, *, out_dtype=None) -> torch.Tensor:
     """y = x * rrt(mean(x^2, last axis) + eps) * gamma."""
+    if (out := _native.rmsnorm(x, gamma, eps, out_dtype)) is not None:
+        return out
     _dev(x, gamma)
     x = x.contiguous()
     cols = x.shape[-1]
@@ -248,6 +263,8 @@ def _op(table, op: str, then) -> int:
 
 
 def unary(op: str, x: torch.Tensor, *, out_dtype=None, then: str | None = None) -> torch.Tensor:
+    if then is None and (out := _native.unary(_UNOP.get(op), x, out_dtype)) is not None:
+        return out
     _dev(x)
     _same_float(x)
     x = x.contiguous()
@@ -258,6 +275,8 @@ def unary(op: str, x: torch.Tensor, *, out_dtype=None, then: str | None = None) 
 
 
 def binary(op: str, x: torch.Tensor, y: torch.Tensor, *, out_dtype=None, then: str | None = None) -> torch.Tensor:
+    if then is None and (out := _native.binary(_BINOP.get(op), x, y, out_dtype)) is not None:
+        return out
     _dev(x, y)
     _same_float(x, y)
     if x.shape != y.shape:
@@ -272,6 +291,8 @@ def binary(op: str, x: torch.Tensor, y: torch.Tensor, *, out_dtype=None, then: s
 def binary_ax(op: str, ax: int, x: torch.Tensor, y: torch.Tensor, *, out_dtype=None, then: str | None = None) -> torch.Tensor:
     """`binary_ax app ax (x, y)`: y lacks axis `ax` of x and is broadcast along it. `then`: a unary operator applied to the
     result in the same pass (a producer inlined into an elementwise consumer)."""
+    if op in _BINOP and (then is None or then in _UNOP) and (out := _native.binary_ax(_op(_BINOP, op, then), ax, x, y, out_dtype)) is not None:
+        return out
     _dev(x, y)
     _same_float(x, y)
     x, y = x.contiguous(), y.contiguous()
@@ -288,6 +309,8 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale: float
               return_lse: bool = False):
     """softmax(scale * q k^T [+ causal mask]) v over the trailing [seq, head_dim] axes; leading axes are batch x head.
     With scale = 1 and causal = False on rank-2 tensors this is lit/tensor/attn_exec.mim:22."""
+    if not return_lse and (out := _native.attention(q, k, v, scale, causal)) is not None:
+        return out
     _dev(q, k, v)
     if q.shape[:-2] != k.shape[:-2] or k.shape != v.shape or q.shape[-1] != k.shape[-1]:
         raise ValueError("contracting dims don't match")
@@ -306,6 +329,8 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale: float
 
 def mlp_gated(x: torch.Tensor, w1: torch.Tensor, w3: torch.Tensor, w2: torch.Tensor, *, h: torch.Tensor | None = None):
     """(silu(x w1) * (x w3)) w2, bf16; weights row-major [in, out] or transpose_2d views of [out, in]."""
+    if h is None and (out := _native.mlp_gated(x, w1, w3, w2)) is not None:
+        return out
     _dev(x, w1, w3, w2, h)
     if x.shape[1] != w1.shape[0] or w1.shape != w3.shape or w1.shape[1] != w2.shape[0]:
         raise ValueError("contracting dims don't match")
@@ -553,6 +578,8 @@ def _copy_fn(t):
 
 def transpose(x: torch.Tensor, perm) -> torch.Tensor:
     """`transpose perm x`: out[o] = x[o[inv perm]] -- output axis i is input axis perm[i] (tensor.mim:1459)."""
+    if (out := _native.transpose(x, perm)) is not None:
+        return out
     perm = [int(p) for p in perm]
     r = x.dim()
     if sorted(perm) != list(range(r)):
