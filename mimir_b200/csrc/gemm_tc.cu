@@ -216,7 +216,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const int64_t row0 = tm * BM + quarter * 32;
             const int64_t row  = row0 + lane;
             const int64_t n0   = tn * BN;
-            if (!(ok = mbar_wait(smem_u32(&bars->acc_full[acc]), acc_phase, abort_flag))) break;
+            float row_operand[8];
+            load_row_256(row_operand, p.post_row, n0, p.N, lane);
+            if (!(ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->acc_full[acc]), acc_phase, abort_flag)))) break;
             tc_fence_after();
             const uint32_t t0 = tmem_base + acc * ACC_COLS + (uint32_t(quarter * 32) << 16);
 #pragma unroll 1
@@ -248,8 +250,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         tc_fence_before();
                         mbar_arrive(smem_u32(&bars->acc_empty[acc]));
                     }
-                    if (p.post != MIMK_POST_ID && row < p.M)
-                        apply_post_32(p.post, v, p.post_row, post_full ? post_full + zoff + row * p.N : nullptr, n0 + c, p.N);
+                    if (p.post != MIMK_POST_ID)
+                        apply_post_32(p.post, v, row_operand, c, post_full && row < p.M ? post_full + zoff + row * p.N + n0 + c : nullptr, p.N - n0 - c);
                     // this thread's row of the piece: 16-byte units at (unit ^ (row & 7)), the 128-byte swizzle
                     const uint32_t row_addr = buf + lane * 128;
                     if (sizeof(TOut) == 2) {
@@ -275,9 +277,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
                 if constexpr (DIRECT) {
                     __syncwarp();
-                    store_piece(smem_raw + (buf - raw_addr), static_cast<TOut*>(p.dst[0]) + zoff + row0 * p.ldc + n0 + c0, p.ldc, p.M - row0,
-                                p.N - n0 - c0, lane);
-                    continue;  // the next piece goes to the other buffer, and the one after waits for this warp above
+                    store_piece(smem_raw + (buf - raw_addr), smem_raw + (out_base + (~chunk_no & 1u) * 4096 - raw_addr), c0 == 0, c0 + CW >= BN,
+                                static_cast<TOut*>(p.dst[0]) + zoff + row0 * p.ldc + n0 + c0, p.ldc, p.M - row0, p.N - n0 - c0, lane);
+                    continue;  // the next piece goes to the other buffer, which all lanes have read when they meet above
                 }
                 fence_proxy_async_smem();  // the bulk store reads shared memory through the async proxy
                 __syncwarp();
@@ -566,7 +568,7 @@ int gemm_tc(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, 
 // pitch first, and the result is written by plain stores. (A result in f32: gemm_bf16_chunked.) Returns MIMK_E_UNSUPPORTED, with nothing launched, where the CUDA-core
 // kernel is the better or the only way.
 //
-// Measured: 2000 x 5003 x 2048, 57 us (2240 on the CUDA cores; 38 with a width of 5008); K = 2047 as well, 75; 3 x 9000 x 5001, 23 to
+// Measured: 2000 x 5003 x 2048, 44 us (2240 on the CUDA cores; 38 with a width of 5008); K = 2047 as well, 60; 3 x 9000 x 5001, 23 to
 // 65 by layout (483 to 508); 37 x 6998 x 546, 20 (54).
 // Floor of the rule: below 2^22 multiply-adds one launch of the CUDA-core kernel is as fast as the copies and the tensor-core
 // kernel's start. Copies are kept in the cached buffer, which a captured graph must not hold on to, and a buffer that cannot be

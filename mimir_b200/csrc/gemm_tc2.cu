@@ -275,7 +275,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             const int64_t row0 = tm * 2 * BM + int64_t(rank) * BM + quarter * 32;
             const int64_t row  = row0 + lane;
             const int64_t n0   = tn * BN;
-            if (!(ok = mbar_wait(smem_u32(&bars->acc_full[acc]), acc_phase, abort_flag))) break;
+            float row_operand[8];
+            load_row_256(row_operand, p.post_row, n0, p.N, lane);
+            if (!(ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars->acc_full[acc]), acc_phase, abort_flag)))) break;
             tc_fence_after();
             const uint32_t t0 = tmem_base + acc * ACC_COLS + (uint32_t(quarter * 32) << 16);
             const uint32_t acc_empty_even = map_to_cta(smem_u32(&bars->acc_empty[acc]), 0);
@@ -310,8 +312,8 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         tc_fence_before();
                         mbar_arrive_cluster(acc_empty_even);
                     }
-                    if (p.post != MIMK_POST_ID && row < p.M)
-                        apply_post_32(p.post, v, p.post_row, post_full ? post_full + row * p.N : nullptr, n0 + c, p.N);
+                    if (p.post != MIMK_POST_ID)
+                        apply_post_32(p.post, v, row_operand, c, post_full && row < p.M ? post_full + row * p.N + n0 + c : nullptr, p.N - n0 - c);
                     // this thread's row of the tile: 16-byte pieces at (piece ^ (row & 7)), the 128-byte swizzle
                     const uint32_t row_addr = buf + lane * 128;
                     if (sizeof(TOut) == 2) {
@@ -337,9 +339,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 }
                 if constexpr (DIRECT) {
                     __syncwarp();
-                    store_piece(smem_raw + (buf - raw_addr), static_cast<TOut*>(p.dst[0]) + row0 * p.ldc + n0 + c0, p.ldc, p.M - row0,
-                                p.N - n0 - c0, lane);
-                    continue;  // the next piece goes to the other buffer, and the one after waits for this warp above
+                    store_piece(smem_raw + (buf - raw_addr), smem_raw + (out_base + (~chunk_no & 1u) * 4096 - raw_addr), c0 == 0, c0 + CW >= BN,
+                                static_cast<TOut*>(p.dst[0]) + row0 * p.ldc + n0 + c0, p.ldc, p.M - row0, p.N - n0 - c0, lane);
+                    continue;  // the next piece goes to the other buffer, which all lanes have read when they meet above
                 }
                 fence_proxy_async_smem();  // the bulk store reads shared memory through the async proxy
                 __syncwarp();
