@@ -463,11 +463,12 @@ int launch(Params& p, __nv_bfloat16* image, __nv_bfloat16* filters, const Sizes&
 
 }  // namespace
 
-// Whether this route takes the convolution: 31-bit rows, a buffer of at most 1 GiB, an estimate below `other_us`, and f32 only where
+// Whether this route takes the convolution: 16 channels and more (a row of fewer takes TMA as long: 25 x 3 x 56 x 61, 128 filters of 3 x 3, 161 us
+// against 106), 31-bit rows, a buffer of at most 1 GiB, an estimate below `other_us`, and f32 only where
 // the accumulators are not many more than one per 64 k, whose sums are what the error comes from (channels in whole blocks; 32 in 25 taps 1.41e-7
 // on either route, but 16 in 25 taps 1.35e-7 against 1.33e-7, 96 in 25 taps 1.75e-7 against 1.68e-7).
 int conv_pieces_preferred(const mimk_conv_desc& d, int sm_count, double other_us) {
-    if (d.n < 1 || d.cout < 1 || d.n >= (1 << 30) || d.cout >= (1 << 30)) return 0;
+    if (d.cin < 16 || d.n < 1 || d.cout < 1 || d.n >= (1 << 30) || d.cout >= (1 << 30)) return 0;
     const double rows = double(d.n) * (double(d.h) + 2.0 * double(d.pad_h) + double(d.stride_h)) * (double(d.w) + 2.0 * double(d.pad_w) + double(d.stride_w));
     if (rows >= double(1 << 30) || double(d.cin + 8) * double(d.kh) * double(d.kw) >= double(1 << 30)) return 0;
     const Shape c    = make_shape(d);

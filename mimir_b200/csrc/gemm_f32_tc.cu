@@ -178,8 +178,9 @@ template <int BN> struct Place {
         tile_coords(item - bz * tiles, p.tiles_m, p.tiles_n, tm, tn);
         m0 = tm * BM, n0 = tn * BN;
         const int all_kb = int((p.K + BK - 1) / BK);
-        // (whole pairs of accumulators to a CTA)
-        chunks = (all_kb + CHUNK - 1) / CHUNK, per = ((chunks + 1) / 2 + p.split - 1) / p.split * 2;
+        // (whole pairs of accumulators to a CTA; a convolution's are added one by one)
+        const int unit = p.conv.cin > 0 ? 1 : 2;
+        chunks = (all_kb + CHUNK - 1) / CHUNK, per = ((chunks + unit - 1) / unit + p.split - 1) / p.split * unit;
         ch0 = rank * per < chunks ? rank * per : chunks, ch1 = ch0 + per < chunks ? ch0 + per : chunks;
         kb0 = ch0 * CHUNK, kb1 = ch1 * CHUNK < all_kb ? ch1 * CHUNK : all_kb;
     }
@@ -239,7 +240,7 @@ __device__ __forceinline__ void store_tile(const Params& p, const Place<BN>& at,
     }
 }
 
-template <int BN, class TIn> __device__ __forceinline__ bool holds(const Params& p, const Place<BN>& at) { return p.split > 1 && at.chunks <= 2 * HELD_PAIRS && at.per <= 2 * Cfg<BN, TIn>::SLOTS; }
+template <int BN, class TIn> __device__ __forceinline__ bool holds(const Params& p, const Place<BN>& at) { return p.split > 1 && p.conv.cin == 0 && at.chunks <= 2 * HELD_PAIRS && at.per <= 2 * Cfg<BN, TIn>::SLOTS; }
 
 // Bits were lost in cutting this CTA's part of the operands: what a sum has to reach for that not to matter, 22 bits above the loss,
 // from the largest finite magnitudes among the CTA's rows, columns and k; a sum of exactly zero can be short of something only if there
@@ -616,18 +617,19 @@ struct Plan {
     int bn, split;
     double us;
 };
-Plan make_plan(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count) {
+// unit: accumulators that go to one CTA together.
+Plan make_plan(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count, int unit) {
     const int64_t tiles_m = (m + BM - 1) / BM;
-    const int kb = int((k + BK - 1) / BK), pairs = (kb + 2 * CHUNK - 1) / (2 * CHUNK);
+    const int kb = int((k + BK - 1) / BK), units = (kb + unit * CHUNK - 1) / (unit * CHUNK);
     Plan best{64, 1, 1e300};
     for (int wide = 0; wide < 2; ++wide)
         for (int split = 1; split <= 8; split *= 2) {
-            if (split > 1 && (pairs + split - 1) / split == (2 * pairs + split - 1) / split) break;  // no fewer for a CTA than with half the CTAs
+            if (split > 1 && (units + split - 1) / split == (2 * units + split - 1) / split) break;  // no fewer for a CTA than with half the CTAs
             const int64_t items = tiles_m * ((n + (wide ? 127 : 63)) / (wide ? 128 : 64)) * batch;
             int64_t room        = split == 1 ? sm_count : split == 2 ? sm_count / 2 - 4 : split == 4 ? sm_count / 4 - 5 : sm_count / 8 - 3;
             if (room < 1) room = 1;  // (a slice of a GPU)
             const double rounds = double((items + room - 1) / room);
-            const int per       = (pairs + split - 1) / split * 2 * CHUNK;
+            const int per       = (units + split - 1) / split * unit * CHUNK;
             const double time   = rounds * ((split > 1 ? 9.0 : 8.0) + (per < kb ? per : kb) * (wide ? 1.15 : 0.95));
             if (time < best.us) best = Plan{wide ? 128 : 64, split, time};
         }
@@ -636,7 +638,7 @@ Plan make_plan(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count) {
 
 template <class TIn, class TOut, bool CONV>
 int plan_and_launch(Params& p, int64_t batch, int sm_count, cudaStream_t s) {
-    const Plan plan = make_plan(p.M, p.N, p.K, batch, sm_count);
+    const Plan plan = make_plan(p.M, p.N, p.K, batch, sm_count, CONV ? 1 : 2);
     p.split = plan.split, p.tiles_m = (p.M + BM - 1) / BM, p.tiles_n = (p.N + plan.bn - 1) / plan.bn;
     const int64_t ctas = p.tiles_m * p.tiles_n * batch * p.split;
     return plan.bn == 128 ? launch<128, TIn, TOut, CONV>(p, ctas, s) : launch<64, TIn, TOut, CONV>(p, ctas, s);
@@ -650,7 +652,8 @@ static int extents_fit(const mimk_gemm_desc& d) {
     const int64_t tiles = ((d.m + BM - 1) / BM) * ((d.n + 63) / 64);
     return tiles < (int64_t(1) << 28) && d.batch < (int64_t(1) << 28) && tiles * d.batch < (int64_t(1) << 28);  // one grid
 }
-double gemm_f32_tc_us(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count) { return make_plan(m, n, k, batch, sm_count).us; }
+// (by single accumulators: the choice against three TF32 products, which are less accurate, is not to move with how pairs fall to CTAs)
+double gemm_f32_tc_us(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count) { return make_plan(m, n, k, batch, sm_count, 1).us; }
 int gemm_f32_tc_supported(const mimk_gemm_desc& d) { return d.in_dtype == MIMK_F32 && extents_fit(d); }
 
 static Params product_params(const mimk_gemm_desc& d, const DeviceInfo& dev) {
@@ -701,7 +704,7 @@ static int64_t conv_ow(const mimk_conv_desc& d) { return (d.w + 2 * d.pad_w - d.
 // sum (4 x 256 x 28 x 28, 256 filters of 3 x 3, 77 us and 1.50e-7 against 73 and 1.65e-7).
 int conv_tc_preferred(const mimk_conv_desc& d, int sm_count) {
     const int64_t pixels = d.n * conv_oh(d) * conv_ow(d), k = d.cin * d.kh * d.kw;
-    const Plan plan = make_plan(pixels, d.cout, k, 1, sm_count);
+    const Plan plan = make_plan(pixels, d.cout, k, 1, sm_count, 1);
     if (d.dtype == MIMK_F32 && plan.split > 1) return 1;
     const int64_t tiles = ((pixels + BM - 1) / BM) * ((d.cout + plan.bn - 1) / plan.bn);
     const double kb = double((k + BK - 1) / BK), round = plan.bn == 128 ? 14.0 + 1.75 * kb : 7.0 + 1.25 * kb;

@@ -688,16 +688,18 @@ def _mrp_into(out, Sr, f, init, post, map_out, maps, ins):
 
 # From this many multiply-adds on a floating-point convolution runs as a contraction on the tensor cores (mimk_conv); below it,
 # and for integers, as ONE map_reduce_post on the per-cell kernel, which keeps the reference's ascending fold per output cell
-# bit for bit.
-CONV_CONTRACTION_MIN_WORK = 1 << 27
+# bit for bit. A cell's fold is a serial chain, about 0.12 us a step: per cell / contraction, us: 1 x 16 x 14 x 14, 32 filters of 3 x 3
+# (2^20) 28 / 22; 1 x 256 x 27 x 27, 64 of 1 x 1 64 / 20; 1 x 64 x 25 x 25, 64 of 5 x 5 157 / 28; 3 x 256 x 16 x 16, 128 of 3 x 3 by 2 333 / 32;
+# the f32 error 2e-7 to 1e-6 against 1.3e-7. Sums of fewer than 64 terms, whose fold is short and rounds less (16 terms: 7e-8 against 1e-7), from 2^27 on.
+CONV_CONTRACTION_MIN_WORK = 1 << 20
 _CONV_PATCH_BYTES = 1 << 30   # patches of at most this many bytes at a time (whole images per piece)
 
 
 def _conv_on_tensor_cores(dtype, n, cin, cout, kh, kw, oh, ow) -> bool:
     k = cin * kh * kw
-    if dtype not in (torch.float32, torch.bfloat16) or n * cout * oh * ow * k < CONV_CONTRACTION_MIN_WORK:
+    if dtype not in (torch.float32, torch.bfloat16) or n * cout * oh * ow * k < CONV_CONTRACTION_MIN_WORK << (7 if k < 64 else 0):
         return False
-    return (cout >= 16 and n * oh * ow >= 128) or (dtype == torch.bfloat16 and _whole_tiles(k, cout))
+    return (cout >= 16 and n * oh * ow >= 16) or (dtype == torch.bfloat16 and _whole_tiles(k, cout))
 
 
 def _whole_tiles(k, cout) -> bool:
