@@ -165,7 +165,8 @@ int mimk_gemm_flat(int64_t m, int64_t n, int64_t k, const void* a, const void* b
 int mimk_reduce(const void* x, void* out, int dtype, int64_t outer, int64_t len, int64_t inner, int monoid,
                 void* stream);
 
-/* How many f32 partial results mimk_reduce / mimk_reduce_static keep for this problem on a device with `sm_count` SMs:
+/* How many f32 partial results mimk_reduce / mimk_reduce_static keep at most for this problem on a device with `sm_count` SMs
+ * (fewer, or none, where rows aligned to 16 bytes are folded four columns to a thread):
  * 0 when the reduced axis is not split (row reductions, or enough columns to fill the machine), else slices * outer *
  * inner. Pure host logic (needs no device): lets a caller of mimk_reduce_static see beforehand whether a plan fits
  * MIMK_REDUCE_STATIC_BYTES. No counterpart in the reference. */

@@ -71,6 +71,36 @@ __device__ __forceinline__ float4 load4_cached(const __nv_bfloat16* p) {
     float2 b = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&u.y));
     return make_float4(a.x, a.y, b.x, b.y);
 }
+// V neighbouring elements as they are loaded, and as f32
+template <class T, int V>
+struct Run;
+template <>
+struct Run<float, 1> {
+    float v;
+    __device__ __forceinline__ void load(const float* p) { v = __ldg(p); }
+    __device__ __forceinline__ float at(int) const { return v; }
+};
+template <>
+struct Run<float, 4> {
+    float4 v;
+    __device__ __forceinline__ void load(const float* p) { v = __ldg(reinterpret_cast<const float4*>(p)); }
+    __device__ __forceinline__ float at(int c) const { return c == 0 ? v.x : c == 1 ? v.y : c == 2 ? v.z : v.w; }
+};
+template <>
+struct Run<__nv_bfloat16, 1> {
+    unsigned short v;
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = __ldg(reinterpret_cast<const unsigned short*>(p)); }
+    __device__ __forceinline__ float at(int) const { return __uint_as_float(uint32_t(v) << 16); }
+};
+template <>
+struct Run<__nv_bfloat16, 4> {
+    uint2 v;
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = __ldg(reinterpret_cast<const uint2*>(p)); }
+    __device__ __forceinline__ float at(int c) const {
+        const uint32_t w = c < 2 ? v.x : v.y;
+        return __uint_as_float(c & 1 ? w & 0xffff0000u : w << 16);
+    }
+};
 __device__ __forceinline__ void store4(float* p, float4 v) { __stcs(reinterpret_cast<float4*>(p), v); }
 __device__ __forceinline__ void store4(__nv_bfloat16* p, float4 v) {
     uint2 u;
@@ -215,9 +245,18 @@ __global__ void softmax_strided_kernel(const TIn* __restrict__ x, TOut* __restri
 // or the address its elements start from (y_mode 0 and 2), from where they lie at the same stride as x's (a * inner).
 struct NoPre {
     struct Cell {};
+    struct Second {};  // nothing to load
+    template <int V>
+    struct Cells {
+        __device__ __forceinline__ Cells(const NoPre&, int64_t, int64_t) {}
+        __device__ __forceinline__ void load(Second&, int64_t) const {}
+        __device__ __forceinline__ float at(const Second&, int) const { return 0.f; }
+    };
+    template <int V>
+    using SecondOf = Second;
     __device__ Cell cell(int64_t, int64_t) const { return Cell{}; }
     __device__ float operator()(float v, const Cell&, int64_t) const { return v; }
-    __device__ bool batched() const { return true; }
+    __host__ __device__ bool batched() const { return true; }
     __device__ float other(const Cell&, int64_t) const { return 0.f; }
     __device__ float first(float v, float) const { return v; }
     __device__ float4 four(float4 v, const Cell&, int64_t) const { return v; }
@@ -245,8 +284,29 @@ struct MapPre {
         else if (mode() == 1) c.yb = ldf(y, o * inner + i);
         return c;
     }
+    // V neighbouring cells of a fold of a middle axis (V = 4: inner % 4 == 0): their second operands at an offset from the first one's start
+    template <int V>
+    using SecondOf = Run<TIn, V>;
+    template <int V>
+    struct Cells {
+        const TIn* yp = nullptr;
+        float yb[V] = {};
+        __device__ __forceinline__ Cells(const MapPre& p, int64_t o, int64_t i) {
+            if (!binary) return;
+            if (p.mode() == 0) yp = p.y + o * p.len * p.inner + i;
+            else if (p.mode() == 2) yp = p.y + i;
+            else if (p.mode() == 1)
+#pragma unroll
+                for (int c = 0; c < V; ++c) yb[c] = ldf(p.y, o * p.inner + i + c);
+        }
+        static constexpr bool each = binary && (YMODE == 0 || YMODE == 2);
+        __device__ __forceinline__ void load(Run<TIn, V>& r, int64_t off) const {
+            if (each) r.load(yp + off);
+        }
+        __device__ __forceinline__ float at(const Run<TIn, V>& r, int c) const { return each ? r.at(c) : yb[c]; }
+    };
     // The first operator alone, with its second operand loaded by the caller: what a fold may batch (no run-time operator).
-    __device__ bool batched() const { return INNER >= 0 && outer_op == MIMK_OP_COPY; }
+    __host__ __device__ bool batched() const { return INNER >= 0 && outer_op == MIMK_OP_COPY; }
     __device__ float other(const Cell& c, int64_t off) const { return per_element() ? ldf(c.yp, off) : c.yb; }
     __device__ float apply(float v, float b) const {
         const float r = first(v, b);
@@ -307,7 +367,7 @@ __global__ void __launch_bounds__(256) reduce_rows_kernel(const TIn* __restrict_
 // results go to `partial` [slice, outer*inner] (or straight to `out` when there is a single slice).
 // Bound by memory latency: a thread has one 4-byte load per element, so it issues BATCH of them before it folds the first
 // (in the same ascending order). Left to the compiler, the loop had one in flight with a producer: the sum of squares of
-// [32, 2048, 512] f32 took 98 us and takes 29 (4.6 TB/s).
+// [32, 2048, 512] f32 took 98 us so and 29 with it (4.6 TB/s; 23 in tiles, below, which this kernel is left out for where they pay).
 // BATCH 0: axes (or slices) of fewer than 16 elements, four at a time with a producer and without one as the compiler does it. There
 // the registers of sixteen loads cost the threads on an SM that hide the latency instead: sum of [1024, 8, 2048] f32 24.2 -> 10.7 us,
 // [4096, 2, 512] 23.7 -> 10.8; sum of squares 24.7 -> 12.2 and 24.0 -> 10.2.
@@ -346,6 +406,70 @@ __global__ void reduce_mid_kernel(const TIn* __restrict__ x, TDst* __restrict__ 
         for (; a < a1; ++a) acc = op(acc, pre(ldf(p, a * inner), cell, a * inner));
         stf(dst, int64_t(blockIdx.y) * total + t, acc);
     }
+}
+
+// inner > 1, V neighbouring columns to a thread: a CTA folds `lanes` x V columns of one outer index over its slice of the axis, 256 / lanes
+// elements of it at a time, and joins the 256 / lanes results of a column at the end. The producer's first operator alone (pre.batched()).
+// Bound by HBM, and for short folds by the launches: a column to a thread of the whole grid needs many slices of the axis, and their partials a
+// second launch. Sum of [32, 2048, 512], inputs not in L2: f32 42 -> 33 us, bf16 36 -> 23; of [1, 128, 1024] f32 14 -> 6, [7, 300, 96]
+// 15 -> 8, [1, 100000, 8] 40 -> 13 (the relative error of the f32 sums is half as large). V = 4: eight loads of 16 (bf16: 8) bytes in flight per thread; four: 34 and 27 us. V = 1, for rows that are
+// not aligned: [32, 2048, 513] f32 44 -> 37, [20, 126, 65] 14 -> 8.
+template <int V, int BATCH, class Op, class TIn, class TDst, class Pre>
+__global__ void __launch_bounds__(256) reduce_tiles_kernel(const TIn* __restrict__ x, TDst* __restrict__ dst, int64_t total, int64_t len, int64_t inner,
+                                                           int64_t slice_len, int tiles, int lanes_log, const Pre pre) {
+    __shared__ float red[V][8 * 32];
+    Op op;
+    const int lanes = 1 << lanes_log, lane = threadIdx.x & (lanes - 1), step = 256 >> lanes_log;
+    const int64_t o = blockIdx.x / tiles, i = (int64_t(blockIdx.x % tiles) * lanes + lane) * V;
+    const int64_t a0 = int64_t(blockIdx.y) * slice_len, a1 = a0 + slice_len < len ? a0 + slice_len : len;
+    float acc[V];
+#pragma unroll
+    for (int c = 0; c < V; ++c) acc[c] = Op::ident();
+    if (i < inner) {
+        const typename Pre::template Cells<V> cells(pre, o, i);
+        int64_t a          = a0 + (threadIdx.x >> lanes_log), off = a * inner;
+        const TIn* p       = x + o * len * inner + i;
+        const int64_t pitch = step * inner;
+        Run<TIn, V> v[BATCH];
+        typename Pre::template SecondOf<V> b[BATCH];
+        auto term = [&](int j, int c) { return pre.first(v[j].at(c), cells.at(b[j], c)); };
+        for (; a + (BATCH - 1) * step < a1; a += BATCH * step, off += BATCH * pitch) {
+#pragma unroll
+            for (int j = 0; j < BATCH; ++j) v[j].load(p + off + j * pitch), cells.load(b[j], off + j * pitch);
+#pragma unroll
+            for (int c = 0; c < V; ++c) {  // in pairs, so that a sum's rounding does not grow with a batch's length
+                float t[BATCH];
+#pragma unroll
+                for (int j = 0; j < BATCH; ++j) t[j] = term(j, c);
+#pragma unroll
+                for (int d = 1; d < BATCH; d <<= 1)
+#pragma unroll
+                    for (int j = 0; j + d < BATCH; j += 2 * d) t[j] = op(t[j], t[j + d]);
+                acc[c] = op(acc[c], t[0]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < BATCH - 1; ++j)
+            if (a + j * step < a1) v[j].load(p + off + j * pitch), cells.load(b[j], off + j * pitch);
+#pragma unroll
+        for (int j = 0; j < BATCH - 1; ++j)
+            if (a + j * step < a1)
+#pragma unroll
+                for (int c = 0; c < V; ++c) acc[c] = op(acc[c], term(j, c));
+    }
+    for (int d = lanes; d < 32; d <<= 1)
+#pragma unroll
+        for (int c = 0; c < V; ++c) acc[c] = op(acc[c], __shfl_xor_sync(0xffffffffu, acc[c], d));
+    if ((threadIdx.x & 31) < lanes)
+#pragma unroll
+        for (int c = 0; c < V; ++c) red[c][(threadIdx.x >> 5) * 32 + lane] = acc[c];
+    __syncthreads();
+    if (threadIdx.x < lanes && i < inner)
+#pragma unroll
+        for (int c = 0; c < V; ++c) {
+            for (int w = 1; w < 8; ++w) acc[c] = op(acc[c], red[c][w * 32 + lane]);
+            stf(dst, int64_t(blockIdx.y) * total + o * inner + i + c, acc[c]);
+        }
 }
 template <class Op, class TOut>
 __global__ void reduce_partials_kernel(const float* __restrict__ partial, TOut* __restrict__ out, int64_t total,
@@ -522,6 +646,41 @@ ReducePlan reduce_plan(int64_t outer, int64_t len, int64_t inner, int sm_count) 
     return p;
 }
 
+// Whether, and with how many lanes (as a power of two), a fold in tiles of v columns to a thread pays. v = 4: 8 lanes (128 bytes of an f32 row to a
+// CTA; 16 and 32 measured the same or up to 30 % more), more where the axis is too short for every thread to have eight elements (sum of
+// [512, 128, 512] f32 47 us with 8 lanes, 33 with 16, 37 untiled), fewer where the row is short. Below that the untiled kernel is as fast or
+// faster: [4096, 32, 512] 62 us, 72 here; [4096, 64, 4] 10, 16 here. v = 1: 32 lanes, and only where the columns alone are few, which is where the
+// untiled kernel needs slices ([2, 64, 1000] 14 us, 8 here; [4096, 64, 301] 74, 137 here).
+inline int fold_tile_lanes(const ReducePlan& p, int64_t len, int64_t inner, int v, int sm_count) {
+    if (v == 1 && p.gx >= 2 * sm_count) return -1;
+    int most = 5;
+    const int least = v == 4 ? 3 : 5;
+    while (most > 0 && (int64_t(v) << (most - 1)) >= inner) --most;
+    for (int lanes = most < least ? most : least; lanes <= most; ++lanes)
+        if (len >= 8 * (256 >> lanes)) return lanes;
+    return -1;
+}
+struct TilePlan {
+    int64_t ctas, slice_len;
+    int tiles, slices;
+};
+// Slices of the axis, of at least 16 (v = 1: 32) elements to a thread, where the tiles alone are fewer than two to an SM (four to an SM: 33 -> 38 us for
+// [32, 2048, 512] f32), never more than `p` has, whose partials are what the caller has room for. Two
+// or three of an axis that is not long save less than the second launch takes: [1, 1024, 1024] f32 13.3 us with two, 10.3 without.
+TilePlan tile_plan(const ReducePlan& p, int64_t outer, int64_t len, int64_t inner, int v, int lanes_log, int sm_count) {
+    TilePlan t;
+    t.tiles = int((inner + (int64_t(v) << lanes_log) - 1) / (int64_t(v) << lanes_log));
+    t.ctas  = outer * t.tiles;
+    int64_t slices = (2LL * sm_count + t.ctas - 1) / t.ctas;
+    const int64_t most = len / ((256 >> lanes_log) * (v == 4 ? 16 : 32));
+    slices      = slices < most ? slices : most;
+    slices      = slices < p.slices ? slices : p.slices;
+    if (slices < 1 || (slices < 4 && len <= 128 * (256 >> lanes_log))) slices = 1;
+    t.slice_len = (len + slices - 1) / slices;
+    t.slices    = int((len + t.slice_len - 1) / t.slice_len);
+    return t;
+}
+
 // `partials(n, &ptr)` supplies room for n floats when the plan splits the axis: the cached allocation for mimk_reduce,
 // the array in the library image for mimk_reduce_static. Nothing there needs clearing: every partial the second kernel
 // reads is written by the first kernel of the same call.
@@ -542,6 +701,25 @@ int reduce_impl(const TIn* x, TOut* out, int64_t outer, int64_t len, int64_t inn
     const int64_t total = outer * inner;
     const int threads   = 256;
     const ReducePlan p  = reduce_plan(outer, len, inner, sm_count);
+    if (pre.batched()) {
+        const bool four = inner % 4 == 0 && reinterpret_cast<uintptr_t>(x) % (4 * sizeof(TIn)) == 0 && pre_vec_ok(pre);
+        const int lanes = fold_tile_lanes(p, len, inner, four ? 4 : 1, sm_count);
+        const TilePlan t = tile_plan(p, outer, len, inner, four ? 4 : 1, lanes < 0 ? 0 : lanes, sm_count);
+        if (lanes >= 0 && t.ctas <= 0x7fffffff) {
+            const dim3 grid{unsigned(t.ctas), unsigned(t.slices)};
+            auto run = [&](auto* dst) {
+                if (four) reduce_tiles_kernel<4, 8, Op><<<grid, threads, 0, s>>>(x, dst, total, len, inner, t.slice_len, t.tiles, lanes, pre);
+                else reduce_tiles_kernel<1, FOLD_BATCH, Op><<<grid, threads, 0, s>>>(x, dst, total, len, inner, t.slice_len, t.tiles, lanes, pre);
+                return launch_status();
+            };
+            if (t.slices == 1) return run(out);
+            float* scratch = nullptr;
+            MIMK_TRY(partials(size_t(t.slices) * size_t(total), &scratch));
+            MIMK_TRY(run(scratch));
+            reduce_partials_kernel<Op><<<p.gx, threads, 0, s>>>(static_cast<const float*>(scratch), out, total, t.slices);
+            return launch_status();
+        }
+    }
     if (p.slices == 1) {
         if (len < FOLD_BATCH) reduce_mid_kernel<0, Op><<<dim3(p.gx, 1), threads, 0, s>>>(x, out, outer, len, inner, len, pre);
         else reduce_mid_kernel<FOLD_BATCH, Op><<<dim3(p.gx, 1), threads, 0, s>>>(x, out, outer, len, inner, len, pre);

@@ -60,6 +60,31 @@ def test_folds_and_maps_along_a_middle_axis(T, outer, length, inner, dtype):
     close_cells(T.binary_ax("mul", 1, x, y, then="relu"), want, want.abs() + 1e-30, tol)
 
 
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("outer,length,inner,offset", [
+    (1, 256, 32, 0), (3, 255, 32, 0), (2, 257, 36, 0), (3, 128, 64, 0), (2, 64, 128, 0), (5, 63, 128, 0), (1, 2048, 4, 0), (2, 2049, 8, 0),
+    (1, 100003, 12, 0), (2, 4100, 260, 0), (1, 20000, 96, 0), (40, 300, 100, 0), (300, 64, 1028, 0),
+    (2, 300, 64, 1), (1, 64, 33, 0), (2, 63, 95, 0), (3, 191, 31, 0), (1, 513, 2, 0), (1, 100003, 7, 0), (2, 4099, 65, 0), (80, 70, 1023, 0)])
+def test_folds_in_tiles_of_columns(T, outer, length, inner, offset, dtype):
+    """One and four columns to a thread, lanes of 1 to 32, slices or none, tails of the axis and of the rows, with each placement of a second
+    operand; extremes are the same values. No term of a sum passes more than length / 8 additions of a thread and 60 of the joins and
+    slices (100 where a column is one thread's), each off by 2^-24 of the sum of the magnitudes at most, and one rounding of its own."""
+    x, y = rnd((outer, length, inner), 1, dtype, offset=offset), rnd((outer, length, inner), 2, dtype, offset=offset)
+    xd, yd, tol = d64(x), d64(y), (length / 8 + 101) * 2.0 ** -24 + (0 if dtype == F32 else BF16_ROUND)
+    close_cells(T.reduce("sum", 1, x), xd.sum(1), xd.abs().sum(1), tol)
+    close_cells(T.reduce_fused("sum", 1, x, "square"), xd.square().sum(1), xd.square().sum(1), tol)
+    close_cells(T.reduce_fused("sum", 1, x, "mul", y), (xd * yd).sum(1), (xd * yd).abs().sum(1), tol)
+    close_cells(T.reduce_fused("sum", 1, x, "mul", y[:, 0]), (xd * yd[:, :1]).sum(1), (xd * yd[:, :1]).abs().sum(1), tol)
+    close_cells(T.reduce_fused("sum", 1, x, "add", y[0]), (xd + yd[0]).sum(1), (xd + yd[0]).abs().sum(1), tol)
+    x[0, length // 2, 0], x[0, length - 1, 1], x[-1, 0, inner - 1] = math.inf, -math.inf, math.nan
+    for monoid in ("max", "min"):
+        want = x.float().nan_to_num(-math.inf if monoid == "max" else math.inf, math.inf, -math.inf)
+        want = want.amax(1) if monoid == "max" else want.amin(1)
+        assert torch.equal(T.reduce(monoid, 1, x).float(), want)
+    got = T.reduce("sum", 1, x).float()
+    assert got[0, 0] == math.inf and (inner == 2 or got[0, 1] == -math.inf) and torch.isnan(got[-1, inner - 1])
+
+
 def attention_reference(q, k, v, scale, causal):
     s = d64(q) @ d64(k).transpose(1, 2) * scale
     if causal:
