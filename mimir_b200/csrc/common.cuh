@@ -137,7 +137,6 @@ int attn_composed(const mimk_attn_desc& d, cudaStream_t s);
 // bf16, head_dim 64 or 128, up to 16 query rows: streams K and V once (attn_few.cu)
 int attn_few_supported(const mimk_attn_desc& d);
 int attn_few(const mimk_attn_desc& d, cudaStream_t s);
-int attn_heads_fill(const mimk_attn_desc& d);  // one head per SM keeps the 128-row kernel's SMs as busy
 // bf16, head_dim 64 or 128: one CTA per SM pulls (head, query-tile pair) items, hand-over between items pipelined
 int attn_tc_persistent_supported(const mimk_attn_desc& d);
 int attn_tc_persistent(const mimk_attn_desc& d, cudaStream_t s);

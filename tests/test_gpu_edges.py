@@ -194,6 +194,21 @@ def test_attention_of_a_few_queries(T, bh, sq, sk, d, causal):
 
 
 @pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("bh,sq,sk,causal", [
+    (1, 8, 16, False), (1, 9, 16, True), (148, 1, 768, False), (128, 8, 1000, False), (128, 9, 1000, True), (2, 8, 3000, True), (3, 7, 47, False), (1, 16, 1, False)])
+def test_attention_of_a_few_queries_in_tiles_of_eight_rows(T, bh, sq, sk, d, causal):
+    # one and two tiles of rows, rings that wrap or are never full, heads that fill the SMs; the bound of test_attention_of_a_few_queries
+    q, k, v = rnd((bh, sq, d), 4, BF16), rnd((bh, sk, d), 5, BF16), rnd((bh, sk, d), 6, BF16)
+    got, lse = T.attention(q, k, v, scale=d ** -0.5, causal=causal, return_lse=True)
+    T.device_status()
+    want, want_lse = attention_reference(q, k, v, d ** -0.5, causal)
+    weights = attention_reference(q, k, v.abs(), d ** -0.5, causal)[0]
+    assert ((d64(got) - want).abs() <= BF16_ROUND * (want.abs() + weights) + 1e-6).all()
+    seen = want_lse.isfinite()
+    assert torch.equal(d64(lse).isfinite(), seen) and ((d64(lse) - want_lse).abs()[seen] <= 1e-4).all()
+
+
+@pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("bh,sq,sk,causal,scale", [(3, 1, 40, True, 0.1), (2, 16, 1000, True, 0.1), (9, 2, 5000, True, 0.1), (200, 3, 300, True, 0.1), (4, 5, 700, False, -0.1)])
 def test_attention_of_a_few_queries_keeps_f32_weights(T, bh, sq, sk, d, causal, scale):
     # fewer queries than keys under a mask, or a negative scale: f32 weights, so that only the result is rounded to bf16
