@@ -9,8 +9,11 @@
 //                 the edge of an image gives a column that is not stored: 7 % at 56 x 56 with a 3 x 3 window).
 //     warps 0..7  add finished accumulators to sums in registers, store the tile by pixels (NCHW)
 //     warp 8      TMA, warp 9 one thread issues the MMAs, 128 x BN x 16
+//     warps 10, 11  read the cut kernel's records (f32) while the first tile is multiplied
 // f32: every block of 64 channels goes into a fresh accumulator, the products of small pieces first, and accumulators are added with
-// ordinary f32 adds (the tensor core does not round its updates to nearest); non-finite cells are folded again by the scalar code.
+// ordinary f32 adds (the tensor core does not round its updates to nearest). Cells that are not finite, or so small that bits lost in
+// cutting tiny values (below 2^-109, f32_split.cuh) could show, are folded again by the scalar code: each block of the cut kernel says
+// whether it lost any, and where one did, the storing warps look for the largest magnitudes that their cells come from.
 // bf16: one accumulator.
 //
 // Against gathering the image by the contraction's own loaders (gemm_f32_tc.cu), where every value is fetched, tested and cut again
@@ -18,6 +21,8 @@
 // 32 x 256 x 28 x 28, 256 of 3 x 3: f32 380 -> 175, bf16 462 -> 68. What bounds the f32 form: shared memory, 116 clocks per MMA of 96 (its
 // operands 10 KB and 5 KB of TMA writes). Also measured: blocks of 32 channels in 64-byte rows, 105 us (TMA takes as long for a row of 64
 // bytes as for one of 128); four accumulators of 128 columns, 114; MMAs issued by lane 0 in a branch of its own, 95.
+#include <math_constants.h>
+
 #include "common.cuh"
 #include "f32_split.cuh"
 #include "sm100.cuh"
@@ -29,7 +34,7 @@ using namespace f32split;
 
 namespace {
 
-constexpr int BM = 128, BKC = 64, NUM_THREADS = 384, TMA_WARP = 8, MMA_WARP = 9;
+constexpr int BM = 128, BKC = 64, NUM_THREADS = 384, TMA_WARP = 8, MMA_WARP = 9, RECORDS_WARP = 10;
 constexpr int STORE_REGS = 224, ISSUE_REGS = 56;  // two warpgroups and one, of 168 a thread at launch
 static_assert(2 * STORE_REGS + ISSUE_REGS <= 3 * 168, "setmaxnreg waits for ever for more than the launch was given");
 constexpr int A_BYTES = BM * BKC * 2;
@@ -50,6 +55,8 @@ struct Bars {
     uint64_t full[6], empty[6], m_full[2], m_empty[2], acc_full[4], acc_empty[4];
     uint32_t tmem_base;
     int abort_flag;
+    uint64_t records;                       // the cut kernel's records have been read
+    uint32_t flags[2];                      // what two warps found there
 };
 struct Ring {  // a place in a ring of N slots
     uint32_t slot = 0, phase = 0;
@@ -64,6 +71,9 @@ struct Shape {
     int n, cin, h, w, cout, kh, kw, oh, ow, stride_h, stride_w, dil_h, dil_w, pad_h, pad_w, by_tap;
     int hp, wp, hq, wq, grids_h, grids_w, pitch;
 };
+// What a block of the cut kernel says (f32): bits of a value were lost; a value was below all its pieces.
+constexpr uint32_t LOST = 1, DEEP = 2;
+
 struct Params {
     Shape c;
     const void* x;
@@ -71,6 +81,9 @@ struct Params {
     void* out;
     int64_t tiles_m, tiles_n;
     int* status;
+    uint32_t* records;             // LOST and DEEP, a word per block of the cut kernel
+    int64_t image_blocks, blocks;  // the image's, then the filters'
+    const __nv_bfloat16 *image_h, *filters_h;  // the first pieces
 };
 
 __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
@@ -83,33 +96,47 @@ __device__ __forceinline__ const TIn* filter_at(const Shape& c, const void* filt
     return static_cast<const TIn*>(filters) + int64_t(co) * c.cin * taps + (c.by_tap ? tap * c.cin + ci : ci * taps + tap);
 }
 
-// neighbouring channels cut and stored, the pieces `piece` elements apart
-template <int PIECES>
-__device__ __forceinline__ void store_pieces(__nv_bfloat16* dst, int64_t piece, float a, float b) {
+// N neighbouring channels cut and stored, the pieces `piece` elements apart; flags: LOST and DEEP.
+template <int PIECES, int N>
+__device__ __forceinline__ void store_pieces(__nv_bfloat16* dst, int64_t piece, const float (&x)[N], uint32_t& flags) {
+    float v[N];
+    uint32_t lost = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = x[i];
 #pragma unroll
     for (int t = 0; t < PIECES; ++t) {
-        *reinterpret_cast<uint32_t*>(dst + t * piece) = upper_halves(a, b);
-        a = lower_part(a), b = lower_part(b);
+        if constexpr (N == 4) *reinterpret_cast<uint2*>(dst + t * piece) = make_uint2(upper_halves(v[0], v[1]), upper_halves(v[2], v[3]));
+        else *reinterpret_cast<uint32_t*>(dst + t * piece) = upper_halves(v[0], v[1]);
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            if (t == 2) lost |= __float_as_uint(v[i]);
+            v[i] = lower_part(v[i]);
+        }
     }
-}
-template <int PIECES>
-__device__ __forceinline__ void store_pieces4(__nv_bfloat16* dst, int64_t piece, float (&v)[4]) {
+    if (PIECES == 3 && (lost & lost_bits)) {
+        flags |= LOST;
 #pragma unroll
-    for (int t = 0; t < PIECES; ++t) {
-        *reinterpret_cast<uint2*>(dst + t * piece) = make_uint2(upper_halves(v[0], v[1]), upper_halves(v[2], v[3]));
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = lower_part(v[i]);
+        for (int i = 0; i < N; ++i) flags |= x[i] != 0.f && fabsf(x[i]) < LOST_ABS ? DEEP : 0u;
     }
 }
 
-// Blocks [0, n hp groups): one padded image row and 64 channels, turned in shared memory; the others: 2048 filter elements each.
+// Blocks [0, image_blocks): one padded image row that some tap reads and 64 channels, turned in shared memory; the others: 2048 filter elements
+// each.
 template <class TIn, int PIECES>
 __global__ void __launch_bounds__(256) conv_cut_kernel(const Params p, __nv_bfloat16* __restrict__ image, __nv_bfloat16* __restrict__ filters,
                                                        int64_t image_piece, int64_t filter_piece) {
     __shared__ float tile[64][65];
     const Shape& c   = p.c;
     const int groups = (c.pitch + 63) / 64, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t rows = int64_t(c.n) * c.hp * groups;
+    uint32_t flags = 0;
+    auto leave = [&]() {  // the block's record
+        if constexpr (PIECES == 3) {
+            uint32_t all = 0;
+            if (__syncthreads_or(flags)) all = LOST | (__syncthreads_or(flags & DEEP) ? DEEP : 0u);
+            if (threadIdx.x == 0) p.records[blockIdx.x] = all;
+        }
+    };
+    const int64_t rows = p.image_blocks;
     if (blockIdx.x >= rows) {
         const int taps = c.kh * c.kw;
         int64_t i      = ((blockIdx.x - rows) * 256 + threadIdx.x) * 2;
@@ -117,21 +144,22 @@ __global__ void __launch_bounds__(256) conv_cut_kernel(const Params p, __nv_bflo
         for (; i < n; i += step) {
             const int64_t t = i / c.pitch;
             const int ci = int(i - t * c.pitch), co = int(t / taps), tap = int(t - int64_t(co) * taps);
-            const float a = ci < c.cin ? load1(filter_at<TIn>(c, p.filters, co, ci, tap)) : 0.f;
-            const float b = ci + 1 < c.cin ? load1(filter_at<TIn>(c, p.filters, co, ci + 1, tap)) : 0.f;
-            store_pieces<PIECES>(filters + i, filter_piece, a, b);
+            const float v[2] = {ci < c.cin ? load1(filter_at<TIn>(c, p.filters, co, ci, tap)) : 0.f,
+                                ci + 1 < c.cin ? load1(filter_at<TIn>(c, p.filters, co, ci + 1, tap)) : 0.f};
+            store_pieces<PIECES>(filters + i, filter_piece, v, flags);
         }
-        return;
+        return leave();
     }
     const int64_t line = blockIdx.x / groups;
-    const int c0 = int(blockIdx.x - line * groups) * 64, img = int(line / c.hp), y = int(line - int64_t(img) * c.hp);
-    const int yi = y - c.pad_h, yg = y % c.stride_h, yq = y / c.stride_h;
-    if (yg >= c.grids_h) return;  // no tap reads the row
+    // (rows and columns behind the padded image, which the grids have where it is no multiple of the strides, are written as zeros too)
+    const int lines = c.hq * c.grids_h, width = c.wq * c.stride_w;
+    const int c0 = int(blockIdx.x - line * groups) * 64, img = int(line / lines), in_image = int(line - int64_t(img) * lines);
+    const int yq = in_image / c.grids_h, yg = in_image - yq * c.grids_h, yi = yq * c.stride_h + yg - c.pad_h;
     const bool inside = unsigned(yi) < unsigned(c.h);
     const int64_t plane = int64_t(c.h) * c.w, grid_rows = int64_t(c.n) * c.hq * c.wq;
     __nv_bfloat16* line_out = image + (int64_t(yg) * c.grids_w * grid_rows + (int64_t(img) * c.hq + yq) * c.wq) * c.pitch + c0;
     const TIn* src = static_cast<const TIn*>(p.x) + (int64_t(img) * c.cin + c0) * plane + int64_t(inside ? yi : 0) * c.w;
-    for (int x0 = 0; x0 < c.wp; x0 += 64) {
+    for (int x0 = 0; x0 < width; x0 += 64) {
         const int xi  = x0 + tx - c.pad_w;
         const bool in0 = inside && unsigned(xi) < unsigned(c.w), in1 = inside && unsigned(xi + 32) < unsigned(c.w);
         float v[16];
@@ -149,17 +177,18 @@ __global__ void __launch_bounds__(256) conv_cut_kernel(const Params p, __nv_bflo
             for (int j = 0; j < 4; ++j) {
                 const int px = j * 16 + ty * 2 + (tx >> 4), x = x0 + px;
                 const int xg = c.stride_w == 1 ? 0 : x % c.stride_w, xq = c.stride_w == 1 ? x : x / c.stride_w;
-                if (x >= c.wp || xg >= c.grids_w) continue;
-                float w[4] = {tile[px][ch], tile[px][ch + 1], tile[px][ch + 2], tile[px][ch + 3]};
-                store_pieces4<PIECES>(line_out + (xg * grid_rows + xq) * c.pitch + ch, image_piece, w);
+                if (x >= width || xg >= c.grids_w) continue;
+                const float w[4] = {tile[px][ch], tile[px][ch + 1], tile[px][ch + 2], tile[px][ch + 3]};
+                store_pieces<PIECES>(line_out + (xg * grid_rows + xq) * c.pitch + ch, image_piece, w, flags);
             }
         }
-        __syncthreads();
+        if (x0 + 64 < width) __syncthreads();
     }
+    leave();
 }
 
 // The scalar fold of one cell, ascending (channel, kh, kw), one fma per step, padding read as zeros: for cells the pieces make
-// non-finite (an operand was inf / NaN, or the sum overflowed).
+// non-finite (an operand was inf / NaN, or the sum overflowed), and for cells as small as the bits lost in cutting.
 template <class TIn>
 __device__ __noinline__ float scalar_fold(const Params& p, int img, int co, int y, int x) {
     const Shape& c = p.c;
@@ -173,6 +202,39 @@ __device__ __noinline__ float scalar_fold(const Params& p, int img, int co, int 
                 v = fmaf(in ? load1(im + (int64_t(ci) * c.h + iy) * c.w + ix) : 0.f, load1(filter_at<TIn>(c, p.filters, co, ci, r * c.kw + q)), v);
             }
     return v;
+}
+
+// Bits were lost in cutting: what the sums of 32 filters from m0 on at `width` positions from n0 on have to reach for that not to matter, 22
+// bits above the loss, from the largest finite magnitudes among those filters and the rows of the grids that their taps read. (A sum of exactly
+// zero can be short of something only if values lie below all their pieces.) By a whole warp, from the first pieces, which are short of
+// a value by less than 2^-7 of it.
+__device__ __noinline__ float lost_bound(const Params& p, int m0, int n0, int width) {
+    const Shape& c = p.c;
+    const int lane = threadIdx.x & 31;
+    auto largest = [&](const __nv_bfloat16* from, int64_t elements) {  // a multiple of eight, 16-byte aligned
+        uint32_t most = 0;
+#pragma unroll 8
+        for (int64_t i = lane * 8; i < elements; i += 256) {
+            const uint4 q       = __ldg(reinterpret_cast<const uint4*>(from + i));
+            const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t lo = w[j] << 16 & 0x7fffffffu, hi = w[j] & 0x7fff0000u;
+                most = max(most, max(lo < 0x7f800000u ? lo : 0u, hi < 0x7f800000u ? hi : 0u));
+            }
+        }
+        return __uint_as_float(__reduce_max_sync(0xffffffffu, most));
+    };
+    const int64_t grid_rows = int64_t(c.n) * c.hq * c.wq, grids = int64_t(c.grids_h) * c.grids_w;
+    const int64_t reach = int64_t((c.kh - 1) * c.dil_h / c.stride_h) * c.wq + (c.kw - 1) * c.dil_w / c.stride_w;
+    float x = 0.f;
+    for (int64_t g = 0; g < grids; ++g) {
+        const int64_t first = g * grid_rows + n0, end = first + width + reach < grids * grid_rows ? first + width + reach : grids * grid_rows;
+        if (first < end) x = fmaxf(x, largest(p.image_h + first * c.pitch, (end - first) * c.pitch));
+    }
+    const int64_t row = int64_t(c.kh) * c.kw * c.pitch;
+    const float w = m0 < c.cout ? largest(p.filters_h + m0 * row, (c.cout - m0 < 32 ? c.cout - m0 : 32) * row) : 0.f;
+    return float(c.cin * c.kh * c.kw) * (0x1p22f * 1.01f * LOST_ABS) * (x + w);
 }
 
 template <int BN, int PIECES, class T>
@@ -202,6 +264,7 @@ conv_pieces_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             mbar_init(smem_u32(&bars->acc_full[b]), 1);
             mbar_init(smem_u32(&bars->acc_empty[b]), 8);
         }
+        mbar_init(smem_u32(&bars->records), 2);
         bars->abort_flag = 0;
         fence_barrier_init();
         tma_prefetch_desc(&tmA);
@@ -318,6 +381,19 @@ conv_pieces_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             }
         }
         __syncwarp();
+    } else if (PIECES == 3) {
+        uint32_t flags = 0;
+#pragma unroll 8
+        for (int64_t i = (threadIdx.x - RECORDS_WARP * 32) * 4; i < p.blocks; i += 256) {
+            const uint4 r = __ldg(reinterpret_cast<const uint4*>(p.records + i));
+            flags |= r.x | (i + 1 < p.blocks ? r.y : 0u) | (i + 2 < p.blocks ? r.z : 0u) | (i + 3 < p.blocks ? r.w : 0u);
+        }
+        flags = __reduce_or_sync(0xffffffffu, flags);
+        if (lane == 0) {
+            bars->flags[warp - RECORDS_WARP] = flags;
+            mbar_arrive(smem_u32(&bars->records));
+        }
+        __syncwarp();
     }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(STORE_REGS));
@@ -350,8 +426,15 @@ conv_pieces_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                 if (lane == 0) mbar_arrive(smem_u32(&bars->acc_empty[acc.slot]));
                 acc.step<C::NACC>();
             }
+            if (PIECES == 3) ok = ok && warp_wait(smem_u32(&bars->records), 0, abort_flag);  // (complete from the first tile on)
             if (!ok) break;
             const int rows = c.cout - (m0 + int(quarter) * 32);
+            float bound = 0.f;
+            bool zeros  = false;
+            if constexpr (PIECES == 3) {
+                const uint32_t flags = bars->flags[0] | bars->flags[1];
+                if (flags) bound = lost_bound(p, m0 + int(quarter) * 32, n0 + int(col0), HALF), zeros = flags & DEEP;
+            }
 #pragma unroll
             for (int i = 0; i < HALF; i += 32) {
 #pragma unroll
@@ -368,9 +451,11 @@ conv_pieces_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 #pragma unroll
                     for (int r = 0; r < 32; ++r)
                         if (r < rows) dst[r * pixels] = T(value[r]);
-                    if (probe != 0.f)
-                        for (int r = 0; r < 32 && r < rows; ++r)
-                            if (!isfinite(block[r * PITCH + lane])) dst[r * pixels] = T(scalar_fold<T>(p, img, co + r, y, x));
+                    if (probe != 0.f || bound > 0.f)
+                        for (int r = 0; r < 32 && r < rows; ++r) {
+                            const float v = block[r * PITCH + lane];
+                            if (!isfinite(v) || (fabsf(v) < bound && (v != 0.f || zeros))) dst[r * pixels] = T(scalar_fold<T>(p, img, co + r, y, x));
+                        }
                 }
                 __syncwarp();
             }
@@ -492,16 +577,20 @@ int conv_pieces(const mimk_conv_desc& d, cudaStream_t s) {
     const int pieces  = d.dtype == MIMK_F32 ? 3 : 1;
     const Sizes sizes = make_sizes(p.c);
     void* scratch     = nullptr;
-    if (get_scratch(sizes.bytes(pieces), &scratch, s) != MIMK_OK) {
+    const Shape& c    = p.c;
+    const int64_t extra = (sizes.filters + 2047) / 2048;
+    p.image_blocks      = int64_t(c.n) * c.hq * c.grids_h * ((c.pitch + 63) / 64);
+    p.blocks            = p.image_blocks + (extra < 1024 ? extra : 1024);
+    if (get_scratch(sizes.bytes(pieces) + size_t(p.blocks) * 4 + 512, &scratch, s) != MIMK_OK) {
         cudaGetLastError();
         return MIMK_E_UNSUPPORTED;
     }
     auto* image   = static_cast<__nv_bfloat16*>(scratch);
     auto* filters = reinterpret_cast<__nv_bfloat16*>((reinterpret_cast<uintptr_t>(image + pieces * sizes.image) + 255) & ~uintptr_t(255));
     p.x = d.x, p.filters = d.filters, p.out = d.out, p.status = dev->status_dev;
-    const Shape& c = p.c;
-    const int64_t rows = int64_t(c.n) * c.hp * ((c.pitch + 63) / 64), extra = (sizes.filters + 2047) / 2048;
-    const unsigned blocks = unsigned(rows + (extra < 1024 ? extra : 1024));
+    p.image_h = image, p.filters_h = filters;
+    p.records = reinterpret_cast<uint32_t*>((reinterpret_cast<uintptr_t>(filters + pieces * sizes.filters) + 255) & ~uintptr_t(255));
+    const unsigned blocks = unsigned(p.blocks);
     if (pieces == 3) conv_cut_kernel<float, 3><<<blocks, 256, 0, s>>>(p, image, filters, sizes.image, sizes.filters);
     else conv_cut_kernel<__nv_bfloat16, 1><<<blocks, 256, 0, s>>>(p, image, filters, sizes.image, sizes.filters);
     MIMK_TRY(launch_status());

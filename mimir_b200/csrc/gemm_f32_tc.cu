@@ -233,7 +233,10 @@ __device__ __forceinline__ void store_tile(const Params& p, const Place<BN>& at,
             const float v[4]  = {q.x, q.y, q.z, q.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-                if (gcol + e < p.N) plane[int64_t(e) * pixels] = TOut(isfinite(v[e]) ? v[e] : scalar_fold<TIn, CONV>(p, at.bz, row, gcol + e));
+                if (gcol + e < p.N) {
+                    const bool again = !isfinite(v[e]) || (fabsf(v[e]) < bound && (v[e] != 0.f || zeros));
+                    plane[int64_t(e) * pixels] = TOut(again ? scalar_fold<TIn, CONV>(p, at.bz, row, gcol + e) : v[e]);
+                }
         } else {
             finish4<TIn, TOut>(p, out, post_full, at.bz, row, gcol, q, bound, zeros);
         }
@@ -246,7 +249,8 @@ template <int BN, class TIn> __device__ __forceinline__ bool holds(const Params&
 // from the largest finite magnitudes among the CTA's rows, columns and k; a sum of exactly zero can be short of something only if there
 // are values below 2^-133. (It finds its place again, and loads four rows at a time: kept for it, or with eight, registers are spilled
 // by the loaders' loop, 1000^3 31 -> 35 us.) By all warps: 16 of 1000 x 1000 x 64 with softmax weights of 1e-38 67 us, 264 by one.
-template <class TIn, int BN>
+// CONV: the largest of the image rows that the tile's windows reach, all channels.
+template <class TIn, int BN, bool CONV>
 __device__ __noinline__ void find_bound(const Params& p, Bars* bars) {
     const Place<BN> at(p);
     const TIn* A = static_cast<const TIn*>(p.A) + at.bz * p.sa;
@@ -271,7 +275,19 @@ __device__ __noinline__ void find_bound(const Params& p, Bars* bars) {
             }
         return __reduce_max_sync(0xffffffffu, most);
     };
-    const uint32_t a = largest(A + at.m0 * p.K + k0, rows, p.K, k1 - k0, p.vec_a);
+    uint32_t a = 0;
+    if (CONV) {
+        const ConvShape& cv  = p.conv;
+        const int64_t pixels = int64_t(cv.oh) * cv.ow, plane = int64_t(cv.h) * cv.w, last = at.m0 + rows - 1;
+        for (int64_t img = at.m0 / pixels; img * pixels <= last; ++img) {
+            const int y0 = img * pixels < at.m0 ? int(at.m0 - img * pixels) / cv.ow : 0;
+            const int y1 = last - img * pixels < pixels ? int(last - img * pixels) / cv.ow : cv.oh - 1;
+            const int top = max(y0 * cv.stride_h - cv.pad_h, 0), bottom = min(y1 * cv.stride_h - cv.pad_h + (cv.kh - 1) * cv.dil_h, cv.h - 1);
+            if (top <= bottom) a = max(a, largest(A + img * cv.cin * plane + int64_t(top) * cv.w, cv.cin, plane, int64_t(bottom - top + 1) * cv.w, false));
+        }
+    } else {
+        a = largest(A + at.m0 * p.K + k0, rows, p.K, k1 - k0, p.vec_a);
+    }
     const TIn* b0    = p.b_nk ? B + at.n0 * p.K + k0 : B + k0 * p.N + at.n0;
     const uint32_t b = p.b_nk ? largest(b0, cols, p.K, k1 - k0, p.vec_b)
                               : largest(b0, k1 - k0, p.N, cols, p.N % 4 == 0 && (reinterpret_cast<uintptr_t>(b0) & 15) == 0);
@@ -286,7 +302,7 @@ template <int BN, class TIn, class TOut, bool CONV>
 __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __grid_constant__ Params p) {
     using C = Cfg<BN, TIn>;
     constexpr int PIECES = C::PIECES;
-    constexpr bool LOSES = PIECES == 3 && !CONV;  // (large convolutions always cut their values, into heads and tails before)
+    constexpr bool LOSES = PIECES == 3;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
     const uint32_t base     = (raw_addr + 1023u) & ~1023u;
@@ -378,20 +394,25 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
         }
     };
     uint32_t lost = 0;
+    // (CONV: at once, for a register that its loaders have not got)
+    auto note = [&](uint32_t bits) {
+        if (!CONV) lost |= bits;
+        else if (LOSES && (bits & lost_bits)) bars->lost = 1;
+    };
     auto store_a = [&](uint32_t at) {
         if (CONV) {
-            split_store8<PIECES>(at + unit_offset(across, unit), A_PIECE, fa);
+            note(split_store8<PIECES>(at + unit_offset(across, unit), A_PIECE, fa));
         } else {
-            lost |= split_store4<PIECES>(at + half_unit_offset(along, half), A_PIECE, fa);
-            lost |= split_store4<PIECES>(at + half_unit_offset(along + 64, half), A_PIECE, fa + 4);
+            note(split_store4<PIECES>(at + half_unit_offset(along, half), A_PIECE, fa));
+            note(split_store4<PIECES>(at + half_unit_offset(along + 64, half), A_PIECE, fa + 4));
         }
     };
     auto store_b = [&](uint32_t at) {
         if (p.b_nk) {
-            lost |= split_store4<PIECES>(at + half_unit_offset(along, half), C::B_PIECE, fb);
-            if (NB == 2) lost |= split_store4<PIECES>(at + half_unit_offset(along + 64, half), C::B_PIECE, fb + 4);
+            note(split_store4<PIECES>(at + half_unit_offset(along, half), C::B_PIECE, fb));
+            if (NB == 2) note(split_store4<PIECES>(at + half_unit_offset(along + 64, half), C::B_PIECE, fb + 4));
         } else if (has_b) {
-            lost |= split_store8<PIECES>(at + unit_offset(across, unit), C::B_PIECE, fb);
+            note(split_store8<PIECES>(at + unit_offset(across, unit), C::B_PIECE, fb));
         }
     };
     if (warp < MMA_WARP && kb0 < kb1) {  // on their way while the barriers and the tensor memory are set up
@@ -568,7 +589,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1) gemm_f32_tc_kernel(const __gri
         }
     }
     __syncthreads();
-    if (LOSES && bars->lost) find_bound<TIn, BN>(p, bars);
+    if (LOSES && bars->lost) find_bound<TIn, BN, CONV>(p, bars);
     // (an abandoned wait leaves MMAs that read the stages; their results are marked invalid by the status word)
     if (p.split > 1) cluster_sync();
     float bound   = 0.f;

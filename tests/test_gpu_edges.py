@@ -432,6 +432,35 @@ def test_convolutions_over_an_image_laid_out_once(T, n, cin, h, w, cout, kh, kw,
     assert torch.equal(d64(conv()).isfinite(), ref(d64(x), d64(f)).isfinite())
 
 
+@pytest.mark.parametrize("n,cin,h,w,cout,k,stride,pad", [
+    (3, 16, 14, 14, 32, 3, 1, 1), (4, 65, 25, 19, 64, 5, 2, 2), (40, 24, 6, 5, 40, 3, 1, 1), (3, 128, 9, 30, 130, 1, 1, 0)])
+@pytest.mark.parametrize("low,high", [(1e-36, 1.0), (1e-38, 1e30), (1.0, 1e-37), (3e-42, 1e10)])
+@pytest.mark.parametrize("laid_out", [False, True])
+def test_f32_convolutions_of_tiny_values(T, n, cin, h, w, cout, k, stride, pad, low, high, laid_out):
+    # as test_f32_products_of_tiny_values, from the least work on that takes the tensor cores, gathered and over an image laid out once
+    x, f = rnd((n, cin, h, w), 1), rnd((cout, cin, k, k), 2)
+    x[n // 3:] *= low
+    f[cout // 3:] *= high
+    f[cout // 2] = 0.0
+    oh, ow = (h + 2 * pad - k) // stride + 1, (w + 2 * pad - k) // stride + 1
+    assert T._conv_on_tensor_cores(F32, n, cin, cout, k, k, oh, ow)
+    if laid_out:
+        run = T.L.lib()["_ZN4mimk11conv_piecesERK14mimk_conv_descP11CUstream_st"]
+        run.restype, run.argtypes = C.c_int, [C.POINTER(T.L.ConvDesc), C.c_void_p]
+        got, d = torch.empty((n, cout, oh, ow), device="cuda"), T.L.ConvDesc()
+        d.n, d.cin, d.h, d.w, d.cout, d.kh, d.kw, d.dtype = n, cin, h, w, cout, k, k, T.L.F32
+        d.stride_h = d.stride_w = stride
+        d.pad_h = d.pad_w = pad
+        d.dil_h = d.dil_w = 1
+        d.x, d.filters, d.out = x.data_ptr(), f.data_ptr(), got.data_ptr()
+        T.L.check(run(C.byref(d), T._stream()), "conv")
+    else:
+        got = T.conv(x, f, stride=(stride, stride), padding=(pad, pad))
+    T.device_status()
+    want, scale = (torch.nn.functional.conv2d(u, v, stride=stride, padding=pad) for u, v in ((d64(x), d64(f)), (d64(x).abs(), d64(f).abs())))
+    close_cells(got, want, scale + cin * k * k * 2.0 ** -149 / F32_CELL, F32_CELL)
+
+
 @pytest.mark.parametrize("m,n,k,b_nk,post,out,offset", [
     (2000, 1003, 520, True, "bias_relu", BF16, 0), (300, 257, 1031, True, None, BF16, 0), (129, 255, 1033, False, "bias", F32, 0),
     (640, 5003, 264, False, None, BF16, 0), (640, 5001, 257, True, "bias_tanh", F32, 1), (65, 2056, 512, True, None, BF16, 1),
