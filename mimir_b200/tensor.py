@@ -690,16 +690,19 @@ def _mrp_into(out, Sr, f, init, post, map_out, maps, ins):
 # and for integers, as ONE map_reduce_post on the per-cell kernel, which keeps the reference's ascending fold per output cell
 # bit for bit. A cell's fold is a serial chain, about 0.12 us a step: per cell / contraction, us: 1 x 16 x 14 x 14, 32 filters of 3 x 3
 # (2^20) 28 / 22; 1 x 256 x 27 x 27, 64 of 1 x 1 64 / 20; 1 x 64 x 25 x 25, 64 of 5 x 5 157 / 28; 3 x 256 x 16 x 16, 128 of 3 x 3 by 2 333 / 32;
-# the f32 error 2e-7 to 1e-6 against 1.3e-7. Sums of fewer than 64 terms, whose fold is short and rounds less (16 terms: 7e-8 against 1e-7), from 2^27 on.
+# the f32 error 2e-7 to 1e-6 against 1.3e-7. Sums of fewer than 64 terms, whose fold is short and rounds less (16 terms: 7e-8 against 1e-7), from 2^27 on;
+# and what mimk_conv does not take: two element types, which only the per-cell kernel accepts, and windows that go through a patch matrix, whose
+# product may round more than the fold (three TF32 products 1.7e-6; bf16 in one accumulator).
 CONV_CONTRACTION_MIN_WORK = 1 << 20
 _CONV_PATCH_BYTES = 1 << 30   # patches of at most this many bytes at a time (whole images per piece)
 
 
-def _conv_on_tensor_cores(dtype, n, cin, cout, kh, kw, oh, ow) -> bool:
+def _conv_on_tensor_cores(dtype, n, cin, cout, kh, kw, oh, ow, gathered=True) -> bool:
+    """gathered: operands that mimk_conv takes."""
     k = cin * kh * kw
-    if dtype not in (torch.float32, torch.bfloat16) or n * cout * oh * ow * k < CONV_CONTRACTION_MIN_WORK << (7 if k < 64 else 0):
+    if dtype not in (torch.float32, torch.bfloat16) or n * cout * oh * ow * k < CONV_CONTRACTION_MIN_WORK << (0 if gathered and k >= 64 else 7):
         return False
-    return (cout >= 16 and n * oh * ow >= 16) or (dtype == torch.bfloat16 and _whole_tiles(k, cout))
+    return (cout >= 16 and n * oh * ow >= (16 if gathered else 128)) or (dtype == torch.bfloat16 and _whole_tiles(k, cout))
 
 
 def _whole_tiles(k, cout) -> bool:
@@ -794,12 +797,12 @@ def conv(x: torch.Tensor, w: torch.Tensor, stride=(1, 1), dilation=(1, 1), paddi
     ow = (wd + 2 * padding[1] - dilation[1] * (kw - 1) - 1) // stride[1] + 1
     k = cin * kh * kw
     contraction = _conv_on_tensor_cores(x.dtype, n, cin, cout, kh, kw, oh, ow)
+    gathered = contraction and x.dtype == w.dtype and _conv_indexable(x, w, oh, ow, stride, dilation, padding)
+    if contraction and not gathered:
+        contraction = _conv_on_tensor_cores(x.dtype, n, cin, cout, kh, kw, oh, ow, gathered=False)
     as_patches = contraction and (x.dtype == torch.float32 or _whole_tiles(k, cout))   # extents the patch matrix is made for
-    gathered = contraction and _conv_indexable(x, w, oh, ow, stride, dilation, padding)
-    if contraction and x.dtype != w.dtype:
-        if as_patches:
-            raise TypeError("conv: both operands share the ring's element type")
-        gathered = False   # the per-cell kernel takes operands of two element types
+    if as_patches and x.dtype != w.dtype:   # (other extents: the per-cell kernel takes operands of two element types)
+        raise TypeError("conv: both operands share the ring's element type")
     laid_out = False
     if gathered:
         d = L.ConvDesc()

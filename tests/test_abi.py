@@ -171,3 +171,14 @@ def test_f32_contraction_estimate_on_any_number_of_sms(lib):
     for sms in list(range(1, 60)) + [132, 148, 160]:
         for m, n, k in ((256, 256, 256), (100, 3000, 4096), (1, 64, 100000)):
             assert 0 < estimate(m, n, k, 1, sms) < 1e12
+
+
+@pytest.mark.parametrize("n,cin,hw,cout,k,gathered,other", [
+    # (multiply-adds, positions): from 2^20 on what mimk_conv takes; two element types and windows through patches from 2^27 on, with 128 positions
+    (1, 16, 14, 32, 3, False, False), (1, 16, 28, 32, 3, True, False), (4, 64, 28, 64, 3, True, False), (4, 64, 56, 64, 3, True, True),
+    (1, 4, 112, 64, 3, False, False), (8, 7, 112, 64, 3, True, True), (1, 4096, 4, 128, 9, True, False), (2, 512, 8, 64, 9, True, True)])
+def test_which_convolutions_leave_the_per_cell_kernel(n, cin, hw, cout, k, gathered, other):
+    import torch
+    from mimir_b200 import tensor as T
+    assert T._conv_on_tensor_cores(torch.float32, n, cin, cout, k, k, hw, hw) == gathered
+    assert T._conv_on_tensor_cores(torch.float32, n, cin, cout, k, k, hw, hw, gathered=False) == other

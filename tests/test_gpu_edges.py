@@ -432,6 +432,17 @@ def test_convolutions_over_an_image_laid_out_once(T, n, cin, h, w, cout, kh, kw,
     assert torch.equal(d64(conv()).isfinite(), ref(d64(x), d64(f)).isfinite())
 
 
+@pytest.mark.parametrize("n,cin,h,w,cout,k,pad", [(1, 16, 28, 28, 32, 3, 1), (2, 64, 20, 21, 24, 3, 0), (1, 128, 17, 16, 64, 1, 0)])
+@pytest.mark.parametrize("dtype,other", [(F32, BF16), (BF16, F32)])
+def test_convolutions_of_two_element_types(T, n, cin, h, w, cout, k, pad, dtype, other):
+    # above the least work of the tensor cores, which take operands of one type: one fold per cell, as below it
+    x, f = rnd((n, cin, h, w), 1, dtype), rnd((cout, cin, k, k), 2, other)
+    got = T.conv(x, f, padding=(pad, pad))
+    T.device_status()
+    want, scale = (torch.nn.functional.conv2d(u, v, padding=pad) for u, v in ((d64(x), d64(f)), (d64(x).abs(), d64(f).abs())))
+    close_cells(got, want, scale, cin * k * k * 2.0 ** -24 if dtype == F32 else BF16_ROUND)
+
+
 @pytest.mark.parametrize("n,cin,h,w,cout,k,stride,pad", [
     (3, 16, 14, 14, 32, 3, 1, 1), (4, 65, 25, 19, 64, 5, 2, 2), (40, 24, 6, 5, 40, 3, 1, 1), (3, 128, 9, 30, 130, 1, 1, 0)])
 @pytest.mark.parametrize("low,high", [(1e-36, 1.0), (1e-38, 1e30), (1.0, 1e-37), (3e-42, 1e10)])
