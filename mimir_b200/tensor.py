@@ -717,7 +717,9 @@ def _sm_count(device: int) -> int:
 
 def _patches_pay(dtype, pixels, cout, k, window, padded, laid_out) -> bool:
     """Whether a patch matrix and the full-rate contraction beat gathering the patches inside the contraction. They never do where
-    the contraction lays the image out first and reads it in place of patches (mimk_conv_laid_out).
+    the contraction lays the image out first and reads it in place of patches (mimk_conv_laid_out), and below 2^27 multiply-adds they are
+    not asked: the patches' product keeps all of K in one accumulator, which rounds more than the per-cell fold that such convolutions
+    had; gathered, accumulators of 64 k are added with f32 adds, which rounds less.
 
     bf16: both estimated, in us. Gathered: rounds of a tile per SM, 14 + 1.85 per k-block of 32 (7 + 1.25 for up to 64 filters).
     Patches: three or four operators' host time, 85 or 112, or where it is more the matrix at 1.3 per MB, the result at 2 (written
@@ -726,7 +728,7 @@ def _patches_pay(dtype, pixels, cout, k, window, padded, laid_out) -> bool:
     1 x 1, 45 / 83.
     f32: the contraction that takes the patches writes two copies of them; only where each pixel is gathered again for many filters
     without a window to blow it up: 32 x 256 x 56 x 56, 512 of 1 x 1, 595 / 536; 256 of them, 307 / 371."""
-    if laid_out:
+    if laid_out or pixels * cout * k < CONV_CONTRACTION_MIN_WORK << 7:
         return False
     if dtype == torch.float32:
         return window == 1 and cout > 256 and cout % 4 == 0 and pixels * cout * k >= 1 << 33

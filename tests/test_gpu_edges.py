@@ -443,6 +443,17 @@ def test_convolutions_of_two_element_types(T, n, cin, h, w, cout, k, pad, dtype,
     close_cells(got, want, scale, cin * k * k * 2.0 ** -24 if dtype == F32 else BF16_ROUND)
 
 
+@pytest.mark.parametrize("n,cin,h,w,cout,k", [(1, 8192, 4, 4, 64, 3), (2, 120, 9, 12, 32, 5)])
+def test_bf16_convolutions_round_like_an_f32_fold(T, n, cin, h, w, cout, k):
+    # off by half a unit of the result's last place and what an f32 sum may lose; operands of one sign, so that what an accumulator cuts off adds up
+    x, f = rnd((n, cin, h, w), 1, BF16).abs_(), rnd((cout, cin, k, k), 2, BF16).abs_()
+    got = T.conv(x, f, padding=(k // 2, k // 2))
+    T.device_status()
+    want = torch.nn.functional.conv2d(d64(x), d64(f), padding=k // 2)
+    half_unit = 2.0 ** (want.log2().floor() - 8)
+    assert ((d64(got) - want).abs() <= half_unit + F32_CELL * want).all()
+
+
 @pytest.mark.parametrize("n,cin,h,w,cout,k,stride,pad", [
     (3, 16, 14, 14, 32, 3, 1, 1), (4, 65, 25, 19, 64, 5, 2, 2), (40, 24, 6, 5, 40, 3, 1, 1), (3, 128, 9, 30, 130, 1, 1, 0)])
 @pytest.mark.parametrize("low,high", [(1e-36, 1.0), (1e-38, 1e30), (1.0, 1e-37), (3e-42, 1e10)])
