@@ -10,15 +10,15 @@
 //     warps 0..7  add finished accumulators to sums in registers, store the tile by pixels (NCHW)
 //     warp 8      TMA, warp 9 one thread issues the MMAs, 128 x BN x 16
 //     warps 10, 11  read the cut kernel's records (f32) while the first tile is multiplied
-// f32: every block of 64 channels goes into a fresh accumulator, the products of small pieces first, and accumulators are added with
-// ordinary f32 adds (the tensor core does not round its updates to nearest). Cells that are not finite, or so small that bits lost in
+// Every block of 64 channels goes into a fresh accumulator, and accumulators are added with ordinary f32 adds (the tensor core does not
+// round its updates to nearest: over all of K in one accumulator a bf16 convolution was off by up to 2e-5 before its result was rounded).
+// f32: the products of small pieces first. Cells that are not finite, or so small that bits lost in
 // cutting tiny values (below 2^-109, f32_split.cuh) could show, are folded again by the scalar code: each block of the cut kernel says
 // whether it lost any, and where one did, the storing warps look for the largest magnitudes that their cells come from.
-// bf16: one accumulator.
 //
 // Against gathering the image by the contraction's own loaders (gemm_f32_tc.cu), where every value is fetched, tested and cut again
-// for each tap that reads it: 16 x 128 x 56 x 56, 128 filters of 3 x 3, f32 214 -> 83 us (cut 16, conv 61), bf16 247 -> 42;
-// 32 x 256 x 28 x 28, 256 of 3 x 3: f32 380 -> 175, bf16 462 -> 68. What bounds the f32 form: shared memory, 116 clocks per MMA of 96 (its
+// for each tap that reads it: 16 x 128 x 56 x 56, 128 filters of 3 x 3, f32 214 -> 83 us (cut 16, conv 61), bf16 247 -> 46;
+// 32 x 256 x 28 x 28, 256 of 3 x 3: f32 380 -> 175, bf16 462 -> 77. What bounds the f32 form: shared memory, 116 clocks per MMA of 96 (its
 // operands 10 KB and 5 KB of TMA writes). Also measured: blocks of 32 channels in 64-byte rows, 105 us (TMA takes as long for a row of 64
 // bytes as for one of 128); four accumulators of 128 columns, 114; MMAs issued by lane 0 in a branch of its own, 95.
 #include <math_constants.h>
@@ -341,7 +341,7 @@ conv_pieces_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                 for (int kb = 0, cb = 0; kb < num_kb; ++kb) {
                     const int left = c.cin - cb * BKC, steps = left >= BKC ? BKC / 16 : (left + 15) / 16;
                     if (++cb == cblocks) cb = 0;
-                    if ((PIECES == 3 || kb == 0) && !wait(bars->acc_empty[acc.slot], acc.phase ^ 1u)) break;
+                    if (!wait(bars->acc_empty[acc.slot], acc.phase ^ 1u)) break;
                     const uint32_t d = tmem_base + acc.slot * BN;
                     if constexpr (PIECES == 3) {
                         const uint32_t lo = x.slot;
@@ -369,14 +369,12 @@ conv_pieces_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                     } else {
                         if (!wait(bars->full[x.slot], x.phase)) break;
                         tc_fence_after();
-                        product(d, x.slot, x.slot, steps, kb == 0);
+                        product(d, x.slot, x.slot, steps, true);
                         commit(smem_u32(&bars->empty[x.slot]));
                         x.step<C::X_SLOTS>();
                     }
-                    if (PIECES == 3 || kb + 1 == num_kb) {
-                        commit(smem_u32(&bars->acc_full[acc.slot]));
-                        acc.step<C::NACC>();
-                    }
+                    commit(smem_u32(&bars->acc_full[acc.slot]));
+                    acc.step<C::NACC>();
                 }
             }
         }
@@ -403,24 +401,29 @@ conv_pieces_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         float* block = reinterpret_cast<float*>(after) + warp * (32 * PITCH);
         Ring acc;
         bool ok      = true;
-        const int chunks = PIECES == 3 ? num_kb : 1, per_image = c.hq * c.wq;
+        const int per_image  = c.hq * c.wq;
         const int64_t pixels = int64_t(c.oh) * c.ow;
         for (int64_t tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
             const int m0 = int(tile % p.tiles_m) * BM, n0 = int(tile / p.tiles_m) * BN;
             float sum[HALF];
 #pragma unroll
             for (int i = 0; i < HALF; ++i) sum[i] = 0.f;
-            for (int ch = 0; ch < chunks; ++ch) {
+            for (int kb = 0; kb < num_kb; ++kb) {
                 if (!(ok = warp_wait(smem_u32(&bars->acc_full[acc.slot]), acc.phase, abort_flag))) break;
                 tc_fence_after();
-                // all columns requested, then one wait: a read of tensor memory stands in line behind the MMAs that are queued
-                const uint32_t t0 = tmem_base + acc.slot * BN + col0 + ((quarter * 32u) << 16);
-                uint32_t r[HALF / 32][32];
+                // as many columns requested as registers allow, then one wait: a read of tensor memory stands in line behind the MMAs that are
+                // queued
+                const uint32_t t0  = tmem_base + acc.slot * BN + col0 + ((quarter * 32u) << 16);
+                constexpr int WIDE = HALF <= 96 ? HALF : 64;
 #pragma unroll
-                for (int i = 0; i < HALF / 32; ++i) tmem_ld_32x32(t0 + i * 32, r[i]);
-                tmem_ld_wait();
+                for (int i0 = 0; i0 < HALF; i0 += WIDE) {
+                    uint32_t r[WIDE / 32][32];
 #pragma unroll
-                for (int i = 0; i < HALF; ++i) sum[i] = PIECES == 3 ? sum[i] + __uint_as_float(r[i / 32][i % 32]) : __uint_as_float(r[i / 32][i % 32]);
+                    for (int i = 0; i < WIDE / 32; ++i) tmem_ld_32x32(t0 + i0 + i * 32, r[i]);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int i = 0; i < WIDE; ++i) sum[i0 + i] += __uint_as_float(r[i / 32][i % 32]);
+                }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&bars->acc_empty[acc.slot]));
@@ -494,7 +497,8 @@ Sizes make_sizes(const Shape& c) {
 
 // Tile width: the one with the least estimated time: launches, a pass over the image at 4.1 TB/s, and rounds of a tile per SM. Measured
 // per block of 64 channels, f32: 1.52 us (128 wide) and 1.85 (192), what the tile's shared-memory traffic takes at 106 bytes a clock
-// (of 288 and 360 KB, a third of it written by TMA); bf16 0.45, 0.55 and 0.7 (256), the loads.
+// (of 288 and 360 KB, a third of it written by TMA); bf16 0.5, 0.63 and 0.82 (256), the loads and what reading the accumulators
+// leaves uncovered (one accumulator over all of K: 0.45, 0.55, 0.7; one per 128 channels saves a third of that, and rounds more).
 struct Plan {
     int bn;
     double us;
@@ -509,7 +513,7 @@ Plan make_plan(const Shape& c, int pieces, int sm_count) {
     for (int bn : {128, 192, 256}) {
         if (pieces == 3 && bn == 256) continue;
         const double rounds = double((tiles_m * ((positions + bn - 1) / bn) + sm_count - 1) / sm_count);
-        const double loads = pieces == 3 ? (bn == 128 ? 0.95 : 1.2) : (bn == 128 ? 0.45 : bn == 192 ? 0.55 : 0.7);
+        const double loads = pieces == 3 ? (bn == 128 ? 0.95 : 1.2) : (bn == 128 ? 0.5 : bn == 192 ? 0.63 : 0.82);
         const double mmas  = (pieces == 3 ? (bn == 128 ? 1.52 : 1.85) : 0.0) * part;
         const double us    = 11.0 + bytes / 4.1e6 + rounds * (4.0 + kb * (mmas > loads ? mmas : loads));
         if (us < best.us) best = Plan{bn, us};

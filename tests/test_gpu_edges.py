@@ -443,7 +443,7 @@ def test_convolutions_of_two_element_types(T, n, cin, h, w, cout, k, pad, dtype,
     close_cells(got, want, scale, cin * k * k * 2.0 ** -24 if dtype == F32 else BF16_ROUND)
 
 
-@pytest.mark.parametrize("n,cin,h,w,cout,k", [(1, 8192, 4, 4, 64, 3), (2, 120, 9, 12, 32, 5)])
+@pytest.mark.parametrize("n,cin,h,w,cout,k", [(1, 8192, 4, 4, 64, 3), (2, 120, 9, 12, 32, 5), (4, 256, 28, 29, 256, 3)])
 def test_bf16_convolutions_round_like_an_f32_fold(T, n, cin, h, w, cout, k):
     # off by half a unit of the result's last place and what an f32 sum may lose; operands of one sign, so that what an accumulator cuts off adds up
     x, f = rnd((n, cin, h, w), 1, BF16).abs_(), rnd((cout, cin, k, k), 2, BF16).abs_()
