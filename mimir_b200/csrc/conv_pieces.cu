@@ -483,7 +483,7 @@ Shape make_shape(const mimk_conv_desc& d) {
     c.oh = (c.hp - c.dil_h * (c.kh - 1) - 1) / c.stride_h + 1, c.ow = (c.wp - c.dil_w * (c.kw - 1) - 1) / c.stride_w + 1;
     c.hq = (c.hp + c.stride_h - 1) / c.stride_h, c.wq = (c.wp + c.stride_w - 1) / c.stride_w;
     c.grids_h = c.kh == 1 ? 1 : c.stride_h, c.grids_w = c.kw == 1 ? 1 : c.stride_w;
-    c.pitch = (c.cin + 7) & ~7;
+    c.pitch = (c.cin + 15) & ~15;  // (whole sectors: 24 channels in rows of 48 bytes 78 us, 45 now; 16 x 24 x 56 x 56, 128 filters of 3 x 3, f32)
     return c;
 }
 
@@ -553,16 +553,19 @@ int launch(Params& p, __nv_bfloat16* image, __nv_bfloat16* filters, const Sizes&
 }  // namespace
 
 // Whether this route takes the convolution: 16 channels and more (a row of fewer takes TMA as long: 25 x 3 x 56 x 61, 128 filters of 3 x 3, 161 us
-// against 106), 31-bit rows, a buffer of at most 1 GiB, an estimate below `other_us`, and f32 only where
-// the accumulators are not many more than one per 64 k, whose sums are what the error comes from (channels in whole blocks; 32 in 25 taps 1.41e-7
-// on either route, but 16 in 25 taps 1.35e-7 against 1.33e-7, 96 in 25 taps 1.75e-7 against 1.68e-7).
+// against 106), 31-bit rows, a buffer of at most 1 GiB, an estimate below `other_us`, and f32 only where the error is no larger than the
+// gathering kernel's. That one's accumulators hold 64 k whatever the channels; here it is one per tap and 64 channels, and the more of them are
+// added the larger the error. Measured, here / gathered, 1e-7: up to nine accumulators 1.15 / 1.26 (16 channels), 1.35 / 1.35 (56); whole blocks of
+// 64 channels the same at any window; 32 channels 1.41 / 1.41 in 25 taps, 1.65 / 1.54 in 49; 24 channels 1.40 / 1.38, 1.65 / 1.48, and 2.20 / 1.74 in
+// 121; 56 in 25 taps 1.53 / 1.51; 72 in 9 taps (18 accumulators) 1.46 / 1.40.
 int conv_pieces_preferred(const mimk_conv_desc& d, int sm_count, double other_us) {
     if (d.cin < 16 || d.n < 1 || d.cout < 1 || d.n >= (1 << 30) || d.cout >= (1 << 30)) return 0;
     const double rows = double(d.n) * (double(d.h) + 2.0 * double(d.pad_h) + double(d.stride_h)) * (double(d.w) + 2.0 * double(d.pad_w) + double(d.stride_w));
-    if (rows >= double(1 << 30) || double(d.cin + 8) * double(d.kh) * double(d.kw) >= double(1 << 30)) return 0;
+    if (rows >= double(1 << 30) || double(d.cin + 16) * double(d.kh) * double(d.kw) >= double(1 << 30)) return 0;
     const Shape c    = make_shape(d);
     const int pieces = d.dtype == MIMK_F32 ? 3 : 1;
-    if (pieces == 3 && c.cin % BKC != 0 && (c.cin <= 16 || c.cin > 32) && c.kh * c.kw * ((c.cin + BKC - 1) / BKC) > 10) return 0;
+    const int accumulators = c.kh * c.kw * ((c.cin + BKC - 1) / BKC);
+    if (pieces == 3 && c.cin % BKC != 0 && accumulators > (c.cin == 32 ? 25 : 10)) return 0;
     if (make_sizes(c).bytes(pieces) > (size_t(1) << 30)) return 0;
     return make_plan(c, pieces, sm_count).us < other_us;
 }

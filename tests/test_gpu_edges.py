@@ -432,6 +432,17 @@ def test_convolutions_over_an_image_laid_out_once(T, n, cin, h, w, cout, kh, kw,
     assert torch.equal(d64(conv()).isfinite(), ref(d64(x), d64(f)).isfinite())
 
 
+@pytest.mark.parametrize("cin,k,laid_out", [
+    (15, 3, False), (17, 3, True), (24, 5, False), (24, 11, False), (32, 5, True), (32, 7, False), (56, 3, True), (64, 7, True), (72, 3, False), (128, 5, True)])
+def test_f32_images_are_laid_out_where_the_error_is_no_larger(T, cin, k, laid_out):
+    n, side, cout = 16, 56, 128
+    d = T.L.ConvDesc()
+    d.n, d.cin, d.h, d.w, d.cout, d.kh, d.kw, d.dtype = n, cin, side, side, cout, k, k, T.L.F32
+    d.stride_h = d.stride_w = d.dil_h = d.dil_w = 1
+    d.pad_h = d.pad_w = k // 2
+    assert T.L.lib().mimk_conv_laid_out(C.byref(d), T._stream()) == laid_out
+
+
 @pytest.mark.parametrize("n,cin,h,w,cout,k,pad", [(1, 16, 28, 28, 32, 3, 1), (2, 64, 20, 21, 24, 3, 0), (1, 128, 17, 16, 64, 1, 0)])
 @pytest.mark.parametrize("dtype,other", [(F32, BF16), (BF16, F32)])
 def test_convolutions_of_two_element_types(T, n, cin, h, w, cout, k, pad, dtype, other):
