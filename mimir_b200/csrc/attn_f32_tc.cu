@@ -693,7 +693,8 @@ int attn_f32_tc(const mimk_attn_desc& d, cudaStream_t s) {
     if (cap == cudaStreamCaptureStatusNone && laid_out_pays(d, p.q_tiles)) {
         const int64_t dp = (d.head_dim + 7) & ~int64_t(7), piece = d.batch_heads * d.seq_k * dp, blocks = (d.seq_k + BKEYS - 1) / BKEYS;
         void* scratch    = nullptr;
-        if (get_scratch(size_t(piece) * 12 + size_t(d.batch_heads * blocks) * 8, &scratch, s) == MIMK_OK) {
+        ScratchLease lease;  // of both launches
+        if (lease.take(size_t(piece) * 12 + size_t(d.batch_heads * blocks) * 8, &scratch, s) == MIMK_OK) {
             auto* pieces = static_cast<__nv_bfloat16*>(scratch);
             auto* most   = reinterpret_cast<float*>(pieces + 6 * piece);
             p.most = most, p.kv_blocks = blocks;

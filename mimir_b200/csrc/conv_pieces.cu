@@ -588,7 +588,8 @@ int conv_pieces(const mimk_conv_desc& d, cudaStream_t s) {
     const int64_t extra = (sizes.filters + 2047) / 2048;
     p.image_blocks      = int64_t(c.n) * c.hq * c.grids_h * ((c.pitch + 63) / 64);
     p.blocks            = p.image_blocks + (extra < 1024 ? extra : 1024);
-    if (get_scratch(sizes.bytes(pieces) + size_t(p.blocks) * 4 + 512, &scratch, s) != MIMK_OK) {
+    ScratchLease lease;  // of both launches
+    if (lease.take(sizes.bytes(pieces) + size_t(p.blocks) * 4 + 512, &scratch, s) != MIMK_OK) {
         cudaGetLastError();
         return MIMK_E_UNSUPPORTED;
     }

@@ -582,12 +582,13 @@ int gemm_tc_ragged(const mimk_gemm_desc& d, cudaStream_t s) {
     int st           = MIMK_OK;
     DeviceInfo* dev  = device_info(&st);
     if (!dev) return st;
+    ScratchLease lease;
     if (r.pack_a || r.pack_b) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         MIMK_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
         if (cap != cudaStreamCaptureStatusNone) return MIMK_E_UNSUPPORTED;
         void* scratch = nullptr;
-        if (get_scratch(r.bytes_a + r.bytes_b, &scratch, s) != MIMK_OK) {
+        if (lease.take(r.bytes_a + r.bytes_b, &scratch, s) != MIMK_OK) {
             cudaGetLastError();
             return MIMK_E_UNSUPPORTED;
         }

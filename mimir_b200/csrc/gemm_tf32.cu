@@ -448,7 +448,8 @@ int gemm_tf32(const mimk_gemm_desc& d, cudaStream_t s) {
     MIMK_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
     if (cap != cudaStreamCaptureStatusNone) return MIMK_E_UNSUPPORTED;
     void* scratch = nullptr;
-    if (get_scratch(2 * a_bytes + 2 * b_bytes, &scratch, s) != MIMK_OK) {
+    ScratchLease lease;
+    if (lease.take(2 * a_bytes + 2 * b_bytes, &scratch, s) != MIMK_OK) {
         cudaGetLastError();
         return MIMK_E_UNSUPPORTED;
     }

@@ -736,9 +736,10 @@ int reduce_impl(const TIn* x, TOut* out, int64_t outer, int64_t len, int64_t inn
 
 struct CachedPartials {
     cudaStream_t stream;
+    mutable ScratchLease lease{};  // (until the fold that it is given to returns)
     int operator()(size_t n, float** out) const {
         void* p = nullptr;
-        MIMK_TRY(get_scratch(n * sizeof(float), &p, stream));
+        MIMK_TRY(lease.take(n * sizeof(float), &p, stream));
         *out = static_cast<float*>(p);
         return MIMK_OK;
     }

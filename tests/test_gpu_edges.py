@@ -611,3 +611,32 @@ def test_two_streams_at_once_give_what_one_gives(T):
         for g, w in zip(got, want):
             assert all(torch.equal(u, v) for u, v in zip(g, w))
     T.device_status()
+
+
+def test_two_threads_on_one_stream_give_what_one_gives(T):
+    # calls of two launches that meet in the stream's cached buffer, of different sizes, so that it also grows under them
+    import threading
+    x = [rnd((n, 64, 56, 56), n) for n in (14, 9)]
+    f, q = rnd((128, 64, 3, 3), 7), [rnd((n, 700, 64), 40 + n) for n in (6, 11)]
+    b = [rnd((1000, 301), i, BF16) for i in (1, 2)]
+    calls = [lambda i=i: [T.conv(x[i], f, padding=(1, 1)), *T.attention(q[i], q[i], q[i], scale=0.1, return_lse=True), T.attention(q[i], q[i], q[i], scale=0.1),
+                          T.product_2d(b[i], b[i].t())] for i in range(2)]
+    want = [c() for c in calls]
+    torch.cuda.synchronize()
+    got, errors = [[], []], []
+
+    def work(i):
+        try:
+            got[i] = [calls[i]() for _ in range(60)]
+        except Exception as e:   # noqa: BLE001 -- shown by the main thread
+            errors.append(e)
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    T.device_status()
+    assert not errors
+    for g, w in zip(got, want):
+        assert len(g) == 60 and all(torch.equal(u, v) for one in g for u, v in zip(one, w))
