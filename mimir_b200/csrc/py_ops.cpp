@@ -62,7 +62,16 @@ bool out_type(PyObject* o, at::ScalarType plain, at::ScalarType& t) {
 }
 
 Tensor empty(at::IntArrayRef shape, at::ScalarType t, const Tensor& like) { return at::detail::empty_cuda(shape, t, like.device(), std::nullopt); }
-void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+// The call into the library, f(stream), without the interpreter's lock: it may wait, for the device where a cached buffer grows, or for room
+// in a launch queue, and what it waits for may be another Python thread's to issue.
+template <class F>
+int unlocked(F&& f) {
+    void* stream         = c10::cuda::getCurrentCUDAStream().stream();
+    PyThreadState* state = PyEval_SaveThread();
+    const int status     = f(stream);
+    PyEval_RestoreThread(state);
+    return status;
+}
 PyObject* result(int status, Tensor&& out) {
     if (status != MIMK_OK) Py_RETURN_NONE;
     return THPVariable_Wrap(std::move(out));
@@ -116,7 +125,7 @@ OP(product_2d, 5)
     d.a = x->data_ptr(), d.b = w->data_ptr(), d.c = out.data_ptr();
     d.in_dtype = dtype_of(x->scalar_type()), d.out_dtype = dtype_of(t), d.b_layout = layout, d.post = int(post);
     d.post_row = bias ? bias->data_ptr() : nullptr;
-    return result(mimk_gemm(&d, stream()), std::move(out));
+    return result(unlocked([&](void* stream) { return mimk_gemm(&d, stream); }), std::move(out));
 END_OP
 
 // a, b, out dtype
@@ -132,7 +141,7 @@ OP(bmm, 3)
     d.batch = batch, d.m = m, d.n = cols, d.k = k, d.stride_a = m * k, d.stride_b = k * cols, d.stride_c = m * cols;
     d.a = x->data_ptr(), d.b = w->data_ptr(), d.c = out.data_ptr();
     d.in_dtype = dtype_of(x->scalar_type()), d.out_dtype = dtype_of(t), d.b_layout = layout, d.post = MIMK_POST_ID;
-    return result(mimk_gemm(&d, stream()), std::move(out));
+    return result(unlocked([&](void* stream) { return mimk_gemm(&d, stream); }), std::move(out));
 END_OP
 
 // monoid id, axis, x
@@ -143,7 +152,7 @@ OP(reduce, 3)
     const View3 v(*x, ax);
     if (!v.good(*x)) Py_RETURN_NONE;
     Tensor out = empty(without(*x, v.ax), x->scalar_type(), *x);
-    return result(mimk_reduce(x->data_ptr(), out.data_ptr(), dtype_of(x->scalar_type()), v.outer, v.len, v.inner, int(monoid), stream()), std::move(out));
+    return result(unlocked([&](void* stream) { return mimk_reduce(x->data_ptr(), out.data_ptr(), dtype_of(x->scalar_type()), v.outer, v.len, v.inner, int(monoid), stream); }), std::move(out));
 END_OP
 
 // monoid id, axis, x, unary inner id, unary outer id
@@ -156,7 +165,7 @@ OP(reduce_of_unary, 5)
     mimk_producer pre = {};
     pre.inner_op = int32_t(inner), pre.outer_op = int32_t(outer), pre.y_mode = 3;
     Tensor out = empty(without(*x, v.ax), x->scalar_type(), *x);
-    return result(mimk_reduce_fused(x->data_ptr(), &pre, out.data_ptr(), dtype_of(x->scalar_type()), v.outer, v.len, v.inner, int(monoid), stream()),
+    return result(unlocked([&](void* stream) { return mimk_reduce_fused(x->data_ptr(), &pre, out.data_ptr(), dtype_of(x->scalar_type()), v.outer, v.len, v.inner, int(monoid), stream); }),
                   std::move(out));
 END_OP
 
@@ -169,7 +178,7 @@ OP(softmax, 3)
     const View3 v(*x, ax);
     if (!v.good(*x)) Py_RETURN_NONE;
     Tensor out = empty(x->sizes(), t, *x);
-    return result(mimk_softmax(x->data_ptr(), out.data_ptr(), dtype_of(x->scalar_type()), dtype_of(t), v.outer, v.len, v.inner, stream()), std::move(out));
+    return result(unlocked([&](void* stream) { return mimk_softmax(x->data_ptr(), out.data_ptr(), dtype_of(x->scalar_type()), dtype_of(t), v.outer, v.len, v.inner, stream); }), std::move(out));
 END_OP
 
 // x, gamma, eps, out dtype
@@ -180,8 +189,8 @@ OP(rmsnorm, 4)
     const int64_t cols = x->size(x->dim() - 1);
     if (gamma->numel() != cols) Py_RETURN_NONE;
     Tensor out = empty(x->sizes(), t, *x);
-    return result(mimk_rmsnorm(x->data_ptr(), gamma->data_ptr(), out.data_ptr(), dtype_of(x->scalar_type()), dtype_of(t), x->numel() / cols, cols,
-                               float(PyFloat_AS_DOUBLE(a[2])), stream()),
+    return result(unlocked([&](void* stream) { return mimk_rmsnorm(x->data_ptr(), gamma->data_ptr(), out.data_ptr(), dtype_of(x->scalar_type()), dtype_of(t), x->numel() / cols, cols,
+                               float(PyFloat_AS_DOUBLE(a[2])), stream); }),
                   std::move(out));
 END_OP
 
@@ -192,7 +201,7 @@ OP(unary, 3)
     at::ScalarType t;
     if (!x || !is_int(a[0], op) || !out_type(a[2], x->scalar_type(), t)) Py_RETURN_NONE;
     Tensor out = empty(x->sizes(), t, *x);
-    return result(mimk_map_t(int(op), x->data_ptr(), nullptr, out.data_ptr(), dtype_of(x->scalar_type()), dtype_of(t), 1, x->numel(), 1, 3, stream()),
+    return result(unlocked([&](void* stream) { return mimk_map_t(int(op), x->data_ptr(), nullptr, out.data_ptr(), dtype_of(x->scalar_type()), dtype_of(t), 1, x->numel(), 1, 3, stream); }),
                   std::move(out));
 END_OP
 
@@ -203,7 +212,7 @@ OP(binary, 4)
     at::ScalarType t;
     if (!x || !y || !is_int(a[0], op) || x->scalar_type() != y->scalar_type() || x->sizes() != y->sizes() || !out_type(a[3], x->scalar_type(), t)) Py_RETURN_NONE;
     Tensor out = empty(x->sizes(), t, *x);
-    return result(mimk_map_t(int(op), x->data_ptr(), y->data_ptr(), out.data_ptr(), dtype_of(x->scalar_type()), dtype_of(t), 1, x->numel(), 1, 0, stream()),
+    return result(unlocked([&](void* stream) { return mimk_map_t(int(op), x->data_ptr(), y->data_ptr(), out.data_ptr(), dtype_of(x->scalar_type()), dtype_of(t), 1, x->numel(), 1, 0, stream); }),
                   std::move(out));
 END_OP
 
@@ -216,7 +225,7 @@ OP(binary_ax, 5)
     const View3 v(*x, ax);
     if (!v.good(*x) || y->sizes() != at::IntArrayRef(without(*x, v.ax))) Py_RETURN_NONE;
     Tensor out = empty(x->sizes(), t, *x);
-    return result(mimk_map_t(int(op), x->data_ptr(), y->data_ptr(), out.data_ptr(), dtype_of(x->scalar_type()), dtype_of(t), v.outer, v.len, v.inner, 1, stream()),
+    return result(unlocked([&](void* stream) { return mimk_map_t(int(op), x->data_ptr(), y->data_ptr(), out.data_ptr(), dtype_of(x->scalar_type()), dtype_of(t), v.outer, v.len, v.inner, 1, stream); }),
                   std::move(out));
 END_OP
 
@@ -237,7 +246,7 @@ OP(attention, 5)
     d.seq_q = q->size(r - 2), d.seq_k = k->size(r - 2), d.head_dim = q->size(r - 1);
     d.q = q->data_ptr(), d.k = k->data_ptr(), d.v = v->data_ptr(), d.o = out.data_ptr();
     d.scale = float(PyFloat_AS_DOUBLE(a[3])), d.causal = a[4] == Py_True, d.dtype = dtype_of(q->scalar_type());
-    return result(mimk_attn_fwd(&d, stream()), std::move(out));
+    return result(unlocked([&](void* stream) { return mimk_attn_fwd(&d, stream); }), std::move(out));
 END_OP
 
 // x, w1, w3, w2
@@ -253,7 +262,7 @@ OP(mlp_gated, 4)
     Tensor out = empty({d.m, d.n}, t, *x);
     d.x = x->data_ptr(), d.w1 = w1->data_ptr(), d.w3 = w3->data_ptr(), d.w2 = w2->data_ptr(), d.y = out.data_ptr();
     d.dtype = dtype_of(t), d.b_layout = layout;
-    return result(mimk_mlp_gated(&d, stream()), std::move(out));
+    return result(unlocked([&](void* stream) { return mimk_mlp_gated(&d, stream); }), std::move(out));
 END_OP
 
 // x, perm (a tuple of ints): the copy-style map_reduce_post that tensor.py's transpose spells
@@ -275,7 +284,7 @@ OP(transpose, 2)
     Tensor out = empty(shape, x->scalar_type(), *x);
     d.in[0] = x->data_ptr(), d.in_dtype[0] = d.out_dtype = dtype_of(x->scalar_type()), d.acc_dtype = MIMK_F32;
     d.comb = MIMK_F_FIRST, d.post = MIMK_P_ID, d.out = out.data_ptr();
-    return result(mimk_map_reduce_post(&d, stream()), std::move(out));
+    return result(unlocked([&](void* stream) { return mimk_map_reduce_post(&d, stream); }), std::move(out));
 END_OP
 
 PyMethodDef methods[] = {

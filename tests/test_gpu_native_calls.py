@@ -128,3 +128,32 @@ def test_watched_calls_are_declined(T):
     answers = []
     torch.func.vmap(lambda t: (answers.append(T._native.unary(T._UNOP["relu"], t, None)), t)[1])(x)
     assert answers == [None]
+
+
+def test_other_threads_run_while_a_call_waits(T):
+    # the library's buffer grows, which waits for the device: the interpreter's lock is not held meanwhile
+    import threading
+    import time
+    a = torch.randn((8192, 8192), device="cuda").to(BF16)
+    small, large = torch.randn((2, 400, 64), device="cuda"), torch.randn((64, 1000, 64), device="cuda")
+    ticks, done = [], threading.Event()
+
+    def tick():
+        while not done.is_set():
+            ticks.append(time.perf_counter())
+            time.sleep(1e-3)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        assert T._native.attention(small, small, small, 0.125, False) is not None
+        thread = threading.Thread(target=tick)
+        thread.start()
+        for _ in range(200):
+            T.product_2d(a, a)
+        start = time.perf_counter()
+        assert T._native.attention(large, large, large, 0.125, False) is not None
+        end = time.perf_counter()
+        done.set()
+        thread.join()
+    torch.cuda.synchronize()
+    assert end - start > 0.05   # (200 products of 0.8 ms were queued)
+    during = [start] + [t for t in ticks if start < t < end] + [end]
+    assert max(v - u for u, v in zip(during, during[1:])) < (end - start) / 2
