@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(THREADS, Ring<D>::CTAS) attn_few_kernel(const 
     int stage  = 0;
     uint32_t phase = 0;
     for (int64_t step = s0; step < s1; ++step) {
-        if (step < issued) alive &= sm100::mbar_wait(bar(stage), phase, &abort_flag);
+        if (step < issued) alive &= bool(__all_sync(0xffffffffu, sm100::mbar_wait(bar(stage), phase, &abort_flag)));  // (one outcome for the warp)
         const uint32_t kt = mine + stage * R::STAGE_BYTES, vt = kt + R::HALVES * R::TILE;
         float s[2][4] = {}, s2[2][4] = {};  // two chains of dependent products for each eight keys
 #pragma unroll
