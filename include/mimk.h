@@ -171,6 +171,9 @@ int mimk_reduce(const void* x, void* out, int dtype, int64_t outer, int64_t len,
  * inner. Pure host logic (needs no device): lets a caller of mimk_reduce_static see beforehand whether a plan fits
  * MIMK_REDUCE_STATIC_BYTES. No counterpart in the reference. */
 int mimk_reduce_plan(int64_t outer, int64_t len, int64_t inner, int sm_count, int64_t* partial_floats);
+/* In how many tiles of columns mimk_reduce folds this problem, 0 where it does not (row reductions, short axes, columns for which one
+ * to a thread is as fast); `aligned`: x starts on four elements. Pure host logic. No counterpart in the reference. */
+int mimk_reduce_tiles(int64_t outer, int64_t len, int64_t inner, int aligned, int sm_count, int64_t* tiles);
 
 /* mimk_reduce for callers that must not have the library allocate: the same arguments and, for F32 operands, the same
  * results bit for bit (one plan, the same kernels) -- F32 ONLY, a BF16 request returns MIMK_E_DTYPE -- but no

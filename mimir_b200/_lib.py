@@ -24,7 +24,7 @@ ROWS_SOFTMAX, ROWS_RMSNORM, ROWS_SOFTMAX_RMSNORM = 0, 1, 2
 # every symbol include/mimk.h declares
 SYMBOLS = (
     "mimk_status_str", "mimk_abi_version", "mimk_last_cuda_error", "mimk_device_check", "mimk_device_status", "mimk_selftest_wait_expiry",
-    "mimk_gemm", "mimk_gemm_flat", "mimk_gemm_gather", "mimk_gemm_reduce_scatter", "mimk_gemm_kpanels", "mimk_reduce", "mimk_reduce_fused", "mimk_reduce_plan", "mimk_reduce_static", "mimk_softmax", "mimk_rmsnorm", "mimk_softmax_rmsnorm", "mimk_map", "mimk_map_t",
+    "mimk_gemm", "mimk_gemm_flat", "mimk_gemm_gather", "mimk_gemm_reduce_scatter", "mimk_gemm_kpanels", "mimk_reduce", "mimk_reduce_fused", "mimk_reduce_plan", "mimk_reduce_tiles", "mimk_reduce_static", "mimk_softmax", "mimk_rmsnorm", "mimk_softmax_rmsnorm", "mimk_map", "mimk_map_t",
     "mimk_splat", "mimk_select", "mimk_generate_affine", "mimk_gather", "mimk_scatter", "mimk_attn_fwd", "mimk_conv", "mimk_conv_laid_out", "mimk_mlp_gated", "mimk_map_reduce_post", "mimk_mrp_classify", "mimk_mrp_cell_kernel", "mimk_program_classify", "mimk_program_run", "mimk_chain_order", "mimk_chain_cost",
     "mimk_host_rows", "mimk_host_rows_pair", "mimk_host_gemm", "mimk_host_attn_fwd", "mimk_host_mlp_gated", "mimk_host_map_reduce_post", "mimk_host_register",
     "mimk_host_unregister", "mimk_host_release",
@@ -151,6 +151,7 @@ def lib() -> C.CDLL:
         L.mimk_reduce_static.argtypes = [vp, vp, ci, i64, i64, i64, ci, vp]
         L.mimk_reduce_fused.argtypes = [vp, C.POINTER(Producer), vp, ci, i64, i64, i64, ci, vp]
         L.mimk_reduce_plan.argtypes = [i64, i64, i64, ci, C.POINTER(i64)]
+        L.mimk_reduce_tiles.argtypes = [i64, i64, i64, ci, ci, C.POINTER(i64)]
         L.mimk_softmax.argtypes = [vp, vp, ci, ci, i64, i64, i64, vp]
         L.mimk_rmsnorm.argtypes = [vp, vp, vp, ci, ci, i64, i64, cf, vp]
         L.mimk_softmax_rmsnorm.argtypes = [vp, vp, vp, ci, ci, i64, i64, cf, vp]

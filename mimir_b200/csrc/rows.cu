@@ -661,21 +661,24 @@ inline int fold_tile_lanes(const ReducePlan& p, int64_t len, int64_t inner, int 
     return -1;
 }
 struct TilePlan {
-    int64_t ctas, slice_len;
-    int tiles, slices;
+    int64_t ctas = 0, slice_len = 0, tiles = 0;  // no CTAs: not in tiles
+    int slices = 1, lanes_log = 0;
 };
 // Slices of the axis, of at least 16 (v = 1: 32) elements to a thread, where the tiles alone are fewer than two to an SM (four to an SM: 33 -> 38 us for
 // [32, 2048, 512] f32), never more than `p` has, whose partials are what the caller has room for. Two
 // or three of an axis that is not long save less than the second launch takes: [1, 1024, 1024] f32 13.3 us with two, 10.3 without.
-TilePlan tile_plan(const ReducePlan& p, int64_t outer, int64_t len, int64_t inner, int v, int lanes_log, int sm_count) {
+TilePlan tile_plan(const ReducePlan& p, int64_t outer, int64_t len, int64_t inner, int v, int sm_count) {
     TilePlan t;
-    t.tiles = int((inner + (int64_t(v) << lanes_log) - 1) / (int64_t(v) << lanes_log));
-    t.ctas  = outer * t.tiles;
+    t.lanes_log = fold_tile_lanes(p, len, inner, v, sm_count);
+    if (t.lanes_log < 0) return t;
+    const int64_t width = int64_t(v) << t.lanes_log, ctas = outer * ((inner + width - 1) / width);
+    if (ctas < 1 || ctas > 0x7fffffff) return t;  // (nothing to fold; more than one grid)
+    t.tiles = (inner + width - 1) / width, t.ctas = ctas;
     int64_t slices = (2LL * sm_count + t.ctas - 1) / t.ctas;
-    const int64_t most = len / ((256 >> lanes_log) * (v == 4 ? 16 : 32));
+    const int64_t most = len / ((256 >> t.lanes_log) * (v == 4 ? 16 : 32));
     slices      = slices < most ? slices : most;
     slices      = slices < p.slices ? slices : p.slices;
-    if (slices < 1 || (slices < 4 && len <= 128 * (256 >> lanes_log))) slices = 1;
+    if (slices < 1 || (slices < 4 && len <= 128 * (256 >> t.lanes_log))) slices = 1;
     t.slice_len = (len + slices - 1) / slices;
     t.slices    = int((len + t.slice_len - 1) / t.slice_len);
     return t;
@@ -703,13 +706,12 @@ int reduce_impl(const TIn* x, TOut* out, int64_t outer, int64_t len, int64_t inn
     const ReducePlan p  = reduce_plan(outer, len, inner, sm_count);
     if (pre.batched()) {
         const bool four = inner % 4 == 0 && reinterpret_cast<uintptr_t>(x) % (4 * sizeof(TIn)) == 0 && pre_vec_ok(pre);
-        const int lanes = fold_tile_lanes(p, len, inner, four ? 4 : 1, sm_count);
-        const TilePlan t = tile_plan(p, outer, len, inner, four ? 4 : 1, lanes < 0 ? 0 : lanes, sm_count);
-        if (lanes >= 0 && t.ctas <= 0x7fffffff) {
+        const TilePlan t = tile_plan(p, outer, len, inner, four ? 4 : 1, sm_count);
+        if (t.ctas > 0) {
             const dim3 grid{unsigned(t.ctas), unsigned(t.slices)};
             auto run = [&](auto* dst) {
-                if (four) reduce_tiles_kernel<4, 8, Op><<<grid, threads, 0, s>>>(x, dst, total, len, inner, t.slice_len, t.tiles, lanes, pre);
-                else reduce_tiles_kernel<1, FOLD_BATCH, Op><<<grid, threads, 0, s>>>(x, dst, total, len, inner, t.slice_len, t.tiles, lanes, pre);
+                if (four) reduce_tiles_kernel<4, 8, Op><<<grid, threads, 0, s>>>(x, dst, total, len, inner, t.slice_len, int(t.tiles), t.lanes_log, pre);
+                else reduce_tiles_kernel<1, FOLD_BATCH, Op><<<grid, threads, 0, s>>>(x, dst, total, len, inner, t.slice_len, int(t.tiles), t.lanes_log, pre);
                 return launch_status();
             };
             if (t.slices == 1) return run(out);
@@ -898,6 +900,14 @@ extern "C" int mimk_reduce_plan(int64_t outer, int64_t len, int64_t inner, int s
     if (outer * inner == 0 || inner == 1) return MIMK_OK;
     const ReducePlan p = reduce_plan(outer, len, inner, sm_count);
     if (p.slices > 1) *partial_floats = int64_t(p.slices) * outer * inner;
+    return MIMK_OK;
+}
+
+extern "C" int mimk_reduce_tiles(int64_t outer, int64_t len, int64_t inner, int aligned, int sm_count, int64_t* tiles) {
+    if (outer < 0 || len < 0 || inner < 0 || sm_count < 1 || !tiles) return MIMK_E_ARG;
+    *tiles = 0;
+    if (outer * inner == 0 || inner == 1) return MIMK_OK;
+    *tiles = tile_plan(reduce_plan(outer, len, inner, sm_count), outer, len, inner, aligned && inner % 4 == 0 ? 4 : 1, sm_count).ctas;
     return MIMK_OK;
 }
 

@@ -182,3 +182,12 @@ def test_which_convolutions_leave_the_per_cell_kernel(n, cin, hw, cout, k, gathe
     from mimir_b200 import tensor as T
     assert T._conv_on_tensor_cores(torch.float32, n, cin, cout, k, k, hw, hw) == gathered
     assert T._conv_on_tensor_cores(torch.float32, n, cin, cout, k, k, hw, hw, gathered=False) == other
+
+
+@pytest.mark.parametrize("outer,length,inner,aligned,tiles", [
+    (32, 2048, 512, 1, 512), (1, 128, 1024, 1, 16), (1, 100, 1000, 0, 32), (4096, 64, 301, 0, 0), (1, 8, 2048, 1, 0), (5, 300, 1, 1, 0), (0, 300, 64, 1, 0),
+    (1, 2, 1 << 34, 1, 0), (1, 2, 1 << 32, 0, 0), (1, 0, 1 << 35, 1, 0), (1, 256, 1 << 36, 1, 0), (1, 256, 1 << 35, 1, 1 << 30)])
+def test_tiles_of_a_fold_for_any_extents(lib, outer, length, inner, aligned, tiles):
+    # (columns whose tiles do not fit 32 bits, or a grid, are folded one to a thread)
+    n = C.c_int64(-1)
+    assert lib.lib().mimk_reduce_tiles(outer, length, inner, aligned, 148, C.byref(n)) == 0 and n.value == tiles
