@@ -1,8 +1,8 @@
 // The operators of mimir_b200/tensor.py for the calls that programs are made of: contiguous CUDA tensors of the right shapes and
 // element types. A call is taken from the Python arguments to the C ABI here, about 3 us of host time instead of 9 through ctypes.
 //
-// Every function returns the result, or None for any call it is not made for (another type, layout, device or shape, a dispatch mode or
-// transform that is active, a status that is not OK): the caller then takes the general path, which makes copies and raises errors.
+// Every function returns the result, or None for any call it is not made for (another type or subclass, layout, device or shape, a dispatch mode
+// or a transform that is active, a status that is not OK): the caller then takes the general path, which makes copies and raises errors.
 // tensor.py alone says what an operator means; nothing is accepted here that it would refuse.
 #include <Python.h>
 
@@ -21,17 +21,20 @@ namespace {
 
 using at::Tensor;
 
-// No transform or mode wants to see the operations (functorch, tracing, fake tensors, autocast ...), nor __torch_function__.
+// No transform or mode wants to see the operations (functorch, tracing, fake tensors ...), nor __torch_function__. Inference mode,
+// which takes one key from the default set, does not: what is allocated in it becomes an inference tensor by itself.
 bool nothing_watches() {
     const auto tls = c10::impl::tls_local_dispatch_key_set();
-    return tls.included_ == c10::default_included_set && !c10::impl::TorchDispatchModeTLS::any_modes_set() && !at::impl::torch_function_mode_enabled();
+    return tls.included_.add(c10::DispatchKey::ADInplaceOrView) == c10::default_included_set && !c10::impl::TorchDispatchModeTLS::any_modes_set() && !at::impl::torch_function_mode_enabled();
 }
 
 int dtype_of(at::ScalarType t) { return t == at::kFloat ? MIMK_F32 : t == at::kBFloat16 ? MIMK_BF16 : -1; }
 
-// A torch.Tensor proper, dense and row-major on a CUDA device, of F32 or BF16 elements; null if not.
+PyTypeObject* parameter_type;  // torch.nn.Parameter, for the life of the module
+
+// A torch.Tensor or torch.nn.Parameter proper, dense and row-major on a CUDA device, of F32 or BF16 elements; null if not.
 const Tensor* dense(PyObject* o, bool any_strides = false) {
-    if (Py_TYPE(o) != reinterpret_cast<PyTypeObject*>(THPVariableClass)) return nullptr;
+    if (Py_TYPE(o) != reinterpret_cast<PyTypeObject*>(THPVariableClass) && Py_TYPE(o) != parameter_type) return nullptr;
     const Tensor& t = THPVariable_Unpack(o);
     if (!t.defined() || !t.is_cuda() || t.layout() != at::kStrided || !t.has_storage() || t.is_neg() || dtype_of(t.scalar_type()) < 0) return nullptr;
     if (t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
@@ -295,4 +298,10 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods};
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__native() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__native() {
+    PyObject* nn = PyImport_ImportModule("torch.nn.parameter");
+    if (!nn) return nullptr;
+    parameter_type = reinterpret_cast<PyTypeObject*>(PyObject_GetAttrString(nn, "Parameter"));
+    Py_DECREF(nn);
+    return parameter_type ? PyModule_Create(&module) : nullptr;
+}

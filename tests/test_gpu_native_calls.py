@@ -52,7 +52,7 @@ def same(T, monkeypatch, f):
         assert got is want
     else:
         assert got.dtype == want.dtype and got.shape == want.shape and got.is_contiguous() == want.is_contiguous()
-        assert got.requires_grad == want.requires_grad and torch.equal(got.nan_to_num(7), want.nan_to_num(7))
+        assert got.requires_grad == want.requires_grad and got.is_inference() == want.is_inference() and torch.equal(got.nan_to_num(7), want.nan_to_num(7))
 
 
 @pytest.mark.parametrize("dtype", [F32, BF16])
@@ -128,6 +128,25 @@ def test_watched_calls_are_declined(T):
     answers = []
     torch.func.vmap(lambda t: (answers.append(T._native.unary(T._UNOP["relu"], t, None)), t)[1])(x)
     assert answers == [None]
+
+
+@pytest.mark.parametrize("mode", [torch.enable_grad, torch.no_grad, torch.inference_mode])
+def test_the_usual_forms_of_weights_and_modes_are_taken(T, monkeypatch, mode):
+    # a program's parameters, and generation in inference mode: taken, with results of the kind that the general path gives
+    class Sub(torch.Tensor):
+        pass
+    x, w = torch.randn((8, 16), device="cuda"), torch.nn.Parameter(torch.randn((16, 24), device="cuda"))
+    gamma = torch.nn.Parameter(torch.ones(16, device="cuda"))
+    with mode():
+        fresh = torch.randn((8, 16), device="cuda")
+        for call in (lambda: T._native.product_2d(x, w, T.L.POST_ID, None, None), lambda: T._native.rmsnorm(fresh, gamma, 1e-6, BF16),
+                     lambda: T._native.attention(x, x, fresh, 0.25, False), lambda: T._native.unary(T._UNOP["relu"], w, None),
+                     lambda: T._native.reduce(T.L.SUM, 0, fresh), lambda: T._native.transpose(w, (1, 0))):
+            got = call()
+            assert got is not None and type(got) is torch.Tensor and not got.requires_grad
+            assert got.is_inference() == torch.is_inference_mode_enabled()
+        same(T, monkeypatch, lambda: T.product_2d(fresh, w))
+        assert T._native.unary(T._UNOP["relu"], x.as_subclass(Sub), None) is None
 
 
 def test_other_threads_run_while_a_call_waits(T):
