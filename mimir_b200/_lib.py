@@ -188,6 +188,15 @@ def lib() -> C.CDLL:
     return _lib
 
 
+def native():
+    """The operators' calls without ctypes (csrc/py_ops.cpp)."""
+    try:
+        from . import _native
+    except ImportError as e:
+        raise ImportError(f"mimir_b200/_native.so is missing, or was built for another torch or interpreter: run `python -m mimir_b200.build` ({e})") from e
+    return _native
+
+
 def check(status: int, where: str) -> None:
     if status != 0:
         raise MimkError(status, where)

@@ -8,6 +8,8 @@ from __future__ import annotations
 
 import concurrent.futures as cf
 import glob
+import importlib.metadata
+import importlib.util
 import os
 import shutil
 import subprocess
@@ -44,11 +46,19 @@ def _stale(target: str, deps) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _native_for() -> str:
+    """What the extension module is built against, found without importing torch."""
+    return "\n".join([sys.version, importlib.metadata.version("torch"), importlib.util.find_spec("torch").origin])
+
+
 def _build_native(force: bool, verbose: bool) -> None:
-    """The extension module, against this interpreter's torch; it finds libmimk.so beside itself."""
-    src = os.path.join(CSRC, "py_ops.cpp")
-    if not force and not _stale(NATIVE, [src, os.path.join(ROOT, "include", "mimk.h")]):
-        return
+    """The extension module, against this interpreter's torch; it finds libmimk.so beside itself. Built anew for a newer source, and for another
+    torch or interpreter than it was built for."""
+    src, built_for = os.path.join(CSRC, "py_ops.cpp"), os.path.join(OBJ, "native_for.txt")
+    if not force and not _stale(NATIVE, [src, os.path.join(ROOT, "include", "mimk.h")]) and os.path.exists(built_for):
+        with open(built_for) as f:
+            if f.read() == _native_for():
+                return
     import sysconfig
 
     import torch
@@ -64,6 +74,8 @@ def _build_native(force: bool, verbose: bool) -> None:
         sys.stderr.write(f"--- py_ops.cpp\n{r.stdout}{r.stderr}\n")
     if r.returncode != 0:
         raise RuntimeError("g++ failed on py_ops.cpp")
+    with open(built_for, "w") as f:
+        f.write(_native_for())
 
 
 def build(force: bool = False, verbose: bool = False) -> str:

@@ -18,7 +18,8 @@ import math
 import torch
 
 from . import _lib as L
-from . import _native
+
+_native = L.native()
 
 _DT = {torch.float32: L.F32, torch.bfloat16: L.BF16, torch.int32: L.I32, torch.int64: L.I64}
 _TORCH = {v: k for k, v in _DT.items()}

@@ -191,3 +191,37 @@ def test_tiles_of_a_fold_for_any_extents(lib, outer, length, inner, aligned, til
     # (columns whose tiles do not fit 32 bits, or a grid, are folded one to a thread)
     n = C.c_int64(-1)
     assert lib.lib().mimk_reduce_tiles(outer, length, inner, aligned, 148, C.byref(n)) == 0 and n.value == tiles
+
+
+@pytest.mark.parametrize("native", [None, b"not a library"])
+def test_a_package_without_its_extension_says_how_to_build_it(tmp_path, native):
+    import shutil
+    import subprocess
+    import sys
+    package = tmp_path / "mimir_b200"
+    package.mkdir()
+    here = os.path.join(ROOT, "mimir_b200")
+    for name in os.listdir(here):
+        if name.endswith(".py"):
+            shutil.copy(os.path.join(here, name), package)
+    if native:
+        (package / "_native.so").write_bytes(native)
+    r = subprocess.run([sys.executable, "-c", "import mimir_b200.tensor"], cwd=tmp_path, capture_output=True, text=True)
+    assert r.returncode != 0 and "run `python -m mimir_b200.build`" in r.stderr
+
+
+def test_the_extension_is_built_anew_for_another_torch(tmp_path, monkeypatch):
+    from mimir_b200 import build as B
+    ran = []
+
+    class Result:
+        returncode, stdout, stderr = 0, "", ""
+    monkeypatch.setattr(B.subprocess, "run", lambda cmd, **kw: ran.append(cmd) or open(B.NATIVE, "w").close() or Result())
+    monkeypatch.setattr(B, "OBJ", str(tmp_path))
+    monkeypatch.setattr(B, "NATIVE", str(tmp_path / "_native.so"))
+    B._build_native(False, False)
+    B._build_native(False, False)
+    assert len(ran) == 1
+    monkeypatch.setattr(B.importlib.metadata, "version", lambda name: "0.0.0")
+    B._build_native(False, False)
+    assert len(ran) == 2
