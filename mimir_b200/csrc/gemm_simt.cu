@@ -261,7 +261,10 @@ int launch_small(const mimk_gemm_desc& d, cudaStream_t s) {
 }
 int launch_small(const mimk_gemm_desc& d, cudaStream_t s) {
     // 16 rows while the device has an SM for each such tile
-    const bool narrow = ((d.m + 15) / 16) * ((d.n + SN - 1) / SN) * d.batch <= 148;
+    int st                = MIMK_OK;
+    const DeviceInfo* dev = device_info(&st);
+    if (!dev) return st;
+    const bool narrow = ((d.m + 15) / 16) * ((d.n + SN - 1) / SN) * d.batch <= dev->sm_count;
     if (d.b_layout == MIMK_B_NK) return narrow ? launch_small<true, 1>(d, s) : launch_small<true, 2>(d, s);
     return narrow ? launch_small<false, 1>(d, s) : launch_small<false, 2>(d, s);
 }
