@@ -467,7 +467,7 @@ def test_bf16_convolutions_round_like_an_f32_fold(T, n, cin, h, w, cout, k):
 
 @pytest.mark.parametrize("n,cin,h,w,cout,k,stride,pad", [
     (3, 16, 14, 14, 32, 3, 1, 1), (4, 65, 25, 19, 64, 5, 2, 2), (40, 24, 6, 5, 40, 3, 1, 1), (3, 128, 9, 30, 130, 1, 1, 0)])
-@pytest.mark.parametrize("low,high", [(1e-36, 1.0), (1e-38, 1e30), (1.0, 1e-37), (3e-42, 1e10)])
+@pytest.mark.parametrize("low,high", [(1.0, 1.0), (1e-36, 1.0), (1e-38, 1e30), (1.0, 1e-37), (3e-42, 1e10)])
 @pytest.mark.parametrize("laid_out", [False, True])
 def test_f32_convolutions_of_tiny_values(T, n, cin, h, w, cout, k, stride, pad, low, high, laid_out):
     # as test_f32_products_of_tiny_values, from the least work on that takes the tensor cores, gathered and over an image laid out once
@@ -517,6 +517,23 @@ def test_bf16_products_of_any_extent(T, m, n, k, b_nk, post, out, offset):
     if post and post.endswith("tanh"):
         want = want.tanh()
     assert got.dtype == out and ((d64(got) - want).abs() <= rounding + scale + 1e-6).all()
+
+
+@pytest.mark.parametrize("m,n,k", [(4864, 576, 64), (8192, 832, 72), (4865, 640, 64), (300, 320, 264)])
+@pytest.mark.parametrize("offset", [1, 2, 7])
+def test_bf16_results_that_start_anywhere(T, m, n, k, offset):
+    # widths of whole 64s, where an odd start leaves the last element of a row to a piece without columns; nothing around the result is touched
+    a, b = rnd((m, k), 1, BF16), rnd((n, k), 2, BF16)
+    want = T.product_2d(a, b.t())
+    room = torch.full((m * n + 64,), 7.0, dtype=BF16, device="cuda")
+    d = T.L.GemmDesc()
+    d.batch, d.m, d.n, d.k, d.stride_c = 1, m, n, k, m * n
+    d.a, d.b, d.c = a.data_ptr(), b.data_ptr(), room.data_ptr() + 2 * offset
+    d.in_dtype, d.out_dtype, d.b_layout, d.post = T.L.BF16, T.L.BF16, T.L.B_NK, T.L.POST_ID
+    T.L.check(T.L.lib().mimk_gemm(C.byref(d), T._stream()), "gemm")
+    T.device_status()
+    assert (room[:offset] == 7.0).all() and (room[offset + m * n:] == 7.0).all()
+    assert ((d64(room[offset:offset + m * n].view(m, n)) - d64(want)).abs() <= BF16_ROUND * d64(want).abs() + 1e-6).all()
 
 
 @pytest.mark.parametrize("batch,m,n,k,b_nk,offset", [
