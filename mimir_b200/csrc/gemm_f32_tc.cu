@@ -13,8 +13,10 @@
 // Accumulators are added in pairs. Few tiles: the pairs of one tile are dealt out to a cluster of two, four or eight CTAs, which exchange
 // them through distributed shared memory (about 14 bytes a clock per SM, what bounds such products: by single accumulators 128 x 1024 x
 // 784 took 17 us). They are added in order whatever the grid as long as each CTA can hold its own to the end and they are at most nine:
-// K <= 1152, with 128 columns K <= 256 * split. Beyond that a CTA adds its own first, and the bits follow the split (300 x 300 x 3000: 24
-// pairs held 31.6 us, eight sums 27).
+// K <= 1152, with 128 columns K <= 256 * split. Up to there a small product has the bits of the same cells of a large one, which programs rely on
+// (and the tests hold, to K = 1028). Beyond that a CTA adds its own first, fewer tiles change hands, the sums round less, and the bits follow the split.
+// That bits agree is what nine is for: 128 x 2048 x 1152, nine pairs held 24.3 us and 1.247e-7, as sums 20.5 and 1.203e-7; 128 x 1024 x 1536,
+// twelve: 24.4 and 1.280e-7, 20.5 and 1.227e-7; 300 x 300 x 3000, 24: 31.6 and 27 us.
 //
 // The operands are read as the caller has them: any extents, strides and alignment, no copies, no scratch. What bounds it:
 // shared-memory bandwidth (a k-block of 128 x 128 moves 96 KB into the MMA and 48 KB from the loaders; measured 100 clocks per

@@ -790,7 +790,8 @@ def _conv_as_contraction(xp, w, n, cin, cout, kh, kw, oh, ow, stride, dilation) 
 def conv(x: torch.Tensor, w: torch.Tensor, stride=(1, 1), dilation=(1, 1), padding=(0, 0)) -> torch.Tensor:
     """`conv R (stride, dilation, padding) (input, weight)`: NCHW input, [Cout, Cin, KH, KW] weight (tensor.mim:434-438).
     Loop vector (n, co, oh, ow, ci, kh, kw); the input is read at (n, ci, oh*s + kh*d, ow*s + kw*d) of the padded tensor
-    (conv_impl, tensor.mim:1254-1282)."""
+    (conv_impl, tensor.mim:1254-1282). Small ones have the reference's ascending fold per cell bit for bit, as conv_grouped always has; larger
+    ones (CONV_CONTRACTION_MIN_WORK) differ from it in the order of their sums."""
     _dev(x, w)
     n, cin, h, wd = x.shape
     cout, cin2, kh, kw = w.shape

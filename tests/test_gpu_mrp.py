@@ -402,8 +402,8 @@ def test_composed_combiners_small_and_large(T, L):
 
 
 def test_large_convolutions_run_as_contractions(T, L):
-    """From 2^27 multiply-adds on, conv gathers its patches with one copy operation and contracts them with the weights on the
-    tensor cores (f32 as 3xTF32, bf16 directly); the result is held to the same tolerance as the per-cell kernel's."""
+    """Large convolutions are contractions on the tensor cores, whatever of gathering, an image laid out once and a patch matrix is
+    chosen; the result is held to the same tolerance as the per-cell kernel's."""
     rng = np.random.default_rng(21)
     x = rng.standard_normal((4, 64, 32, 32)).astype(np.float32)
     w = (rng.standard_normal((128, 64, 3, 3)) * 0.05).astype(np.float32)
