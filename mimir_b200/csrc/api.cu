@@ -74,9 +74,13 @@ int ScratchLease::take(size_t bytes, void** out, cudaStream_t stream, bool secon
     int st        = MIMK_OK;
     DeviceInfo* d = device_info(&st);
     if (!d) return st;
+    // (by the stream's number, not its handle: cudaStreamPerThread names another stream in each thread, and a handle may come back for a new stream
+    // while the work of the one before is not done)
+    unsigned long long id = 0;
+    MIMK_CUDA_TRY(cudaStreamGetId(stream, &id));
     Pool* pool       = &g_scratch[d->device][second];
     Pool::Slot* slot = nullptr;
-    MIMK_TRY(pool->acquire(bytes, stream, &slot));
+    MIMK_TRY(pool->acquire(bytes, reinterpret_cast<void*>(id), &slot));
     pool_ = pool, slot_ = slot;
     *out = slot->ptr;
     return MIMK_OK;

@@ -657,3 +657,37 @@ def test_two_threads_on_one_stream_give_what_one_gives(T):
     assert not errors
     for g, w in zip(got, want):
         assert len(g) == 60 and all(torch.equal(u, v) for one in g for u, v in zip(one, w))
+
+
+def test_a_handle_that_names_a_stream_per_thread(T):
+    # cudaStreamPerThread is another stream in each thread: calls of two launches do not meet in one buffer there
+    import threading
+    per_thread, convs = 2, []
+    for n in (14, 9):
+        x, f = rnd((n, 64, 56, 56), n), rnd((128, 64, 3, 3), 7 + n)
+        outs = [torch.empty((n, 128, 56, 56), device="cuda") for _ in range(21)]
+        d = T.L.ConvDesc()
+        d.n, d.cin, d.h, d.w, d.cout, d.kh, d.kw, d.dtype = n, 64, 56, 56, 128, 3, 3, T.L.F32
+        d.stride_h = d.stride_w = d.dil_h = d.dil_w = d.pad_h = d.pad_w = 1
+        d.x, d.filters = x.data_ptr(), f.data_ptr()
+        assert T.L.lib().mimk_conv_laid_out(C.byref(d), T._stream()) == 1
+        convs.append((d, outs, x, f))
+    statuses = [[], []]
+
+    def run(i, outs, stream):
+        d = convs[i][0]
+        for out in outs:
+            d.out = out.data_ptr()
+            statuses[i].append(T.L.lib().mimk_conv(C.byref(d), stream))
+    for i in range(2):
+        run(i, convs[i][1][:1], T._stream())
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=run, args=(i, convs[i][1][1:], per_thread)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    T.device_status()
+    for (_, outs, _, _), status in zip(convs, statuses):
+        assert status == [0] * 21 and all(torch.equal(out, outs[0]) for out in outs[1:])
