@@ -270,7 +270,7 @@ extern "C" int mimk_attn_fwd(const mimk_attn_desc* d, void* stream) {
         paired        = (e && e[0] == '1') ? 1 : 0;
     }
     if (paired && attn_tc_pair_supported(*d)) return attn_tc_pair(*d, s);
-    if (attn_few_supported(*d)) return attn_few(*d, s);
+    if (attn_few_supported(*d) && !(attn_tc_persistent_supported(*d) && attn_heads_fill(*d, dev->sm_count))) return attn_few(*d, s);
     if (attn_tc_persistent_supported(*d)) return attn_tc_persistent(*d, s);
     static int composed = -1;  // MIMK_ATTN_COMPOSED=0 keeps every such problem on the one-launch CUDA-core kernel
     if (f32_on_tensor_cores() && attn_f32_tc_supported(*d)) return attn_simt_preferred(*d, dev->sm_count) ? attn_simt(*d, s) : attn_f32_tc(*d, s);

@@ -353,6 +353,16 @@ int attn_few_supported(const mimk_attn_desc& d) {
     return aligned16(d.q) && aligned16(d.k) && aligned16(d.v);
 }
 
+// With more than eight rows the second tile of rows makes this kernel's steps twice as long, while the 128-row kernel (attn_tc_p.cu) gives a
+// head to each SM whatever its rows: it is ahead where one round of heads leaves few SMs idle, the longer the fewer the keys. Its time / this
+// kernel's, us, 128 heads x 128: 16 rows, 100 keys 7.9 / 10.3, 400 12.6 / 16.3, 1000 18.7 / 19.7, 2500 no more; 11 rows, 400 12.5 / 13.8, 1000
+// 18.7 / 17.1; 10 rows, 400 12.5 / 13.1, 1000 18.7 / 16.5. With a head on every SM there are no idle SMs whose share of the memory's rate the others take: 148
+// heads, 4096 keys, 16 rows 56.0 / 60.4, 12 rows 56.1 / 58.4, 5500 keys no more. At head_dim 64, with more or with fewer heads it is behind (200 heads x 16 x 1000 36.9 / 24.4).
+int attn_heads_fill(const mimk_attn_desc& d, int sm_count) {
+    if (d.head_dim != 128 || d.seq_q <= 10 || d.batch_heads > sm_count || d.batch_heads * 5 < sm_count * 4) return 0;
+    return d.seq_k <= 75 * d.seq_q || (d.batch_heads * 20 >= sm_count * 19 && d.seq_k >= 2000 && d.seq_k <= 5000);
+}
+
 int attn_few(const mimk_attn_desc& d, cudaStream_t s) {
     int st          = MIMK_OK;
     DeviceInfo* dev = device_info(&st);

@@ -133,6 +133,7 @@ int attn_composed(const mimk_attn_desc& d, cudaStream_t s);
 // bf16, head_dim 64 or 128, up to 16 query rows: streams K and V once (attn_few.cu)
 int attn_few_supported(const mimk_attn_desc& d);
 int attn_few(const mimk_attn_desc& d, cudaStream_t s);
+int attn_heads_fill(const mimk_attn_desc& d, int sm_count);  // ... whose heads keep the 128-row kernel's SMs busy, which is ahead then
 // bf16, head_dim 64 or 128: one CTA per SM pulls (head, query-tile pair) items, hand-over between items pipelined
 int attn_tc_persistent_supported(const mimk_attn_desc& d);
 int attn_tc_persistent(const mimk_attn_desc& d, cudaStream_t s);

@@ -208,6 +208,18 @@ def test_attention_of_a_few_queries_in_tiles_of_eight_rows(T, bh, sq, sk, d, cau
     assert torch.equal(d64(lse).isfinite(), seen) and ((d64(lse) - want_lse).abs()[seen] <= 1e-4).all()
 
 
+@pytest.mark.parametrize("bh,sq,sk", [(118, 16, 400), (120, 10, 400), (120, 11, 825), (120, 11, 826), (128, 16, 1), (128, 16, 1200), (148, 12, 1999), (148, 14, 4097), (149, 16, 130)])
+def test_attention_of_a_few_queries_where_heads_fill_the_chip(T, bh, sq, sk):
+    # on both sides of the line between the streaming kernel and the 128-row kernel; the bound of test_attention_of_a_few_queries
+    q, k, v = rnd((bh, sq, 128), 7, BF16), rnd((bh, sk, 128), 8, BF16), rnd((bh, sk, 128), 9, BF16)
+    got, lse = T.attention(q, k, v, scale=128 ** -0.5, return_lse=True)
+    T.device_status()
+    want, want_lse = attention_reference(q, k, v, 128 ** -0.5, False)
+    weights = attention_reference(q, k, v.abs(), 128 ** -0.5, False)[0]
+    assert ((d64(got) - want).abs() <= BF16_ROUND * (want.abs() + weights) + 1e-6).all()
+    assert ((d64(lse) - want_lse).abs() <= 1e-4).all()
+
+
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("bh,sq,sk,causal,scale", [(3, 1, 40, True, 0.1), (2, 16, 1000, True, 0.1), (9, 2, 5000, True, 0.1), (200, 3, 300, True, 0.1), (4, 5, 700, False, -0.1)])
 def test_attention_of_a_few_queries_keeps_f32_weights(T, bh, sq, sk, d, causal, scale):
