@@ -143,8 +143,9 @@ __device__ __forceinline__ void stage_part(float* to, int to_pitch, const float*
     }
 }
 
-// RT: rows of a thread
-template <bool B_NK, int RT>
+// RT: rows of a thread. VEC: both operands by 16 bytes, which K is a multiple of then. (B stored [N, K]: tested at run time, with a loop for the
+// rest of K, 733 x 634 x 16 4.9 -> 5.1 us, 4 of 107 x 204 x 188 5.7 -> 6.3. Stored [K, N] such an instance is slower: 41 x 168 x 252 5.2 -> 5.6.)
+template <bool B_NK, int RT, bool VEC>
 __global__ void __launch_bounds__(256) gemm_simt_small_kernel(const float* __restrict__ A, const float* __restrict__ B,
                                                              float* __restrict__ C, int64_t M, int64_t N, int64_t K,
                                                              int64_t sa, int64_t sb, int64_t sc, int post, int vec_a, int vec_b,
@@ -163,9 +164,9 @@ __global__ void __launch_bounds__(256) gemm_simt_small_kernel(const float* __res
     auto stage = [&](int buf, int64_t k0) {
         float* As = smem + buf * (A_FLOATS + B_FLOATS);
         float* Bs = As + A_FLOATS;
-        stage_part<SM, KC>(As, KP, A + m0 * K + k0, K, M - m0, K - k0, vec_a);
-        if (B_NK) stage_part<SN, KC>(Bs, KP, B + n0 * K + k0, K, N - n0, K - k0, vec_b);
-        else stage_part<KC, SN>(Bs, NP, B + k0 * N + n0, N, K - k0, N - n0, vec_b);
+        stage_part<SM, KC>(As, KP, A + m0 * K + k0, K, M - m0, K - k0, VEC || vec_a);
+        if (B_NK) stage_part<SN, KC>(Bs, KP, B + n0 * K + k0, K, N - n0, K - k0, VEC || vec_b);
+        else stage_part<KC, SN>(Bs, NP, B + k0 * N + n0, N, K - k0, N - n0, VEC || vec_b);
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
@@ -182,7 +183,7 @@ __global__ void __launch_bounds__(256) gemm_simt_small_kernel(const float* __res
         const int kn    = int(K - c * KC < KC ? K - c * KC : KC);
         int k           = 0;
 #pragma unroll 4
-        for (; k + 4 <= kn; k += 4) {
+        for (; VEC ? k < kn : k + 4 <= kn; k += 4) {
             float av[RT][4];
 #pragma unroll
             for (int i = 0; i < RT; ++i) {
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(256) gemm_simt_small_kernel(const float* __res
                 }
             }
         }
-        for (; k < kn; ++k) {
+        for (; !VEC && k < kn; ++k) {
             const float b0 = B_NK ? Bs[tx * KP + k] : Bs[k * NP + tx * 2], b1 = B_NK ? Bs[(tx + 16) * KP + k] : Bs[k * NP + tx * 2 + 1];
 #pragma unroll
             for (int i = 0; i < RT; ++i) {
@@ -235,17 +236,22 @@ __global__ void __launch_bounds__(256) gemm_simt_small_kernel(const float* __res
 bool vec_a(const mimk_gemm_desc& d) { return d.k % 4 == 0 && aligned16(d.a) && d.stride_a % 4 == 0; }
 bool vec_b(const mimk_gemm_desc& d) { return (d.b_layout == MIMK_B_NK ? d.k : d.n) % 4 == 0 && aligned16(d.b) && d.stride_b % 4 == 0; }
 
-// Worth it while the 64 x 64 tiling leaves most SMs without a tile.
+// Worth it while the 64 x 64 tiling leaves most SMs without a tile. With copies of 4 bytes, which take as long as a short K, not with many tiles
+// either. This kernel / the one above, us: 217 x 1298 x 17 (287 tiles of 32 x 32) 4.6 / 6.7, 303 x 1139 x 21 (360) 6.2 / 6.8, 2070 x 194 x 20 (455) 5.9 / 6.8, 2152 x 197 x 13
+// (476) 7.3 / 5.8, 693 x 731 x 15 (506) 7.2 / 5.7; 1978 x 347 x 109 (682) 13.9 / 17.0, 697 x 1101 x 83 (770) 13.3 / 14.8, 808 x 1267 x 195 (1040)
+// 33.7 / 27.8.
 bool small_tiles_apply(const mimk_gemm_desc& d) {
     if (d.in_dtype != MIMK_F32 || d.out_dtype != MIMK_F32 || d.k < 1) return false;
     const int64_t big = ((d.m + TM - 1) / TM) * ((d.n + TN - 1) / TN) * d.batch;
-    return big < 2 * 148 && (d.m + 31) / 32 <= 65535 && d.batch <= 65535;
+    if (big >= 2 * 148 || (d.m + 31) / 32 > 65535 || d.batch > 65535) return false;
+    const int64_t tiles = ((d.m + 31) / 32) * ((d.n + SN - 1) / SN) * d.batch;
+    return (vec_a(d) && vec_b(d)) || tiles * 10 <= 31 * 148 || (tiles <= 6 * 148 && d.k >= 48);
 }
 
-template <bool B_NK, int RT>
+template <bool B_NK, int RT, bool VEC>
 int launch_small(const mimk_gemm_desc& d, cudaStream_t s) {
     constexpr int SMEM = 2 * (16 * RT * KP + (B_NK ? SN * KP : KC * NP)) * int(sizeof(float));
-    auto kern          = gemm_simt_small_kernel<B_NK, RT>;
+    auto kern          = gemm_simt_small_kernel<B_NK, RT, VEC>;
     static bool configured[64] = {};  // per instance and device: the attribute is a per-device setting
     int dev = 0;
     MIMK_CUDA_TRY(cudaGetDevice(&dev));
@@ -259,14 +265,21 @@ int launch_small(const mimk_gemm_desc& d, cudaStream_t s) {
                                  static_cast<const float*>(d.post_row), static_cast<const float*>(d.post_full));
     return launch_status();
 }
+template <bool B_NK, int RT>
+int launch_small(const mimk_gemm_desc& d, bool vec, cudaStream_t s) {
+    if constexpr (B_NK)
+        if (vec) return launch_small<true, RT, true>(d, s);
+    return launch_small<B_NK, RT, false>(d, s);
+}
 int launch_small(const mimk_gemm_desc& d, cudaStream_t s) {
     // 16 rows while the device has an SM for each such tile
     int st                = MIMK_OK;
     const DeviceInfo* dev = device_info(&st);
     if (!dev) return st;
     const bool narrow = ((d.m + 15) / 16) * ((d.n + SN - 1) / SN) * d.batch <= dev->sm_count;
-    if (d.b_layout == MIMK_B_NK) return narrow ? launch_small<true, 1>(d, s) : launch_small<true, 2>(d, s);
-    return narrow ? launch_small<false, 1>(d, s) : launch_small<false, 2>(d, s);
+    const bool vec = vec_a(d) && vec_b(d);
+    if (d.b_layout == MIMK_B_NK) return narrow ? launch_small<true, 1>(d, vec, s) : launch_small<true, 2>(d, vec, s);
+    return narrow ? launch_small<false, 1>(d, vec, s) : launch_small<false, 2>(d, vec, s);
 }
 
 template <class TIn, class TOut>

@@ -335,6 +335,20 @@ def test_small_f32_products_of_any_alignment(T, m, n, k, offset, nk):
     close_cells(got, d64(a[:m]) @ bd, d64(a[:m]).abs() @ bd.abs(), k * 2.0 ** -24)
 
 
+@pytest.mark.parametrize("nk", [False, True])
+@pytest.mark.parametrize("m,n,k", [(416, 1121, 17), (448, 1057, 17), (448, 1057, 48), (880, 1053, 47), (960, 931, 50), (733, 635, 16), (107, 205, 188), (33, 65, 256)])
+def test_small_f32_products_on_either_kernel_have_one_result(T, m, n, k, nk):
+    # both sides of the lines between tiles of 32 x 32 and of 64 x 64, with copies of 4 and of 16 bytes: a corner has the same bits
+    a, b = rnd((m, k), 1), rnd((n, k) if nk else (k, n), 2)
+    got = T.product_2d(a, b.t() if nk else b)
+    corner = b[:21].contiguous() if nk else b[:, :21].contiguous()
+    part = T.product_2d(a[:33].contiguous(), corner.t() if nk else corner)
+    T.device_status()
+    assert torch.equal(part, got[:33, :21])
+    bd = d64(b).t() if nk else d64(b)
+    close_cells(got, d64(a) @ bd, d64(a).abs() @ bd.abs(), k * 2.0 ** -24)
+
+
 def test_f32_products_keep_infinities_and_extremes(T):
     a, b = rnd((200, 600), 1), rnd((600, 300), 2)
     a[3, 5], a[7, 0], b[9, 11] = math.inf, math.nan, -math.inf
