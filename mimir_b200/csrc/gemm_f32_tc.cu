@@ -167,6 +167,14 @@ __device__ __noinline__ float scalar_fold(const Params& p, int64_t bz, int64_t r
     return v;
 }
 
+// How many of a tile's accumulators go to each CTA of a cluster: whole pairs, so that half as many partial tiles change hands; one each where
+// there are CTAs enough, and the pairs are added when the tile is stored; one by one in convolutions, and beyond HELD_PAIRS, where
+// each CTA adds up its own in any case. (Always whole pairs, us: 1710 x 104 x 233 9.9 -> 12.0, 23 x 719 x 472 10.2 -> 11.0, 62 x 36 x 2364 18.4 -> 19.3.)
+__host__ __device__ inline int share_of(int chunks, int split, bool conv) {
+    if (conv || chunks > 2 * HELD_PAIRS || chunks <= split) return (chunks + split - 1) / split;
+    return ((chunks + 1) / 2 + split - 1) / split * 2;
+}
+
 // What a CTA works on: a tile of a batch entry, and of its k-blocks the accumulators [ch0, ch1).
 template <int BN> struct Place {
     int rank, ch0, ch1, kb0, kb1, per, chunks;
@@ -180,9 +188,7 @@ template <int BN> struct Place {
         tile_coords(item - bz * tiles, p.tiles_m, p.tiles_n, tm, tn);
         m0 = tm * BM, n0 = tn * BN;
         const int all_kb = int((p.K + BK - 1) / BK);
-        // (whole pairs of accumulators to a CTA; a convolution's are added one by one)
-        const int unit = p.conv.cin > 0 ? 1 : 2;
-        chunks = (all_kb + CHUNK - 1) / CHUNK, per = ((chunks + unit - 1) / unit + p.split - 1) / p.split * unit;
+        chunks = (all_kb + CHUNK - 1) / CHUNK, per = share_of(chunks, p.split, p.conv.cin > 0);
         ch0 = rank * per < chunks ? rank * per : chunks, ch1 = ch0 + per < chunks ? ch0 + per : chunks;
         kb0 = ch0 * CHUNK, kb1 = ch1 * CHUNK < all_kb ? ch1 * CHUNK : all_kb;
     }
@@ -206,11 +212,12 @@ __device__ __forceinline__ void finish4(const Params& p, TOut* out, const TOut* 
 }
 
 // The accumulators of a tile in order, each CTA of the cluster a share of the rows. hold: every pair of them has a partial tile of its
-// own, else each CTA has one.
+// own, or each of them, where each is a CTA's only one; else each CTA has one.
 template <int BN, class TIn, class TOut, bool CONV>
 __device__ __forceinline__ void store_tile(const Params& p, const Place<BN>& at, uint32_t base, bool hold, float bound, bool zeros) {
     using C = Cfg<BN, TIn>;
-    const int rows = BM / p.split, held = hold ? at.per / 2 : 1, used = hold ? (at.chunks + 1) / 2 : (at.chunks + at.per - 1) / at.per;
+    const bool pairs = hold && at.per > 1, singles = hold && at.per == 1;
+    const int rows = BM / p.split, held = pairs ? at.per / 2 : 1, used = pairs ? (at.chunks + 1) / 2 : (at.chunks + at.per - 1) / at.per;
     TOut* out             = static_cast<TOut*>(p.C) + at.bz * p.sc;
     const TOut* post_full = p.post_full ? static_cast<const TOut*>(p.post_full) + at.bz * p.sc : nullptr;
     for (int i = threadIdx.x; i < rows * (BN / 4); i += NUM_THREADS) {
@@ -225,6 +232,12 @@ __device__ __forceinline__ void store_tile(const Params& p, const Place<BN>& at,
 #pragma unroll
             for (int t = 0; t < 4; ++t)
                 w[t] = t0 + t < used ? ld_cluster4(a + ((t0 + t) % held) * C::PART_BYTES, uint32_t((t0 + t) / held)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            if (singles)  // (the same adds as where a pair is one CTA's)
+#pragma unroll
+                for (int t = 0; t < 4; t += 2) {
+                    w[t].x += w[t + 1].x, w[t].y += w[t + 1].y, w[t].z += w[t + 1].z, w[t].w += w[t + 1].w;
+                    w[t + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
 #pragma unroll
             for (int t = 0; t < 4; ++t) q.x += w[t].x, q.y += w[t].y, q.z += w[t].z, q.w += w[t].w;
         }
@@ -640,20 +653,21 @@ struct Plan {
     int bn, split;
     double us;
 };
-// unit: accumulators that go to one CTA together.
-Plan make_plan(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count, int unit) {
+// singly: accumulators are dealt out one by one.
+Plan make_plan(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count, bool singly) {
     const int64_t tiles_m = (m + BM - 1) / BM;
-    const int kb = int((k + BK - 1) / BK), units = (kb + unit * CHUNK - 1) / (unit * CHUNK);
+    const int kb = int((k + BK - 1) / BK), chunks = (kb + CHUNK - 1) / CHUNK;
     Plan best{64, 1, 1e300};
     for (int wide = 0; wide < 2; ++wide)
         for (int split = 1; split <= 8; split *= 2) {
-            if (split > 1 && (units + split - 1) / split == (2 * units + split - 1) / split) break;  // no fewer for a CTA than with half the CTAs
+            if (split > 1 && share_of(chunks, split, singly) == share_of(chunks, split / 2, singly)) break;  // no fewer for a CTA than with half the CTAs
             const int64_t items = tiles_m * ((n + (wide ? 127 : 63)) / (wide ? 128 : 64)) * batch;
             int64_t room        = split == 1 ? sm_count : split == 2 ? sm_count / 2 - 4 : split == 4 ? sm_count / 4 - 5 : sm_count / 8 - 3;
             if (room < 1) room = 1;  // (a slice of a GPU)
             const double rounds = double((items + room - 1) / room);
-            const int per       = (units + split - 1) / split * unit * CHUNK;
-            const double time   = rounds * ((split > 1 ? 9.0 : 8.0) + (per < kb ? per : kb) * (wide ? 1.15 : 0.95));
+            const int per       = share_of(chunks, split, singly) * CHUNK;
+            const bool singles  = !singly && split > 1 && per == CHUNK;  // of 128 columns: twice the bytes to exchange (172 x 740 x 340 10.2 -> 11.1 us)
+            const double time   = rounds * ((split > 1 ? 9.0 : 8.0) + (per < kb ? per : kb) * (wide ? 1.15 : 0.95) + (singles && wide ? 1.6 : 0.0));
             if (time < best.us) best = Plan{wide ? 128 : 64, split, time};
         }
     return best;
@@ -661,7 +675,7 @@ Plan make_plan(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count, int
 
 template <class TIn, class TOut, bool CONV>
 int plan_and_launch(Params& p, int64_t batch, int sm_count, cudaStream_t s) {
-    const Plan plan = make_plan(p.M, p.N, p.K, batch, sm_count, CONV ? 1 : 2);
+    const Plan plan = make_plan(p.M, p.N, p.K, batch, sm_count, CONV);
     p.split = plan.split, p.tiles_m = (p.M + BM - 1) / BM, p.tiles_n = (p.N + plan.bn - 1) / plan.bn;
     const int64_t ctas = p.tiles_m * p.tiles_n * batch * p.split;
     return plan.bn == 128 ? launch<128, TIn, TOut, CONV>(p, ctas, s) : launch<64, TIn, TOut, CONV>(p, ctas, s);
@@ -676,7 +690,7 @@ static int extents_fit(const mimk_gemm_desc& d) {
     return tiles < (int64_t(1) << 28) && d.batch < (int64_t(1) << 28) && tiles * d.batch < (int64_t(1) << 28);  // one grid
 }
 // (by single accumulators: the choice against three TF32 products, which are less accurate, is not to move with how pairs fall to CTAs)
-double gemm_f32_tc_us(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count) { return make_plan(m, n, k, batch, sm_count, 1).us; }
+double gemm_f32_tc_us(int64_t m, int64_t n, int64_t k, int64_t batch, int sm_count) { return make_plan(m, n, k, batch, sm_count, true).us; }
 int gemm_f32_tc_supported(const mimk_gemm_desc& d) { return d.in_dtype == MIMK_F32 && extents_fit(d); }
 
 static Params product_params(const mimk_gemm_desc& d, const DeviceInfo& dev) {
@@ -727,7 +741,7 @@ static int64_t conv_ow(const mimk_conv_desc& d) { return (d.w + 2 * d.pad_w - d.
 // sum (4 x 256 x 28 x 28, 256 filters of 3 x 3, 77 us and 1.50e-7 against 73 and 1.65e-7).
 int conv_tc_preferred(const mimk_conv_desc& d, int sm_count) {
     const int64_t pixels = d.n * conv_oh(d) * conv_ow(d), k = d.cin * d.kh * d.kw;
-    const Plan plan = make_plan(pixels, d.cout, k, 1, sm_count, 1);
+    const Plan plan = make_plan(pixels, d.cout, k, 1, sm_count, true);
     if (d.dtype == MIMK_F32 && plan.split > 1) return 1;
     const int64_t tiles = ((pixels + BM - 1) / BM) * ((d.cout + plan.bn - 1) / plan.bn);
     const double kb = double((k + BK - 1) / BK), round = plan.bn == 128 ? 14.0 + 1.75 * kb : 7.0 + 1.25 * kb;

@@ -349,6 +349,18 @@ def test_small_f32_products_on_either_kernel_have_one_result(T, m, n, k, nk):
     close_cells(got, d64(a) @ bd, d64(a).abs() @ bd.abs(), k * 2.0 ** -24)
 
 
+@pytest.mark.parametrize("m,n,k,tiles", [
+    (1710, 104, 233, 30), (23, 720, 472, 10), (172, 740, 340, 6), (260, 1268, 115, 3), (100, 320, 512, 20), (129, 256, 577, 15), (96, 80, 520, 30)])
+def test_f32_products_dealt_out_by_pairs_and_singly_have_one_result(T, m, n, k, tiles):
+    # whatever share of a tile's accumulators each CTA of a cluster has, a product has the bits of the same rows of one with more tiles (with
+    # fewer than three TF32 products per term are made for)
+    a, b = rnd((m, k), 1), rnd((n, k), 2)
+    got, large = T.product_2d(a, b.t()), T.product_2d(torch.cat([a, rnd((128 * tiles, k), 3)]), b.t())
+    T.device_status()
+    assert torch.equal(got, large[:m])
+    close_cells(got, d64(a) @ d64(b).t(), d64(a).abs() @ d64(b).t().abs(), F32_CELL)
+
+
 def test_f32_products_keep_infinities_and_extremes(T):
     a, b = rnd((200, 600), 1), rnd((600, 300), 2)
     a[3, 5], a[7, 0], b[9, 11] = math.inf, math.nan, -math.inf
