@@ -532,6 +532,23 @@ def test_f32_convolutions_of_tiny_values(T, n, cin, h, w, cout, k, stride, pad, 
     close_cells(got, want, scale + cin * k * k * 2.0 ** -149 / F32_CELL, F32_CELL)
 
 
+@pytest.mark.parametrize("n,cin,side,cout,k,tiny", [(16, 64, 30, 130, 3, 1e-40), (16, 64, 30, 128, 3, 3e-42), (16, 128, 28, 100, 5, 1e-40)])
+def test_f32_convolutions_of_a_few_tiny_values(T, n, cin, side, cout, k, tiny):
+    # a few positions whose cells are folded again for all filters, beside zeros and ordinary cells
+    x, f = rnd((n, cin, side, side), 1), rnd((cout, cin, k, k), 2)
+    x[0], x[1, :, 2:] = 0.0, 0.0
+    x[0, 0, 0, 0], x[0, 3, 9, 9], x[1, 5, side - 1, side - 1] = tiny, -tiny, tiny
+    d = T.L.ConvDesc()
+    d.n, d.cin, d.h, d.w, d.cout, d.kh, d.kw, d.dtype = n, cin, side, side, cout, k, k, T.L.F32
+    d.stride_h = d.stride_w = d.dil_h = d.dil_w = 1
+    d.pad_h = d.pad_w = k // 2
+    assert T.L.lib().mimk_conv_laid_out(C.byref(d), T._stream()) == 1
+    got = T.conv(x, f, padding=(k // 2, k // 2))
+    T.device_status()
+    want, scale = (torch.nn.functional.conv2d(u, v, padding=k // 2) for u, v in ((d64(x), d64(f)), (d64(x).abs(), d64(f).abs())))
+    close_cells(got, want, scale + cin * k * k * 2.0 ** -149 / F32_CELL, F32_CELL)
+
+
 @pytest.mark.parametrize("m,n,k,b_nk,post,out,offset", [
     (2000, 1003, 520, True, "bias_relu", BF16, 0), (300, 257, 1031, True, None, BF16, 0), (129, 255, 1033, False, "bias", F32, 0),
     (640, 5003, 264, False, None, BF16, 0), (640, 5001, 257, True, "bias_tanh", F32, 1), (65, 2056, 512, True, None, BF16, 1),
