@@ -10,10 +10,14 @@
  *     the call is asynchronous on `stream` (a cudaStream_t passed as void*; NULL = the default stream);
  *   - every call returns an int status (0 = ok) instead of aborting, so emitted code can pipe it to
  *     `mim_cu_check(int)` (src/mim/plug/nvptx/rt/mim_cuda_rt.c:16-21) exactly like a CUresult;
- *   - entry points that need scratch beyond their arguments (f32 contractions on the tensor cores, split-axis
- *     reductions, mimk_mlp_gated without `h`, composed attention, large scatters) take it from a cached buffer that belongs
+ *   - entry points that need scratch beyond their arguments (f32 contractions with many tiles, bf16 ones whose operands have to be
+ *     copied, split-axis reductions, mimk_mlp_gated without `h`, f32 attention from 384 keys on and convolutions laid out
+ *     beforehand (up to 1 GiB each), composed attention, large scatters) take it from a cached buffer that belongs
  *     to the stream of the call: calls on different streams never share one (up to 8 streams per device keep a buffer;
- *     a ninth takes over the least recently used after a device-wide wait), calls on one stream are ordered by it;
+ *     a ninth takes over the least recently used after a device-wide wait), calls on one stream are ordered by it. A buffer grows
+ *     when a call needs more, after a device-wide wait, and is kept until the process ends, outside any other allocator;
+ *   - any entry point may be called from any host thread, on one stream too: a call has its buffer from its first launch to its
+ *     last, and another thread's call on the same stream waits for it (cudaStreamPerThread counts as each thread's own stream);
  *   - nothing here falls back to the CPU: without a usable sm_100 device every compute call fails with
  *     MIMK_E_NO_DEVICE.
  */
@@ -276,7 +280,9 @@ int mimk_scatter(const void* input, const void* index, const void* updates, void
  * Replaces: the composed program `softmax (q * transpose_2d k) * v` (lit/tensor/attn_exec.mim:20-22), seven
  * map_reduce_post ops with a materialised score matrix; scale, mask and batching are extensions.
  * q,o: [batch_heads, seq_q, head_dim]; k,v: [batch_heads, seq_k, head_dim]; dtype F32 or BF16 (o same dtype);
- * bf16 with head_dim 64 or 128 and f32 with head_dim up to 128 run fused on the tensor cores; other head dims from 2^24
+ * bf16 with head_dim 64 or 128 and f32 with head_dim up to 128 run fused on the tensor cores (f32, where several tiles of 128
+ * queries read at least 384 keys: K and V cut into bf16 pieces once beforehand, in the library's cached buffer; not under stream
+ * capture, where every tile cuts them again: longer, and other last bits); other head dims from 2^24
  * score-products on run as the composition S = Q K^T, softmax, O = P V on the contraction and row kernels (the score
  * matrix lives in a cached library buffer; not when lse is requested); everything else on a warp-per-query CUDA-core kernel;
  * lse (optional, f32 [batch_heads, seq_q]) receives log-sum-exp of the scaled scores. */
@@ -298,7 +304,7 @@ int mimk_attn_fwd(const mimk_attn_desc* desc, void* stream);
  * by_tap: the filters are given as [co, kh, kw, ci], ci a multiple of 8; then each load's place in the window is tested once for
  * eight channels.
  * Where an estimate says so, the image is laid out for the tensor cores first, in the library's cached buffer (not under stream
- * capture); mimk_conv_laid_out tells (1 / 0) whether a call with these sizes on this stream would do that, when the order of the
+ * capture: longer there, and other last bits); mimk_conv_laid_out tells (1 / 0) whether a call with these sizes on this stream would do that, when the order of the
  * filters makes no difference. */
 typedef struct mimk_conv_desc {
     int64_t n, cin, h, w, cout, kh, kw;

@@ -13,8 +13,8 @@
 // and head_dim <= 64 has two CTAs per SM.
 // What bounds it: LAID with two tiles the MMAs (N = 64: 46 clocks each with P in tensor memory, 57 with Q in shared memory, against 32
 // of arithmetic; 4600 clocks a block for both tiles), else the chain score -> softmax -> P V (3400 a block).
-// Measured (K and V cut by the workers before): 32 heads x 1000 x 64 73 us (119); 128 x 1024 x 64 251 (416); 128 x 2000 x 32 causal 339 (655);
-// 8 x 2048 x 128 124 (188); 11 x 1047 x 128 81 (107). 2-norm error 1.7e-7 to 4e-7.
+// Measured (K and V cut by the workers before): 32 heads x 1000 x 64 65 us (119); 128 x 1024 x 64 241 (410); 128 x 2000 x 32 causal 329 (651);
+// 8 x 2048 x 128 110 (175); 11 x 1047 x 128 71 (99). 2-norm error 1.7e-7 to 4e-7.
 //
 // Rows whose result is not finite (an infinite or NaN operand, an overflow), or so small that bits lost in the cutting of tiny
 // values (and weights) would show, are computed again by the general path.

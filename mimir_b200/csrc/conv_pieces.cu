@@ -17,8 +17,8 @@
 // whether it lost any, and where one did, the storing warps look for the largest magnitudes that their cells come from.
 //
 // Against gathering the image by the contraction's own loaders (gemm_f32_tc.cu), where every value is fetched, tested and cut again
-// for each tap that reads it: 16 x 128 x 56 x 56, 128 filters of 3 x 3, f32 214 -> 83 us (cut 16, conv 61), bf16 247 -> 46;
-// 32 x 256 x 28 x 28, 256 of 3 x 3: f32 380 -> 175, bf16 462 -> 77. What bounds the f32 form: shared memory, 116 clocks per MMA of 96 (its
+// for each tap that reads it: 16 x 128 x 56 x 56, 128 filters of 3 x 3, f32 214 -> 82 us (cut 16, conv 61), bf16 247 -> 40;
+// 32 x 256 x 28 x 28, 256 of 3 x 3: f32 380 -> 195, bf16 462 -> 67. What bounds the f32 form: shared memory, 116 clocks per MMA of 96 (its
 // operands 10 KB and 5 KB of TMA writes). Also measured: blocks of 32 channels in 64-byte rows, 105 us (TMA takes as long for a row of 64
 // bytes as for one of 128); four accumulators of 128 columns, 114; MMAs issued by lane 0 in a branch of its own, 95.
 #include <math_constants.h>

@@ -40,7 +40,7 @@ __device__ __forceinline__ void apply_post_32(int post, float (&v)[32], const fl
 // cannot write (a row pitch that is no multiple of 16 bytes, or a base that is not aligned): the warp stores each row with neighbouring lanes
 // on neighbouring words. Where a row starts in the middle of a word, its last element waits for the next piece, so that single elements are
 // stored at the ends of the tile only. Eight rows' words are read before the first is stored. What bounds it: the instructions per row (2000 x
-// 5003 x 2048, at first row by row with tests of its own for each: 62 us; 49 now; 43 by bulk stores, for a width of 5008; storing
+// 5003 x 2048, at first row by row with tests of its own for each: 60 us; 47 now; 39 by bulk stores, for a width of 5008; storing
 // whole sectors only, carried from piece to piece, gains nothing).
 __device__ __forceinline__ void store_piece(const uint8_t* buf, const uint8_t* before, bool first, bool last, __nv_bfloat16* c, int64_t ldc, int64_t rows,
                                             int64_t cols, int lane) {

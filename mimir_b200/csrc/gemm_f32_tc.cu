@@ -12,7 +12,7 @@
 // small terms first) and ordinary f32 adds between accumulators, the error stays below that of an f32 fold for any K.
 // Accumulators are added in pairs. Few tiles: the pairs of one tile are dealt out to a cluster of two, four or eight CTAs, which exchange
 // them through distributed shared memory (about 14 bytes a clock per SM, what bounds such products: by single accumulators 128 x 1024 x
-// 784 took 17 us). They are added in order whatever the grid as long as each CTA can hold its own to the end and they are at most nine:
+// 784 took 17 us), or one accumulator to a CTA where there are as many, their pairs added at the end. They are added in order whatever the grid as long as each CTA can hold its own to the end and they are at most nine:
 // K <= 1152, with 128 columns K <= 256 * split. Up to there a small product has the bits of the same cells of a large one, which programs rely on
 // (and the tests hold, to K = 1028). Beyond that a CTA adds its own first, fewer tiles change hands, the sums round less, and the bits follow the split.
 // That bits agree is what nine is for: 128 x 2048 x 1152, nine pairs held 24.3 us and 1.247e-7, as sums 20.5 and 1.203e-7; 128 x 1024 x 1536,

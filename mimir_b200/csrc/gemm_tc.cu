@@ -568,7 +568,7 @@ int gemm_tc(const mimk_gemm_desc& d, cudaStream_t s, int gated, const void* b2, 
 // pitch first, and the result is written by plain stores. (A result in f32: gemm_bf16_chunked.) Returns MIMK_E_UNSUPPORTED, with nothing launched, where the CUDA-core
 // kernel is the better or the only way.
 //
-// Measured: 2000 x 5003 x 2048, 44 us (2240 on the CUDA cores; 38 with a width of 5008); K = 2047 as well, 60; 3 x 9000 x 5001, 23 to
+// Measured: 2000 x 5003 x 2048, 47 us, 50 with bias and relu (2240 on the CUDA cores; 39 with a width of 5008); K = 2047 as well, 62; 3 x 9000 x 5001, 23 to
 // 65 by layout (483 to 508); 37 x 6998 x 546, 20 (54).
 // Floor of the rule: below 2^22 multiply-adds one launch of the CUDA-core kernel is as fast as the copies and the tensor-core
 // kernel's start. Copies are kept in the cached buffer, which a captured graph must not hold on to, and a buffer that cannot be

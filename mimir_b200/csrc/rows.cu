@@ -411,9 +411,9 @@ __global__ void reduce_mid_kernel(const TIn* __restrict__ x, TDst* __restrict__ 
 // inner > 1, V neighbouring columns to a thread: a CTA folds `lanes` x V columns of one outer index over its slice of the axis, 256 / lanes
 // elements of it at a time, and joins the 256 / lanes results of a column at the end. The producer's first operator alone (pre.batched()).
 // Bound by HBM, and for short folds by the launches: a column to a thread of the whole grid needs many slices of the axis, and their partials a
-// second launch. Sum of [32, 2048, 512], inputs not in L2: f32 42 -> 33 us, bf16 36 -> 23; of [1, 128, 1024] f32 14 -> 6, [7, 300, 96]
-// 15 -> 8, [1, 100000, 8] 40 -> 13 (the relative error of the f32 sums is half as large). V = 4: eight loads of 16 (bf16: 8) bytes in flight per thread; four: 34 and 27 us. V = 1, for rows that are
-// not aligned: [32, 2048, 513] f32 44 -> 37, [20, 126, 65] 14 -> 8.
+// second launch. Sum of [32, 2048, 512], inputs not in L2: f32 32 -> 24 us; of [1, 128, 1024] f32 12 -> 5, [7, 300, 96]
+// 14 -> 5, [1, 100000, 8] 38 -> 11 (the relative error of the f32 sums is half as large). V = 4: eight loads of 16 (bf16: 8) bytes in flight per thread; four take 3 to 17 % longer. V = 1, for rows that are
+// not aligned: [32, 2048, 513] f32 33 -> 26, [20, 126, 65] 12 -> 4. (Per call in a stream of calls.)
 template <int V, int BATCH, class Op, class TIn, class TDst, class Pre>
 __global__ void __launch_bounds__(256) reduce_tiles_kernel(const TIn* __restrict__ x, TDst* __restrict__ dst, int64_t total, int64_t len, int64_t inner,
                                                            int64_t slice_len, int tiles, int lanes_log, const Pre pre) {
