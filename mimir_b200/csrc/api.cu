@@ -1,4 +1,6 @@
 // C-ABI entry points that only validate and dispatch, plus the per-device state of the library.
+#include <atomic>
+#include <cstdint>
 #include <cstdlib>
 #include <mutex>
 
@@ -70,17 +72,21 @@ using Pool = ScratchPool<DeviceMemory, SCRATCH_SLOTS>;
 Pool g_scratch[MAX_DEVICES][2];
 }  // namespace
 
+// What a stream's buffers go by: its handle, but for cudaStreamPerThread, which names another stream in each thread, the thread's number, odd as
+// no handle from 3 on is. (Not cudaStreamGetId: a stream that is being captured refuses it, and a call that has its buffer may be captured.)
+static void* stream_key(cudaStream_t stream) {
+    static std::atomic<uintptr_t> threads{0};
+    thread_local const uintptr_t number = ++threads;
+    return stream == cudaStreamPerThread ? reinterpret_cast<void*>(2 * number + 1) : static_cast<void*>(stream);
+}
+
 int ScratchLease::take(size_t bytes, void** out, cudaStream_t stream, bool second) {
     int st        = MIMK_OK;
     DeviceInfo* d = device_info(&st);
     if (!d) return st;
-    // (by the stream's number, not its handle: cudaStreamPerThread names another stream in each thread, and a handle may come back for a new stream
-    // while the work of the one before is not done)
-    unsigned long long id = 0;
-    MIMK_CUDA_TRY(cudaStreamGetId(stream, &id));
     Pool* pool       = &g_scratch[d->device][second];
     Pool::Slot* slot = nullptr;
-    MIMK_TRY(pool->acquire(bytes, reinterpret_cast<void*>(id), &slot));
+    MIMK_TRY(pool->acquire(bytes, stream_key(stream), &slot));
     pool_ = pool, slot_ = slot;
     *out = slot->ptr;
     return MIMK_OK;

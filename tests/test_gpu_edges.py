@@ -746,3 +746,23 @@ def test_a_handle_that_names_a_stream_per_thread(T):
     T.device_status()
     for (_, outs, _, _), status in zip(convs, statuses):
         assert status == [0] * 21 and all(torch.equal(out, outs[0]) for out in outs[1:])
+
+
+@pytest.mark.parametrize("what", ["reduce", "mlp", "attention", "scatter"])
+def test_calls_that_have_their_buffer_may_be_captured(T, what):
+    x, h, q = rnd((1, 60000, 8), 1), [rnd(s, 2, BF16) for s in ((256, 512), (512, 512), (512, 512), (512, 256))], rnd((4, 512, 160), 3)
+    big, index, updates = rnd((5000, 8), 4), (rnd((5000, 8), 5).abs() * 40).long().clamp_(max=4999), rnd((5000, 8), 6)
+    call = {"reduce": lambda: T.reduce("sum", 1, x), "mlp": lambda: T.mlp_gated(*h), "attention": lambda: T.attention(q, q, q, scale=0.1),
+            "scatter": lambda: T.scatter(0, big, index, updates)}[what]
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        want = call()
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            got = call()
+    graph.replay()
+    torch.cuda.synchronize()
+    T.device_status()
+    assert torch.equal(got, want)
